@@ -1,23 +1,16 @@
 // kb_batch.cu -- many independent 1D2F1V solves (uneven cell counts and
-// velocity grids) advanced by ONE persistent kernel launch per time step.
+// velocity grids) advanced by one fused kernel launch per time step.
 //
 // Ragged layout: instance b owns cells [cell_off[b], cell_off[b] + nxt[b])
 // (ghosts included) and a velocity table at vel_off[b] of length nu[b]; its
 // distributions start at elem_off[b] in the flat h / b arrays and are
 // [cell][nus[b]] (velocity fastest, rows padded to a multiple of 4 values so
-// every row starts 16-byte aligned for bulk copies).  Each step runs three
-// phases per instance:
-//   A  face moments fw (blocked compensated sums over velocities) and the
-//      old heat flux q
-//   C  cell parameters: w, prim, tau, residual terms, the instance's
-//      residual and convergence flag
-//   D  pointwise KFVS flux + BGK / Shakhov relaxation (one thread per
-//      velocity, marching the cells)
-// FP32 split form: k_batch_seg fuses A, C and D for one 16-cell segment of
-// one instance per CTA (one pass over HBM), and k_batch_seg_res forms each
-// instance's residual from its segments' partial sums.  FP64 form
-// (k_batch_step, the comparator): a CTA takes whole instances from a work
-// counter (largest first).
+// every row starts 16-byte aligned for bulk copies).  A CTA fuses the whole
+// step of one segment of one instance: face moments and old heat flux, cell
+// parameters (w, prim, tau), pointwise KFVS flux + BGK / Shakhov relaxation,
+// in one pass over HBM (k_batch_seg in FP32, k_batch_seg64 in FP64);
+// k_batch_seg_res forms each instance's residual and convergence flag from its
+// segments' partial sums.
 // Covers the configuration of the batched shock-structure ensemble: KFVS,
 // BGK or Shakhov, fixed boundaries, van Leer, up to 256 velocities.
 #include <cuda_runtime.h>
@@ -26,229 +19,14 @@
 #include <cmath>
 #include <map>
 #include <cstring>
-#include <numeric>
 #include <string>
 #include <vector>
 
 #include "../../include/kitgpu.h"
 #include "kb_batch.cuh"
+#include "kb_batch64.cuh"
 
 namespace kb {
-
-template <typename R, int BS>
-__global__ void __launch_bounds__(BS) k_batch_step(BatchDev B, const R* __restrict__ Hin,
-                                                    const R* __restrict__ Bin, R* __restrict__ Hout,
-                                                    R* __restrict__ Bout) {
-  __shared__ int s_b;
-  __shared__ double red[BS / 32][8];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  for (;;) {
-    if (tid == 0) s_b = atomicAdd(B.counter, 1);
-    __syncthreads();
-    const int slot = s_b;
-    __syncthreads();
-    if (slot >= B.n) return;
-    const int b = B.order[slot];
-    const int nx = B.nx[b], ng = B.ng[b], nu = B.nu[b], ns = B.nus[b];
-    const long c0 = B.cell_off[b], e0 = B.elem_off[b];
-    const int nxt = nx + 2 * ng;
-    const R* Hi = Hin + e0;
-    const R* Bi = Bin + e0;
-    R* Ho = Hout + e0;
-    R* Bo = Bout + e0;
-    if (!B.active[b]) {  // converged: carry the state over
-      for (long k = tid; k < (long)nxt * ns; k += BS) {
-        Ho[k] = Hi[k];
-        Bo[k] = Bi[k];
-      }
-      continue;
-    }
-    const R* U = btab<R>(B, 0) + B.vel_off[b];
-    const R* W = btab<R>(B, 1) + B.vel_off[b];
-    const double dx = B.dx[b], dt = B.dt[b];
-    const R epsd = R(1.e-7 * dx);
-    double* fw = B.fw + B.face_off[b] * 4;
-    // ---- A: face moments (faces 1 .. nx-1 bound the stepped cells) and q
-    const R T3 = R(dt), T4 = R(0.5 * dt * dt / dx);
-    for (int f = 1 + tid; f <= nx - 1; f += BS) {
-      BSum<R> s0, s1, s2;
-      s0.init();
-      s1.init();
-      s2.init();
-      const int iL = f - 1, iR = f;
-      const int rL = brule(iL, nx, ng), rR = brule(iR, nx, ng);
-      const R* hL = Hi + (long)(iL + ng) * ns;
-      const R* bL = Bi + (long)(iL + ng) * ns;
-      for (int v = 0; v < nu; ++v) {
-        R u = U[v];
-        bool pos = u >= R(0);
-        const R* hc = pos ? hL : hL + ns;
-        const R* bc = pos ? bL : bL + ns;
-        int r = pos ? rL : rR;
-        R h0 = hc[v], b0 = bc[v];
-        R sh = R(0), sb = R(0);
-        if (r == 1) {
-          sh = bvl<R>(1, hc[v - ns], h0, hc[v + ns], epsd);
-          sb = bvl<R>(1, bc[v - ns], b0, bc[v + ns], epsd);
-        }
-        R side = pos ? R(0.5) : R(-0.5);
-        R hf = h0 + side * sh, bf = b0 + side * sb;
-        R fh = T3 * u * hf - T4 * (u * u) * sh;
-        R fb = T3 * u * bf - T4 * (u * u) * sb;
-        R wf = W[v] * fh;
-        s0.add(wf);
-        s1.add(wf * u);
-        s2.add(wf * u * u + W[v] * fb);
-        if ((v & 7) == 7) {
-          s0.flush();
-          s1.flush();
-          s2.flush();
-        }
-      }
-      double* o = fw + (long)f * 4;
-      o[0] = s0.get();
-      o[1] = s1.get();
-      o[2] = 0.5 * s2.get();
-    }
-    if (B.coll == COLL_SHAKHOV) {
-      for (int i = 1 + tid; i <= nx - 2; i += BS) {
-        BSum<R> s;
-        s.init();
-        const R* hc = Hi + (long)(i + ng) * ns;
-        const R* bc = Bi + (long)(i + ng) * ns;
-        R Uc = R(B.prim[(c0 + i + ng) * 4 + 1]);
-        for (int v = 0; v < nu; ++v) {
-          R cu = U[v] - Uc;
-          s.add(W[v] * cu * (cu * cu * hc[v] + bc[v]));
-          if ((v & 7) == 7) s.flush();
-        }
-        B.q[c0 + i + ng] = 0.5 * s.get();
-      }
-    }
-    __syncthreads();
-    // ---- C: cell parameters of the stepped cells 1 .. nx-2 (fixed ends)
-    double rr[6] = {0, 0, 0, 0, 0, 0};
-    for (int i = 1 + tid; i <= nx - 2; i += BS) {
-      const long c = c0 + i + ng;
-      double* w = B.w + c * 4;
-      double* p = B.prim + c * 4;
-      const double* fL = fw + (long)i * 4;
-      const double* fR = fw + (long)(i + 1) * 4;
-      double wo[3] = {w[0], w[1], w[2]};
-      double lo = p[2], rho_o = p[0], Uo = p[1];
-      for (int k = 0; k < 3; ++k) w[k] += (fL[k] - fR[k]) / dx;
-      double pn[4];
-      conserve_prim(w, 3, B.gamma, pn);
-      p[0] = pn[0];
-      p[1] = pn[1];
-      p[2] = pn[2];
-      for (int k = 0; k < 3; ++k) {
-        double d = w[k] - wo[k];
-        rr[k] += d * d;
-        rr[3 + k] += fabs(w[k]);
-      }
-      double lam = pn[2];
-      double tau = vhs_time(pn[0], lam, B.mu[b], B.omega);
-      if (!(pn[0] > 0.0) || !(lam > 0.0) || !isfinite(pn[0]) || !isfinite(lam)) atomicOr(B.status, 1);
-      double* k = B.cp + c * 16;
-      k[0] = pn[0] * sqrt(lam / PI);  // new Maxwellian
-      k[1] = pn[1];
-      k[2] = lam;
-      k[3] = B.K / (2.0 * lam);
-      k[4] = dt / tau;
-      k[5] = 1.0 / (1.0 + dt / tau);
-      k[6] = rho_o * sqrt(lo / PI);  // old Maxwellian (Shakhov)
-      k[7] = Uo;
-      k[8] = lo;
-      k[9] = B.K / (2.0 * lo);
-      k[10] = B.coll == COLL_SHAKHOV ? 0.8 * (1.0 - B.Pr) * (lo * lo) / rho_o * B.q[c] : 0.0;
-    }
-    // residual (src/Solver/solver_update.jl:86-88; fixed ends add zero)
-    for (int k = 0; k < 6; ++k) {
-#pragma unroll
-      for (int m = 16; m >= 1; m >>= 1) rr[k] += __shfl_xor_sync(0xffffffffu, rr[k], m);
-    }
-    if (lane == 0)
-      for (int k = 0; k < 6; ++k) red[wid][k] = rr[k];
-    __syncthreads();
-    if (tid == 0) {
-      double t[6] = {0, 0, 0, 0, 0, 0};
-      for (int w8 = 0; w8 < BS / 32; ++w8)
-        for (int k = 0; k < 6; ++k) t[k] += red[w8][k];
-      double mx = 0.0;
-      for (int k = 0; k < 3; ++k) {
-        // fixed ends contribute sqrt(0 * 2) / (0 + 1e-7) = 0 (update_boundary.jl:41-44)
-        double r = sqrt(t[k] * nx) / (t[3 + k] + 1.e-7);
-        B.residual[b * 4 + k] = r;
-        mx = fmax(mx, r);
-      }
-      if (mx < B.tol) B.active[b] = 0;
-    }
-    __syncthreads();
-    // ---- D: pointwise update, one thread per velocity marching the cells
-    for (int v = tid; v < nu; v += BS) {
-      const R u = U[v];
-      const bool pos = u >= R(0);
-      const R side = pos ? R(0.5) : R(-0.5);
-      auto at = [&](const R* q, int i) { return q[(long)(i + ng) * ns + v]; };
-      // fixed end cells keep their state
-      Ho[(long)ng * ns + v] = at(Hi, 0);
-      Bo[(long)ng * ns + v] = at(Bi, 0);
-      Ho[(long)(nx - 1 + ng) * ns + v] = at(Hi, nx - 1);
-      Bo[(long)(nx - 1 + ng) * ns + v] = at(Bi, nx - 1);
-      // window: cells i-1, i, i+1 around the upwind cell of face i (between i-1 and i)
-      auto face = [&](int f, R& fh, R& fb) {
-        int up = pos ? f - 1 : f;
-        int r = brule(up, nx, ng);
-        R h0 = at(Hi, up), b0 = at(Bi, up);
-        R sh = R(0), sb = R(0);
-        if (r == 1) {
-          sh = bvl<R>(1, at(Hi, up - 1), h0, at(Hi, up + 1), epsd);
-          sb = bvl<R>(1, at(Bi, up - 1), b0, at(Bi, up + 1), epsd);
-        }
-        R hf = h0 + side * sh, bf = b0 + side * sb;
-        fh = T3 * u * hf - T4 * (u * u) * sh;
-        fb = T3 * u * bf - T4 * (u * u) * sb;
-      };
-      R fhL, fbL;
-      face(1, fhL, fbL);
-      for (int i = 1; i <= nx - 2; ++i) {
-        R fhR, fbR;
-        face(i + 1, fhR, fbR);
-        const long c = c0 + i + ng;
-        const double* k = B.cp + c * 16;
-        R h0 = at(Hi, i), b0 = at(Bi, i);
-        R du = u - R(k[1]);
-        R M = R(k[0]) * mexp(-R(k[2]) * du * du);
-        R MH = M, MB = M * R(k[3]);
-        if (B.coll == COLL_SHAKHOV) {
-          R ou = u - R(k[7]);
-          R OH = R(k[6]) * mexp(-R(k[8]) * ou * ou);
-          R cq = R(k[10]) * ou;
-          R tl = R(2) * R(k[8]) * ou * ou + R(B.K);
-          MH += cq * (tl - R(5)) * OH;
-          MB += cq * (tl - R(3)) * OH * R(k[9]);
-        }
-        R dtau = R(k[4]);
-        R hn, bn;
-        if (sizeof(R) == 8) {
-          hn = (h0 + (fhL - fhR) / R(dx) + dtau * MH) / (R(1) + dtau);
-          bn = (b0 + (fbL - fbR) / R(dx) + dtau * MB) / (R(1) + dtau);
-        } else {
-          R idx = R(1.0 / dx), inv = R(k[5]);
-          hn = (h0 + (fhL - fhR) * idx + dtau * MH) * inv;
-          bn = (b0 + (fbL - fbR) * idx + dtau * MB) * inv;
-        }
-        Ho[(long)(i + ng) * ns + v] = hn;
-        Bo[(long)(i + ng) * ns + v] = bn;
-        fhL = fhR;
-        fbL = fbR;
-      }
-    }
-    __syncthreads();
-  }
-}
-
 
 // Residual of each active instance of the segment form
 // (src/Solver/solver_update.jl:86-88) and its convergence flag.  One warp per
@@ -274,6 +52,10 @@ __global__ void k_batch_seg_res(BatchDev B) {
     }
     if (mx < B.tol) B.active[b] = 0;
   }
+}
+
+void seg_res_launch(const BatchDev& B, cudaStream_t st) {
+  k_batch_seg_res<<<(unsigned)((B.n + 3) / 4), 128, 0, st>>>(B);
 }
 
 __global__ void k_batch_timestep(BatchDev B, const double* umax, double cfl, double* dt_out,
@@ -315,6 +97,10 @@ __global__ void k_batch_mcache(BatchDev B) {
   SegMax m;
   m.set(B.prim + cell * 4, B.K);
   seg_store_coef(B, cell, m);
+}
+
+void seg_mcache_launch(const BatchDev& B, int n, int max_cells, cudaStream_t st) {
+  k_batch_mcache<<<dim3((unsigned)((max_cells + 127) / 128), (unsigned)n), 128, 0, st>>>(B);
 }
 
 // FP64 form: h = maxwellian(u, prim), b = h K / (2 lambda) in FP64
@@ -360,7 +146,7 @@ struct kb_batch {
   kb::BatchDev d;
   int prec = 0;
   int n = 0;
-  long ncell = 0, nelem = 0, nface = 0, nvel = 0;
+  long ncell = 0, nelem = 0, nvel = 0;
   void* h[2] = {nullptr, nullptr};
   void* bq[2] = {nullptr, nullptr};
   int cur = 0;
@@ -372,8 +158,7 @@ struct kb_batch {
   double* d_stage = nullptr;
   double* d_umax = nullptr;
   cudaGraphExec_t graph = nullptr;
-  int graph_cur = -1;
-  int grid = 0;
+  int graph_cur = -1, graph_launches = 0;
   int64_t launches = 0;
   // FP32 segment kernel: shape (cells per segment, threads, persistent grid)
   // and its launch; segment tables are rebuilt when the shape changes
@@ -419,7 +204,7 @@ extern "C" int kb_batch_destroy(kb_batch_t* B) {
 }
 
 // Compiled shapes of the FP32 segment kernel (kb_batch_seg_a.cu, _b.cu).
-static const std::vector<kb::SegVariant>& seg_variants() {
+const std::vector<kb::SegVariant>& kb::seg_variants() {
   static const std::vector<kb::SegVariant> v = [] {
     std::vector<kb::SegVariant> out;
     kb::seg_variants_a(out);
@@ -429,17 +214,9 @@ static const std::vector<kb::SegVariant>& seg_variants() {
   return v;
 }
 
-// Select the segment kernel's shape: segment tables for `seg` cells per
-// segment (instances in processing order, their segments consecutive),
-// the kernel's shared-memory limit, and the grid -- one CTA per segment, or
-// (persist) as many CTAs as fit on the GPU at once, each looping over
-// segments.  Runs outside any stream capture; invalidates the step graph.
-static int batch_set_shape(kb_batch* B, int seg, int threads, int persist) {
-  const kb::SegVariant* var = nullptr;
-  for (const auto& v : seg_variants())
-    if (v.seg == seg && v.threads == threads) var = &v;
-  if (!var) return bfail(KB_ERR_ARG, "batch shape: no segment kernel for " + std::to_string(seg) +
-                                         " cells x " + std::to_string(threads) + " threads");
+// Segment tables for `seg` cells per segment (an instance's segments are
+// consecutive).  Waits for the stream; invalidates the step graph.
+static int batch_tables(kb_batch* B, int seg) {
   std::vector<int> seg_b, seg_i0, seg_first(B->n), nseg(B->n);
   for (int b = 0; b < B->n; ++b) {
     seg_first[b] = (int)seg_b.size();
@@ -456,6 +233,33 @@ static int batch_set_shape(kb_batch* B, int seg, int threads, int persist) {
   ok &= cudaMemcpy(B->d_segi0, seg_i0.data(), sizeof(int) * seg_i0.size(), cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(B->d_segfirst, seg_first.data(), sizeof(int) * B->n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(B->d_nseg, nseg.data(), sizeof(int) * B->n, cudaMemcpyHostToDevice) == cudaSuccess;
+  if (!ok) {
+    cudaGetLastError();
+    return bfail(KB_ERR_CUDA, "batch shape: segment table upload failed");
+  }
+  B->nseg = (long)seg_b.size();
+  B->d.nseg_all = (int)B->nseg;
+  B->seg = seg;
+  if (B->graph) {
+    cudaGraphExecDestroy(B->graph);
+    B->graph = nullptr;
+  }
+  return KB_OK;
+}
+
+// Select the FP32 segment kernel's shape: its segment tables, the kernel's
+// shared-memory limit, and the grid -- one CTA per segment, or (persist) as
+// many CTAs as fit on the GPU at once, each looping over segments.  Runs
+// outside any stream capture.
+static int batch_set_shape(kb_batch* B, int seg, int threads, int persist) {
+  const kb::SegVariant* var = nullptr;
+  for (const auto& v : kb::seg_variants())
+    if (v.seg == seg && v.threads == threads) var = &v;
+  if (!var) return bfail(KB_ERR_ARG, "batch shape: no segment kernel for " + std::to_string(seg) +
+                                         " cells x " + std::to_string(threads) + " threads");
+  int rc = batch_tables(B, seg);
+  if (rc != KB_OK) return rc;
+  bool ok = true;
   const int smem = var->smem(B->d.sst_max, B->d.nu4_max);
   ok &= cudaFuncSetAttribute(var->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, var->smem_max) ==
         cudaSuccess;
@@ -469,21 +273,14 @@ static int batch_set_shape(kb_batch* B, int seg, int threads, int persist) {
   ok &= cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, var->fn, threads, smem) == cudaSuccess;
   if (!ok || per < 1) {
     cudaGetLastError();
-    return bfail(KB_ERR_CUDA, "batch shape: segment tables or kernel attributes refused");
+    return bfail(KB_ERR_CUDA, "batch shape: kernel attributes refused");
   }
-  B->nseg = (long)seg_b.size();
-  B->d.nseg_all = (int)B->nseg;
-  B->seg = seg;
   B->seg_t = threads;
   B->persist = persist ? 1 : 0;
   B->seg_fn = var->fn;
   B->seg_smem = smem;
   B->seg_grid = persist ? (int)std::min<long>(B->nseg, (long)sms * per) : (int)B->nseg;
   if (B->pool && persist) B->seg_grid = sms * per;  // fixed, whatever the membership
-  if (B->graph) {
-    cudaGraphExecDestroy(B->graph);
-    B->graph = nullptr;
-  }
   return KB_OK;
 }
 
@@ -512,12 +309,11 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   B->nx.assign(nx, nx + n);
   B->ng.assign(ngx, ngx + n);
   B->nu.assign(nu, nu + n);
-  std::vector<long> face_off(n), vel_off_l(n);
   std::vector<int> vel_off(n);
   std::vector<double> dx(n), dt(n, 0.0), mu(mu_ref, mu_ref + n);
   B->cell_off.resize(n);
   B->elem_off.resize(n);
-  long cells = 0, elems = 0, faces = 0, vels = 0;
+  long cells = 0, elems = 0, vels = 0;
   B->nus.resize(n);
   B->dense_off.resize(n);
   long dense = 0;
@@ -526,30 +322,29 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
     B->cell_off[b] = cells;
     B->elem_off[b] = elems;
     B->dense_off[b] = dense;
-    face_off[b] = faces;
     vel_off[b] = (int)vels;
     long nxt = nx[b] + 2 * ngx[b];
     B->nus[b] = (nu[b] + 3) / 4 * 4;
     cells += nxt;
     elems += nxt * B->nus[b];
     dense += nxt * nu[b];
-    faces += nx[b] + 1;
     vels += nu[b];
     dx[b] = (x1[b] - x0[b]) / nx[b];
     seg_cap += (nx[b] + 7) / 8;  // the shortest segment length the tuner offers
+  }
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int seg64 = kb::seg64_cells(cells, sms);
+  if (B->prec == KB_PREC_FP64) {
+    seg_cap = 0;
+    for (int b = 0; b < n; ++b) seg_cap += (nx[b] + seg64 - 1) / seg64;
   }
   B->ndense = dense;
   B->seg_cap = seg_cap;
   B->ncell = cells;
   B->nelem = elems;
-  B->nface = faces;
   B->nvel = vels;
-  // largest instances first
-  std::vector<int> order(n);
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int a, int c) {
-    return (long)nx[a] * nu[a] > (long)nx[c] * nu[c];
-  });
   auto fail_out = [&](int rc) {
     kb_batch_destroy(B);
     return rc;
@@ -561,13 +356,12 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
 #define BALLOC(dst, T, count)                                              \
   if ((rc = balloc(B, &p, sizeof(T) * (size_t)(count))) != KB_OK) return fail_out(rc); \
   dst = (T*)p;
-  int *d_order, *d_nx, *d_ng, *d_nu, *d_vo, *d_active, *d_counter, *d_status;
+  int *d_nx, *d_ng, *d_nu, *d_vo, *d_active, *d_status;
   int *d_nus, *d_segb, *d_segi0, *d_segfirst, *d_nseg;
   double* d_respart;
-  long *d_co, *d_eo, *d_fo;
-  double *d_dx, *d_dt, *d_mu, *d_u, *d_w, *d_wv, *d_prim, *d_fw, *d_q, *d_cp, *d_res;
+  long *d_co, *d_eo;
+  double *d_dx, *d_dt, *d_mu, *d_u, *d_w, *d_wv, *d_prim, *d_res;
   float *d_uf, *d_wf, *d_ul, *d_mc;
-  BALLOC(d_order, int, n);
   BALLOC(d_nx, int, n);
   BALLOC(d_ng, int, n);
   BALLOC(d_nu, int, n);
@@ -579,11 +373,9 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   BALLOC(d_respart, double, B->seg_cap * 8);
   BALLOC(d_vo, int, n);
   BALLOC(d_active, int, n);
-  BALLOC(d_counter, int, 2);
   BALLOC(d_status, int, 1);
   BALLOC(d_co, long, n);
   BALLOC(d_eo, long, n);
-  BALLOC(d_fo, long, n);
   BALLOC(d_dx, double, n);
   BALLOC(d_dt, double, n);
   BALLOC(d_mu, double, n);
@@ -594,9 +386,6 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   BALLOC(d_wf, float, vels);
   BALLOC(d_w, double, cells * 4);
   BALLOC(d_prim, double, cells * 4);
-  BALLOC(d_fw, double, faces * 4);
-  BALLOC(d_q, double, cells);
-  BALLOC(d_cp, double, cells * 16);
   BALLOC(d_mc, float, cells * 8);
   BALLOC(d_res, double, (size_t)n * 4);
   BALLOC(B->d_umax, double, n);
@@ -616,7 +405,6 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   for (long k = 0; k < vels; ++k) ul[k] = float(u_all[k] - (double)uf[k]);
   std::vector<int> ones(n, 1);
   bool ok = true;
-  ok &= cudaMemcpy(d_order, order.data(), sizeof(int) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_nx, nx, sizeof(int) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_ng, ngx, sizeof(int) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_nu, nu, sizeof(int) * n, cudaMemcpyHostToDevice) == cudaSuccess;
@@ -626,7 +414,6 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   ok &= cudaMemcpy(d_active, ones.data(), sizeof(int) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_co, B->cell_off.data(), sizeof(long) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_eo, B->elem_off.data(), sizeof(long) * n, cudaMemcpyHostToDevice) == cudaSuccess;
-  ok &= cudaMemcpy(d_fo, face_off.data(), sizeof(long) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_dx, dx.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_dt, dt.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_mu, mu.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
@@ -637,13 +424,10 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   ok &= cudaMemcpy(d_wf, wf.data(), sizeof(float) * vels, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(B->d_umax, umax, sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemset(d_status, 0, sizeof(int)) == cudaSuccess;
-  ok &= cudaMemset(d_q, 0, sizeof(double) * cells) == cudaSuccess;
-  ok &= cudaMemset(d_fw, 0, sizeof(double) * faces * 4) == cudaSuccess;
   ok &= cudaMemset(d_res, 0, sizeof(double) * n * 4) == cudaSuccess;
   if (!ok) return fail_out(bfail(KB_ERR_CUDA, "batch table upload failed"));
   kb::BatchDev& d = B->d;
   d.n = n;
-  d.order = d_order;
   d.nx = d_nx;
   d.ng = d_ng;
   d.nu = d_nu;
@@ -676,14 +460,9 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   d.wtf = d_wf;
   d.w = d_w;
   d.prim = d_prim;
-  d.fw = d_fw;
-  d.face_off = d_fo;
-  d.q = d_q;
-  d.cp = d_cp;
   d.mc = d_mc;
   d.residual = d_res;
   d.active = d_active;
-  d.counter = d_counter;
   d.status = d_status;
   d.K = base->K;
   d.gamma = base->gamma;
@@ -691,14 +470,11 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   d.Pr = base->Pr;
   d.tol = 0.0;
   d.coll = base->collision;
-  int dev = 0, sms = 1, per = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (B->prec == KB_PREC_FP64)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb::k_batch_step<double, 256>, 256, 0);
-  else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb::k_batch_step<float, 256>, 256, 0);
-  B->grid = std::min(n, std::max(1, sms * per));
+  d.clock = nullptr;
+  if (B->prec == KB_PREC_FP64) {
+    if (!kb::seg64_prepare()) return fail_out(bfail(KB_ERR_CUDA, "FP64 segment kernel attributes refused"));
+    if ((rc = batch_tables(B, seg64)) != KB_OK) return fail_out(rc);
+  }
   if (B->prec == KB_PREC_FP32 && (rc = batch_set_shape(B, 16, 128, 0)) != KB_OK)
     return fail_out(rc);
   *out = B;
@@ -744,7 +520,7 @@ extern "C" int kb_batch_upload(kb_batch_t* B, const double* w, const double* pri
   if (B->prec == KB_PREC_FP32) {  // the FP32 step reads each cell's Maxwellian coefficients
     int maxc = 1;
     for (int b = 0; b < B->n; ++b) maxc = std::max(maxc, B->nx[b] + 2 * B->ng[b]);
-    kb::k_batch_mcache<<<dim3((unsigned)((maxc + 127) / 128), (unsigned)B->n), 128, 0, B->stream>>>(B->d);
+    kb::seg_mcache_launch(B->d, B->n, maxc, B->stream);
     B->launches++;
     cudaStreamSynchronize(B->stream);
   }
@@ -846,32 +622,33 @@ extern "C" int kb_batch_set_dt(kb_batch_t* B, const double* dt) {
   return KB_OK;
 }
 
-// Kernels batch_launch issues per step: the FP32 segment form adds the
-// per-instance residual kernel.
-static int batch_kernels_per_step(const kb_batch* B) { return B->prec == KB_PREC_FP32 ? 2 : 1; }
-
-static void batch_launch(kb_batch* B, int cur) {
+// One step from buffer `cur`.  The residual kernel sets residuals and
+// convergence flags; with tol = 0 no flag can change, so only the last step of
+// a call needs it (res).  Returns the kernels launched.
+static int batch_launch(kb_batch* B, int cur, bool res) {
+  int n = 0;
   if (B->prec == KB_PREC_FP32) {  // fused segments (one pass over HBM)
     const float* hin = (const float*)B->h[cur];
     const float* bin = (const float*)B->bq[cur];
     float* hout = (float*)B->h[cur ^ 1];
     float* bout = (float*)B->bq[cur ^ 1];
-    void* args[] = {(void*)&B->d, (void*)&hin, (void*)&bin, (void*)&hout, (void*)&bout};
-    if (B->seg_grid > 0)  // an empty pool has no segments
+    int slot = -1;
+    void* args[] = {(void*)&B->d, (void*)&hin, (void*)&bin, (void*)&hout, (void*)&bout, (void*)&slot};
+    if (B->seg_grid > 0) {  // an empty pool has no segments
       cudaLaunchKernel(B->seg_fn, dim3((unsigned)B->seg_grid), dim3((unsigned)B->seg_t), args,
                        (size_t)B->seg_smem, B->stream);
-    kb::k_batch_seg_res<<<(unsigned)((B->n + 3) / 4), 128, 0, B->stream>>>(B->d);
-    return;
+      ++n;
+    }
+  } else {
+    kb::seg64_launch(B->d, B->seg, (const double*)B->h[cur], (const double*)B->bq[cur],
+                     (double*)B->h[cur ^ 1], (double*)B->bq[cur ^ 1], res, -1, B->stream);
+    ++n;
   }
-  cudaMemsetAsync(B->d.counter, 0, sizeof(int), B->stream);
-  if (B->prec == KB_PREC_FP64)
-    kb::k_batch_step<double, 256><<<B->grid, 256, 0, B->stream>>>(
-        B->d, (const double*)B->h[cur], (const double*)B->bq[cur], (double*)B->h[cur ^ 1],
-        (double*)B->bq[cur ^ 1]);
-  else
-    kb::k_batch_step<float, 256><<<B->grid, 256, 0, B->stream>>>(
-        B->d, (const float*)B->h[cur], (const float*)B->bq[cur], (float*)B->h[cur ^ 1],
-        (float*)B->bq[cur ^ 1]);
+  if (res) {
+    kb::seg_res_launch(B->d, B->stream);
+    ++n;
+  }
+  return n;
 }
 
 // Two steps (ping and pong) captured once as a CUDA graph and replayed.
@@ -884,8 +661,9 @@ static int batch_graph(kb_batch* B) {
   cudaGraph_t g;
   if (cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
     return bfail(KB_ERR_CUDA, "graph capture failed to start");
-  batch_launch(B, B->cur);
-  batch_launch(B, B->cur ^ 1);
+  const bool res = B->d.tol > 0.0;  // flags may change at every step
+  B->graph_launches = batch_launch(B, B->cur, res);
+  B->graph_launches += batch_launch(B, B->cur ^ 1, res);
   if (cudaStreamEndCapture(B->stream, &g) != cudaSuccess)
     return bfail(KB_ERR_CUDA, "graph capture failed");
   cudaError_t e = cudaGraphInstantiate(&B->graph, g, 0);
@@ -906,17 +684,19 @@ extern "C" int kb_batch_step(kb_batch_t* B, int32_t nsteps, double tol, double* 
       B->graph = nullptr;
     }
   }
-  int rc = batch_graph(B);
-  if (rc != KB_OK) return rc;
-  int pairs = nsteps / 2;
-  for (int k = 0; k < pairs; ++k) {
-    if (cudaGraphLaunch(B->graph, B->stream) != cudaSuccess)
-      return bfail(KB_ERR_CUDA, "graph launch failed");
-    B->launches += 2 * batch_kernels_per_step(B);
+  // pairs of steps replayed, the last one or two launched with the residual
+  int left = nsteps;
+  if (left > 2) {
+    int rc = batch_graph(B);
+    if (rc != KB_OK) return rc;
+    for (; left > 2; left -= 2) {
+      if (cudaGraphLaunch(B->graph, B->stream) != cudaSuccess)
+        return bfail(KB_ERR_CUDA, "graph launch failed");
+      B->launches += B->graph_launches;
+    }
   }
-  if (nsteps & 1) {
-    batch_launch(B, B->cur);
-    B->launches += batch_kernels_per_step(B);
+  for (; left > 0; --left) {
+    B->launches += batch_launch(B, B->cur, left == 1 || tol > 0.0);
     B->cur ^= 1;
   }
   if (cudaStreamSynchronize(B->stream) != cudaSuccess)
@@ -932,7 +712,7 @@ extern "C" int kb_batch_step(kb_batch_t* B, int32_t nsteps, double tol, double* 
 
 extern "C" int kb_batch_set_tuning(kb_batch_t* B, const int32_t* params, int32_t n) {
   if (!B || !params || n < 1) return bfail(KB_ERR_ARG, "kb_batch_set_tuning: null argument");
-  if (B->prec != KB_PREC_FP32) return KB_OK;  // the FP64 comparator has one shape
+  if (B->prec != KB_PREC_FP32) return KB_OK;  // the FP64 form has one shape
   const int seg = params[0] > 0 ? params[0] : 16;
   const int thr = n > 1 && params[1] > 0 ? params[1] : 128;
   const int per = n > 2 ? params[2] : 0;

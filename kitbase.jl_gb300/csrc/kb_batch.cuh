@@ -17,7 +17,6 @@ namespace kb {
 
 struct BatchDev {
   int n;                 // instances
-  const int* order;      // processing order (largest first)
   const int* nx;         // physical cells
   const int* ng;         // ghost layers
   const int* nu;         // velocities
@@ -35,17 +34,19 @@ struct BatchDev {
   const float* wtf;
   double* w;             // [cell][4] (3 used)
   double* prim;          // [cell][4]
-  double* fw;            // [instance faces][4] scratch: face flux per instance (nx+1 each)
-  const long* face_off;
-  double* q;             // [cell] old heat flux
-  double* cp;            // [cell][16] cell coefficients (see k_batch_step)
   float* mc;             // [cell][8] FP32 Maxwellian coefficients of the cell's current prim
                          // (SegMax: rn, U hi, lambda, K / (2 lambda), U lo), kept with prim
   double* residual;      // [n][4]
+  // Per-step time step of a single solve (kb_step_cfl), null otherwise.  Step
+  // number m has slot m mod 3: [slot] the CFL rate of the state before it,
+  // [3 + slot] the time before it; then cfl, the end time, umax and the number
+  // of steps taken.  A step reads its slot, collects the rate of its new state
+  // in the next slot (atomic maximum over the segments) and clears the one
+  // after, so no kernel stands between two steps and no host wait.
+  double* clock;         // [10]
   int* active;           // [n] 1 while not converged
-  int* counter;          // work counter
   int* status;
-  // FP32 segment form: segment k covers cells [seg_i0[k], seg_i0[k] + SEG) of
+  // Segment k covers cells [seg_i0[k], seg_i0[k] + cells per segment) of
   // instance seg_b[k]; an instance's segments are consecutive from
   // seg_first[b] (nseg[b] of them)
   const int* seg_b;
@@ -60,18 +61,10 @@ struct BatchDev {
   int coll;
 };
 
-template <typename R>
-__device__ __forceinline__ R bvl(int rule, R qm, R q0, R qp, R epsd) {
-  R a = q0 - qm, b = qp - q0;
-  if (rule == 1) return (a * fabs(b) + b * fabs(a)) / (fabs(a) + fabs(b) + epsd);
-  return R(0);
-}
-// FP32 form: one reciprocal and one multiply (subnormals flushed), the
-// division the FP32 passes of the 2D solver use as well
-template <>
-__device__ __forceinline__ float bvl<float>(int rule, float qm, float q0, float qp, float epsd) {
-  float a = q0 - qm, b = qp - q0;
-  if (rule != 1) return 0.f;
+// van Leer slope times dx: one reciprocal and one multiply (subnormals
+// flushed), the division the FP32 passes of the 2D solver use as well
+__device__ __forceinline__ float bvl(float qm, float q0, float qp, float epsd) {
+  const float a = q0 - qm, b = qp - q0;
   float r;
   asm("div.approx.ftz.f32 %0, %1, %2;"
       : "=f"(r)
@@ -87,37 +80,14 @@ __device__ __forceinline__ int brule(int i, int nx, int ng) {
   return 1;
 }
 
-template <typename R>
-struct BSum;
-template <>
-struct BSum<float> {
+// Blocked FP32 sum, flushed into a double-float accumulator.
+struct BSum {
   float p;
   DF d;
   __device__ __forceinline__ void init() { p = 0.f; d.hi = d.lo = 0.f; }
   __device__ __forceinline__ void add(float x) { p += x; }
   __device__ __forceinline__ void flush() { df_add(d, p); p = 0.f; }
-  __device__ __forceinline__ double get() { flush(); return (double)d.hi + (double)d.lo; }
 };
-template <>
-struct BSum<double> {
-  double p;
-  __device__ __forceinline__ void init() { p = 0.0; }
-  __device__ __forceinline__ void add(double x) { p += x; }
-  __device__ __forceinline__ void flush() {}
-  __device__ __forceinline__ double get() { return p; }
-};
-
-template <typename R>
-__device__ __forceinline__ const R* btab(const BatchDev& B, int which);
-template <>
-__device__ __forceinline__ const double* btab<double>(const BatchDev& B, int which) {
-  return which == 0 ? B.u : B.wt;
-}
-template <>
-__device__ __forceinline__ const float* btab<float>(const BatchDev& B, int which) {
-  return which == 0 ? B.uf : B.wtf;
-}
-
 
 // e^x on the MUFU unit (2^(x log2 e), results below 2^-126 flushed to zero)
 __device__ __forceinline__ float fexp(float x) {
@@ -184,6 +154,46 @@ __device__ __forceinline__ void seg_init_cell(const BatchDev& B, int b, int c, f
   }
 }
 
+// ---- per-step time step (BatchDev::clock)
+struct SegClock {
+  double dt, t;
+  bool stop;  // the end time is reached: the state is carried over
+};
+// timestep (src/Solver/solver_main.jl:240-288) from the collected rate
+__device__ __forceinline__ SegClock seg_clock(const BatchDev& B, int slot) {
+  SegClock c;
+  const double tend = B.clock[7];
+  c.t = B.clock[3 + slot];
+  c.dt = B.clock[6] / B.clock[slot];
+  c.dt = c.dt < tend - c.t ? c.dt : tend - c.t;
+  c.stop = !(c.t < tend - 1e-14 * fabs(tend)) || !(c.dt > 0.0);
+  return c;
+}
+// by one thread of the launch
+__device__ __forceinline__ void seg_clock_next(const BatchDev& B, int slot, const SegClock& c) {
+  const int nx = (slot + 1) % 3, clear = (slot + 2) % 3;
+  B.clock[3 + nx] = c.stop ? c.t : c.t + c.dt;
+  if (c.stop) B.clock[nx] = B.clock[slot];
+  else B.clock[9] += 1.0;
+  B.clock[clear] = 0.0;
+}
+__device__ __forceinline__ double seg_rate(const BatchDev& B, const double* p, double rdx) {
+  return (fmax(B.clock[8], fabs(p[1])) + sqrt(0.5 * B.gamma / p[2])) * rdx;
+}
+// The largest rate of a segment's cells (`rate`: the stepped cell of this
+// lane) and of the fixed ends among them into the next slot; one warp.  Rates
+// are positive, so their bits order like unsigned integers.
+__device__ __forceinline__ void seg_clock_rate(const BatchDev& B, int slot, double rate, long c0, int ng,
+                                               int i0, int i1, int nx, double rdx, int lane) {
+  if (i0 == 0 && lane == 0) rate = fmax(rate, seg_rate(B, B.prim + (c0 + ng) * 4, rdx));
+  if (i1 == nx && lane == 1) rate = fmax(rate, seg_rate(B, B.prim + (c0 + nx - 1 + ng) * 4, rdx));
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) rate = fmax(rate, __shfl_xor_sync(0xffffffffu, rate, o));
+  if (lane == 0)
+    atomicMax((unsigned long long*)(B.clock + (slot + 1) % 3),
+              (unsigned long long)__double_as_longlong(rate));
+}
+
 // ---- FP32 form: one CTA per segment of SEG cells, the whole step fused.
 // In 1D an instance has at most 256 velocities, so a segment's stencil window
 // (SEG + 4 cells x all velocities, h and b) fits in shared memory: the face
@@ -229,11 +239,12 @@ __host__ __device__ inline int seg_smem_max() {
 // A CTA takes segments k = blockIdx.x, blockIdx.x + gridDim.x, ...: one
 // segment each when the grid has a CTA per segment, or a persistent loop
 // when the grid is the number of CTAs that fit on the GPU at once.
+// slot: see BatchDev::clock (-1: the instances' own dt).
 template <int SEG, int SEG_T>
 __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __restrict__ Hin,
                                                      const float* __restrict__ Bin,
                                                      float* __restrict__ Hout,
-                                                     float* __restrict__ Bout) {
+                                                     float* __restrict__ Bout, int slot) {
   using SH = SegShape<SEG, SEG_T>;
   constexpr int SEG_ROWS = SH::ROWS;
   constexpr int SEG_FT = SH::FT;
@@ -241,6 +252,7 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ unsigned long long bar;
   __shared__ float sconst[4];  // T3, T4, 1/dx, 1e-7 dx
+  __shared__ double sdt;       // the instance's time step
   // GB300 runs FP64 at 1/64 of the FP32 rate: FP64 work below is done by as
   // few warps as possible (the per-instance constants by one thread, the
   // cell update and its residual by the first warp)
@@ -260,7 +272,13 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
   const float* Bi = Bin + e0;
   float* Ho = Hout + e0;
   float* Bo = Bout + e0;
-  if (!B.active[b]) {  // converged: carry this segment's cells over
+  bool skip = !B.active[b];
+  if (slot >= 0) {
+    const SegClock c = seg_clock(B, slot);
+    skip = skip || c.stop;
+    if (k == 0 && tid == 0) seg_clock_next(B, slot, c);
+  }
+  if (skip) {  // converged or past the end: carry this segment's cells over
     for (long t = tid; t < (long)(i1 - i0) * ns; t += SEG_T) {
       const long o = (long)(i0 + ng) * ns + t;
       Ho[o] = Hi[o];
@@ -296,7 +314,8 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
     sW[v] = B.wtf[B.vel_off[b] + v];
   }
   if (tid == 0) {
-    const double dx0 = B.dx[b], dt0 = B.dt[b];
+    const double dx0 = B.dx[b], dt0 = slot >= 0 ? seg_clock(B, slot).dt : B.dt[b];
+    sdt = dt0;
     sconst[0] = float(dt0);
     sconst[1] = float(0.5 * dt0 * dt0 / dx0);
     sconst[2] = float(1.0 / dx0);
@@ -348,8 +367,8 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
         const float h0 = hc[v], b0 = bc[v];
         float sh = 0.f, sb = 0.f;
         if (r == 1) {
-          sh = bvl<float>(1, hc[v - sst], h0, hc[v + sst], epsd);
-          sb = bvl<float>(1, bc[v - sst], b0, bc[v + sst], epsd);
+          sh = bvl(hc[v - sst], h0, hc[v + sst], epsd);
+          sb = bvl(bc[v - sst], b0, bc[v + sst], epsd);
         }
         const float side = pos ? 0.5f : -0.5f;
         const float hf = h0 + side * sh, bf = b0 + side * sb;
@@ -398,6 +417,7 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
   if (wid == 0) {
     // residual terms of the cell: a convergence monitor, summed in FP32 below
     float rr[6] = {0, 0, 0, 0, 0, 0};
+    double rate = 0.0;  // CFL rate of the cell's new state (slot >= 0)
     // face f = fa + jf, moment m: the SEG_FT partials of its threads, in order
     for (int t0 = lane; t0 < 3 * (SEG + 1); t0 += 32) {
       const int jf = t0 / 3, m = t0 - 3 * jf;
@@ -419,7 +439,7 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
     __syncwarp();
     // ---- cell parameters of the stepped cells (one lane per cell, FP64)
     if (lane < cb - ca) {
-      const double dx = B.dx[b], dt = B.dt[b];
+      const double dx = B.dx[b], dt = sdt;
       const int i = ca + lane;
       const long c = c0 + i + ng;
       double* w = B.w + c * 4;
@@ -435,6 +455,7 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
       p[0] = pn[0];
       p[1] = pn[1];
       p[2] = pn[2];
+      if (slot >= 0) rate = seg_rate(B, pn, idx);
       for (int m = 0; m < 3; ++m) {
         double d = w[m] - wo[m];
         rr[m] = float(d * d);
@@ -492,6 +513,7 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
 #pragma unroll
       for (int m = 0; m < 6; ++m) pr[m] = (double)rr[m];
     }
+    if (slot >= 0) seg_clock_rate(B, slot, rate, c0, ng, i0, i1, nx, 1.0 / B.dx[b], lane);
   } else if (wid <= SH::NWH) {
     // ---- old heat flux of the stepped cells, QT threads per cell, and the
     // Shakhov factor 0.8 (1 - Pr) lambda^2 / rho q of the cell coefficients
@@ -499,7 +521,7 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
     const int i = ca + jc;
     float qf = 0.f;
     if (B.coll == COLL_SHAKHOV) {
-      BSum<float> sm4;
+      BSum sm4;
       sm4.init();
       if (i < cb) {
         const double Ud = spo[jc * 3 + 1];
@@ -551,8 +573,8 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
         const float h0 = hc[0], b0 = bc[0];
         float sh = 0.f, sb = 0.f;
         if (VL || brule(pos ? f - 1 : f, nx, ng) == 1) {
-          sh = bvl<float>(1, hc[-sst], h0, hc[sst], epsd);
-          sb = bvl<float>(1, bc[-sst], b0, bc[sst], epsd);
+          sh = bvl(hc[-sst], h0, hc[sst], epsd);
+          sb = bvl(bc[-sst], b0, bc[sst], epsd);
         }
         fh = Tu * (h0 + side * sh) - Tuu * sh;
         fbv = Tu * (b0 + side * sb) - Tuu * sb;
@@ -606,6 +628,8 @@ struct SegVariant {
   int (*smem)(int sst_max, int nu4_max);
   int smem_max;
 };
+// The compiled shapes (kb_batch.cu).
+const std::vector<SegVariant>& seg_variants();
 void seg_variants_a(std::vector<SegVariant>& out);
 void seg_variants_b(std::vector<SegVariant>& out);
 

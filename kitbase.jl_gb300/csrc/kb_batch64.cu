@@ -1,0 +1,297 @@
+// kb_batch64.cu -- FP64 step of 1D2F1V solves (KFVS, fixed ends, van Leer),
+// one CTA per segment of a few cells, the whole step fused in one launch.
+#include "kb_batch64.cuh"
+
+#include <algorithm>
+
+#include "kb_f64.cuh"
+
+namespace kb {
+
+constexpr int SEG64_T = 128;
+constexpr int SEG64_CC = 12;  // doubles of coefficients per cell
+
+int seg64_smem(int seg, int ns) {
+  return 8 * ((2 * (seg + 4) + 2 * (seg + 1) + 5) * ns + (seg + 1) * 4 + seg * (SEG64_CC + 4) + 8);
+}
+
+// The FP64 pipe (two lanes per clock on each multiprocessor) bounds the step,
+// so the cells should spread over all multiprocessors; a shorter segment
+// forms more faces twice, (seg + 1) / seg of them, and a longer one holds
+// more shared memory.  Four CTAs per multiprocessor overlap one another's
+// copies, barriers and the serial cell phase.
+int seg64_cells(long cells, int sms) {
+  const long s = cells / (4L * std::max(1, sms));
+  return (int)std::min<long>(SEG64_MAX, std::max<long>(1, s));
+}
+
+// Sum of four values over the warp: a reduce-scatter (two exchanges that
+// halve the number of values a lane carries, then three plain levels), 6
+// FP64 additions instead of 20.  Lanes 0 .. 7 return the total of a, 8 .. 15 of
+// b, 16 .. 23 of c, 24 .. 31 of d.
+__device__ __forceinline__ double warp_sum4(double a, double b, double c, double d, int lane) {
+  const unsigned all = 0xffffffffu;
+  const bool hi = lane & 16, mid = lane & 8;
+  // level 16: the lower half keeps (a, b), the upper half (c, d)
+  double k0 = hi ? c : a, k1 = hi ? d : b;
+  const double g0 = hi ? a : c, g1 = hi ? b : d;
+  k0 += __shfl_xor_sync(all, g0, 16);
+  k1 += __shfl_xor_sync(all, g1, 16);
+  // level 8: bit 8 clear keeps the first of the two, set the second
+  double k = mid ? k1 : k0;
+  const double g = mid ? k0 : k1;
+  k += __shfl_xor_sync(all, g, 8);
+  k += __shfl_xor_sync(all, k, 4);
+  k += __shfl_xor_sync(all, k, 2);
+  k += __shfl_xor_sync(all, k, 1);
+  return k;
+}
+
+// Segment k covers cells [seg_i0[k], seg_i0[k] + seg) of instance seg_b[k];
+// its window (two more cells on each side, h and b, all velocities) arrives
+// by two bulk copies.  Phases, a CTA barrier between them:
+//   1  flux of every face of the segment at every velocity into shared memory
+//      (each is used twice below: by its moments and by the two cells)
+//   2  a warp per face: the three moments, and with them the old heat flux of
+//      the cell to the right of the face
+//   3  a lane per cell: w, prim, tau and the coefficients of the relaxation
+//   4  relaxation of every (cell, velocity)
+// Bound by the FP64 pipe: about 50 (BGK) or 80 (Shakhov) FP64 instructions per
+// cell and velocity.  One CTA per instance, which formed every face flux twice
+// with two IEEE divisions each, left 24 instances (7.5e5 cell-velocity points)
+// on 24 multiprocessors: 4.24 ms a step, now 0.21 ms.  Results do not depend on the
+// segment length or on what else is in the launch: a face's moments are
+// summed in the same lane order wherever the segment starts.
+__global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, int nsm,
+                                                         const double* __restrict__ Hin,
+                                                         const double* __restrict__ Bin,
+                                                         double* __restrict__ Hout,
+                                                         double* __restrict__ Bout, int want_res,
+                                                         int slot) {
+  extern __shared__ __align__(16) unsigned char sm64[];
+  __shared__ unsigned long long bar;
+  __shared__ double sdt[3];  // dt, time before the step, 1: the step is skipped
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int k = blockIdx.x;
+  const int b = B.seg_b[k], i0 = B.seg_i0[k];
+  const int nx = B.nx[b], ng = B.ng[b], nu = B.nu[b], ns = B.nus[b];
+  const int i1 = min(i0 + seg, nx);
+  const long c0 = B.cell_off[b], e0 = B.elem_off[b];
+  const double* Hi = Hin + e0;
+  const double* Bi = Bin + e0;
+  double* Ho = Hout + e0;
+  double* Bo = Bout + e0;
+  if (tid == 0) {
+    sdt[0] = B.dt[b];
+    sdt[2] = B.active[b] ? 0.0 : 1.0;
+    if (slot >= 0) {
+      const SegClock c = seg_clock(B, slot);
+      sdt[0] = c.dt;
+      sdt[1] = c.t;
+      if (c.stop) sdt[2] = 1.0;
+      if (k == 0) seg_clock_next(B, slot, c);
+    }
+    mbar_init(&bar, 1);
+    fence_async_smem();
+  }
+  __syncthreads();
+  if (sdt[2] != 0.0) {  // converged or past the end: carry this segment's cells over
+    for (long t = tid; t < (long)(i1 - i0) * ns; t += SEG64_T) {
+      const long o = (long)(i0 + ng) * ns + t;
+      Ho[o] = Hi[o];
+      Bo[o] = Bi[o];
+    }
+    return;
+  }
+  double* sH = (double*)sm64;
+  double* sB = sH + (seg + 4) * nsm;
+  double* sF = sB + (seg + 4) * nsm;  // fh [face][v]
+  double* sG = sF + (seg + 1) * nsm;  // fb
+  double* sU = sG + (seg + 1) * nsm;
+  double* sW = sU + nsm;
+  double* sWu = sW + nsm;             // weight * u
+  double* sT = sWu + nsm;             // dt u
+  double* sK = sT + nsm;              // +-dt u / 2 - dt^2 u^2 / (2 dx): factor of the slope
+  double* sfw = sK + nsm;             // [face][4]
+  double* sq = sfw + (seg + 1) * 4;   // [cell][4] old heat flux (first value)
+  double* scc = sq + seg * 4;         // [cell][SEG64_CC]
+  // window rows r0 .. r1-1 (cells incl. ghosts) are contiguous in h and b
+  const int r0 = max(i0 - 2, -ng), r1 = min(i1 + 2, nx + ng), nrow = r1 - r0;
+  if (tid == 0) {
+    const unsigned bytes = (unsigned)nrow * ns * 8u;
+    mbar_expect(&bar, 2u * bytes);
+    bulk_g2s(sH, Hi + (long)(r0 + ng) * ns, bytes, &bar);
+    bulk_g2s(sB, Bi + (long)(r0 + ng) * ns, bytes, &bar);
+  }
+  const double dx = B.dx[b], dt = sdt[0];
+  const double rdx = 1.0 / dx;
+  const double T4 = 0.5 * dt * dt * rdx;
+  for (int v = tid; v < nu; v += SEG64_T) {
+    const double u = B.u[B.vel_off[b] + v], w = B.wt[B.vel_off[b] + v];
+    const double tu = dt * u;
+    sU[v] = u;
+    sW[v] = w;
+    sWu[v] = w * u;
+    sT[v] = tu;
+    sK[v] = (u >= 0.0 ? 0.5 : -0.5) * tu - T4 * (u * u);
+  }
+  const bool ok = tid == 0 ? mbar_wait(&bar, 0) : true;
+  if (__syncthreads_or(!ok)) {  // CTA-uniform: bounded clean-up, then leave
+    if (tid == 0) {
+      atomicOr(B.status, 2);
+      mbar_wait(&bar, 0);
+    }
+    return;
+  }
+  const double epsd = 1.e-7 * dx;
+  const int ca = max(i0, 1), cb = min(i1, nx - 1);  // stepped cells [ca, cb)
+  const int nc = max(0, cb - ca), nf = nc > 0 ? nc + 1 : 0;  // faces ca .. cb
+  // ---- 1: fluxes.  fh = dt u (h + side s) - dt^2 u^2 / (2 dx) s = T h + K s
+  for (int t = tid; t < nf * nu; t += SEG64_T) {
+    const int j = t / nu, v = t - j * nu;
+    const int up = ca + j - (sU[v] >= 0.0 ? 1 : 0);  // upwind cell
+    const int o = (up - r0) * ns + v;
+    const double h0 = sH[o], b0 = sB[o];
+    double sh = 0.0, sb = 0.0;
+    if (brule(up, nx, ng) == 1) {
+      sh = vl64(sH[o - ns], h0, sH[o + ns], epsd);
+      sb = vl64(sB[o - ns], b0, sB[o + ns], epsd);
+    }
+    sF[j * ns + v] = fma(sK[v], sh, sT[v] * h0);
+    sG[j * ns + v] = fma(sK[v], sb, sT[v] * b0);
+  }
+  __syncthreads();
+  // ---- 2: moments of face ca + j and heat flux of cell ca + j
+  const bool shak = B.coll == COLL_SHAKHOV;
+  for (int j = wid; j < nf; j += SEG64_T / 32) {
+    double m0 = 0.0, m1 = 0.0, m2 = 0.0, q = 0.0;
+    const double* F = sF + j * ns;
+    const double* G = sG + j * ns;
+    for (int v = lane; v < nu; v += 32) {
+      const double fh = F[v], w = sW[v], wu = sWu[v];
+      m0 = fma(w, fh, m0);
+      m1 = fma(wu, fh, m1);
+      m2 = fma(wu * sU[v], fh, fma(w, G[v], m2));
+    }
+    if (shak && j < nc) {
+      const int o = (ca + j - r0) * ns;
+      const double Uc = B.prim[(c0 + ca + j + ng) * 4 + 1];
+      for (int v = lane; v < nu; v += 32) {
+        const double cu = sU[v] - Uc;
+        q = fma(sW[v] * cu, fma(cu * cu, sH[o + v], sB[o + v]), q);
+      }
+    }
+    const double s = warp_sum4(m0, m1, m2, q, lane);
+    if ((lane & 7) == 0) {
+      const int m = lane >> 3;
+      if (m < 3) sfw[j * 4 + m] = m == 2 ? 0.5 * s : s;
+      else if (j < nc) sq[j * 4] = 0.5 * s;
+    }
+  }
+  __syncthreads();
+  // ---- 3: cell parameters, one lane of warp 0 per cell
+  if (wid == 0) {
+    double rr[6] = {0, 0, 0, 0, 0, 0};
+    double rate = 0.0;
+    if (lane < nc) {
+      const long c = c0 + ca + lane + ng;
+      double* w = B.w + c * 4;
+      double* p = B.prim + c * 4;
+      const double* fL = sfw + lane * 4;
+      const double* fR = fL + 4;
+      const double wo[3] = {w[0], w[1], w[2]};
+      const double rho_o = p[0], Uo = p[1], lo = p[2];
+      double wn[3], pn[4];
+      for (int m = 0; m < 3; ++m) {
+        wn[m] = wo[m] + (fL[m] - fR[m]) * rdx;
+        w[m] = wn[m];
+      }
+      conserve_prim(wn, 3, B.gamma, pn);
+      p[0] = pn[0];
+      p[1] = pn[1];
+      p[2] = pn[2];
+      for (int m = 0; m < 3; ++m) {
+        const double d = wn[m] - wo[m];
+        rr[m] = d * d;
+        rr[3 + m] = fabs(wn[m]);
+      }
+      const double lam = pn[2];
+      if (!(pn[0] > 0.0) || !(lam > 0.0) || !isfinite(pn[0]) || !isfinite(lam)) atomicOr(B.status, 1);
+      const double dtau = dt / vhs_time(pn[0], lam, B.mu[b], B.omega);
+      double* cc = scc + lane * SEG64_CC;
+      cc[0] = pn[0] * sqrt(lam / PI);  // new Maxwellian
+      cc[1] = pn[1];
+      cc[2] = -lam;
+      cc[3] = B.K / (2.0 * lam);
+      cc[4] = dtau;
+      cc[5] = 1.0 / (1.0 + dtau);
+      if (shak) {  // old Maxwellian and the factor of the heat flux
+        cc[6] = rho_o * sqrt(lo / PI);
+        cc[7] = Uo;
+        cc[8] = -lo;
+        cc[9] = B.K / (2.0 * lo);
+        cc[10] = 0.8 * (1.0 - B.Pr) * (lo * lo) / rho_o * sq[lane * 4];
+      }
+      if (slot >= 0) rate = seg_rate(B, pn, rdx);
+    }
+    if (want_res) {
+#pragma unroll
+      for (int m = 0; m < 6; ++m) rr[m] = warp_sum(rr[m]);
+      if (lane == 0) {
+        double* pr = B.respart + (long)k * 8;
+#pragma unroll
+        for (int m = 0; m < 6; ++m) pr[m] = rr[m];
+      }
+    }
+    if (slot >= 0) seg_clock_rate(B, slot, rate, c0, ng, i0, i1, nx, rdx, lane);
+  }
+  __syncthreads();
+  // ---- 4: relaxation; fixed end cells keep their state
+  for (int v = tid; v < nu; v += SEG64_T) {
+    if (i0 == 0) {
+      Ho[(long)ng * ns + v] = sH[(0 - r0) * ns + v];
+      Bo[(long)ng * ns + v] = sB[(0 - r0) * ns + v];
+    }
+    if (i1 == nx) {
+      Ho[(long)(nx - 1 + ng) * ns + v] = sH[(nx - 1 - r0) * ns + v];
+      Bo[(long)(nx - 1 + ng) * ns + v] = sB[(nx - 1 - r0) * ns + v];
+    }
+  }
+  for (int t = tid; t < nc * nu; t += SEG64_T) {
+    const int j = t / nu, v = t - j * nu;
+    const double* cc = scc + j * SEG64_CC;
+    const int o = (ca + j - r0) * ns + v;
+    const double u = sU[v];
+    const double du = u - cc[1];
+    double MH = cc[0] * exp(cc[2] * (du * du));
+    double MB = MH * cc[3];
+    if (shak) {
+      const double ou = u - cc[7], l2 = cc[8] * (ou * ou);  // -lambda c^2
+      const double S = cc[10] * ou * (cc[6] * exp(l2));
+      const double tl = fma(-2.0, l2, B.K);
+      MH = fma(S, tl - 5.0, MH);
+      MB = fma(S * (tl - 3.0), cc[9], MB);
+    }
+    const long g = (long)(ca + j + ng) * ns + v;
+    const double* F = sF + j * ns + v;
+    const double* G = sG + j * ns + v;
+    Ho[g] = fma(cc[4], MH, fma(F[0] - F[ns], rdx, sH[o])) * cc[5];
+    Bo[g] = fma(cc[4], MB, fma(G[0] - G[ns], rdx, sB[o])) * cc[5];
+  }
+}
+
+bool seg64_prepare() {
+  const bool ok = cudaFuncSetAttribute(k_batch_seg64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       seg64_smem(SEG64_MAX, SEG_MAXNU)) == cudaSuccess;
+  prefer_max_shared((const void*)k_batch_seg64);
+  return ok;
+}
+
+void seg64_launch(const BatchDev& B, int seg, const double* hin, const double* bin, double* hout,
+                  double* bout, bool want_res, int slot, cudaStream_t st) {
+  if (B.nseg_all <= 0) return;
+  k_batch_seg64<<<(unsigned)B.nseg_all, SEG64_T, seg64_smem(seg, B.nu4_max), st>>>(
+      B, seg, B.nu4_max, hin, bin, hout, bout, want_res ? 1 : 0, slot);
+}
+
+}  // namespace kb

@@ -7,7 +7,7 @@ import pytest
 
 import kitgpu
 from kitgpu import batch as KB
-from cases import rho_u_t_error
+from cases import oracle_for, rho_u_t_error
 
 pytestmark = pytest.mark.gpu
 
@@ -77,6 +77,37 @@ def test_batch_fp32_edge_sizes(gpu_lib, coll):
     for k, KS in enumerate(sets):
         ref = single(KS, dt[k], 40)
         assert max(rho_u_t_error(outs[k]["prim"], ref["prim"])) < 1e-5, k
+
+
+@pytest.mark.parametrize("coll", ["shakhov", "bgk"])
+def test_batch_fp64_edge_sizes(gpu_lib, coll):
+    """Edges of the FP64 segment form against the oracle (1e-12): the smallest
+    grid, grids of one cell more or less than whole segments, last segments
+    that hold the fixed end alone, velocity counts odd, not a multiple of 4 and
+    around the warp and CTA sizes; ghosts and none.  The same instances are
+    stepped in a small batch (one cell per segment) and beside enough cells
+    for the longest segments: bit-identical."""
+    cfgs = [dict(KB.shock_config(Ma, nx, nu, coll=coll), nxg=ng) for Ma, nx, nu, ng in
+            [(1.5, 3, 5, 0), (2.0, 8, 31, 0), (3.0, 9, 33, 2), (4.0, 17, 128, 0), (6.0, 10, 256, 1),
+             (1.2, 16, 1 + 64, 0), (2.5, 25, 7, 0)]]
+    filler = [KB.shock_config(1.5, 400, 16, coll=coll) for _ in range(16)]
+    outs = []
+    for sets in (KB.solver_sets(cfgs), KB.solver_sets(cfgs + filler)):
+        bt = KB.Batch(sets, "fp64")
+        bt.init_initial()
+        dt = bt.timestep()
+        bt.step(13)
+        outs.append(bt.download()[:len(cfgs)])
+        bt.close()
+    for k, KS in enumerate(KB.solver_sets(cfgs)):
+        for key in ("w", "prim", "h", "b"):
+            assert np.array_equal(outs[0][k][key], outs[1][k][key]), (k, key)
+        orc = oracle_for(KS)
+        orc.step(dt[k], 13)
+        ref = dict(zip(("w", "prim", "h", "b"), orc.get_state()))
+        assert max(rho_u_t_error(outs[0][k]["prim"], ref["prim"])) < 1e-12, k
+        for key in ("h", "b"):
+            assert np.max(np.abs(outs[0][k][key] - ref[key])) < 1e-12 * np.max(ref[key]), (k, key)
 
 
 def test_instance_independent_of_batch(gpu_lib):
