@@ -346,6 +346,12 @@ int kb_create(const kb_config_t* cfg, const double* u, const double* v, const do
         return bail(fail(KB_ERR_CUDA, "wall face list upload failed"));
     }
   }
+  if (kb::line_covers(c)) {
+    const int seg = kb::line_seg(c.precision, c.nx, h->s.sm_count);
+    if ((rc = dev_alloc(h, &p, kb::line_bytes(c, (int)h->ncell, seg))) != KB_OK) return bail(rc);
+    if (!kb::line_init(h->line, c, h->s, (int)h->ncell, seg, p))
+      return bail(fail(KB_ERR_CUDA, "segment kernel set-up failed"));
+  }
   // the set-up copies above are synchronous; wait for this handle's stream
   // only, so that creating a handle never waits for other solves' work
   if (cudaStreamSynchronize(h->stream) != cudaSuccess || cudaGetLastError() != cudaSuccess)
@@ -595,7 +601,7 @@ static int timed_step(kb_handle* h, double dt, cudaEvent_t* ev) {
   return n;
 }
 
-static int enqueue_steps(kb_handle* h, double dt, int nsteps);
+static int enqueue_steps(kb_handle* h, double dt, int nsteps, bool res);
 static void drop_step_graphs(kb_handle* h);
 
 // Two steps from the current buffer recorded as a CUDA graph for kb_step,
@@ -610,7 +616,7 @@ static cudaGraphExec_t step_pair_graph(kb_handle* h, double dt) {
   if (h->sgraph[c]) return h->sgraph[c];
   cudaGraph_t gr = nullptr;
   bool ok = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-  const int n = ok ? enqueue_steps(h, dt, 2) : 0;
+  const int n = ok ? enqueue_steps(h, dt, 2, false) : 0;
   ok = cudaStreamEndCapture(h->stream, &gr) == cudaSuccess && ok;
   h->s.cur = c;  // two recorded steps leave the buffer index where it was
   if (ok && cudaGraphInstantiate(&h->sgraph[c], gr, 0) == cudaSuccess) {
@@ -652,17 +658,15 @@ int kb_step(kb_handle_t* h, double dt, int32_t nsteps, double* residual) {
     // are bound by their kernels rather than by launch latency.  The first
     // two steps run eagerly (modules load and function attributes are set
     // outside any capture); results are those of the eager steps, bit for bit.
+    // Only the last step, which runs eagerly, forms the residual: the call
+    // returns no other.
+    if (h->line.on && nsteps > 0) KB_TRY(check_launch(h, kb::line_begin(h->line, h->s, dt, h->stream)));
     int s = 0;
-    auto eager = [&]() -> int {
-      int n = kb::launch_reconstruct(h->s, h->stream);
-      n += kb::launch_evolve(h->s, dt, h->stream);
-      n += kb::launch_update(h->s, dt, h->stream);
-      return check_launch(h, n);
-    };
+    auto eager = [&]() -> int { return check_launch(h, enqueue_steps(h, dt, 1, s == nsteps - 1)); };
     for (; s < nsteps && s < 2; ++s) KB_TRY(eager());
-    if (nsteps - s >= 4) {
+    if (nsteps - s >= 5) {
       cudaGraphExec_t gx = step_pair_graph(h, dt);
-      for (; gx && s + 2 <= nsteps; s += 2) {
+      for (; gx && s + 2 < nsteps; s += 2) {
         KB_CUDA(cudaGraphLaunch(gx, h->stream));
         h->launches += h->sgraph_launches;
       }
@@ -679,6 +683,35 @@ int kb_step_cfl(kb_handle_t* h, double cfl, double sim_time, double max_time, in
   if (!(cfl > 0.0) || nsteps < 0) return fail(KB_ERR_ARG, "kb_step_cfl: cfl must be positive, nsteps >= 0");
   double t = sim_time;
   double r[4] = {0.0, 0.0, 0.0, 0.0};
+  if (h->line.on && !h->timing) {
+    // The segment kernels find the time step on the device (BatchDev::clock):
+    // steps are enqueued a chunk at a time, with one wait per chunk.
+    kb::Line& L = h->line;
+    constexpr int CHUNK = 64;
+    const double c0[10] = {0.0, 0.0, 0.0, sim_time, 0.0, 0.0, cfl, max_time, h->cfg.umax, 0.0};
+    KB_CUDA(cudaMemcpyAsync(L.d.clock, c0, sizeof(c0), cudaMemcpyHostToDevice, h->stream));
+    KB_TRY(check_launch(h, kb::launch_timestep(h->s, h->cfg.umax, 0.0, L.d.clock, h->stream)));
+    KB_TRY(check_launch(h, kb::line_begin(L, h->s, L.dt, h->stream)));
+    double c[10] = {0.0};
+    int done = 0;  // steps taken
+    for (int s = 0; s < nsteps && done == s;) {
+      const int m = std::min(CHUNK, nsteps - s);
+      for (int k = 0; k < m; ++k, ++s)
+        KB_TRY(check_launch(h, kb::line_step(L, h->s, k == m - 1, s % 3, h->stream)));
+      KB_CUDA(cudaMemcpyAsync(c, L.d.clock, sizeof(c), cudaMemcpyDeviceToHost, h->stream));
+      double rs[4] = {0.0, 0.0, 0.0, 0.0};
+      KB_TRY(read_residual(h, rs));
+      h->evolved = false;
+      done = (int)c[9];
+      t = c[3 + s % 3];
+      if (done > 0)
+        for (int k = 0; k < 4; ++k) r[k] = rs[k];
+    }
+    *time_out = t;
+    if (residual)
+      for (int k = 0; k < h->s.g.NW; ++k) residual[k] = r[k];
+    return KB_OK;
+  }
   // stop at max_time (within rounding of the accumulated time)
   const double t_eps = 1e-14 * fabs(max_time);
   for (int s = 0; s < nsteps && t < max_time - t_eps; ++s) {
@@ -711,13 +744,19 @@ static void drop_step_graphs(kb_handle* h) {
     }
 }
 
-// nsteps steps enqueued kernel by kernel on the handle stream.
-static int enqueue_steps(kb_handle* h, double dt, int nsteps) {
+// nsteps steps enqueued kernel by kernel on the handle stream; res: the last
+// one with its residual.  A line's time step is set by line_begin.
+static int enqueue_steps(kb_handle* h, double dt, int nsteps, bool res) {
   int n = 0;
   for (int s = 0; s < nsteps; ++s) {
+    const bool rs = res && s == nsteps - 1;
+    if (h->line.on) {
+      n += kb::line_step(h->line, h->s, rs, -1, h->stream);
+      continue;
+    }
     n += kb::launch_reconstruct(h->s, h->stream);
     n += kb::launch_evolve(h->s, dt, h->stream);
-    n += kb::launch_update(h->s, dt, h->stream);
+    n += kb::launch_update(h->s, dt, h->stream, rs);
   }
   return n;
 }
@@ -737,6 +776,7 @@ int kb_step_async(kb_handle_t* h, double dt, int32_t nsteps) {
   // first chunk of a shape runs eagerly (module loading and function
   // attributes happen outside a capture) and is recorded for the next one.
   const int c = h->s.cur;
+  if (h->line.on && nsteps > 0) KB_TRY(check_launch(h, kb::line_begin(h->line, h->s, dt, h->stream)));
   if (nsteps > 0 && h->agraph[c] && h->agraph_dt == dt && h->agraph_n == nsteps) {
     KB_CUDA(cudaGraphLaunch(h->agraph[c], h->stream));
     h->launches += h->agraph_launches;
@@ -750,14 +790,14 @@ int kb_step_async(kb_handle_t* h, double dt, int32_t nsteps) {
       h->agraph_dt = dt;
       h->agraph_n = nsteps;
     }
-    KB_TRY(check_launch(h, enqueue_steps(h, dt, nsteps)));
+    KB_TRY(check_launch(h, enqueue_steps(h, dt, nsteps, true)));
     if (again && nsteps > 0 && !h->agraph[c]) {
       // record the same chunk from buffer c for the next calls
       const int after = h->s.cur;
       h->s.cur = c;
       cudaGraph_t gr = nullptr;
       bool ok = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-      int n = ok ? enqueue_steps(h, dt, nsteps) : 0;
+      int n = ok ? enqueue_steps(h, dt, nsteps, true) : 0;
       ok = cudaStreamEndCapture(h->stream, &gr) == cudaSuccess && ok;
       if (ok && cudaGraphInstantiate(&h->agraph[c], gr, 0) == cudaSuccess) {
         h->agraph_launches = n;

@@ -10,6 +10,7 @@
 
 #include "../../include/kitgpu.h"
 #include "kb_kernels.cuh"
+#include "kb_line.cuh"
 
 struct kb_handle {
   kb_config_t cfg;
@@ -40,6 +41,8 @@ struct kb_handle {
   double agraph_dt = 0.0;
   int agraph_n = 0;
   int64_t agraph_launches = 0;
+  // 1D solves the fused segment kernels cover (kb_line.cu)
+  kb::Line line;
   // per-stage kernel timing (kb_set_timing): CUDA events on the handle stream
   bool timing = false;
   std::vector<cudaEvent_t> events;

@@ -989,7 +989,7 @@ int launch_cell_param(DevState& s, double dt, cudaStream_t st) {
 }
 
 template <typename R, int D>
-static int finish_t(DevState& s, cudaStream_t st) {
+static int finish_t(DevState& s, cudaStream_t st, bool res) {
   int n = 0;
   s.cur ^= 1;
   bool fill = false;
@@ -1004,9 +1004,11 @@ static int finish_t(DevState& s, cudaStream_t st) {
     if (s.g.ngx > 0) { k_ghost<R><<<2 * s.g.ngx * nrow, 128, 0, st>>>(t, 0); ++n; }
     if (D == 2 && s.g.ngy > 0) { k_ghost<R><<<2 * s.g.ngy * s.g.nxt, 128, 0, st>>>(t, 1); ++n; }
   }
-  prefer_max_shared((const void*)k_residual<false>);
-  k_residual<false><<<1, 256, 0, st>>>(s);
-  ++n;
+  if (res) {
+    prefer_max_shared((const void*)k_residual<false>);
+    k_residual<false><<<1, 256, 0, st>>>(s);
+    ++n;
+  }
   return n;
 }
 
@@ -1050,15 +1052,15 @@ void group_small(int kind, const DevState& ls, int flux, int blocks, cudaStream_
   }
 }
 
-int launch_finish(DevState& s, cudaStream_t st) {
-  if (s.prec == 0) return s.g.D == 1 ? finish_t<double, 1>(s, st) : finish_t<double, 2>(s, st);
-  return s.g.D == 1 ? finish_t<float, 1>(s, st) : finish_t<float, 2>(s, st);
+int launch_finish(DevState& s, cudaStream_t st, bool res) {
+  if (s.prec == 0) return s.g.D == 1 ? finish_t<double, 1>(s, st, res) : finish_t<double, 2>(s, st, res);
+  return s.g.D == 1 ? finish_t<float, 1>(s, st, res) : finish_t<float, 2>(s, st, res);
 }
 
-int launch_update(DevState& s, double dt, cudaStream_t st) {
+int launch_update(DevState& s, double dt, cudaStream_t st, bool res) {
   int n = launch_cell_param(s, dt, st);
   n += launch_march(s, dt, st);
-  n += launch_finish(s, st);
+  n += launch_finish(s, st, res);
   return n;
 }
 

@@ -130,17 +130,18 @@ void group_small(int kind, const DevState& ls, int flux, int blocks, cudaStream_
 void face_kinds_host(const Geo& g, signed char* kind);
 
 // One time step (reconstruct! -> evolve! -> update!) on `stream`.
-// Returns the number of kernel launches.
+// Returns the number of kernel launches.  res: with the residual (only the
+// last step of a run is asked for it).
 int launch_reconstruct(DevState& s, cudaStream_t st);
 int launch_evolve(DevState& s, double dt, cudaStream_t st);
-int launch_update(DevState& s, double dt, cudaStream_t st);
+int launch_update(DevState& s, double dt, cudaStream_t st, bool res = true);
 
 // The same step split into its kernel groups (per-stage timing):
 // evolve = face_param + moments + wall; update = cell_param + march + finish.
 int launch_face_param(DevState& s, double dt, cudaStream_t st);
 int launch_wall(DevState& s, double dt, cudaStream_t st);
 int launch_cell_param(DevState& s, double dt, cudaStream_t st);
-int launch_finish(DevState& s, cudaStream_t st);
+int launch_finish(DevState& s, cudaStream_t st, bool res = true);
 
 // Pass A (face moments, heat flux) and pass B (pointwise update), kb_march.cu.
 int launch_moments(DevState& s, cudaStream_t st);

@@ -1,0 +1,141 @@
+// kb_line.cu -- single 1D2F1V solves through the fused segment kernels.
+//
+// A 1D solve has a few tens of thousands of cell-velocity points: its step is
+// bound by the latency of the kernels it is made of, not by their work.  The
+// general form launches five (face parameters, face moments, cell parameters,
+// update, residual), each a chain of global loads and FP64 divisions on a
+// handful of CTAs; the segment kernels of the batch do the step in one launch,
+// with the same layout of w, prim, h and b.
+#include "kb_line.cuh"
+
+#include <vector>
+
+namespace kb {
+
+bool line_covers(const kb_config_t& c) {
+  return c.dim == 1 && c.nf != 1 && c.flux == KB_FLUX_KFVS && c.interp_order == 2 &&
+         c.bc[0] == KB_BC_FIX && c.bc[1] == KB_BC_FIX && c.nu <= SEG_MAXNU;
+}
+
+static const SegVariant kLine32 = {4, 128, (const void*)k_batch_seg<4, 128>, seg_smem<4, 128>,
+                                   seg_smem_max<4, 128>()};
+
+int line_seg(int prec, int nx, int sms) {
+  return prec == KB_PREC_FP64 ? seg64_cells(nx, sms) : kLine32.seg;
+}
+
+// ints: nx, ng, nu, nus, vel_off, active, seg_first, nseg, then seg_b and
+// seg_i0; longs: cell_off, elem_off; doubles: dx, dt, mu, clock[10], respart;
+// floats: ul, mc
+static int line_nseg(const kb_config_t& c, int seg) { return (c.nx + seg - 1) / seg; }
+static size_t line_doubles(const kb_config_t& c, int seg) { return 2 + 3 + 11 + 8 * (size_t)line_nseg(c, seg); }
+static size_t line_floats(const kb_config_t& c, int ncell) { return (size_t)(c.nu + 3) / 4 * 4 + 8 * (size_t)ncell; }
+static size_t line_ints(const kb_config_t& c, int seg) { return 8 + 2 * (size_t)line_nseg(c, seg); }
+size_t line_bytes(const kb_config_t& c, int ncell, int seg) {
+  return 8 * line_doubles(c, seg) + 4 * line_floats(c, ncell) + 4 * line_ints(c, seg);
+}
+
+bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int seg, void* mem) {
+  const int ns = line_nseg(c, seg);
+  double* D = (double*)mem;
+  float* F = (float*)(D + line_doubles(c, seg));
+  int* I = (int*)(F + line_floats(c, ncell));
+  std::vector<double> hd(line_doubles(c, seg), 0.0);
+  std::vector<float> hf(line_floats(c, ncell), 0.f);
+  std::vector<int> hi(line_ints(c, seg), 0);
+  hd[2] = s.g.dx;
+  hd[4] = s.g.mu_ref;
+  std::vector<double> u(c.nu);
+  if (cudaMemcpy(u.data(), s.u, sizeof(double) * c.nu, cudaMemcpyDeviceToHost) != cudaSuccess) return false;
+  for (int k = 0; k < c.nu; ++k) hf[k] = float(u[k] - (double)(float)u[k]);
+  const int head[8] = {c.nx, c.ngx, c.nu, s.g.vstride, 0, 1, 0, ns};
+  for (int k = 0; k < 8; ++k) hi[k] = head[k];
+  for (int k = 0; k < ns; ++k) hi[8 + ns + k] = k * seg;  // seg_b stays 0
+  if (cudaMemcpy(D, hd.data(), 8 * hd.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(F, hf.data(), 4 * hf.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(I, hi.data(), 4 * hi.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+    return false;
+  BatchDev& d = L.d;
+  d.n = 1;
+  d.nx = I;
+  d.ng = I + 1;
+  d.nu = I + 2;
+  d.nus = I + 3;
+  d.vel_off = I + 4;
+  d.active = I + 5;
+  d.seg_first = I + 6;
+  d.nseg = I + 7;
+  d.seg_b = I + 8;
+  d.seg_i0 = I + 8 + ns;
+  d.cell_off = (const long*)D;
+  d.elem_off = (const long*)(D + 1);
+  d.dx = D + 2;
+  d.dt = D + 3;
+  d.mu = D + 4;
+  d.clock = D + 5;
+  d.respart = D + 16;
+  d.u = s.u;
+  d.wt = s.wt;
+  d.uf = s.uf;
+  d.wtf = s.wtf;
+  d.ul = F;
+  d.mc = F + (c.nu + 3) / 4 * 4;
+  d.w = s.w;
+  d.prim = s.prim;
+  d.residual = s.residual;
+  d.status = s.status;
+  d.nseg_all = ns;
+  d.sst_max = seg_stride(s.g.vstride);
+  d.nu4_max = s.g.vstride;
+  d.K = s.g.K;
+  d.gamma = s.g.gamma;
+  d.omega = s.g.omega;
+  d.Pr = s.g.Pr;
+  d.tol = 0.0;
+  d.coll = s.coll;
+  L.seg = seg;
+  if (s.prec == 0) {
+    if (!seg64_prepare()) return false;
+  } else {
+    L.f32 = &kLine32;
+    L.smem = kLine32.smem(d.sst_max, d.nu4_max);
+    if (cudaFuncSetAttribute(kLine32.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kLine32.smem_max) !=
+        cudaSuccess)
+      return false;
+    prefer_max_shared(kLine32.fn);
+  }
+  L.on = true;
+  return true;
+}
+
+int line_begin(Line& L, const DevState& s, double dt, cudaStream_t st) {
+  if (L.dt != dt) {
+    cudaMemcpyAsync((void*)L.d.dt, &dt, sizeof(double), cudaMemcpyHostToDevice, st);
+    L.dt = dt;
+  }
+  if (s.prec == 0) return 0;
+  seg_mcache_launch(L.d, 1, s.ncell, st);
+  return 1;
+}
+
+int line_step(Line& L, DevState& s, bool res, int slot, cudaStream_t st) {
+  const int cur = s.cur;
+  if (s.prec == 0) {
+    seg64_launch(L.d, L.seg, (const double*)s.h[cur], (const double*)s.b[cur], (double*)s.h[cur ^ 1],
+                 (double*)s.b[cur ^ 1], res || slot >= 0, slot, st);
+  } else {
+    const float* hin = (const float*)s.h[cur];
+    const float* bin = (const float*)s.b[cur];
+    float* hout = (float*)s.h[cur ^ 1];
+    float* bout = (float*)s.b[cur ^ 1];
+    void* args[] = {(void*)&L.d, (void*)&hin, (void*)&bin, (void*)&hout, (void*)&bout, (void*)&slot};
+    cudaLaunchKernel(L.f32->fn, dim3((unsigned)L.d.nseg_all), dim3((unsigned)L.f32->threads), args,
+                     (size_t)L.smem, st);
+  }
+  s.cur = cur ^ 1;
+  if (!res) return 1;
+  seg_res_launch(L.d, st);
+  return 2;
+}
+
+}  // namespace kb
