@@ -310,7 +310,7 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   B->ng.assign(ngx, ngx + n);
   B->nu.assign(nu, nu + n);
   std::vector<int> vel_off(n);
-  std::vector<double> dx(n), dt(n, 0.0), mu(mu_ref, mu_ref + n);
+  std::vector<double> dx(n), rdx(n), dt(n, 0.0), mu(mu_ref, mu_ref + n), rmu(n);
   B->cell_off.resize(n);
   B->elem_off.resize(n);
   long cells = 0, elems = 0, vels = 0;
@@ -330,6 +330,8 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
     dense += nxt * nu[b];
     vels += nu[b];
     dx[b] = (x1[b] - x0[b]) / nx[b];
+    rdx[b] = 1.0 / dx[b];
+    rmu[b] = 1.0 / (2.0 * mu[b]);
     seg_cap += (nx[b] + 7) / 8;  // the shortest segment length the tuner offers
   }
   int dev = 0, sms = 1;
@@ -360,7 +362,7 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   int *d_nus, *d_segb, *d_segi0, *d_segfirst, *d_nseg;
   double* d_respart;
   long *d_co, *d_eo;
-  double *d_dx, *d_dt, *d_mu, *d_u, *d_w, *d_wv, *d_prim, *d_res;
+  double *d_dx, *d_rdx, *d_dt, *d_mu, *d_rmu, *d_mc64, *d_u, *d_w, *d_wv, *d_prim, *d_res;
   float *d_uf, *d_wf, *d_ul, *d_mc;
   BALLOC(d_nx, int, n);
   BALLOC(d_ng, int, n);
@@ -379,6 +381,8 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   BALLOC(d_dx, double, n);
   BALLOC(d_dt, double, n);
   BALLOC(d_mu, double, n);
+  BALLOC(d_rdx, double, n);
+  BALLOC(d_rmu, double, n);
   BALLOC(d_u, double, vels);
   BALLOC(d_wv, double, vels);
   BALLOC(d_uf, float, vels);
@@ -386,7 +390,8 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   BALLOC(d_wf, float, vels);
   BALLOC(d_w, double, cells * 4);
   BALLOC(d_prim, double, cells * 4);
-  BALLOC(d_mc, float, cells * 8);
+  BALLOC(d_mc, float, B->prec == KB_PREC_FP32 ? cells * 8 : 0);
+  BALLOC(d_mc64, double, B->prec == KB_PREC_FP64 ? cells * 4 : 0);
   BALLOC(d_res, double, (size_t)n * 4);
   BALLOC(B->d_umax, double, n);
   size_t esz = B->prec == KB_PREC_FP64 ? 8 : 4;
@@ -417,6 +422,8 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   ok &= cudaMemcpy(d_dx, dx.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_dt, dt.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_mu, mu.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
+  ok &= cudaMemcpy(d_rdx, rdx.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
+  ok &= cudaMemcpy(d_rmu, rmu.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_u, u_all, sizeof(double) * vels, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_wv, w_all, sizeof(double) * vels, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_uf, uf.data(), sizeof(float) * vels, cudaMemcpyHostToDevice) == cudaSuccess;
@@ -453,6 +460,8 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   d.dx = d_dx;
   d.dt = d_dt;
   d.mu = d_mu;
+  d.rdx = d_rdx;
+  d.rmu = d_rmu;
   d.u = d_u;
   d.wt = d_wv;
   d.uf = d_uf;
@@ -461,6 +470,7 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   d.w = d_w;
   d.prim = d_prim;
   d.mc = d_mc;
+  d.mc64 = d_mc64;
   d.residual = d_res;
   d.active = d_active;
   d.status = d_status;
@@ -468,6 +478,7 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   d.gamma = base->gamma;
   d.omega = base->omega;
   d.Pr = base->Pr;
+  kb::seg_gas(d);
   d.tol = 0.0;
   d.coll = base->collision;
   d.clock = nullptr;
@@ -517,10 +528,11 @@ extern "C" int kb_batch_upload(kb_batch_t* B, const double* w, const double* pri
     }
     cudaStreamSynchronize(B->stream);
   }
-  if (B->prec == KB_PREC_FP32) {  // the FP32 step reads each cell's Maxwellian coefficients
+  {  // the step reads each cell's Maxwellian coefficients
     int maxc = 1;
     for (int b = 0; b < B->n; ++b) maxc = std::max(maxc, B->nx[b] + 2 * B->ng[b]);
-    kb::seg_mcache_launch(B->d, B->n, maxc, B->stream);
+    if (B->prec == KB_PREC_FP32) kb::seg_mcache_launch(B->d, B->n, maxc, B->stream);
+    else kb::seg64_mcache_launch(B->d, B->n, maxc, B->stream);
     B->launches++;
     cudaStreamSynchronize(B->stream);
   }
@@ -547,10 +559,12 @@ extern "C" int kb_batch_init_equilibrium(kb_batch_t* B, const double* w, const d
   int maxc = 1;
   for (int b = 0; b < B->n; ++b) maxc = std::max(maxc, B->nx[b] + 2 * B->ng[b]);
   const dim3 grid((unsigned)maxc, (unsigned)B->n);
-  if (B->prec == KB_PREC_FP64)
+  if (B->prec == KB_PREC_FP64) {
     kb::k_batch_init_eq64<<<grid, 128, 0, B->stream>>>(B->d, (double*)B->h[0], (double*)B->bq[0],
                                                        (double*)B->h[1], (double*)B->bq[1]);
-  else
+    kb::seg64_mcache_launch(B->d, B->n, maxc, B->stream);
+    B->launches++;
+  } else
     kb::k_batch_init_eq32<<<grid, 128, 0, B->stream>>>(B->d, 0, (float*)B->h[0], (float*)B->bq[0],
                                                        (float*)B->h[1], (float*)B->bq[1]);
   B->launches++;
@@ -851,6 +865,7 @@ extern "C" int kb_pool_add(kb_batch_t* B, int32_t nx, int32_t ngx, int32_t nu, d
   bool ok = put1(B->d.nx, b, (int)nx) && put1(B->d.ng, b, (int)ngx) && put1(B->d.nu, b, (int)nu) &&
             put1(B->d.nus, b, (int)nus) && put1(B->d.cell_off, b, co) && put1(B->d.elem_off, b, eo) &&
             put1(B->d.vel_off, b, (int)vo) && put1(B->d.dx, b, dx) && put1(B->d.mu, b, mu_ref) &&
+            put1(B->d.rdx, b, 1.0 / dx) && put1(B->d.rmu, b, 1.0 / (2.0 * mu_ref)) &&
             put1((const double*)B->d_umax, b, umax);
   std::vector<float> uf(nu), ul(nu), wf(nu);
   for (int k = 0; k < nu; ++k) {

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "kb_device.cuh"
+#include "kb_f64.cuh"
 #include "kb_kernels.cuh"
 #include "kb_tma.cuh"
 
@@ -25,8 +26,10 @@ struct BatchDev {
   const long* elem_off;  // first distribution element
   const int* vel_off;    // velocity table offset
   const double* dx;      // cell size
+  const double* rdx;     // 1 / dx
   const double* dt;      // time step
   const double* mu;      // reference viscosity
+  const double* rmu;     // 1 / (2 mu)
   const double* u;       // velocity tables (FP64)
   const double* wt;
   const float* uf;       // FP32 copies
@@ -58,8 +61,22 @@ struct BatchDev {
   int sst_max;           // largest shared-memory row stride of the batch (floats)
   int nu4_max;           // largest velocity count, rounded up to 4
   double K, gamma, omega, Pr, tol;
+  double hg;             // 0.5 / (gamma - 1)
+  float Kf, om1f, prf;   // K, 1 - omega and 0.8 (1 - Pr) in FP32
+  double* mc64;          // [cell][4] FP64 Maxwellian coefficients of the cell's current prim
+                         // (seg_coef64), kept with prim
+  Pow64 tau_pow;         // lambda^(omega - 1) of the collision time
   int coll;
 };
+
+// The gas constants that follow from K, gamma, omega and Pr.
+inline void seg_gas(BatchDev& d) {
+  d.hg = 0.5 / (d.gamma - 1.0);
+  d.Kf = float(d.K);
+  d.om1f = float(1.0 - d.omega);
+  d.prf = float(0.8 * (1.0 - d.Pr));
+  d.tau_pow = pow64_of(d.omega - 1.0);
+}
 
 // van Leer slope times dx: one reciprocal and one multiply (subnormals
 // flushed), the division the FP32 passes of the 2D solver use as well
@@ -115,11 +132,11 @@ __device__ __forceinline__ float seg_maxwell(float u, float ulo, float rn, float
 struct SegMax {
   float rn, Uh, Ul, lam, cB;
   __device__ __forceinline__ void set(const double* p, double K) {
-    rn = float(p[0] * sqrt(p[2] * (1.0 / PI)));
-    Uh = float(p[1]);
-    Ul = float(p[1] - (double)Uh);
-    lam = float(p[2]);
-    cB = float(K / (2.0 * p[2]));
+    rn = f32_of(p[0] * sqrt64(p[2] * (1.0 / PI)));
+    Uh = f32_of(p[1]);
+    Ul = f32_of(p[1] - f64_of(Uh));
+    lam = f32_of(p[2]);
+    cB = f32_of((0.5 * K) * rcp64(p[2]));
   }
 };
 
@@ -178,7 +195,7 @@ __device__ __forceinline__ void seg_clock_next(const BatchDev& B, int slot, cons
   B.clock[clear] = 0.0;
 }
 __device__ __forceinline__ double seg_rate(const BatchDev& B, const double* p, double rdx) {
-  return (fmax(B.clock[8], fabs(p[1])) + sqrt(0.5 * B.gamma / p[2])) * rdx;
+  return (fmax(B.clock[8], fabs(p[1])) + sqrt64((0.5 * B.gamma) * rcp64(p[2]))) * rdx;
 }
 // The largest rate of a segment's cells (`rate`: the stepped cell of this
 // lane) and of the fixed ends among them into the next slot; one warp.  Rates
@@ -208,9 +225,10 @@ constexpr int SEG_MAXNU = 256;
 constexpr int SEG_CC = 4;  // float4 coefficient blocks per cell
 __host__ __device__ inline int seg_stride(int nus) { return (nus + 31) / 32 * 32 + 4; }
 // Thread mapping of a segment CTA of SEG cells and T threads: FT threads per
-// face in the face-moment phase (SEG + 1 faces), QT threads per cell in the
-// heat-flux phase (warps 1 .. NWH), one lane per cell of warp 0 in the cell
-// phase, one thread per velocity in the pointwise phase.
+// face in the face-moment phase (SEG + 1 faces), then one warp of the CTA with
+// a lane per cell in the cell phase and beside it NWH warps with QT threads
+// per cell in the heat-flux phase, one thread per velocity in the pointwise
+// phase.
 template <int SEG, int T>
 struct SegShape {
   static constexpr int ROWS = SEG + 4;  // window cells
@@ -218,17 +236,19 @@ struct SegShape {
   static constexpr int QRAW = (T - 32) / SEG;
   static constexpr int QT = QRAW >= 8 ? 8 : (QRAW >= 4 ? 4 : (QRAW >= 2 ? 2 : 1));
   static constexpr int NWH = (QT * SEG + 31) / 32;
+  static constexpr int NV = 3 * (SEG + 1);  // face moments merged by the cell warp
+  static constexpr int ML = 8 * NV <= 32 ? 8 : (4 * NV <= 32 ? 4 : (2 * NV <= 32 ? 2 : 1));  // lanes for each
   static_assert(SEG <= 32 && T % 32 == 0 && FT >= 1 && QRAW >= 1 && 1 + NWH <= T / 32,
                 "segment shape");
 };
 // Dynamic shared memory of a segment CTA, sized by the batch's largest row
 // stride and velocity count: h and b windows, velocity tables (hi, weight,
-// lo), fw, the 16-byte aligned cell coefficients, the face-moment partials
-// and the old prim of the stepped cells.
+// lo), fw, the 16-byte aligned cell coefficients, the face-moment partials,
+// the old w of the stepped cells and their old Maxwellian coefficients.
 template <int SEG, int T>
 __host__ __device__ inline int seg_smem(int sst_max, int nu4_max) {
   return 2 * (SEG + 4) * sst_max * 4 + 3 * nu4_max * 4 + (SEG + 1) * 3 * 8 + 16 +
-         SEG * SEG_CC * 16 + T * 6 * 4 + SEG * 3 * 8 + 8 * 8;
+         SEG * SEG_CC * 16 + T * 6 * 4 + SEG * 3 * 8 + SEG * 32 + 8 * 8;
 }
 template <int SEG, int T>
 __host__ __device__ inline int seg_smem_max() {
@@ -251,11 +271,14 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
   constexpr int QT = SH::QT;
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ unsigned long long bar;
-  __shared__ float sconst[4];  // T3, T4, 1/dx, 1e-7 dx
-  __shared__ double sdt;       // the instance's time step
-  // GB300 runs FP64 at 1/64 of the FP32 rate: FP64 work below is done by as
-  // few warps as possible (the per-instance constants by one thread, the
-  // cell update and its residual by the first warp)
+  __shared__ float sconst[5];  // T3, T4, 1/dx, 1e-7 dx, 2 mu
+  __shared__ double srdx;      // 1/dx
+  // An FP64 instruction holds a quarter of the multiprocessor for 64 cycles
+  // whatever its active lanes, so the FP64 cell phase is one warp's, written
+  // for few instructions (about 30; the divisions, conversions and compares
+  // of the plain form took 140), and which warp it is changes from segment to
+  // segment: a CTA's warp number decides its quarter, and one fixed warp would
+  // queue every resident CTA's cell phase on the same one.
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if (tid == 0) {
     mbar_init(&bar, 1);
@@ -295,7 +318,6 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
   double* sfw = (double*)(sUl + B.nu4_max);  // [SEG + 1][3]
   // [SEG][SEG_CC] float4 cell coefficients, 16-byte aligned
   float4* scc = (float4*)(((unsigned long long)(sfw + (SEG + 1) * 3) + 15) & ~15ull);
-  float* sred = (float*)(scc + SEG * SEG_CC);  // [SEG_T][6]: face-moment DF partials
   // window rows r0 .. r1-1 (cells incl. ghosts), smem row = cell - r0
   const int r0 = max(i0 - 2, -ng), r1 = min(i1 + 2, nx + ng), nrow = r1 - r0;
   if (tid < 32) {
@@ -314,12 +336,28 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
     sW[v] = B.wtf[B.vel_off[b] + v];
   }
   if (tid == 0) {
-    const double dx0 = B.dx[b], dt0 = slot >= 0 ? seg_clock(B, slot).dt : B.dt[b];
-    sdt = dt0;
-    sconst[0] = float(dt0);
-    sconst[1] = float(0.5 * dt0 * dt0 / dx0);
-    sconst[2] = float(1.0 / dx0);
-    sconst[3] = float(1.e-7 * dx0);
+    const double rdx0 = B.rdx[b], dt0 = slot >= 0 ? seg_clock(B, slot).dt : B.dt[b];
+    sconst[0] = f32_of(dt0);
+    sconst[1] = f32_of(0.5 * dt0 * dt0 * rdx0);
+    sconst[2] = f32_of(rdx0);
+    sconst[3] = f32_of(1.e-7 * B.dx[b]);
+    sconst[4] = f32_of(B.mu[b]) * 2.f;
+    srdx = rdx0;
+  }
+  // the old w and Maxwellian coefficients of the stepped cells, while the
+  // window is on its way
+  const int fa = max(i0, 1), fb = min(i1, nx - 1);
+  const int ca = max(i0, 1), cb = min(i1, nx - 1);  // stepped cells [ca, cb)
+  float* sred = (float*)(scc + SEG * SEG_CC);  // [SEG_T][6]: face-moment DF partials
+  double* swo = (double*)(sred + SEG_T * 6);   // [SEG][3] w
+  float4* smc = (float4*)(((unsigned long long)(swo + SEG * 3) + 15) & ~15ull);  // [SEG][2] see B.mc
+  if (tid < cb - ca) {
+    const long c = c0 + ca + tid + ng;
+    swo[tid * 3 + 0] = B.w[c * 4 + 0];
+    swo[tid * 3 + 1] = B.w[c * 4 + 1];
+    swo[tid * 3 + 2] = B.w[c * 4 + 2];
+    smc[tid * 2] = ((const float4*)(B.mc + c * 8))[0];
+    smc[tid * 2 + 1] = ((const float4*)(B.mc + c * 8))[1];
   }
   // one thread waits for the window; the others wait at the CTA barrier
   const bool ok = tid == 0 ? mbar_wait(&bar, phase & 1) : true;
@@ -338,8 +376,6 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
 
   // ---- face moments of faces fa .. fb: SEG_FT threads per face (velocities
   // v = q mod SEG_FT), so the SEG + 1 faces keep all four warps busy
-  const int fa = max(i0, 1), fb = min(i1, nx - 1);
-  const int ca = max(i0, 1), cb = min(i1, nx - 1);  // stepped cells [ca, cb)
   {
     const int j = tid / SEG_FT, q = tid - j * SEG_FT;
     const int f = fa + j;
@@ -402,67 +438,67 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
     o[4] = m2.hi;
     o[5] = m2.lo + l2;
   }
-  // the old prim of the stepped cells, read before warp 0 overwrites it
-  // (warps 1 and 2 need the old U while warp 0 updates the cells)
-  double* spo = (double*)(sred + SEG_T * 6);  // [SEG][3] rho, U, lambda
-  if (tid < cb - ca) {
-    const double* p = B.prim + (c0 + ca + tid + ng) * 4;
-    spo[tid * 3 + 0] = p[0];
-    spo[tid * 3 + 1] = p[1];
-    spo[tid * 3 + 2] = p[2];
-  }
-  __syncthreads();  // face partials and old prim in shared memory
-  // Warp 0: merge the face moments, then the FP64 cell update; warps 1 and 2
-  // meanwhile: the old heat flux (Shakhov) of the stepped cells.
-  if (wid == 0) {
+  __syncthreads();  // face partials in shared memory
+  // The cell warp: merge the face moments, then the FP64 cell update; NWH other
+  // warps meanwhile: the old heat flux (Shakhov) of the stepped cells.
+  constexpr int NW = SEG_T / 32;
+  const int role = (wid + (int)(((unsigned)k * 2654435761u) >> 29)) % NW;
+  if (role == 0) {
     // residual terms of the cell: a convergence monitor, summed in FP32 below
     float rr[6] = {0, 0, 0, 0, 0, 0};
     double rate = 0.0;  // CFL rate of the cell's new state (slot >= 0)
     // face f = fa + jf, moment m: the SEG_FT partials of its threads, in order
-    for (int t0 = lane; t0 < 3 * (SEG + 1); t0 += 32) {
+    // (ML lanes take every ML-th and join)
+    for (int r = 0; r < SH::NV; r += 32 / SH::ML) {
+      const int t0 = r + lane / SH::ML, ql = lane % SH::ML;
       const int jf = t0 / 3, m = t0 - 3 * jf;
-      if (fa + jf <= fb) {
-        const float* o = sred + jf * SEG_FT * 6 + 2 * m;
-        DF d;
-        d.hi = o[0];
-        d.lo = o[1];
-        for (int t = 1; t < SEG_FT; ++t) {
-          DF e;
-          e.hi = o[6 * t];
-          e.lo = o[6 * t + 1];
-          d = df_merge(d, e);
-        }
-        const double v = (double)d.hi + (double)d.lo;
-        sfw[jf * 3 + m] = m == 2 ? 0.5 * v : v;
+      const float* o = sred + jf * SEG_FT * 6 + 2 * m;
+      const bool live = t0 < SH::NV && fa + jf <= fb;
+      DF d;
+      d.hi = live ? o[6 * ql] : 0.f;
+      d.lo = live ? o[6 * ql + 1] : 0.f;
+      for (int t = ql + SH::ML; live && t < SEG_FT; t += SH::ML) {
+        DF e;
+        e.hi = o[6 * t];
+        e.lo = o[6 * t + 1];
+        d = df_merge(d, e);
       }
+#pragma unroll
+      for (int x = 1; x < SH::ML; x <<= 1) d = df_merge(d, df_shfl_xor(d, x));
+      const float half = m == 2 ? 0.5f : 1.f;
+      if (live && ql == 0) sfw[jf * 3 + m] = f64_of(half * d.hi) + f64_of(half * d.lo);
     }
     __syncwarp();
     // ---- cell parameters of the stepped cells (one lane per cell, FP64)
     if (lane < cb - ca) {
-      const double dx = B.dx[b], dt = sdt;
+      const double rdx = srdx;
       const int i = ca + lane;
       const long c = c0 + i + ng;
       double* w = B.w + c * 4;
       double* p = B.prim + c * 4;
       const double* fL = sfw + (i - fa) * 3;
       const double* fR = sfw + (i + 1 - fa) * 3;
-      double wo[3] = {w[0], w[1], w[2]};
-      const double rho_o = spo[lane * 3 + 0], Uo = spo[lane * 3 + 1], lo = spo[lane * 3 + 2];
-      const double idx = 1.0 / dx;
-      for (int m = 0; m < 3; ++m) w[m] += (fL[m] - fR[m]) * idx;
-      double pn[4];
-      conserve_prim<true>(w, 3, B.gamma, pn);
+      double wn[3];
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        const double d = fL[m] - fR[m];
+        wn[m] = fma(d, rdx, swo[lane * 3 + m]);
+        const float df = f32_of(d) * sconst[2];  // the change of w
+        rr[m] = df * df;
+        rr[3 + m] = fabsf(f32_of(wn[m]));
+        w[m] = wn[m];
+      }
+      // conserve_prim (src/Theory/theory_macro.jl:185-206), hg = 0.5 / (gamma - 1)
+      double pn[3];
+      const double rr0 = rcp64(wn[0]);
+      pn[0] = wn[0];
+      pn[1] = wn[1] * rr0;
+      pn[2] = wn[0] * B.hg * rcp64(fma(-0.5 * wn[1], pn[1], wn[2]));
       p[0] = pn[0];
       p[1] = pn[1];
       p[2] = pn[2];
-      if (slot >= 0) rate = seg_rate(B, pn, idx);
-      for (int m = 0; m < 3; ++m) {
-        double d = w[m] - wo[m];
-        rr[m] = float(d * d);
-        rr[3 + m] = float(fabs(w[m]));
-      }
-      double lam = pn[2];
-      if (!(pn[0] > 0.0) || !(lam > 0.0) || !isfinite(pn[0]) || !isfinite(lam)) atomicOr(B.status, 1);
+      if (slot >= 0) rate = seg_rate(B, pn, rdx);
+      if (!pos64(pn[0]) || !pos64(pn[2])) atomicOr(B.status, 1);
       // w, prim and q stay FP64; the coefficients below feed only the FP32
       // pointwise update.  The Maxwellian's density factor, U and lambda are
       // formed in FP64 and rounded once, and U is carried as an FP32 pair
@@ -470,38 +506,30 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
       // at high Mach the energy is mostly kinetic, and an FP32-rounded U or
       // density factor would bias the moments of the equilibrium by more
       // than the FP32 split form's 1e-5 budget in T.  tau only sets the
-      // relaxation rate and is formed in FP32 (GB300's FP64 rate is 1/64 of
-      // its FP32 rate).
-      const float rf = float(pn[0]), lf = float(lam);
-      const float tau = float(B.mu[b]) * 2.f * powf(lf, float(1.0 - B.omega)) / rf;
-      const float dtt = float(dt) / tau;
-      const double Kd = B.K;
-      float4* kc = scc + lane * SEG_CC;
+      // relaxation rate and is formed in FP32.
+      SegMax mn;  // the new Maxwellian
+      mn.set(pn, B.K);
+      const float tau = sconst[4] * powf(mn.lam, B.om1f) / f32_of(pn[0]);
+      const float dtt = sconst[0] / tau;
       // the old Maxwellian's coefficients are the ones this cell's update
       // formed from the same prim one step earlier (or the set-up formed from
-      // the initial prim): read instead of recomputed, which saves an FP64
-      // square root and division per cell, bit for bit the same values
-      float4* mcc = (float4*)(B.mc + c * 8);
-      const float4 mo = mcc[0];
-      const float mUl = mcc[1].x;
+      // the initial prim): read instead of recomputed
+      const float4 mo = smc[lane * 2];
+      float4* kc = scc + lane * SEG_CC;
       // new Maxwellian: density factor, U (hi), lambda, K / (2 lambda)
-      SegMax mn;
-      mn.set(pn, Kd);
       kc[0] = make_float4(mn.rn, mn.Uh, mn.lam, mn.cB);
       // dt / tau, 1 / (1 + dt / tau), old Maxwellian (Shakhov) density factor and U (hi)
       kc[1] = make_float4(dtt, 1.f / (1.f + dtt), mo.x, mo.y);
       // old lambda, K / (2 lambda); .z (the Shakhov heat-flux factor) comes
-      // from warps 1-2; .w the low part of U
+      // from the heat-flux warps; .w the low part of U
       float* k2 = (float*)(kc + 2);
       k2[0] = mo.z;
       k2[1] = mo.w;
       k2[3] = mn.Ul;
-      kc[3] = make_float4(mUl, 0.f, 0.f, 0.f);
-      mcc[0] = make_float4(mn.rn, mn.Uh, mn.lam, mn.cB);
-      mcc[1] = make_float4(mn.Ul, 0.f, 0.f, 0.f);
+      kc[3] = make_float4(smc[lane * 2 + 1].x, 0.f, 0.f, 0.f);
+      seg_store_coef(B, c, mn);
     }
-    // residual partial sums of the segment, in a fixed shuffle order (FP32:
-    // GB300's FP64 pipe would make this tree the longest chain of the phase)
+    // residual partial sums of the segment, in a fixed shuffle order
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
 #pragma unroll
@@ -511,21 +539,20 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
     if (lane == 0) {
       double* pr = B.respart + (long)k * 8;
 #pragma unroll
-      for (int m = 0; m < 6; ++m) pr[m] = (double)rr[m];
+      for (int m = 0; m < 6; ++m) pr[m] = f64_of(rr[m]);
     }
-    if (slot >= 0) seg_clock_rate(B, slot, rate, c0, ng, i0, i1, nx, 1.0 / B.dx[b], lane);
-  } else if (wid <= SH::NWH) {
+    if (slot >= 0) seg_clock_rate(B, slot, rate, c0, ng, i0, i1, nx, srdx, lane);
+  } else if (role <= SH::NWH) {
     // ---- old heat flux of the stepped cells, QT threads per cell, and the
     // Shakhov factor 0.8 (1 - Pr) lambda^2 / rho q of the cell coefficients
-    const int lt = tid - 32, jc = lt / QT, q = lt % QT;
+    const int lt = (role - 1) * 32 + lane, jc = lt / QT, q = lt % QT;
     const int i = ca + jc;
     float qf = 0.f;
     if (B.coll == COLL_SHAKHOV) {
       BSum sm4;
       sm4.init();
       if (i < cb) {
-        const double Ud = spo[jc * 3 + 1];
-        const float Uc = float(Ud), Ul = float(Ud - (double)Uc);  // U as an FP32 pair
+        const float Uc = smc[jc * 2].y, Ul = smc[jc * 2 + 1].x;  // U as an FP32 pair
         const float* hc = rowH(i);
         const float* bc = rowB(i);
         int it = 0;
@@ -540,9 +567,8 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
 #pragma unroll
       for (int m = 1; m < QT; m <<= 1) d = df_merge(d, df_shfl_xor(d, m));
       if (i < cb) {
-        const double qc = 0.5 * ((double)d.hi + (double)d.lo);
-        const float rof = float(spo[jc * 3 + 0]), lof = float(spo[jc * 3 + 2]);
-        qf = float(0.8 * (1.0 - B.Pr)) * (lof * lof) / rof * float(qc);
+        const float lof = smc[jc * 2].z;
+        qf = B.prf * (lof * lof) / f32_of(swo[jc * 3]) * (0.5f * (d.hi + d.lo));
       }
     }
     if (q == 0 && jc < SEG && i < cb) ((float*)(scc + jc * SEG_CC + 2))[2] = qf;
@@ -601,7 +627,7 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
           const float ou = (u - k1.w) + (ulo - kc[3].x);
           const float OH = k1.z * fexp(-k2.x * ou * ou);
           const float cq = k2.z * ou;
-          const float tl = 2.f * k2.x * ou * ou + float(B.K);
+          const float tl = 2.f * k2.x * ou * ou + B.Kf;
           MH += cq * (tl - 5.f) * OH;
           MB += cq * (tl - 3.f) * OH * k2.y;
         }

@@ -12,7 +12,7 @@ constexpr int SEG64_T = 128;
 constexpr int SEG64_CC = 12;  // doubles of coefficients per cell
 
 int seg64_smem(int seg, int ns) {
-  return 8 * ((2 * (seg + 4) + 2 * (seg + 1) + 5) * ns + (seg + 1) * 4 + seg * (SEG64_CC + 4) + 8);
+  return 8 * ((2 * (seg + 4) + 2 * (seg + 1) + 5) * ns + (seg + 1) * 4 + seg * (SEG64_CC + 4) + EXP64_N + 8);
 }
 
 // The FP64 pipe (two lanes per clock on each multiprocessor) bounds the step,
@@ -45,6 +45,16 @@ __device__ __forceinline__ double warp_sum4(double a, double b, double c, double
   k += __shfl_xor_sync(all, k, 2);
   k += __shfl_xor_sync(all, k, 1);
   return k;
+}
+
+// Coefficients of a cell's Maxwellian from its prim [rho, U, lambda]: density
+// factor, K / (2 lambda), and the Shakhov factor 0.8 (1 - Pr) lambda^2 / rho.
+// A step needs them for the new state and for the old; the old ones are those
+// that the step before formed from the same prim (BatchDev::mc64).
+__device__ __forceinline__ void seg_coef64(const BatchDev& B, const double* p, double rrho, double* m) {
+  m[0] = p[0] * sqrt64(p[2] * (1.0 / PI));
+  m[1] = (0.5 * B.K) * rcp64(p[2]);
+  m[2] = (0.8 * (1.0 - B.Pr)) * (p[2] * p[2]) * rrho;
 }
 
 // Segment k covers cells [seg_i0[k], seg_i0[k] + seg) of instance seg_b[k];
@@ -115,6 +125,7 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
   double* sfw = sK + nsm;             // [face][4]
   double* sq = sfw + (seg + 1) * 4;   // [cell][4] old heat flux (first value)
   double* scc = sq + seg * 4;         // [cell][SEG64_CC]
+  double* stab = scc + seg * SEG64_CC;  // 2^(j / 64)
   // window rows r0 .. r1-1 (cells incl. ghosts) are contiguous in h and b
   const int r0 = max(i0 - 2, -ng), r1 = min(i1 + 2, nx + ng), nrow = r1 - r0;
   if (tid == 0) {
@@ -124,8 +135,26 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
     bulk_g2s(sB, Bi + (long)(r0 + ng) * ns, bytes, &bar);
   }
   const double dx = B.dx[b], dt = sdt[0];
-  const double rdx = 1.0 / dx;
+  const double rdx = B.rdx[b];
   const double T4 = 0.5 * dt * dt * rdx;
+  const int ca = max(i0, 1), cb = min(i1, nx - 1);  // stepped cells [ca, cb)
+  const int nc = max(0, cb - ca), nf = nc > 0 ? nc + 1 : 0;  // faces ca .. cb
+  // the lane that updates a cell (of a warp that changes from segment to
+  // segment: its number decides which quarter of the multiprocessor works)
+  // reads its w and prim while the window is on its way
+  const bool shak = B.coll == COLL_SHAKHOV;
+  const int role = (wid + (int)(((unsigned)k * 2654435761u) >> 30)) % (SEG64_T / 32);
+  const bool mine = role == 0 && lane < nc;
+  const long cell = c0 + ca + lane + ng;
+  double wo[3] = {1.0, 0.0, 1.0}, po[3] = {1.0, 0.0, 1.0}, mo[3] = {1.0, 0.0, 0.0}, rmu = 1.0;
+  if (mine) {
+    for (int m = 0; m < 3; ++m) {
+      wo[m] = B.w[cell * 4 + m];
+      po[m] = B.prim[cell * 4 + m];
+      mo[m] = B.mc64[cell * 4 + m];
+    }
+    rmu = B.rmu[b];
+  }
   for (int v = tid; v < nu; v += SEG64_T) {
     const double u = B.u[B.vel_off[b] + v], w = B.wt[B.vel_off[b] + v];
     const double tu = dt * u;
@@ -133,7 +162,16 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
     sW[v] = w;
     sWu[v] = w * u;
     sT[v] = tu;
-    sK[v] = (u >= 0.0 ? 0.5 : -0.5) * tu - T4 * (u * u);
+    sK[v] = fma(nonneg64(u) ? 0.5 : -0.5, tu, -T4 * (u * u));
+  }
+  exp64_load(stab, tid, SEG64_T);
+  if (mine && shak) {  // the old Maxwellian
+    double* cc = scc + lane * SEG64_CC;
+    cc[7] = po[1];
+    cc[8] = EXP64_LOG2E * po[2];
+    cc[9] = mo[1];
+    cc[10] = mo[0] * mo[2];
+    cc[11] = 2.0 * po[2];
   }
   const bool ok = tid == 0 ? mbar_wait(&bar, 0) : true;
   if (__syncthreads_or(!ok)) {  // CTA-uniform: bounded clean-up, then leave
@@ -144,12 +182,10 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
     return;
   }
   const double epsd = 1.e-7 * dx;
-  const int ca = max(i0, 1), cb = min(i1, nx - 1);  // stepped cells [ca, cb)
-  const int nc = max(0, cb - ca), nf = nc > 0 ? nc + 1 : 0;  // faces ca .. cb
   // ---- 1: fluxes.  fh = dt u (h + side s) - dt^2 u^2 / (2 dx) s = T h + K s
   for (int t = tid; t < nf * nu; t += SEG64_T) {
     const int j = t / nu, v = t - j * nu;
-    const int up = ca + j - (sU[v] >= 0.0 ? 1 : 0);  // upwind cell
+    const int up = ca + j - (nonneg64(sU[v]) ? 1 : 0);  // upwind cell
     const int o = (up - r0) * ns + v;
     const double h0 = sH[o], b0 = sB[o];
     double sh = 0.0, sb = 0.0;
@@ -162,7 +198,6 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
   }
   __syncthreads();
   // ---- 2: moments of face ca + j and heat flux of cell ca + j
-  const bool shak = B.coll == COLL_SHAKHOV;
   for (int j = wid; j < nf; j += SEG64_T / 32) {
     double m0 = 0.0, m1 = 0.0, m2 = 0.0, q = 0.0;
     const double* F = sF + j * ns;
@@ -175,7 +210,7 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
     }
     if (shak && j < nc) {
       const int o = (ca + j - r0) * ns;
-      const double Uc = B.prim[(c0 + ca + j + ng) * 4 + 1];
+      const double Uc = scc[j * SEG64_CC + 7];
       for (int v = lane; v < nu; v += 32) {
         const double cu = sU[v] - Uc;
         q = fma(sW[v] * cu, fma(cu * cu, sH[o + v], sB[o + v]), q);
@@ -189,49 +224,50 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
     }
   }
   __syncthreads();
-  // ---- 3: cell parameters, one lane of warp 0 per cell
-  if (wid == 0) {
+  // ---- 3: cell parameters, one lane per cell
+  if (role == 0) {
     double rr[6] = {0, 0, 0, 0, 0, 0};
     double rate = 0.0;
-    if (lane < nc) {
-      const long c = c0 + ca + lane + ng;
-      double* w = B.w + c * 4;
-      double* p = B.prim + c * 4;
+    if (mine) {
+      double* w = B.w + cell * 4;
+      double* p = B.prim + cell * 4;
       const double* fL = sfw + lane * 4;
       const double* fR = fL + 4;
-      const double wo[3] = {w[0], w[1], w[2]};
-      const double rho_o = p[0], Uo = p[1], lo = p[2];
-      double wn[3], pn[4];
-      for (int m = 0; m < 3; ++m) {
-        wn[m] = wo[m] + (fL[m] - fR[m]) * rdx;
-        w[m] = wn[m];
-      }
-      conserve_prim(wn, 3, B.gamma, pn);
-      p[0] = pn[0];
-      p[1] = pn[1];
-      p[2] = pn[2];
-      for (int m = 0; m < 3; ++m) {
-        const double d = wn[m] - wo[m];
-        rr[m] = d * d;
-        rr[3 + m] = fabs(wn[m]);
-      }
-      const double lam = pn[2];
-      if (!(pn[0] > 0.0) || !(lam > 0.0) || !isfinite(pn[0]) || !isfinite(lam)) atomicOr(B.status, 1);
-      const double dtau = dt / vhs_time(pn[0], lam, B.mu[b], B.omega);
+      double wn[3], pn[3];
+      for (int m = 0; m < 3; ++m) wn[m] = wo[m] + (fL[m] - fR[m]) * rdx;
+      // conserve_prim (src/Theory/theory_macro.jl:185-206) with hg = 0.5 / (gamma - 1)
+      const double rr0 = rcp64(wn[0]), hr = wn[0] * B.hg;
+      pn[0] = wn[0];
+      pn[1] = wn[1] * rr0;
+      const double ei = fma(-0.5 * wn[1], pn[1], wn[2]);
+      const double lam = hr * rcp64(ei);
+      pn[2] = lam;
+      // dt / tau, tau = 2 mu lambda^(1 - omega) / rho (vhs_collision_time,
+      // src/Theory/theory_relaxation.jl:28)
+      const double dtau = (dt * rmu) * (pn[0] * pow_tab(lam, B.tau_pow, stab));
+      double mn[3];
+      seg_coef64(B, pn, rr0, mn);
       double* cc = scc + lane * SEG64_CC;
-      cc[0] = pn[0] * sqrt(lam / PI);  // new Maxwellian
+      cc[0] = mn[0];  // new Maxwellian
       cc[1] = pn[1];
-      cc[2] = -lam;
-      cc[3] = B.K / (2.0 * lam);
+      cc[2] = EXP64_LOG2E * lam;
+      cc[3] = mn[1];
       cc[4] = dtau;
-      cc[5] = 1.0 / (1.0 + dtau);
-      if (shak) {  // old Maxwellian and the factor of the heat flux
-        cc[6] = rho_o * sqrt(lo / PI);
-        cc[7] = Uo;
-        cc[8] = -lo;
-        cc[9] = B.K / (2.0 * lo);
-        cc[10] = 0.8 * (1.0 - B.Pr) * (lo * lo) / rho_o * sq[lane * 4];
+      cc[5] = rcp64(1.0 + dtau);
+      if (shak) cc[10] *= sq[lane * 4];  // the factor of the heat flux
+      for (int m = 0; m < 3; ++m) {
+        w[m] = wn[m];
+        p[m] = pn[m];
+        B.mc64[cell * 4 + m] = mn[m];
       }
+      if (want_res) {
+        for (int m = 0; m < 3; ++m) {
+          const double d = wn[m] - wo[m];
+          rr[m] = d * d;
+          rr[3 + m] = fabs(wn[m]);
+        }
+      }
+      if (!pos64(pn[0]) || !pos64(lam)) atomicOr(B.status, 1);
       if (slot >= 0) rate = seg_rate(B, pn, rdx);
     }
     if (want_res) {
@@ -257,20 +293,21 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
       Bo[(long)(nx - 1 + ng) * ns + v] = sB[(nx - 1 - r0) * ns + v];
     }
   }
+  const double K3 = B.K - 3.0;
   for (int t = tid; t < nc * nu; t += SEG64_T) {
     const int j = t / nu, v = t - j * nu;
     const double* cc = scc + j * SEG64_CC;
     const int o = (ca + j - r0) * ns + v;
     const double u = sU[v];
     const double du = u - cc[1];
-    double MH = cc[0] * exp(cc[2] * (du * du));
+    double MH = cc[0] * exp2_tab(cc[2], du * du, stab);
     double MB = MH * cc[3];
     if (shak) {
-      const double ou = u - cc[7], l2 = cc[8] * (ou * ou);  // -lambda c^2
-      const double S = cc[10] * ou * (cc[6] * exp(l2));
-      const double tl = fma(-2.0, l2, B.K);
-      MH = fma(S, tl - 5.0, MH);
-      MB = fma(S * (tl - 3.0), cc[9], MB);
+      const double ou = u - cc[7], o2 = ou * ou;
+      const double S = cc[10] * ou * exp2_tab(cc[8], o2, stab);
+      const double tl = fma(cc[11], o2, K3);  // 2 lambda c^2 + K - 3
+      MH = fma(S, tl - 2.0, MH);
+      MB = fma(S * tl, cc[9], MB);
     }
     const long g = (long)(ca + j + ng) * ns + v;
     const double* F = sF + j * ns + v;
@@ -278,6 +315,19 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
     Ho[g] = fma(cc[4], MH, fma(F[0] - F[ns], rdx, sH[o])) * cc[5];
     Bo[g] = fma(cc[4], MB, fma(G[0] - G[ns], rdx, sB[o])) * cc[5];
   }
+}
+
+__global__ void k_batch_mcache64(BatchDev B) {
+  const int b = blockIdx.y;
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= B.nx[b] + 2 * B.ng[b]) return;
+  const long cell = B.cell_off[b] + c;
+  double mn[3];
+  seg_coef64(B, B.prim + cell * 4, rcp64(B.prim[cell * 4]), mn);
+  for (int m = 0; m < 3; ++m) B.mc64[cell * 4 + m] = mn[m];
+}
+void seg64_mcache_launch(const BatchDev& B, int n, int max_cells, cudaStream_t st) {
+  k_batch_mcache64<<<dim3((unsigned)((max_cells + 31) / 32), (unsigned)n), 32, 0, st>>>(B);
 }
 
 bool seg64_prepare() {

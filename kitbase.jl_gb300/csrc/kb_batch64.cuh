@@ -22,7 +22,8 @@ void seg64_launch(const BatchDev& B, int seg, const double* hin, const double* b
                   double* bout, bool want_res, int slot, cudaStream_t st);
 // Per-instance residual of the last step that left its sums (k_batch_seg_res).
 void seg_res_launch(const BatchDev& B, cudaStream_t st);
-// FP32 Maxwellian coefficients of every cell from its prim (BatchDev::mc).
+// Maxwellian coefficients of every cell from its prim (BatchDev::mc64, mc).
+void seg64_mcache_launch(const BatchDev& B, int n, int max_cells, cudaStream_t st);
 void seg_mcache_launch(const BatchDev& B, int n, int max_cells, cudaStream_t st);
 
 }  // namespace kb

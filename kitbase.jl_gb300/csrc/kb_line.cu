@@ -25,10 +25,11 @@ int line_seg(int prec, int nx, int sms) {
 }
 
 // ints: nx, ng, nu, nus, vel_off, active, seg_first, nseg, then seg_b and
-// seg_i0; longs: cell_off, elem_off; doubles: dx, dt, mu, clock[10], respart;
-// floats: ul, mc
+// seg_i0; longs: cell_off, elem_off; doubles: dx, dt, mu, 1/dx, 1/(2 mu),
+// clock[10], respart, FP64 mc64; floats: ul, FP32 mc
 static int line_nseg(const kb_config_t& c, int seg) { return (c.nx + seg - 1) / seg; }
-static size_t line_doubles(const kb_config_t& c, int seg) { return 2 + 3 + 11 + 8 * (size_t)line_nseg(c, seg); }
+static size_t line_doubles(const kb_config_t& c, int seg) { return 18 + 8 * (size_t)line_nseg(c, seg); }
+// (8 floats or 4 doubles of Maxwellian coefficients per cell: the same room)
 static size_t line_floats(const kb_config_t& c, int ncell) { return (size_t)(c.nu + 3) / 4 * 4 + 8 * (size_t)ncell; }
 static size_t line_ints(const kb_config_t& c, int seg) { return 8 + 2 * (size_t)line_nseg(c, seg); }
 size_t line_bytes(const kb_config_t& c, int ncell, int seg) {
@@ -45,6 +46,8 @@ bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int 
   std::vector<int> hi(line_ints(c, seg), 0);
   hd[2] = s.g.dx;
   hd[4] = s.g.mu_ref;
+  hd[5] = 1.0 / s.g.dx;
+  hd[6] = 1.0 / (2.0 * s.g.mu_ref);
   std::vector<double> u(c.nu);
   if (cudaMemcpy(u.data(), s.u, sizeof(double) * c.nu, cudaMemcpyDeviceToHost) != cudaSuccess) return false;
   for (int k = 0; k < c.nu; ++k) hf[k] = float(u[k] - (double)(float)u[k]);
@@ -72,14 +75,17 @@ bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int 
   d.dx = D + 2;
   d.dt = D + 3;
   d.mu = D + 4;
-  d.clock = D + 5;
-  d.respart = D + 16;
+  d.rdx = D + 5;
+  d.rmu = D + 6;
+  d.clock = D + 7;
+  d.respart = D + 18;
   d.u = s.u;
   d.wt = s.wt;
   d.uf = s.uf;
   d.wtf = s.wtf;
   d.ul = F;
   d.mc = F + (c.nu + 3) / 4 * 4;
+  d.mc64 = (double*)d.mc;
   d.w = s.w;
   d.prim = s.prim;
   d.residual = s.residual;
@@ -91,6 +97,7 @@ bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int 
   d.gamma = s.g.gamma;
   d.omega = s.g.omega;
   d.Pr = s.g.Pr;
+  seg_gas(d);
   d.tol = 0.0;
   d.coll = s.coll;
   L.seg = seg;
@@ -113,8 +120,8 @@ int line_begin(Line& L, const DevState& s, double dt, cudaStream_t st) {
     cudaMemcpyAsync((void*)L.d.dt, &dt, sizeof(double), cudaMemcpyHostToDevice, st);
     L.dt = dt;
   }
-  if (s.prec == 0) return 0;
-  seg_mcache_launch(L.d, 1, s.ncell, st);
+  if (s.prec == 0) seg64_mcache_launch(L.d, 1, s.ncell, st);
+  else seg_mcache_launch(L.d, 1, s.ncell, st);
   return 1;
 }
 

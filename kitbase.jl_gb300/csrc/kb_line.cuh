@@ -28,8 +28,8 @@ size_t line_bytes(const kb_config_t& c, int ncell, int seg);
 // Fill `mem` (line_bytes) and L for the solve in s; outside any capture.
 bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int seg, void* mem);
 // Before steps with time step dt (outside any capture): the step in device
-// memory and, FP32, the Maxwellian coefficients of the current prim.  Returns
-// the number of launches.
+// memory and the Maxwellian coefficients of the current prim.  Returns the
+// number of launches.
 int line_begin(Line& L, const DevState& s, double dt, cudaStream_t st);
 // One step (advances s.cur); res: with its residual.  slot: BatchDev::clock.
 int line_step(Line& L, DevState& s, bool res, int slot, cudaStream_t st);
