@@ -604,21 +604,29 @@ static int timed_step(kb_handle* h, double dt, cudaEvent_t* ev) {
 static int enqueue_steps(kb_handle* h, double dt, int nsteps, bool res);
 static void drop_step_graphs(kb_handle* h);
 
-// Two steps from the current buffer recorded as a CUDA graph for kb_step,
-// cached per starting buffer and dt; null when recording failed (the caller
-// then steps eagerly).
-static cudaGraphExec_t step_pair_graph(kb_handle* h, double dt) {
+// Steps per recorded graph of kb_step (even, so that the buffer index comes
+// back).  Between two graphs the GPU idles for some microseconds: a line's
+// step takes about ten, so 16 of its one-kernel steps share a graph (FP32
+// 200 x 101: 9.9 -> 8.8 us a step); longer steps gain nothing from more than
+// two, and every new dt pays for the recording.
+static int graph_steps(const kb_handle* h) { return h->line.on ? 16 : 2; }
+
+// graph_steps steps from the current buffer recorded as a CUDA graph for
+// kb_step, cached per starting buffer and dt (a line's dt is in device memory,
+// so its graph serves any); null when recording failed (the caller then steps
+// eagerly).
+static cudaGraphExec_t step_graph(kb_handle* h, double dt) {
   const int c = h->s.cur;
-  if (h->sgraph_dt != dt) {
+  if (h->sgraph_dt != dt && !h->line.on) {
     drop_step_graphs(h);
     h->sgraph_dt = dt;
   }
   if (h->sgraph[c]) return h->sgraph[c];
   cudaGraph_t gr = nullptr;
   bool ok = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-  const int n = ok ? enqueue_steps(h, dt, 2, false) : 0;
+  const int n = ok ? enqueue_steps(h, dt, graph_steps(h), false) : 0;
   ok = cudaStreamEndCapture(h->stream, &gr) == cudaSuccess && ok;
-  h->s.cur = c;  // two recorded steps leave the buffer index where it was
+  h->s.cur = c;  // the recorded steps leave the buffer index where it was
   if (ok && cudaGraphInstantiate(&h->sgraph[c], gr, 0) == cudaSuccess) {
     h->sgraph_launches = n;
   } else {
@@ -653,8 +661,8 @@ int kb_step(kb_handle_t* h, double dt, int32_t nsteps, double* residual) {
       }
     }
   } else {
-    // A long run replays two steps recorded as a CUDA graph: one graph
-    // launch per two steps instead of ~16 kernel launches, so small solves
+    // A long run replays steps recorded as a CUDA graph: one graph launch for
+    // several steps instead of ~8 kernel launches per step, so small solves
     // are bound by their kernels rather than by launch latency.  The first
     // two steps run eagerly (modules load and function attributes are set
     // outside any capture); results are those of the eager steps, bit for bit.
@@ -664,9 +672,10 @@ int kb_step(kb_handle_t* h, double dt, int32_t nsteps, double* residual) {
     int s = 0;
     auto eager = [&]() -> int { return check_launch(h, enqueue_steps(h, dt, 1, s == nsteps - 1)); };
     for (; s < nsteps && s < 2; ++s) KB_TRY(eager());
-    if (nsteps - s >= 5) {
-      cudaGraphExec_t gx = step_pair_graph(h, dt);
-      for (; gx && s + 2 < nsteps; s += 2) {
+    const int gs = graph_steps(h);
+    if (nsteps - s > 2 * gs) {
+      cudaGraphExec_t gx = step_graph(h, dt);
+      for (; gx && s + gs < nsteps; s += gs) {
         KB_CUDA(cudaGraphLaunch(gx, h->stream));
         h->launches += h->sgraph_launches;
       }

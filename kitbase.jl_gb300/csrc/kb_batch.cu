@@ -36,6 +36,8 @@ namespace kb {
 // an atomic counter of the others.
 __global__ void k_batch_seg_res(BatchDev B) {
   const int b = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_next();
   if (b >= B.n || !B.active[b]) return;  // warp-uniform
   double t[6] = {0, 0, 0, 0, 0, 0};
   const int s0 = B.seg_first[b], s1 = s0 + B.nseg[b];
@@ -55,7 +57,8 @@ __global__ void k_batch_seg_res(BatchDev B) {
 }
 
 void seg_res_launch(const BatchDev& B, cudaStream_t st) {
-  k_batch_seg_res<<<(unsigned)((B.n + 3) / 4), 128, 0, st>>>(B);
+  void* args[] = {(void*)&B};
+  launch_after((const void*)k_batch_seg_res, dim3((unsigned)((B.n + 3) / 4)), dim3(128), 0, st, args);
 }
 
 __global__ void k_batch_timestep(BatchDev B, const double* umax, double cfl, double* dt_out,
@@ -649,8 +652,8 @@ static int batch_launch(kb_batch* B, int cur, bool res) {
     int slot = -1;
     void* args[] = {(void*)&B->d, (void*)&hin, (void*)&bin, (void*)&hout, (void*)&bout, (void*)&slot};
     if (B->seg_grid > 0) {  // an empty pool has no segments
-      cudaLaunchKernel(B->seg_fn, dim3((unsigned)B->seg_grid), dim3((unsigned)B->seg_t), args,
-                       (size_t)B->seg_smem, B->stream);
+      kb::launch_after(B->seg_fn, dim3((unsigned)B->seg_grid), dim3((unsigned)B->seg_t),
+                       (size_t)B->seg_smem, B->stream, args);
       ++n;
     }
   } else {

@@ -295,6 +295,20 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
   const float* Bi = Bin + e0;
   float* Ho = Hout + e0;
   float* Bo = Bout + e0;
+  const int sst = seg_stride(ns);
+  float* sH = (float*)sm;
+  float* sB = sH + SEG_ROWS * B.sst_max;
+  float* sU = sB + SEG_ROWS * B.sst_max;
+  float* sW = sU + B.nu4_max;
+  float* sUl = sW + B.nu4_max;               // low parts of the velocities
+  for (int v = tid; v < nu; v += SEG_T) {
+    sU[v] = B.uf[B.vel_off[b] + v];
+    sUl[v] = B.ul[B.vel_off[b] + v];
+    sW[v] = B.wtf[B.vel_off[b] + v];
+  }
+  // up to here only what no step writes
+  pdl_wait();
+  pdl_next();
   bool skip = !B.active[b];
   if (slot >= 0) {
     const SegClock c = seg_clock(B, slot);
@@ -307,14 +321,9 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
       Ho[o] = Hi[o];
       Bo[o] = Bi[o];
     }
+    __syncthreads();  // the velocity tables are reused by the next segment
     continue;  // CTA-uniform
   }
-  const int sst = seg_stride(ns);
-  float* sH = (float*)sm;
-  float* sB = sH + SEG_ROWS * B.sst_max;
-  float* sU = sB + SEG_ROWS * B.sst_max;
-  float* sW = sU + B.nu4_max;
-  float* sUl = sW + B.nu4_max;               // low parts of the velocities
   double* sfw = (double*)(sUl + B.nu4_max);  // [SEG + 1][3]
   // [SEG][SEG_CC] float4 cell coefficients, 16-byte aligned
   float4* scc = (float4*)(((unsigned long long)(sfw + (SEG + 1) * 3) + 15) & ~15ull);
@@ -329,11 +338,6 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
       float* dst = ((r & 1) ? sB : sH) + row * sst;
       bulk_g2s(dst, src, (unsigned)ns * 4u, &bar);
     }
-  }
-  for (int v = tid; v < nu; v += SEG_T) {
-    sU[v] = B.uf[B.vel_off[b] + v];
-    sUl[v] = B.ul[B.vel_off[b] + v];
-    sW[v] = B.wtf[B.vel_off[b] + v];
   }
   if (tid == 0) {
     const double rdx0 = B.rdx[b], dt0 = slot >= 0 ? seg_clock(B, slot).dt : B.dt[b];

@@ -8,21 +8,33 @@
 
 namespace kb {
 
-constexpr int SEG64_T = 128;
+constexpr int SEG64_T = 256;  // against 128: 700 x 200 points 34.1 -> 28.3 us a step
 constexpr int SEG64_CC = 12;  // doubles of coefficients per cell
 
 int seg64_smem(int seg, int ns) {
   return 8 * ((2 * (seg + 4) + 2 * (seg + 1) + 5) * ns + (seg + 1) * 4 + seg * (SEG64_CC + 4) + EXP64_N + 8);
 }
 
-// The FP64 pipe (two lanes per clock on each multiprocessor) bounds the step,
-// so the cells should spread over all multiprocessors; a shorter segment
-// forms more faces twice, (seg + 1) / seg of them, and a longer one holds
-// more shared memory.  Four CTAs per multiprocessor overlap one another's
-// copies, barriers and the serial cell phase.
+// The FP64 pipe bounds the step, and one warp on each quarter of a
+// multiprocessor nearly fills it: the segments should give every
+// multiprocessor the same work.  A segment of s cells forms s + 1 faces and
+// has a fixed part worth about one more, so the length with the smallest
+// (segments of the busiest multiprocessor) (s + 2) is taken.  Against four or
+// more short segments per multiprocessor: 700 x 64 points 25.1 -> 13.8 us a
+// step, 700 x 200 46.1 -> 28.3, 2048 x 256 106.8 -> 91.5; up to 16 cells a
+// segment, whose memory leaves one CTA on a multiprocessor, are slower for
+// ensembles (128 shocks: 753 against 650 us).
 int seg64_cells(long cells, int sms) {
-  const long s = cells / (4L * std::max(1, sms));
-  return (int)std::min<long>(SEG64_MAX, std::max<long>(1, s));
+  long best = 0;
+  int seg = 1;
+  for (int s = 1; s <= SEG64_MAX; ++s) {
+    const long ctas = (cells + s - 1) / s, t = (ctas + sms - 1) / std::max(1, sms) * (s + 2);
+    if (s == 1 || t <= best) {
+      best = t;
+      seg = s;
+    }
+  }
+  return seg;
 }
 
 // Sum of four values over the warp: a reduce-scatter (two exchanges that
@@ -69,7 +81,7 @@ __device__ __forceinline__ void seg_coef64(const BatchDev& B, const double* p, d
 // Bound by the FP64 pipe: about 50 (BGK) or 80 (Shakhov) FP64 instructions per
 // cell and velocity.  One CTA per instance, which formed every face flux twice
 // with two IEEE divisions each, left 24 instances (7.5e5 cell-velocity points)
-// on 24 multiprocessors: 4.24 ms a step, now 0.21 ms.  Results do not depend on the
+// on 24 multiprocessors: 4.24 ms a step, now 0.15 ms.  Results do not depend on the
 // segment length or on what else is in the launch: a face's moments are
 // summed in the same lane order wherever the segment starts.
 __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, int nsm,
@@ -91,6 +103,29 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
   const double* Bi = Bin + e0;
   double* Ho = Hout + e0;
   double* Bo = Bout + e0;
+  double* sH = (double*)sm64;
+  double* sB = sH + (seg + 4) * nsm;
+  double* sF = sB + (seg + 4) * nsm;  // fh [face][v]
+  double* sG = sF + (seg + 1) * nsm;  // fb
+  double* sU = sG + (seg + 1) * nsm;
+  double* sW = sU + nsm;
+  double* sWu = sW + nsm;             // weight * u
+  double* sT = sWu + nsm;             // dt u
+  double* sK = sT + nsm;              // +-dt u / 2 - dt^2 u^2 / (2 dx): factor of the slope
+  double* sfw = sK + nsm;             // [face][4]
+  double* sq = sfw + (seg + 1) * 4;   // [cell][4] old heat flux (first value)
+  double* scc = sq + seg * 4;         // [cell][SEG64_CC]
+  double* stab = scc + seg * SEG64_CC;  // 2^(j / 256)
+  for (int v = tid; v < nu; v += SEG64_T) {
+    const double u = B.u[B.vel_off[b] + v], w = B.wt[B.vel_off[b] + v];
+    sU[v] = u;
+    sW[v] = w;
+    sWu[v] = w * u;
+  }
+  exp64_load(stab, tid, SEG64_T);
+  // up to here only what no step writes
+  pdl_wait();
+  pdl_next();
   if (tid == 0) {
     sdt[0] = B.dt[b];
     sdt[2] = B.active[b] ? 0.0 : 1.0;
@@ -113,19 +148,6 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
     }
     return;
   }
-  double* sH = (double*)sm64;
-  double* sB = sH + (seg + 4) * nsm;
-  double* sF = sB + (seg + 4) * nsm;  // fh [face][v]
-  double* sG = sF + (seg + 1) * nsm;  // fb
-  double* sU = sG + (seg + 1) * nsm;
-  double* sW = sU + nsm;
-  double* sWu = sW + nsm;             // weight * u
-  double* sT = sWu + nsm;             // dt u
-  double* sK = sT + nsm;              // +-dt u / 2 - dt^2 u^2 / (2 dx): factor of the slope
-  double* sfw = sK + nsm;             // [face][4]
-  double* sq = sfw + (seg + 1) * 4;   // [cell][4] old heat flux (first value)
-  double* scc = sq + seg * 4;         // [cell][SEG64_CC]
-  double* stab = scc + seg * SEG64_CC;  // 2^(j / 64)
   // window rows r0 .. r1-1 (cells incl. ghosts) are contiguous in h and b
   const int r0 = max(i0 - 2, -ng), r1 = min(i1 + 2, nx + ng), nrow = r1 - r0;
   if (tid == 0) {
@@ -156,15 +178,11 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
     rmu = B.rmu[b];
   }
   for (int v = tid; v < nu; v += SEG64_T) {
-    const double u = B.u[B.vel_off[b] + v], w = B.wt[B.vel_off[b] + v];
+    const double u = sU[v];
     const double tu = dt * u;
-    sU[v] = u;
-    sW[v] = w;
-    sWu[v] = w * u;
     sT[v] = tu;
     sK[v] = fma(nonneg64(u) ? 0.5 : -0.5, tu, -T4 * (u * u));
   }
-  exp64_load(stab, tid, SEG64_T);
   if (mine && shak) {  // the old Maxwellian
     double* cc = scc + lane * SEG64_CC;
     cc[7] = po[1];
@@ -340,8 +358,10 @@ bool seg64_prepare() {
 void seg64_launch(const BatchDev& B, int seg, const double* hin, const double* bin, double* hout,
                   double* bout, bool want_res, int slot, cudaStream_t st) {
   if (B.nseg_all <= 0) return;
-  k_batch_seg64<<<(unsigned)B.nseg_all, SEG64_T, seg64_smem(seg, B.nu4_max), st>>>(
-      B, seg, B.nu4_max, hin, bin, hout, bout, want_res ? 1 : 0, slot);
+  int nsm = B.nu4_max, res = want_res ? 1 : 0;
+  void* args[] = {(void*)&B, &seg, &nsm, &hin, &bin, &hout, &bout, &res, &slot};
+  launch_after((const void*)k_batch_seg64, dim3((unsigned)B.nseg_all), dim3(SEG64_T),
+               (size_t)seg64_smem(seg, B.nu4_max), st, args);
 }
 
 }  // namespace kb

@@ -136,8 +136,7 @@ int line_step(Line& L, DevState& s, bool res, int slot, cudaStream_t st) {
     float* hout = (float*)s.h[cur ^ 1];
     float* bout = (float*)s.b[cur ^ 1];
     void* args[] = {(void*)&L.d, (void*)&hin, (void*)&bin, (void*)&hout, (void*)&bout, (void*)&slot};
-    cudaLaunchKernel(L.f32->fn, dim3((unsigned)L.d.nseg_all), dim3((unsigned)L.f32->threads), args,
-                     (size_t)L.smem, st);
+    launch_after(L.f32->fn, dim3((unsigned)L.d.nseg_all), dim3((unsigned)L.f32->threads), (size_t)L.smem, st, args);
   }
   s.cur = cur ^ 1;
   if (!res) return 1;

@@ -8,6 +8,29 @@
 
 namespace kb {
 
+// ---- programmatic dependent launch.  A step is a chain of short kernels; a
+// kernel launched with launch_after starts when every CTA of the one before it
+// has called pdl_next, so its CTAs are placed, and set up what no kernel of the
+// chain writes, while that one still runs.  pdl_wait returns once the kernels
+// before are complete and their writes are visible: every kernel of a chain
+// calls it, in every thread that reads or writes what they do, before anything
+// else of theirs.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+inline cudaError_t launch_after(const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t st, void** args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelExC(&c, fn, args);
+}
+
 // ---- bulk async copies (TMA engine) into shared memory, completed on an mbarrier.
 // Every wait is bounded by the global timer: after KB_WAIT_NS the waiter
 // gives up, and the caller records KB status bit 2 (timeout).
