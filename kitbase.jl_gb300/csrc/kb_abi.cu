@@ -211,6 +211,7 @@ int kb_create(const kb_config_t* cfg, const double* u, const double* v, const do
   g.mu_ref = c.mu_ref;
   g.omega = c.omega;
   g.Pr = c.Pr;
+  kb::geo_consts(g);
   h->nvel = g.nvel;
   h->vstride = g.vstride;
   h->ncell = (long)g.nxt * g.nyt;
@@ -270,16 +271,16 @@ int kb_create(const kb_config_t* cfg, const double* u, const double* v, const do
   ALLOC(h->s.prim, double, h->ncell * 4);
   ALLOC(h->s.sw, double, h->ncell * 8);
   ALLOC(h->s.fp, kb::FaceParam, h->nface);
-  ALLOC(h->s.fpf, kb::FaceParamF, h->nface);
   ALLOC(h->s.fw, double, (size_t)h->nface * 4);
   ALLOC(h->s.wall, double, (size_t)h->nface * 4);
   ALLOC(h->s.rhow, double, h->nface);
   ALLOC(h->s.kind, signed char, h->nface);
   ALLOC(h->s.q, double, h->ncell * 2);
-  ALLOC(h->s.cp, kb::CellParam, h->ncell);
-  ALLOC(h->s.cpf, kb::CellParamF, h->ncell);
-  ALLOC(h->s.fc, kb::FaceCoef32, h->nface);
-  ALLOC(h->s.cc, kb::CellCoef32, h->ncell);
+  ALLOC(h->s.cp, kb::CellParam, c.precision == KB_PREC_FP32 ? 0 : h->ncell);
+  const bool f32 = c.precision == KB_PREC_FP32;
+  ALLOC(h->s.fc, kb::FaceCoef32, f32 ? h->nface : 0);
+  ALLOC(h->s.fc64, kb::FaceCoef64, f32 ? 0 : h->nface);
+  ALLOC(h->s.cc, kb::CellCoef32, f32 ? h->ncell : 0);
   ALLOC(h->s.blockres, double, (size_t)h->s.res_blocks * 16);
   h->s.mpart = nullptr;
   h->s.grp = nullptr;
@@ -304,8 +305,10 @@ int kb_create(const kb_config_t* cfg, const double* u, const double* v, const do
   cudaMemset(h->s.wall, 0, sizeof(double) * h->nface * 4);
   cudaMemset(h->s.rhow, 0, sizeof(double) * h->nface);
   cudaMemset(h->s.status, 0, sizeof(int));
-  cudaMemset(h->s.fc, 0, sizeof(kb::FaceCoef32) * h->nface);
-  cudaMemset(h->s.cc, 0, sizeof(kb::CellCoef32) * h->ncell);
+  if (f32) {
+    cudaMemset(h->s.fc, 0, sizeof(kb::FaceCoef32) * h->nface);
+    cudaMemset(h->s.cc, 0, sizeof(kb::CellCoef32) * h->ncell);
+  }
   cudaMemset(h->s.fp, 0, sizeof(kb::FaceParam) * h->nface);
   cudaMemset(h->s.residual, 0, sizeof(double) * 4);
 

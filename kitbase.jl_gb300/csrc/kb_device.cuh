@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "kb_f64.cuh"
+
 namespace kb {
 
 constexpr double PI = 3.141592653589793238462643383279502884;
@@ -38,7 +40,27 @@ struct Geo {
   // 2F models, 0 for the 1F models, which carry no b (src/Solver/step_1f.jl)
   double Kb;
   int nf;  // distributions per cell: 2 (h, b) or 1 (f, held in h; b stays 0)
+  // formed once on the host (geo_consts): FP64 divisions are dear on the device
+  double rdx, rdy;   // 1 / dx, 1 / dy
+  double rds;        // 1 / cell size (dx, or dx dy)
+  double hg;         // 0.5 / (gamma - 1)
+  double rmu;        // 1 / (2 mu_ref)
+  double sfac;       // 0.8 (1 - Pr)
+  double rKD;        // 1 / (K + D)
+  float om1f;        // omega - 1
+  Pow64 tau_pow;     // lambda^(omega - 1) of the collision time
 };
+inline void geo_consts(Geo& g) {
+  g.rdx = 1.0 / g.dx;
+  g.rdy = 1.0 / g.dy;
+  g.rds = 1.0 / (g.D == 1 ? g.dx : g.dx * g.dy);
+  g.hg = 0.5 / (g.gamma - 1.0);
+  g.rmu = 1.0 / (2.0 * g.mu_ref);
+  g.sfac = 0.8 * (1.0 - g.Pr);
+  g.rKD = 1.0 / (g.K + double(g.D));
+  g.om1f = float(g.omega - 1.0);
+  g.tau_pow = pow64_of(g.omega - 1.0);
+}
 
 // Interface quantities of one face in the face-local frame.  KFVS uses only
 // `mult`; KCU adds the equilibrium part (prim, Mt[0..1], fwa); UGKS all of it.
@@ -53,35 +75,16 @@ struct FaceParam {
   double tr[2];     // transport coefficients incl. len: Th = tr0 un h_face - tr1 un^2 sh
 };
 
-// FP32 copy of the per-v coefficients of FaceParam, read by the FP32 kernels.
-struct FaceParamF {
-  float rho_n;      // rho * (lambda/pi)^(D/2)
-  float U, V, lam;  // interface velocity (local frame) and lambda
-  float cB;         // K / (2 lambda)
-  float Mt[5];
-  float aL[4], aR[4], aT[4];
-  float Mxi2;
-  float len;
-  float pad[2];
-};
-
-// Per-cell quantities of the update: new Maxwellian, relaxation factor,
-// Shakhov coefficients at the old state.
+// Per-cell quantities of the FP64 update: new Maxwellian, relaxation factors,
+// old Maxwellian with the Shakhov factors.
 struct CellParam {
-  double rho_n, U, V, lam, cB;  // new Maxwellian: rho*(lam/pi)^(D/2), U, V, lambda, K/(2 lambda)
+  double rho_n, U, V, l2, cB;  // new Maxwellian: rho*(lam/pi)^(D/2), U, V, EXP64_LOG2E lambda, K/(2 lambda)
   double dtau;                  // dt / tau
   double inv;                   // 1 / (1 + dt / tau)
   double o_rho_n, oU, oV, olam, ocB;  // old Maxwellian (Shakhov term)
-  double sfac;                  // 0.8 (1 - Pr) lambda^2 / rho (old)
-  double q0, q1;                // old heat flux
+  double s0, s1;                // 0.8 (1 - Pr) lambda^2 / rho (old) times the old heat flux
   int upd;                      // 0: copied unchanged, 1: stepped
   int coll;                     // collision model used for this cell
-};
-
-struct CellParamF {
-  float rho_n, U, V, lam, cB, dtau, inv;
-  float o_rho_n, oU, oV, olam, ocB, sf0, sf1;  // sf0/1 = sfac * q0/1
-  int upd, coll;
 };
 
 // FP32 coefficient block of one face for the velocity-owning kernels.  With
@@ -104,6 +107,18 @@ struct __align__(16) FaceCoef32 {
   float4 Cm;  // C2..C5 for un < 0
   float4 Dm;  // D2..D5 for un < 0
 };
+
+// The same block in FP64, with the Maxwellian as rho (lam/pi)^(D/2), U, V and
+// EXP64_LOG2E lambda (exp2_tab).
+struct Quad64 {
+  double x, y, z, w;
+};
+struct FaceCoef64 {
+  Quad64 E, T, G, Cp, Dp, Cm, Dm;
+};
+template <typename R> struct FaceCoefOf;
+template <> struct FaceCoefOf<float> { using T = FaceCoef32; };
+template <> struct FaceCoefOf<double> { using T = FaceCoef64; };
 
 // FP32 coefficients of the pointwise cell update (velocity (u, v), c2):
 //   M   = 2^(EM.x + EM.y u + EM.z v + EM.w c2),  MB = M A.x
@@ -177,181 +192,130 @@ __device__ __forceinline__ double slope_of<double>(int rule, double qm, double q
 
 // ---------------------------------------------------- scalar FP64 physics
 
-// conserve_prim!, src/Theory/theory_macro.jl:185-206.  FAST (the FP32 split
-// form) multiplies by 1 / rho instead of dividing: GB300 runs FP64 at 1/64 of
-// the FP32 rate and each FP64 division costs several FP64 operations.
-template <bool FAST = false>
-__device__ inline void conserve_prim(const double* W, int nw, double g, double* p) {
-  if (FAST) {
-    const double r = 1.0 / W[0];
-    p[0] = W[0];
-    p[1] = W[1] * r;
-    if (nw == 3) {
-      p[2] = 0.5 * W[0] / ((g - 1.0) * (W[2] - 0.5 * (W[1] * W[1]) * r));
-      p[3] = 0.0;
-    } else {
-      p[2] = W[2] * r;
-      p[3] = 0.5 * W[0] / ((g - 1.0) * (W[3] - 0.5 * (W[1] * W[1] + W[2] * W[2]) * r));
-    }
-    return;
-  }
-  if (nw == 3) {
-    p[0] = W[0];
-    p[1] = W[1] / W[0];
-    p[2] = 0.5 * W[0] / (g - 1.0) / (W[2] - 0.5 * (W[1] * W[1]) / W[0]);
+// conserve_prim!, src/Theory/theory_macro.jl:185-206, with hg = 0.5 / (gamma - 1).
+template <int NW>
+__device__ __forceinline__ void conserve_prim(const double* W, double hg, double* p) {
+  const double r = rcp64(W[0]);
+  p[0] = W[0];
+  p[1] = W[1] * r;
+  if (NW == 3) {
+    p[2] = W[0] * hg * rcp64(fma(-0.5 * W[1], p[1], W[2]));
     p[3] = 0.0;
   } else {
-    p[0] = W[0];
-    p[1] = W[1] / W[0];
-    p[2] = W[2] / W[0];
-    p[3] = 0.5 * W[0] / (g - 1.0) / (W[3] - 0.5 * (W[1] * W[1] + W[2] * W[2]) / W[0]);
+    p[2] = W[2] * r;
+    p[3] = W[0] * hg * rcp64(fma(-0.5, fma(W[1], p[1], W[2] * p[2]), W[3]));
   }
 }
 
 // Transcendental functions of the face and cell parameters.  FAST (the FP32
 // split form, whose fluxes are FP32 anyway) evaluates them in FP32 and widens
-// the result; otherwise the FP64 library functions.  Arithmetic, divisions
-// and the moment recursions stay FP64 either way.
+// the result; otherwise FP64 (tab: exp64_load).  Arithmetic and the moment
+// recursions stay FP64 either way.
 template <bool FAST>
-__device__ __forceinline__ double t_exp(double x) { return FAST ? (double)expf((float)x) : exp(x); }
+__device__ __forceinline__ double t_exp_neg(double x, const double* tab) {  // e^-x, x >= 0
+  return FAST ? f64_of(expf(f32_of(-x))) : exp2_tab(EXP64_LOG2E, x, tab);
+}
 template <bool FAST>
-__device__ __forceinline__ double t_erfc(double x) { return FAST ? (double)erfcf((float)x) : erfc(x); }
+__device__ __forceinline__ double t_erfc(double x) { return FAST ? f64_of(erfcf(f32_of(x))) : erfc(x); }
 template <bool FAST>
-__device__ __forceinline__ double t_sqrt(double x) { return FAST ? (double)sqrtf((float)x) : sqrt(x); }
+__device__ __forceinline__ double t_sqrt(double x) { return FAST ? f64_of(sqrtf(f32_of(x))) : sqrt64(x); }
+
+// 1 / tau of vhs_collision_time, tau = 2 mu lambda^(1 - omega) / rho
+// (src/Theory/theory_relaxation.jl:28)
 template <bool FAST>
-__device__ __forceinline__ double t_pow(double x, double y) {
-  return FAST ? (double)powf((float)x, (float)y) : pow(x, y);
+__device__ __forceinline__ double vhs_rate(const Geo& g, double rho, double lam, const double* tab) {
+  const double p = FAST ? f64_of(powf(f32_of(lam), g.om1f)) : pow_tab(lam, g.tau_pow, tab);
+  return g.rmu * rho * p;
 }
 
-// vhs_collision_time, src/Theory/theory_relaxation.jl:28
-template <bool FAST = false>
-__device__ inline double vhs_time(double rho, double lam, double mu, double om) {
-  return mu * 2.0 * t_pow<FAST>(lam, 1.0 - om) / rho;
+// Half-range moments of the Gaussian (gauss_moments,
+// src/Theory/theory_moments.jl:10-86) of orders 0 and 1: over u > 0,
+// L0 = erfc(-s) / 2 with s = sqrt(lambda) U, L1 = U L0 + e, over u < 0,
+// R0 = erfc(s) / 2, R1 = U R0 - e, e = exp(-s^2) / (2 sqrt(pi lambda)).  The
+// smaller of L0 and R0 is evaluated and the other is 1 less it.
+// hl = 1 / (2 lambda).
+template <bool FAST>
+__device__ __forceinline__ void half_range(double l, double U, double hl, const double* tab, double& L0,
+                                           double& L1, double& R0, double& R1) {
+  const double sl = t_sqrt<FAST>(l), x = l * (U * U);
+  const double e = FAST ? f64_of(0.5f * expf(f32_of(-x)) * rsqrtf(f32_of(PI * l)))
+                        : exp2_tab(EXP64_LOG2E, x, tab) * (hl * sl * 0.56418958354775628695);  // 1 / sqrt(pi)
+  const double a = 0.5 * t_erfc<FAST>(sl * fabs(U)), b = 1.0 - a;
+  const bool up = nonneg64(U);
+  L0 = up ? b : a;
+  R0 = up ? a : b;
+  L1 = fma(U, L0, e);
+  R1 = fma(U, R0, -e);
 }
 
-// Moments of the Gaussian: orders 0..6 of the full / left / right half
-// range in u, orders 0..6 in v, orders 0..2 of the internal energy
-// (gauss_moments, src/Theory/theory_moments.jl:10-86).
-struct GM {
-  double Mu[7], MuL[7], MuR[7], Mv[7], Mxi[3];
+// Conserved moments of u^al (slope . psi) of a Maxwellian
+// (moments_conserve_slope, src/Theory/theory_moments.jl:335-369), psi =
+// (1, u, [v,] (u^2 + [v^2 +] xi^2) / 2): the tangential and internal parts
+// depend on the slope and the Maxwellian alone (SlopeV), so one slope's
+// half- and full-range moments of several orders share them.
+template <int NW>
+struct SlopeV {
+  double a0, a1, c, x1, x2, V0, V1, V2, v1, v2;
+  // a: slope; V: tangential velocity; hl = 1 / (2 lambda); x1, x2: <xi^2>, <xi^4>
+  __device__ __forceinline__ void set(const double* a, double V, double hl, double x1_, double x2_) {
+    x1 = x1_;
+    x2 = x2_;
+    a0 = a[0];
+    a1 = a[1];
+    c = 0.5 * a[NW - 1];
+    const double A = fma(c, x1, a0);
+    if (NW == 3) {
+      V0 = A;
+      return;
+    }
+    const double a2 = a[2];
+    v1 = V;
+    v2 = fma(V, V, hl);
+    const double v3 = fma(V, v2, 2.0 * hl * v1), v4 = fma(V, v3, 3.0 * hl * v2);
+    V0 = fma(c, v2, fma(a2, v1, A));
+    V1 = fma(c, v3, fma(a2, v2, A * v1));
+    V2 = fma(c, v4, fma(a2, v3, A * v2));
+  }
+  // M: u moments of orders al .. al + 4
+  __device__ __forceinline__ void get(const double* M, double* o) const {
+    const double U0 = fma(a1, M[1], c * M[2]), U1 = fma(a1, M[2], c * M[3]), U2 = fma(a1, M[3], c * M[4]);
+    const double s0 = fma(M[0], V0, U0);
+    o[0] = s0;
+    o[1] = fma(M[1], V0, U1);
+    // <xi^2 ...> = x1 (s0 - c x1 M0) + c x2 M0
+    double e = fma(M[2], V0, U2) + fma(x1, s0, c * fma(-x1, x1, x2) * M[0]);
+    if (NW == 4) {
+      o[2] = fma(M[0], V1, v1 * U0);
+      e += fma(M[0], V2, v2 * U0);
+    }
+    o[NW - 1] = 0.5 * e;
+  }
 };
 
-// half: 1 the left half range only (MuL, Mv, Mxi), 2 the right half only,
-// 3 everything.  1 / (2 lambda) is formed once and multiplied in.
-template <bool FAST = false>
-__device__ inline void gauss_moments(const double* p, int nw, double inK, GM& m, int half = 3) {
-  double l = p[nw - 1], U = p[1];
-  const double hl = 0.5 / l;
-  const double sl = t_sqrt<FAST>(l);
-  // e = exp(-l U^2) / (2 sqrt(pi l)); FAST evaluates it in FP32 like its exp
-  const double e = FAST ? double(0.5f * expf(float(-l * (U * U))) * rsqrtf(float(PI * l)))
-                        : 0.5 * exp(-l * (U * U)) / sqrt(PI * l);
-  if (half & 1) {
-    m.MuL[0] = 0.5 * t_erfc<FAST>(-sl * U);
-    m.MuL[1] = U * m.MuL[0] + e;
-    for (int i = 2; i <= 6; ++i) m.MuL[i] = U * m.MuL[i - 1] + (i - 1) * hl * m.MuL[i - 2];
+// pdf_slope(prim, sw, inK) (src/Theory/theory_pdf.jl:11-49).  r0 = 1 / rho,
+// hl = 1 / (2 lambda), rk = 1 / (K + D), Kd = K + D.
+template <int NW>
+__device__ __forceinline__ void pdf_slope(const double* p, const double* s, double r0, double hl, double rk,
+                                          double Kd, double* sl) {
+  constexpr int E = NW - 1;  // energy slot
+  const double l = p[E], U = p[1], V = NW == 4 ? p[2] : 0.0, sv = NW == 4 ? s[2] : 0.0;
+  const double q2 = NW == 4 ? fma(U, U, V * V) : U * U, c = Kd * hl;
+  double t = fma(s[0], q2 - c, 2.0 * s[E]);
+  t = fma(-2.0 * U, s[1], t);
+  if (NW == 4) t = fma(-2.0 * V, sv, t);
+  const double tl = 2.0 * l * r0;
+  const double se = (2.0 * l * rk) * tl * t;
+  const double s1 = fma(tl, fma(-U, s[0], s[1]), -U * se);
+  double z = fma(s[0], r0, -U * s1);
+  if (NW == 4) {
+    const double s2 = fma(tl, fma(-V, s[0], sv), -V * se);
+    z = fma(-V, s2, z);
+    sl[2] = s2;
   }
-  if (half & 2) {
-    m.MuR[0] = 0.5 * t_erfc<FAST>(sl * U);
-    m.MuR[1] = U * m.MuR[0] - e;
-    for (int i = 2; i <= 6; ++i) m.MuR[i] = U * m.MuR[i - 1] + (i - 1) * hl * m.MuR[i - 2];
-  }
-  if (half == 3)
-    for (int i = 0; i <= 6; ++i) m.Mu[i] = m.MuL[i] + m.MuR[i];
-  double V = nw == 4 ? p[2] : 0.0;
-  m.Mv[0] = 1.0;
-  m.Mv[1] = V;
-  for (int i = 2; i <= 6; ++i) m.Mv[i] = V * m.Mv[i - 1] + (i - 1) * hl * m.Mv[i - 2];
-  m.Mxi[0] = 1.0;
-  m.Mxi[1] = inK * hl;
-  m.Mxi[2] = (inK * inK + 2.0 * inK) * (hl * hl);
-}
-
-// moments_conserve(Mu[, Mv], Mxi, alpha[, beta], delta) for the internal-energy
-// forms (src/Theory/theory_moments.jl:98-145).  In 1D Mv is ignored.
-__device__ inline void moments_conserve(const double* Mu, const double* Mv, const double* Mxi,
-                                        int nw, int a, int bb, int d, double* uv) {
-  if (nw == 3) {
-    uv[0] = Mu[a] * Mxi[d / 2];
-    uv[1] = Mu[a + 1] * Mxi[d / 2];
-    uv[2] = 0.5 * (Mu[a + 2] * Mxi[d / 2] + Mu[a] * Mxi[(d + 2) / 2]);
-    uv[3] = 0.0;
-  } else {
-    uv[0] = Mu[a] * Mv[bb] * Mxi[d / 2];
-    uv[1] = Mu[a + 1] * Mv[bb] * Mxi[d / 2];
-    uv[2] = Mu[a] * Mv[bb + 1] * Mxi[d / 2];
-    uv[3] = 0.5 * (Mu[a + 2] * Mv[bb] * Mxi[d / 2] + Mu[a] * Mv[bb + 2] * Mxi[d / 2] +
-                   Mu[a] * Mv[bb] * Mxi[(d + 2) / 2]);
-  }
-}
-
-// moments_conserve_slope (src/Theory/theory_moments.jl:335-369)
-__device__ inline void moments_conserve_slope(const double* a, const double* Mu,
-                                              const double* Mv, const double* Mxi, int nw,
-                                              int al, double* out) {
-  double t0[4], t1[4], t2[4], t3[4], t4[4], t5[4];
-  if (nw == 3) {
-    moments_conserve(Mu, Mv, Mxi, 3, al, 0, 0, t0);
-    moments_conserve(Mu, Mv, Mxi, 3, al + 1, 0, 0, t1);
-    moments_conserve(Mu, Mv, Mxi, 3, al + 2, 0, 0, t2);
-    moments_conserve(Mu, Mv, Mxi, 3, al, 0, 2, t3);
-    for (int k = 0; k < 3; ++k)
-      out[k] = a[0] * t0[k] + a[1] * t1[k] + 0.5 * a[2] * t2[k] + 0.5 * a[2] * t3[k];
-    out[3] = 0.0;
-  } else {
-    moments_conserve(Mu, Mv, Mxi, 4, al, 0, 0, t0);
-    moments_conserve(Mu, Mv, Mxi, 4, al + 1, 0, 0, t1);
-    moments_conserve(Mu, Mv, Mxi, 4, al, 1, 0, t2);
-    moments_conserve(Mu, Mv, Mxi, 4, al + 2, 0, 0, t3);
-    moments_conserve(Mu, Mv, Mxi, 4, al, 2, 0, t4);
-    moments_conserve(Mu, Mv, Mxi, 4, al, 0, 2, t5);
-    for (int k = 0; k < 4; ++k)
-      out[k] = a[0] * t0[k] + a[1] * t1[k] + a[2] * t2[k] + 0.5 * a[3] * t3[k] +
-               0.5 * a[3] * t4[k] + 0.5 * a[3] * t5[k];
-  }
-}
-
-// pdf_slope(prim, sw, inK) (src/Theory/theory_pdf.jl:11-49); FAST forms the
-// three reciprocals once (see conserve_prim)
-template <bool FAST = false>
-__device__ inline void pdf_slope(const double* p, const double* s, int nw, double inK,
-                                 double* sl) {
-  if (FAST) {
-    const int e = nw - 1;  // energy slot
-    const double r0 = 1.0 / p[0], rl = 1.0 / p[e], rk = 1.0 / (inK + double(nw - 2));
-    const double U = p[1], V = nw == 4 ? p[2] : 0.0, sv = nw == 4 ? s[2] : 0.0;
-    const double q2 = U * U + V * V, c = 0.5 * (inK + double(nw - 2)) * rl;
-    const double se = 4.0 * (p[e] * p[e]) * rk * r0 *
-                      (2.0 * s[e] - 2.0 * U * s[1] - 2.0 * V * sv + s[0] * (q2 - c));
-    const double tl = 2.0 * p[e] * r0;
-    const double s1 = tl * (s[1] - U * s[0]) - U * se;
-    const double s2 = tl * (sv - V * s[0]) - V * se;
-    sl[0] = s[0] * r0 - U * s1 - V * s2 - 0.5 * (q2 + c) * se;
-    sl[1] = s1;
-    if (nw == 4) {
-      sl[2] = s2;
-      sl[3] = se;
-    } else {
-      sl[2] = se;
-      sl[3] = 0.0;
-    }
-    return;
-  }
-  if (nw == 3) {
-    sl[2] = 4.0 * (p[2] * p[2]) / (inK + 1.0) / p[0] *
-            (2.0 * s[2] - 2.0 * p[1] * s[1] + s[0] * ((p[1] * p[1]) - 0.5 * (inK + 1.0) / p[2]));
-    sl[1] = 2.0 * p[2] / p[0] * (s[1] - p[1] * s[0]) - p[1] * sl[2];
-    sl[0] = s[0] / p[0] - p[1] * sl[1] - 0.5 * ((p[1] * p[1]) + 0.5 * (inK + 1.0) / p[2]) * sl[2];
-    sl[3] = 0.0;
-  } else {
-    sl[3] = 4.0 * (p[3] * p[3]) / (inK + 2.0) / p[0] *
-            (2.0 * s[3] - 2.0 * p[1] * s[1] - 2.0 * p[2] * s[2] +
-             s[0] * ((p[1] * p[1]) + (p[2] * p[2]) - 0.5 * (inK + 2.0) / p[3]));
-    sl[2] = 2.0 * p[3] / p[0] * (s[2] - p[2] * s[0]) - p[2] * sl[3];
-    sl[1] = 2.0 * p[3] / p[0] * (s[1] - p[1] * s[0]) - p[1] * sl[3];
-    sl[0] = s[0] / p[0] - p[1] * sl[1] - p[2] * sl[2] -
-            0.5 * ((p[1] * p[1]) + (p[2] * p[2]) + 0.5 * (inK + 2.0) / p[3]) * sl[3];
-  }
+  sl[0] = fma(-0.5 * (q2 + c), se, z);
+  sl[1] = s1;
+  sl[E] = se;
+  if (NW == 3) sl[3] = 0.0;
 }
 
 // ------------------------------------------- compensated FP32 accumulation
@@ -391,8 +355,37 @@ __device__ __forceinline__ DF df_shfl_xor(DF a, int m) {
 __device__ __forceinline__ double df_warp_sum(DF a) {
 #pragma unroll
   for (int m = 16; m >= 1; m >>= 1) a = df_merge(a, df_shfl_xor(a, m));
-  return (double)a.hi + (double)a.lo;
+  return f64_of(a.hi) + f64_of(a.lo);
 }
+
+// Sums of N values over the warp (N a power of two, at most 32): a
+// reduce-scatter whose first log2 N levels halve the number of values a lane
+// carries, then plain levels: N - 1 + 5 - log2 N additions instead of 5 N.
+// Lane l returns the total of value l >> (5 - log2 N), in a fixed order.
+__device__ __forceinline__ double join(double a, double b) { return a + b; }
+__device__ __forceinline__ DF join(DF a, DF b) { return df_merge(a, b); }
+__device__ __forceinline__ double shfl_xor_of(double a, int m) { return __shfl_xor_sync(0xffffffffu, a, m); }
+__device__ __forceinline__ DF shfl_xor_of(DF a, int m) { return df_shfl_xor(a, m); }
+template <int N, typename T>
+__device__ __forceinline__ T warp_sums(T* x, int lane) {
+#pragma unroll
+  for (int m = 16, n = N; m >= 1; m >>= 1) {
+    if (n > 1) {
+      n >>= 1;
+      const bool up = lane & m;  // the upper lanes keep the upper half
+#pragma unroll
+      for (int k = 0; k < n; ++k) {
+        const T keep = up ? x[n + k] : x[k], give = up ? x[k] : x[n + k];
+        x[k] = join(keep, shfl_xor_of(give, m));
+      }
+    } else {
+      x[0] = join(x[0], shfl_xor_of(x[0], m));
+    }
+  }
+  return x[0];
+}
+__device__ __forceinline__ double f64_total(double x) { return x; }
+__device__ __forceinline__ double f64_total(DF x) { return f64_of(x.hi) + f64_of(x.lo); }
 
 __device__ __forceinline__ double warp_sum(double x) {
 #pragma unroll
@@ -419,8 +412,7 @@ struct Acc<float> {
   __device__ __forceinline__ double total() { return df_warp_sum(s); }
 };
 
-// exp of a Maxwellian exponent: accurate FP64 exp on the FP64 path, ex2.approx
-// with a pre-scaled argument on the FP32 path.
+// exp of a Maxwellian exponent
 __device__ __forceinline__ double mexp(double x) { return exp(x); }
 __device__ __forceinline__ float mexp(float x) { return exp2f(x * float(LOG2E)); }
 

@@ -97,43 +97,22 @@ struct FP {
   R aL[4], aR[4], aT[4];
 };
 template <typename R>
-__device__ __forceinline__ FP<R> load_fp(const DevState& s, int f);
-template <>
-__device__ __forceinline__ FP<double> load_fp<double>(const DevState& s, int f) {
+__device__ __forceinline__ FP<R> load_fp(const DevState& s, int f) {
   const FaceParam& p = s.fp[f];
-  FP<double> r;
-  double lam = p.prim[3];
-  r.rho_n = s.g.D == 1 ? p.prim[0] * sqrt(lam / PI) : p.prim[0] * (lam / PI);
-  r.U = p.prim[1];
-  r.V = p.prim[2];
-  r.lam = lam;
-  r.cB = s.g.Kb / (2.0 * lam);
-  r.Mxi2 = p.Mxi2;
-  r.len = p.len;
-  for (int k = 0; k < 5; ++k) r.Mt[k] = p.Mt[k];
+  FP<R> r;
+  const double lam = p.prim[3] > 0 ? p.prim[3] : 1.0;  // KFVS has no interface state
+  r.rho_n = R(s.g.D == 1 ? p.prim[0] * sqrt64(lam * (1.0 / PI)) : p.prim[0] * (lam * (1.0 / PI)));
+  r.U = R(p.prim[1]);
+  r.V = R(p.prim[2]);
+  r.lam = R(p.prim[3]);
+  r.cB = R(s.g.Kb * (0.5 * rcp64(lam)));
+  r.Mxi2 = R(p.Mxi2);
+  r.len = R(p.len);
+  for (int k = 0; k < 5; ++k) r.Mt[k] = R(p.Mt[k]);
   for (int k = 0; k < 4; ++k) {
-    r.aL[k] = p.aL[k];
-    r.aR[k] = p.aR[k];
-    r.aT[k] = p.aT[k];
-  }
-  return r;
-}
-template <>
-__device__ __forceinline__ FP<float> load_fp<float>(const DevState& s, int f) {
-  const FaceParamF& p = s.fpf[f];
-  FP<float> r;
-  r.rho_n = p.rho_n;
-  r.U = p.U;
-  r.V = p.V;
-  r.lam = p.lam;
-  r.cB = p.cB;
-  r.Mxi2 = p.Mxi2;
-  r.len = p.len;
-  for (int k = 0; k < 5; ++k) r.Mt[k] = p.Mt[k];
-  for (int k = 0; k < 4; ++k) {
-    r.aL[k] = p.aL[k];
-    r.aR[k] = p.aR[k];
-    r.aT[k] = p.aT[k];
+    r.aL[k] = R(p.aL[k]);
+    r.aR[k] = R(p.aR[k]);
+    r.aT[k] = R(p.aT[k]);
   }
   return r;
 }
@@ -202,36 +181,5 @@ __device__ __forceinline__ void face_flux(const FP<R>& P, R dt, R un, R ut, bool
     }
   }
 }
-
-template <typename R>
-struct CP {
-  R rho_n, U, V, lam, cB, dtau, inv, o_rho_n, oU, oV, olam, ocB, s0, s1;
-  int upd, coll;
-};
-template <typename R>
-__device__ __forceinline__ CP<R> load_cp(const DevState& s, int c);
-template <>
-__device__ __forceinline__ CP<double> load_cp<double>(const DevState& s, int c) {
-  const CellParam& p = s.cp[c];
-  CP<double> r;
-  r.rho_n = p.rho_n; r.U = p.U; r.V = p.V; r.lam = p.lam; r.cB = p.cB;
-  r.dtau = p.dtau; r.inv = p.inv;
-  r.o_rho_n = p.o_rho_n; r.oU = p.oU; r.oV = p.oV; r.olam = p.olam; r.ocB = p.ocB;
-  r.s0 = p.sfac * p.q0; r.s1 = p.sfac * p.q1;
-  r.upd = p.upd; r.coll = p.coll;
-  return r;
-}
-template <>
-__device__ __forceinline__ CP<float> load_cp<float>(const DevState& s, int c) {
-  const CellParamF& p = s.cpf[c];
-  CP<float> r;
-  r.rho_n = p.rho_n; r.U = p.U; r.V = p.V; r.lam = p.lam; r.cB = p.cB;
-  r.dtau = p.dtau; r.inv = p.inv;
-  r.o_rho_n = p.o_rho_n; r.oU = p.oU; r.oV = p.oV; r.olam = p.olam; r.ocB = p.ocB;
-  r.s0 = p.sf0; r.s1 = p.sf1;
-  r.upd = p.upd; r.coll = p.coll;
-  return r;
-}
-
 
 }  // namespace kb

@@ -66,7 +66,8 @@ void launch_mom(const DevState& ls, int blocks, cudaStream_t st) {
   });
   CUtensorMap unused;  // the grouped kernel reads the members' maps from the table
   std::memset(&unused, 0, sizeof(unused));
-  kern<<<(unsigned)blocks, kb::MOM_THREADS, SL::BYTES, st>>>(unused, unused, ls);
+  void* args[] = {(void*)&unused, (void*)&unused, (void*)&ls};
+  kb::launch_after((const void*)kern, dim3((unsigned)blocks), dim3(kb::MOM_THREADS), SL::BYTES, st, args);
 }
 
 void launch_march(const DevState& ls, int blocks, cudaStream_t st) {
@@ -82,7 +83,9 @@ void launch_march(const DevState& ls, int blocks, cudaStream_t st) {
   });
   CUtensorMap unused;
   std::memset(&unused, 0, sizeof(unused));
-  kern<<<(unsigned)blocks, kb::M3_BS, L::BYTES, st>>>(unused, unused, ls, G_RY);
+  int ry = G_RY;
+  void* args[] = {(void*)&unused, (void*)&unused, (void*)&ls, (void*)&ry};
+  kb::launch_after((const void*)kern, dim3((unsigned)blocks), dim3(kb::M3_BS), L::BYTES, st, args);
 }
 
 }  // namespace
@@ -282,16 +285,17 @@ int kb_group_step_async(kb_group_t* G, int32_t nsteps) {
   int64_t nl = 0;
   for (int k = 0; k < nsteps; ++k) {
     const DevState& ls = G->ls[(G->parity + k) & 1];
-    kb::group_small(kb::GK_WSLOPE, ls, G->flux, G->blocks[kb::GK_WSLOPE], G->stream);
-    kb::group_small(kb::GK_FACE, ls, G->flux, G->blocks[kb::GK_FACE], G->stream);
+    kb::group_small(kb::GK_WSLOPE, ls, G->flux, G->blocks[kb::GK_WSLOPE], false, G->stream);
+    kb::group_small(kb::GK_FACE, ls, G->flux, G->blocks[kb::GK_FACE], false, G->stream);
     if (shak) launch_mom<true, 0>(ls, G->blocks[kb::GK_MOMX], G->stream);
     else launch_mom<false, 0>(ls, G->blocks[kb::GK_MOMX], G->stream);
     launch_mom<false, 1>(ls, G->blocks[kb::GK_MOMY], G->stream);
-    kb::group_small(kb::GK_WALL, ls, G->flux, G->blocks[kb::GK_WALL], G->stream);
-    kb::group_small(kb::GK_CELL, ls, G->flux, G->blocks[kb::GK_CELL], G->stream);
+    kb::group_small(kb::GK_WALL, ls, G->flux, G->blocks[kb::GK_WALL], false, G->stream);
+    const bool last = k == nsteps - 1;  // the chunk reports the last step's residual
+    kb::group_small(kb::GK_CELL, ls, G->flux, G->blocks[kb::GK_CELL], last, G->stream);
     launch_march(ls, G->blocks[kb::GK_MARCH], G->stream);
-    kb::group_small(kb::GK_RES, ls, G->flux, G->blocks[kb::GK_RES], G->stream);
-    nl += 6 + (G->blocks[kb::GK_WSLOPE] > 0) + (G->blocks[kb::GK_WALL] > 0);
+    if (last) kb::group_small(kb::GK_RES, ls, G->flux, G->blocks[kb::GK_RES], true, G->stream);
+    nl += 5 + last + (G->blocks[kb::GK_WSLOPE] > 0) + (G->blocks[kb::GK_WALL] > 0);
   }
   // the members' current buffers moved with the steps
   G->parity = (G->parity + nsteps) & 1;

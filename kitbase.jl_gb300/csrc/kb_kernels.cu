@@ -12,11 +12,13 @@
 #include <cstdint>
 #include <mutex>
 #include <set>
+#include <tuple>
 #include <utility>
 #include <stdio.h>
 
 #include "kb_kernels.cuh"
 #include "kb_flux.cuh"
+#include "kb_tma.cuh"
 
 namespace kb {
 
@@ -43,10 +45,10 @@ void face_kinds_host(const Geo& g, signed char* kind) {
 
 // reconstruct! for w (src/Solver/solver_reconstruction.jl:111-122 1D, :496-537 2D):
 // one thread per (physical cell, direction).
-// FAST (the FP32 split form): one reciprocal of the cell size per thread in
-// place of two FP64 divisions per component.
-template <bool FAST, bool GRP = false>
+template <bool GRP = false>
 __global__ void k_wslope(DevState sp) {
+  pdl_wait();
+  pdl_next();
   int lb;
   const int gr = group_member<GRP, GK_WSLOPE>(sp, lb);
   KB_GROUP_STATE(GRP, sp, gr);
@@ -59,91 +61,107 @@ __global__ void k_wslope(DevState sp) {
   int c = cell_index(g, i, j);
   int rule = slope_rule(g, d, d == 0 ? i : j);
   int step = d == 0 ? 1 : g.nxt;
-  double dd = d == 0 ? g.dx : g.dy;  // 0.5 * (dx[i-1] + dx[i]) on a uniform mesh
+  // dx = 0.5 * (dx[i-1] + dx[i]) on a uniform mesh
   double* out = s.sw + ((long)c * 2 + d) * 4;
-  const double rd = FAST ? 1.0 / dd : 0.0;
+  const double rd = d == 0 ? g.rdx : g.rdy;
+  const double eps = 1.e-7 * (d == 0 ? g.dx : g.dy);
   for (int k = 0; k < g.NW; ++k) {
     double q0 = s.w[(long)c * 4 + k];
     double qm = (rule == 1 || rule == 3) ? s.w[(long)(c - step) * 4 + k] : 0.0;
     double qp = (rule == 1 || rule == 2) ? s.w[(long)(c + step) * 4 + k] : 0.0;
-    if (FAST) {
-      const double a = (q0 - qm) * rd, b = (qp - q0) * rd;
-      out[k] = rule == 1 ? vanleer(a, b) : (rule == 2 ? b : (rule == 3 ? a : 0.0));
-    } else {
-      out[k] = slope_of<double>(rule, qm, q0, qp, dd);
-    }
+    out[k] = rd * (rule == 1 ? vl64(qm, q0, qp, eps) : (rule == 2 ? qp - q0 : (rule == 3 ? q0 - qm : 0.0)));
   }
 }
 
 // ------------------------------------------------------- face parameters
 
 // log2-form exponent of rho (lam/pi)^(D/2) exp(-lam ((un-U)^2 + (ut-V)^2)) as
-// E.x + E.y un + E.z ut + E.w c2.
-// FAST (the FP32 split form): log2 of the density factor in FP32.
-template <bool FAST = false>
-__device__ inline float4 maxwell_exp2(double rho_n, double U, double V, double lam) {
+// E.x + E.y un + E.z ut + E.w c2; the log2 of the density factor in FP32.
+__device__ __forceinline__ float4 maxwell_exp2(double rho_n, double U, double V, double lam) {
   float4 E;
-  const double l2r = rho_n > 0.0 ? (FAST ? double(log2f(float(rho_n))) : log2(rho_n)) : 0.0;
-  E.x = rho_n > 0.0 ? float(l2r - lam * (U * U + V * V) * LOG2E) : -200.f;
-  E.y = float(2.0 * lam * U * LOG2E);
-  E.z = float(2.0 * lam * V * LOG2E);
-  E.w = float(-lam * LOG2E);
+  const float rf = f32_of(rho_n);
+  const double ll = lam * LOG2E, lU = ll * U, lV = ll * V;
+  E.x = rf > 0.f ? f32_of(f64_of(log2f(rf)) - fma(lU, U, lV * V)) : -200.f;
+  E.y = f32_of(lU + lU);
+  E.z = f32_of(lV + lV);
+  E.w = f32_of(-ll);
   return E;
 }
 
-// FP32 monomial coefficients of the interface flux (see FaceCoef32).
-template <bool FAST = false>
-__device__ __forceinline__ FaceCoef32 face_coef32(const Geo& g, const FaceParam& P, int flux, double dd) {
-  FaceCoef32 c;
-  float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-  c.E = c.T = c.G = c.Cp = c.Dp = c.Cm = c.Dm = z;
-  double len = P.len;
-  c.T.x = float(P.tr[0]);
-  c.T.y = float(P.tr[1] / dd);
-  if (flux == FLUX_KFVS) return c;
-  double lam = P.prim[3], rho = P.prim[0];
-  double rho_n = g.D == 1 ? rho * t_sqrt<FAST>(lam / PI) : rho * (lam / PI);
-  c.E = maxwell_exp2<FAST>(rho_n, P.prim[1], P.prim[2], lam);
-  double cB = g.Kb / (2.0 * lam);
-  const double* Mt = P.Mt;
-  if (flux == FLUX_KCU) {
-    c.T.z = float(Mt[0] * len);
-    c.T.w = float(Mt[0] * cB * len);
-    return c;
+// One coefficient in the block's precision.
+__device__ __forceinline__ void put(float& o, double x) { o = f32_of(x); }
+__device__ __forceinline__ void put(double& o, double x) { o = x; }
+__device__ __forceinline__ void put_maxwell(float4& E, double rho_n, double U, double V, double lam) {
+  E = maxwell_exp2(rho_n, U, V, lam);
+}
+__device__ __forceinline__ void put_maxwell(Quad64& E, double rho_n, double U, double V, double lam) {
+  E.x = rho_n;
+  E.y = U;
+  E.z = V;
+  E.w = EXP64_LOG2E * lam;
+}
+
+// Monomial coefficients of the interface flux (see FaceCoef32, FaceCoef64); rdd
+// = 1 / cell size along the normal, hl = 1 / (2 lambda).
+template <int D, int FLUX, typename FC>
+__device__ __forceinline__ void face_coef(FC& c, const Geo& g, const FaceParam& P, double rdd, double hl) {
+  constexpr bool FAST = sizeof(c.E.x) == 4;
+  c = FC{};
+  put(c.T.x, P.tr[0]);
+  put(c.T.y, P.tr[1] * rdd);
+  if (FLUX == FLUX_KFVS) return;
+  const double lam = P.prim[3], rho = P.prim[0], len = P.len;
+  const double rho_n = D == 1 ? rho * t_sqrt<FAST>(lam * (1.0 / PI)) : rho * (lam * (1.0 / PI));
+  put_maxwell(c.E, rho_n, P.prim[1], P.prim[2], lam);
+  const double cB = g.Kb * hl, M0 = P.Mt[0] * len;
+  if (FLUX == FLUX_KCU) {
+    put(c.T.z, M0);
+    put(c.T.w, M0 * cB);
+    return;
   }
-  // the energy slope sits at index D + 1; selected between constant indices
-  // (a run-time index would place the slope arrays in local memory)
   const double* t = P.aT;
-  const double tt = g.D == 2 ? t[2] : 0.0, te = g.D == 2 ? t[3] : t[2], Mxi2 = P.Mxi2;
-  c.T.z = float((Mt[0] + Mt[2] * (t[0] + 0.5 * te * cB)) * len);
-  c.T.w = float((Mt[0] * cB + Mt[2] * (cB * t[0] + 0.5 * te * Mxi2)) * len);
-  c.G.x = float(Mt[2] * tt * len);
-  c.G.y = float(0.5 * Mt[2] * te * len);
-  c.G.z = float(Mt[2] * cB * tt * len);
-  c.G.w = float(0.5 * Mt[2] * cB * te * len);
+  const double M1 = P.Mt[1] * len, M2 = P.Mt[2] * len, M1B = M1 * cB, M2B = M2 * cB, X2 = P.Mxi2;
+  const double te = 0.5 * t[D + 1];
+  put(c.T.z, fma(M2, fma(te, cB, t[0]), M0));
+  put(c.T.w, fma(M0, cB, fma(M2B, t[0], M2 * te * X2)));
+  if (D == 2) {
+    put(c.G.x, M2 * t[2]);
+    put(c.G.z, M2B * t[2]);
+  }
+  put(c.G.y, M2 * te);
+  put(c.G.w, M2B * te);
+  const double M2t = M2 * t[1], M2Bt = M2B * t[1];
   // one upwind side's slope terms (a = aL for un >= 0, aR otherwise)
-  auto side = [&](const double (&a)[4], float4& C, float4& Dd) {
-    const double at = g.D == 2 ? a[2] : 0.0, ae = g.D == 2 ? a[3] : a[2];
-    C.x = float((Mt[1] * (a[0] + 0.5 * ae * cB) + Mt[2] * t[1]) * len);
-    C.y = float(Mt[1] * a[1] * len);
-    C.z = float(Mt[1] * at * len);
-    C.w = float(0.5 * Mt[1] * ae * len);
-    Dd.x = float((Mt[1] * (cB * a[0] + 0.5 * ae * Mxi2) + Mt[2] * cB * t[1]) * len);
-    Dd.y = float(Mt[1] * cB * a[1] * len);
-    Dd.z = float(Mt[1] * cB * at * len);
-    Dd.w = float(0.5 * Mt[1] * cB * ae * len);
+  auto side = [&](const double (&a)[4], auto& C, auto& Dd) {
+    const double ae = 0.5 * a[D + 1];
+    put(C.x, fma(M1, fma(ae, cB, a[0]), M2t));
+    put(C.y, M1 * a[1]);
+    if (D == 2) put(C.z, M1 * a[2]);
+    put(C.w, M1 * ae);
+    put(Dd.x, fma(M1B, a[0], fma(M1 * ae, X2, M2Bt)));
+    put(Dd.y, M1B * a[1]);
+    if (D == 2) put(Dd.z, M1B * a[2]);
+    put(Dd.w, M1B * ae);
   };
   side(P.aL, c.Cp, c.Dp);
   side(P.aR, c.Cm, c.Dm);
-  return c;
 }
 
 // Interface equilibrium from the two half Maxwellians (flux_kcu.jl:480-495,
 // flux_ugks.jl:47-56), then the KCU / UGKS time integrals, UGKS slopes and
 // the analytic part of fw.  One thread per face.
-// FAST: the FP32 split form (transcendentals in FP32, see t_exp).
+// FAST: the FP32 split form (transcendentals in FP32, see t_exp_neg).
+// Bound by the FP64 pipe: about 320 (UGKS) or 110 (KCU) FP64 instructions per
+// face where moment by moment evaluation with divisions took 800 and 300.
 template <int D, int FLUX, bool FAST, bool GRP = false>
 __global__ void k_face_param(DevState sp, double dt_arg) {
+  __shared__ double tab[FAST || FLUX == FLUX_KFVS ? 1 : EXP64_N];
+  if (!FAST && FLUX != FLUX_KFVS) {
+    exp64_load(tab, threadIdx.x, blockDim.x);
+    __syncthreads();
+  }
+  pdl_wait();
+  pdl_next();
   int lb;
   const int gr = group_member<GRP, GK_FACE>(sp, lb);
   KB_GROUP_STATE(GRP, sp, gr);
@@ -153,9 +171,9 @@ __global__ void k_face_param(DevState sp, double dt_arg) {
   if (f >= s.nface_x + s.nface_y) return;
   if (s.kind[f] != 1) return;
   FaceGeo r = face_geo(g, f);
-  constexpr int NW = D + 2;
-  double dxh = 0.5 * (r.d == 0 ? g.dx : g.dy);
-  double len = face_len(g, r.d, r.fi, r.fj);
+  constexpr int NW = D + 2, E = D + 1;
+  const double dxh = 0.5 * (r.d == 0 ? g.dx : g.dy), rdd = r.d == 0 ? g.rdx : g.rdy;
+  const double len = D == 1 ? 1.0 : face_len(g, r.d, r.fi, r.fj);
   FaceParam P;
   for (int k = 0; k < 4; ++k) {
     P.prim[k] = 0;
@@ -165,6 +183,7 @@ __global__ void k_face_param(DevState sp, double dt_arg) {
   P.len = len;
   P.Mxi2 = 0;
   P.tr[0] = P.tr[1] = 0;
+  double hl = 0.0;
   if (FLUX == FLUX_KFVS) {
     P.mult = 1.0;
     P.tr[0] = dt * len;
@@ -175,8 +194,8 @@ __global__ void k_face_param(DevState sp, double dt_arg) {
     const double* sl = s.sw + ((long)r.cL * 2 + r.d) * 4;
     const double* sr = s.sw + ((long)r.cR * 2 + r.d) * 4;
     for (int k = 0; k < 4; ++k) {
-      wl[k] = k < NW ? s.w[(long)r.cL * 4 + k] + dxh * sl[k] : 0.0;
-      wr[k] = k < NW ? s.w[(long)r.cR * 4 + k] - dxh * sr[k] : 0.0;
+      wl[k] = k < NW ? fma(dxh, sl[k], s.w[(long)r.cL * 4 + k]) : 0.0;
+      wr[k] = k < NW ? fma(-dxh, sr[k], s.w[(long)r.cR * 4 + k]) : 0.0;
     }
     if (NW == 4 && r.d == 1) {  // local_frame with n = (0, 1)
       wL[0] = wl[0]; wL[1] = wl[2]; wL[2] = -wl[1]; wL[3] = wl[3];
@@ -184,96 +203,102 @@ __global__ void k_face_param(DevState sp, double dt_arg) {
     } else {
       for (int k = 0; k < 4; ++k) { wL[k] = wl[k]; wR[k] = wr[k]; }
     }
-    double pL[4], pR[4], wi[4], p[4], M1[4], M2[4];
-    conserve_prim<FAST>(wL, NW, g.gamma, pL);
-    conserve_prim<FAST>(wR, NW, g.gamma, pR);
-    GM m;
-    gauss_moments<FAST>(pL, NW, g.K, m, 1);
-    moments_conserve(m.MuL, m.Mv, m.Mxi, NW, 0, 0, 0, M1);
-    gauss_moments<FAST>(pR, NW, g.K, m, 2);
-    moments_conserve(m.MuR, m.Mv, m.Mxi, NW, 0, 0, 0, M2);
-    for (int k = 0; k < 4; ++k) wi[k] = k < NW ? pL[0] * M1[k] + pR[0] * M2[k] : 0.0;
-    conserve_prim<FAST>(wi, NW, g.gamma, p);
-    double lam = p[NW - 1];
+    double wi[4] = {0.0, 0.0, 0.0, 0.0}, p[4], pj = 0.0, ps = 0.0;  // pj, ps: pressure jump and sum (KCU)
+    // the half of one side's Maxwellian that crosses the face (its conserved moments)
+    auto half = [&](const double* w, bool left) {
+      double q[4], L0, L1, R0, R1;
+      conserve_prim<NW>(w, g.hg, q);
+      const double h = 0.5 * rcp64(q[E]);
+      half_range<FAST>(q[E], q[1], h, tab, L0, L1, R0, R1);
+      const double m0 = q[0] * (left ? L0 : R0), m1 = q[0] * (left ? L1 : R1);
+      const double V = NW == 4 ? q[2] : 0.0;
+      wi[0] += m0;
+      wi[1] += m1;
+      if (NW == 4) wi[2] = fma(m0, V, wi[2]);
+      // <u^2> + <v^2> + <xi^2>
+      const double t = NW == 4 ? fma(V, V, h + g.K * h) : g.K * h;
+      wi[E] = fma(0.5, fma(q[1], m1, fma(h, m0, m0 * t)), wi[E]);
+      if (FLUX == FLUX_KCU) {
+        const double pr = q[0] * h;  // pressure: rho / (2 lambda)
+        pj = left ? pr : pj - pr;
+        ps += pr;
+      }
+    };
+    half(wL, true);
+    half(wR, false);
+    conserve_prim<NW>(wi, g.hg, p);
+    const double lam = p[E], U = p[1], V = NW == 4 ? p[2] : 0.0;
+    hl = 0.5 * rcp64(lam);
     P.prim[0] = p[0];
-    P.prim[1] = p[1];
-    P.prim[2] = NW == 4 ? p[2] : 0.0;
+    P.prim[1] = U;
+    P.prim[2] = V;
     P.prim[3] = lam;
-    double tau = vhs_time<FAST>(p[0], lam, g.mu_ref, g.omega);
-    GM mi;
+    const double itau = vhs_rate<FAST>(g, p[0], lam, tab);
+    const double x1 = g.K * hl, x2 = fma(2.0 * hl, x1, x1 * x1);  // <xi^2>, <xi^4>
+    const double v2 = NW == 4 ? fma(V, V, hl) : 0.0;
+    double Mu[7];
+    Mu[0] = 1.0;
+    Mu[1] = U;
+    Mu[2] = fma(U, U, hl);
+    Mu[3] = fma(U, Mu[2], 2.0 * hl * U);
+    // u times the conserved moments of the interface Maxwellian
+    double Muv[4] = {Mu[1], Mu[2], 0.0, 0.0};
+    if (NW == 4) Muv[2] = Mu[1] * V;
+    Muv[E] = 0.5 * fma(Mu[1], v2 + x1, Mu[3]);
+    P.mult = len;
     if (FLUX == FLUX_KCU) {
-      tau += fabs(pL[0] / pL[NW - 1] - pR[0] / pR[NW - 1]) /
-             (pL[0] / pL[NW - 1] + pR[0] / pR[NW - 1]) * dt * 2.0;
-      P.Mt[1] = tau * (1.0 - t_exp<FAST>(-dt / tau));
+      const double tau = rcp64(itau) + fabs(pj) * rcp64(ps) * (2.0 * dt);
+      P.Mt[1] = tau * (1.0 - t_exp_neg<FAST>(dt * rcp64(tau), tab));
       P.Mt[0] = dt - P.Mt[1];
-      gauss_moments<FAST>(p, NW, g.K, mi);
-      double Muv[4];
-      moments_conserve(mi.Mu, mi.Mv, mi.Mxi, NW, 1, 0, 0, Muv);
-      for (int k = 0; k < NW; ++k) P.fwa[k] = P.Mt[0] * p[0] * Muv[k] * len;
-      P.mult = len;
+      const double m = P.Mt[0] * p[0] * len;
+      for (int k = 0; k < NW; ++k) P.fwa[k] = m * Muv[k];
       P.tr[0] = P.Mt[1] * len;
     } else {
-      double dL[4], dR[4];
-      const double rdx = FAST ? 1.0 / dxh : 0.0;
-      for (int k = 0; k < 4; ++k) {
-        dL[k] = k < NW ? (FAST ? (wi[k] - wL[k]) * rdx : (wi[k] - wL[k]) / dxh) : 0.0;
-        dR[k] = k < NW ? (FAST ? (wR[k] - wi[k]) * rdx : (wR[k] - wi[k]) / dxh) : 0.0;
+      const double tau = rcp64(itau), rh = 2.0 * rdd, r0 = rcp64(p[0]), Kd = g.K + double(D), rk = g.rKD;
+      double dL[4] = {0.0, 0.0, 0.0, 0.0}, dR[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int k = 0; k < NW; ++k) {
+        dL[k] = (wi[k] - wL[k]) * rh;
+        dR[k] = (wR[k] - wi[k]) * rh;
       }
-      double aL[4], aR[4], aT[4];
-      pdf_slope<FAST>(p, dL, NW, g.K, aL);
-      pdf_slope<FAST>(p, dR, NW, g.K, aR);
-      gauss_moments<FAST>(p, NW, g.K, mi);
-      double MauL[4], MauR[4], MauT[4], Muv[4], tmp[4];
-      moments_conserve_slope(aL, mi.MuL, mi.Mv, mi.Mxi, NW, 1, MauL);
-      moments_conserve_slope(aR, mi.MuR, mi.Mv, mi.Mxi, NW, 1, MauR);
-      for (int k = 0; k < 4; ++k) tmp[k] = -p[0] * (MauL[k] + MauR[k]);
-      pdf_slope<FAST>(p, tmp, NW, g.K, aT);
-      double ex = t_exp<FAST>(-dt / tau);
-      double Mt[5];
-      Mt[3] = tau * (1.0 - ex);
-      Mt[4] = -tau * dt * ex + tau * Mt[3];
-      Mt[0] = dt - Mt[3];
-      Mt[1] = -tau * Mt[0] + Mt[4];
-      Mt[2] = (dt * dt) / 2.0 - tau * Mt[0];
-      moments_conserve(mi.Mu, mi.Mv, mi.Mxi, NW, 1, 0, 0, Muv);
-      moments_conserve_slope(aL, mi.MuL, mi.Mv, mi.Mxi, NW, 2, MauL);
-      moments_conserve_slope(aR, mi.MuR, mi.Mv, mi.Mxi, NW, 2, MauR);
-      moments_conserve_slope(aT, mi.Mu, mi.Mv, mi.Mxi, NW, 1, MauT);
-      for (int k = 0; k < NW; ++k)
-        P.fwa[k] = (Mt[0] * p[0] * Muv[k] + Mt[1] * p[0] * (MauL[k] + MauR[k]) +
-                    Mt[2] * p[0] * MauT[k]) * len;
-      for (int k = 0; k < 5; ++k) P.Mt[k] = Mt[k];
-      // slopes stored with the energy slope at index D+1 for both dimensions
-      for (int k = 0; k < 4; ++k) {
-        P.aL[k] = aL[k];
-        P.aR[k] = aR[k];
-        P.aT[k] = aT[k];
+      pdf_slope<NW>(p, dL, r0, hl, rk, Kd, P.aL);
+      pdf_slope<NW>(p, dR, r0, hl, rk, Kd, P.aR);
+      double ML[7], MR[7];
+      half_range<FAST>(lam, U, hl, tab, ML[0], ML[1], MR[0], MR[1]);
+      for (int i = 2; i <= 6; ++i) {
+        const double q = double(i - 1) * hl;
+        if (i > 3) Mu[i] = fma(U, Mu[i - 1], q * Mu[i - 2]);
+        ML[i] = fma(U, ML[i - 1], q * ML[i - 2]);
+        MR[i] = Mu[i] - ML[i];
       }
-      P.Mxi2 = mi.Mxi[2];
-      P.mult = len;
-      P.tr[0] = Mt[3] * len;
-      P.tr[1] = Mt[4] * len;
+      SlopeV<NW> sL, sR, sT;
+      sL.set(P.aL, V, hl, x1, x2);
+      sR.set(P.aR, V, hl, x1, x2);
+      double a[4], b[4], tmp[4] = {0.0, 0.0, 0.0, 0.0};
+      sL.get(ML + 1, a);
+      sR.get(MR + 1, b);
+      for (int k = 0; k < NW; ++k) tmp[k] = -p[0] * (a[k] + b[k]);
+      pdf_slope<NW>(p, tmp, r0, hl, rk, Kd, P.aT);
+      const double ex = t_exp_neg<FAST>(dt * itau, tab);
+      P.Mt[3] = tau * (1.0 - ex);
+      P.Mt[4] = fma(-tau * dt, ex, tau * P.Mt[3]);
+      P.Mt[0] = dt - P.Mt[3];
+      P.Mt[1] = fma(-tau, P.Mt[0], P.Mt[4]);
+      P.Mt[2] = fma(-tau, P.Mt[0], 0.5 * (dt * dt));
+      sT.set(P.aT, V, hl, x1, x2);
+      double c[4];
+      sL.get(ML + 2, a);
+      sR.get(MR + 2, b);
+      sT.get(Mu + 1, c);
+      const double m = p[0] * len, m0 = m * P.Mt[0], m1 = m * P.Mt[1], m2 = m * P.Mt[2];
+      for (int k = 0; k < NW; ++k) P.fwa[k] = fma(m0, Muv[k], fma(m1, a[k] + b[k], m2 * c[k]));
+      P.Mxi2 = x2;
+      P.tr[0] = P.Mt[3] * len;
+      P.tr[1] = P.Mt[4] * len;
     }
   }
   s.fp[f] = P;
-  s.fc[f] = face_coef32<FAST>(g, P, FLUX, r.d == 0 ? g.dx : g.dy);
-  FaceParamF F;
-  double lam = P.prim[3] > 0 ? P.prim[3] : 1.0;
-  F.rho_n = float(g.D == 1 ? P.prim[0] * sqrt(lam / PI) : P.prim[0] * (lam / PI));
-  F.U = float(P.prim[1]);
-  F.V = float(P.prim[2]);
-  F.lam = float(P.prim[3]);
-  F.cB = float(g.Kb / (2.0 * lam));
-  for (int k = 0; k < 5; ++k) F.Mt[k] = float(P.Mt[k]);
-  for (int k = 0; k < 4; ++k) {
-    F.aL[k] = float(P.aL[k]);
-    F.aR[k] = float(P.aR[k]);
-    F.aT[k] = float(P.aT[k]);
-  }
-  F.Mxi2 = float(P.Mxi2);
-  F.len = float(len);
-  F.pad[0] = F.pad[1] = 0.f;
-  s.fpf[f] = F;
+  if constexpr (FAST) face_coef<D, FLUX>(s.fc[f], g, P, rdd, hl);
+  else face_coef<D, FLUX>(s.fc64[f], g, P, rdd, hl);
 }
 
 // ------------------------------------------------------------ Maxwell walls
@@ -285,9 +310,19 @@ __global__ void k_face_param(DevState sp, double dt_arg) {
 // shared by all its warps, each warp sums its part, and thread 0 adds the
 // warps' sums in warp order (deterministic) and finishes the face.
 constexpr int WALL_T = 128;
+// exp(-lw e) from lw scaled to the base-two exponent of each form
+__device__ __forceinline__ float wall_exp(float l2, float e, const double*) { return exp2f(l2 * e); }
+__device__ __forceinline__ double wall_exp(double l2, double e, const double* tab) { return exp2_tab(l2, e, tab); }
 template <typename R, int D, bool GRP = false>
 __global__ void __launch_bounds__(WALL_T) k_wall(DevState sp, double dt_arg) {
   __shared__ double part[WALL_T / 32][8];
+  __shared__ double tab[sizeof(R) == 8 ? EXP64_N : 1];
+  if (sizeof(R) == 8) {
+    exp64_load(tab, threadIdx.x, WALL_T);
+    __syncthreads();
+  }
+  pdl_wait();
+  pdl_next();
   int lb;
   const int gr = group_member<GRP, GK_WALL>(sp, lb);
   KB_GROUP_STATE(GRP, sp, gr);
@@ -315,25 +350,26 @@ __global__ void __launch_bounds__(WALL_T) k_wall(DevState sp, double dt_arg) {
   const R* V = vtab<R>(s, 1);
   const R* W = vtab<R>(s, 2);
   long vs = g.vstride;
-  R Uw = R(bw[1]), Vw = R(bw[2]), Lw = R(lw);
+  R Uw = R(bw[1]), Vw = R(bw[2]);
   // One pass: the outgoing half from the interior cell's h, b; the incoming
   // half as moments of the unit-density wall Maxwellian, scaled by the wall
   // density afterwards in FP64.  The mass flux S0 = SF + rho_n * I0 then
   // cancels to FP64 round-off by construction (the density is chosen so that
   // no mass crosses the wall), also when h is stored in FP32.
   Acc<R> o0, o1, o2, o3, i0, i1, i2, i3;
+  const R Lw2 = R(lw * (sizeof(R) == 8 ? EXP64_LOG2E : -LOG2E));
   for (int v = threadIdx.x; v < g.nvel; v += WALL_T) {
     R un, ut;
     if (D == 1) { un = U[v]; ut = R(0); }
     else if (r.d == 0) { un = U[v]; ut = V[v]; }
     else { un = V[v]; ut = -U[v]; }
-    const bool in = un * R(rot) >= R(0);
+    const bool in = rot > 0 ? !(un < R(0)) : !(un > R(0));
     R c2 = un * un;
     if (D == 2) c2 += ut * ut;
     if (in) {
       R du = un - Uw, e = du * du;
       if (D == 2) { R dv = ut - Vw; e += dv * dv; }
-      const R t = W[v] * un * mexp(-Lw * e);
+      const R t = W[v] * un * wall_exp(Lw2, e, tab);
       i0.add(t);
       i1.add(t * un);
       if (D == 2) i2.add(t * ut);
@@ -347,25 +383,23 @@ __global__ void __launch_bounds__(WALL_T) k_wall(DevState sp, double dt_arg) {
     }
   }
   {
-    const double t0 = o0.total(), t1 = o1.total(), t2 = D == 2 ? o2.total() : 0.0, t3 = o3.total();
-    const double t4 = i0.total(), t5 = i1.total(), t6 = D == 2 ? i2.total() : 0.0, t7 = i3.total();
-    if (lane == 0) {
-      part[wid][0] = t0; part[wid][1] = t1; part[wid][2] = t2; part[wid][3] = t3;
-      part[wid][4] = t4; part[wid][5] = t5; part[wid][6] = t6; part[wid][7] = t7;
-    }
+    decltype(o0.s) x[8] = {o0.s, o1.s, o2.s, o3.s, i0.s, i1.s, i2.s, i3.s};
+    const double t = f64_total(warp_sums<8>(x, lane));
+    if ((lane & 3) == 0) part[wid][lane >> 2] = t;
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
+  // lane k of the first warp adds the warps' sums k in warp order
+  if (wid != 0) return;
+  double Tk = part[0][lane & 7];
+  for (int w = 1; w < WALL_T / 32; ++w) Tk += part[w][lane & 7];
   double T[8];
-  for (int k = 0; k < 8; ++k) {
-    T[k] = part[0][k];
-    for (int w = 1; w < WALL_T / 32; ++w) T[k] += part[w][k];
-  }
-  const double norm = D == 1 ? sqrt(lw / PI) : (lw / PI);
+  for (int k = 0; k < 8; ++k) T[k] = __shfl_sync(0xffffffffu, Tk, k);
+  if (lane != 0) return;
+  const double norm = D == 1 ? sqrt64(lw * (1.0 / PI)) : lw * (1.0 / PI);
   const double SF = T[0], I0 = T[4];
-  const double rho = -SF / (I0 * norm);
-  const double rn = rho * norm;  // wall density times the Maxwellian's normalisation
-  const double cBw = g.Kb / (2.0 * lw);
+  const double rn = -SF * rcp64(I0);  // wall density times the Maxwellian's normalisation
+  const double rho = rn * rcp64(norm);
+  const double cBw = g.Kb * (0.5 * rcp64(lw));
   double len = D == 2 ? (r.d == 0 ? g.dy : g.dx) : 1.0;
   double sc = D == 2 ? len * dt : dt;
   const double S0 = SF + rn * I0;
@@ -373,12 +407,21 @@ __global__ void __launch_bounds__(WALL_T) k_wall(DevState sp, double dt_arg) {
   const double S2 = D == 2 ? T[2] + rn * T[6] : 0.0;
   const double S3 = T[3] + rn * (T[7] + cBw * I0);
   s.rhow[f] = rho;
-  FaceCoef32 wc;
-  float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-  wc.G = wc.Cp = wc.Dp = wc.Cm = wc.Dm = z;
-  wc.E = maxwell_exp2(D == 1 ? rho * sqrt(lw / PI) : rho * (lw / PI), bw[1], bw[2], lw);
-  wc.T = make_float4(float(sc), 0.f, float(g.Kb / (2.0 * lw)), float(rot));
-  s.fc[f] = wc;
+  if (sizeof(R) == 4) {
+    FaceCoef32 wc;
+    float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    wc.G = wc.Cp = wc.Dp = wc.Cm = wc.Dm = z;
+    wc.E = maxwell_exp2(rn, bw[1], bw[2], lw);
+    wc.T = make_float4(f32_of(sc), 0.f, f32_of(cBw), rot > 0 ? 1.f : -1.f);
+    s.fc[f] = wc;
+  } else {
+    FaceCoef64 wc{};
+    put_maxwell(wc.E, rn, bw[1], bw[2], lw);
+    wc.T.x = sc;
+    wc.T.z = cBw;
+    wc.T.w = rot > 0 ? 1.0 : -1.0;
+    s.fc64[f] = wc;
+  }
   double fl[4] = {S0 * sc, S1 * sc, 0.0, 0.0};
   if (D == 1) {
     fl[2] = 0.5 * S3 * sc;
@@ -414,20 +457,29 @@ __device__ inline int update_group(const Geo& g, int i, int j) {
 }
 
 // step! scalar part (src/Solver/step_2f.jl:6-64, :179-249): Shakhov factors of
-// the old state, w += flux divergence, prim, tau, residual terms.  One thread
-// per physical cell; each block writes its residual partials in a fixed order.
-// FAST (the FP32 split form): tau, the density factors and the exponent
-// offsets of the coefficient blocks with FP32 transcendentals, conserve_prim
-// by reciprocals (see t_exp); w and prim stay FP64.  BS threads per block
-// (32 on small grids, 256 otherwise: DevState::cell_bs).
+// the old state, w += flux divergence, prim, tau.  One thread per physical
+// cell; res: each block writes its residual partials in a fixed order.  FAST
+// (the FP32 split form): tau and the exponent offsets of the coefficient
+// blocks with FP32 transcendentals; w and prim stay FP64.  BS threads per
+// block (32 on small grids, 256 otherwise: DevState::cell_bs).  Bound by the
+// FP64 pipe and, on small grids, by its latency: about 55 FP64 instructions a
+// cell (FP32 split, BGK) where divisions, conversions and the unused form's
+// coefficients took 350.
 template <int D, bool FAST, int BS, bool GRP = false>
-__global__ void __launch_bounds__(BS) k_cell_param(DevState sp, double dt_arg) {
+__global__ void __launch_bounds__(BS) k_cell_param(DevState sp, double dt_arg, int res) {
+  __shared__ double tab[FAST ? 1 : EXP64_N];
+  if (!FAST) {
+    exp64_load(tab, threadIdx.x, BS);
+    __syncthreads();
+  }
+  pdl_wait();
+  pdl_next();
   int lb;
   const int gr = group_member<GRP, GK_CELL>(sp, lb);
   KB_GROUP_STATE(GRP, sp, gr);
   const double dt = GRP ? sp.grp->dt[gr] : dt_arg;
   const Geo& g = s.g;
-  __shared__ double red[BS][8];
+  __shared__ double red[BS / 32][16];
   int t = lb * BS + threadIdx.x;
   double rr[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   int grp = 0;
@@ -435,149 +487,146 @@ __global__ void __launch_bounds__(BS) k_cell_param(DevState sp, double dt_arg) {
     int i = t % g.nx, j = t / g.nx;
     int c = cell_index(g, i, j);
     grp = update_group(g, i, j);
-    CellParam P;
-    P.upd = grp ? 1 : 0;
-    int coll = (D == 1 && grp == 2) ? COLL_BGK : s.coll;
-    P.coll = coll;
+    constexpr int NW = D + 2;  // compile-time, so the small arrays stay in registers
+    const int coll = (D == 1 && grp == 2) ? COLL_BGK : s.coll;
+    const bool shak = grp && coll == COLL_SHAKHOV;
     double* w = s.w + (long)c * 4;
     double* p = s.prim + (long)c * 4;
-    constexpr int NW = D + 2;  // compile-time, so the small arrays stay in registers
-    double lo = p[NW - 1];
-    P.o_rho_n = D == 1 ? p[0] * t_sqrt<FAST>(lo / PI) : p[0] * (lo / PI);
-    P.oU = p[1];
-    P.oV = D == 2 ? p[2] : 0.0;
-    P.olam = lo;
-    P.ocB = g.Kb / (2.0 * lo);
-    P.sfac = 0.8 * (1.0 - g.Pr) * (lo * lo) / p[0];
-    P.q0 = s.q[(long)c * 2 + 0];
-    P.q1 = s.q[(long)c * 2 + 1];
+    double po[4] = {1.0, 0.0, 0.0, 1.0}, q0 = 0.0, q1 = 0.0;
+    if (shak) {
+      for (int k = 0; k < NW; ++k) po[k] = p[k];
+      q0 = s.q[(long)c * 2 + 0];
+      q1 = D == 2 ? s.q[(long)c * 2 + 1] : 0.0;
+    }
+    double pn[4] = {0.0, 0.0, 0.0, 0.0}, rho_n = 0.0, cB = 0.0, dtau = 0.0, inv = 1.0;
     if (grp) {
-      double wo[4] = {w[0], w[1], w[2], w[3]};
-      double ds;
-      const double *fL, *fR, *fD = nullptr, *fU = nullptr;
-      int fx = j * (g.nx + 1) + i;
-      fL = s.fw + (long)fx * 4;
-      fR = s.fw + (long)(fx + 1) * 4;
-      if (D == 1) {
-        ds = g.dx;
-        for (int k = 0; k < 3; ++k) w[k] += (fL[k] - fR[k]) / ds;
-      } else {
-        int fy = s.nface_x + j * g.nx + i;
-        fD = s.fw + (long)fy * 4;
-        fU = s.fw + (long)(fy + g.nx) * 4;
-        ds = g.dx * g.dy;
-        for (int k = 0; k < 4; ++k) w[k] += (fL[k] - fR[k] + fD[k] - fU[k]) / ds;
-      }
-      double pn[4];
-      conserve_prim<FAST>(w, NW, g.gamma, pn);
-      for (int k = 0; k < NW; ++k) p[k] = pn[k];
+      double wn[4];
+      const int fx = j * (g.nx + 1) + i;
+      const double* fL = s.fw + (long)fx * 4;
+      const double* fR = s.fw + (long)(fx + 1) * 4;
+      const int fy = D == 2 ? s.nface_x + j * g.nx + i : 0;
+      const double* fD = s.fw + (long)fy * 4;
+      const double* fU = s.fw + (long)(fy + g.nx) * 4;
       for (int k = 0; k < NW; ++k) {
-        double dw = w[k] - wo[k];
-        rr[k] = dw * dw;
-        rr[4 + k] = fabs(w[k]);
+        double d = fL[k] - fR[k];
+        if (D == 2) d = d + fD[k] - fU[k];
+        const double wo = w[k];
+        wn[k] = fma(d, g.rds, wo);
+        w[k] = wn[k];
+        if (res) {
+          const double dw = wn[k] - wo;
+          rr[k] = dw * dw;
+          rr[4 + k] = fabs(wn[k]);
+        }
       }
-      double lam = pn[NW - 1];
-      double tau = vhs_time<FAST>(pn[0], lam, g.mu_ref, g.omega);
-      P.rho_n = D == 1 ? pn[0] * t_sqrt<FAST>(lam / PI) : pn[0] * (lam / PI);
-      P.U = pn[1];
-      P.V = D == 2 ? pn[2] : 0.0;
-      P.lam = lam;
-      P.cB = g.Kb / (2.0 * lam);
-      P.dtau = dt / tau;
-      P.inv = 1.0 / (1.0 + dt / tau);
-      bool bad = !(pn[0] > 0.0) || !(lam > 0.0) || !isfinite(pn[0]) || !isfinite(lam) ||
-                 !isfinite(pn[1]);
-      if (bad) atomicOr(s.status, 1);
-    } else {
-      P.rho_n = P.U = P.V = P.lam = P.cB = P.dtau = 0.0;
-      P.inv = 1.0;
+      conserve_prim<NW>(wn, g.hg, pn);
+      for (int k = 0; k < NW; ++k) p[k] = pn[k];
+      const double lam = pn[NW - 1];
+      const double lp = lam * (1.0 / PI);
+      rho_n = D == 1 ? pn[0] * t_sqrt<FAST>(lp) : pn[0] * lp;
+      cB = g.Kb * (0.5 * rcp64(lam));
+      dtau = dt * vhs_rate<FAST>(g, pn[0], lam, tab);
+      inv = rcp64(1.0 + dtau);
+      if (!pos64(pn[0]) || !pos64(lam) || !isfinite(f32_of(pn[1]))) atomicOr(s.status, 1);
     }
-    s.cp[c] = P;
-    CellParamF F;
-    F.rho_n = float(P.rho_n);
-    F.U = float(P.U);
-    F.V = float(P.V);
-    F.lam = float(P.lam);
-    F.cB = float(P.cB);
-    F.dtau = float(P.dtau);
-    F.inv = float(P.inv);
-    F.o_rho_n = float(P.o_rho_n);
-    F.oU = float(P.oU);
-    F.oV = float(P.oV);
-    F.olam = float(P.olam);
-    F.ocB = float(P.ocB);
-    F.sf0 = float(P.sfac * P.q0);
-    F.sf1 = float(P.sfac * P.q1);
-    F.upd = P.upd;
-    F.coll = P.coll;
-    s.cpf[c] = F;
-    CellCoef32 K;
-    float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    K.EM = K.EO = K.Q = K.TL = z;
-    if (P.upd) {
-      K.EM = maxwell_exp2<FAST>(P.rho_n, P.U, P.V, P.lam);
-      double ds = D == 1 ? g.dx : g.dx * g.dy;
-      K.A = make_float4(float(P.cB), float(P.dtau), float(P.inv), float(1.0 / ds));
-      if (P.coll == COLL_SHAKHOV) {
-        K.EO = maxwell_exp2<FAST>(P.o_rho_n, P.oU, P.oV, P.olam);
-        double s0 = P.sfac * P.q0, s1 = P.sfac * P.q1;
-        K.Q = make_float4(float(-(s0 * P.oU + s1 * P.oV)), float(s0), float(s1), float(P.ocB));
-        double l2 = 2.0 * P.olam;
-        K.TL = make_float4(float(l2 * (P.oU * P.oU + P.oV * P.oV) + g.Kb), float(-2.0 * l2 * P.oU),
-                           float(-2.0 * l2 * P.oV), float(l2));
-      } else {
-        K.EO.x = -200.f;
-      }
-    } else {
-      K.EM.x = -200.f;
-      K.EO.x = -200.f;
+    const double lo = po[NW - 1], lop = lo * (1.0 / PI), oV = D == 2 ? po[2] : 0.0;
+    double o_rho_n = 0.0, ocB = 0.0, s0 = 0.0, s1 = 0.0;
+    if (shak) {
+      o_rho_n = D == 1 ? po[0] * t_sqrt<FAST>(lop) : po[0] * lop;
+      ocB = g.Kb * (0.5 * rcp64(lo));
+      const double sf = g.sfac * (lo * lo) * rcp64(po[0]);
+      s0 = sf * q0;
+      s1 = sf * q1;
+    }
+    const double lam = pn[NW - 1], V = D == 2 ? pn[2] : 0.0;
+    if (FAST) {
+      CellCoef32 K;
+      float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+      K.EM = K.EO = K.Q = K.TL = z;
+      K.EM.x = K.EO.x = -200.f;
       K.A = make_float4(0.f, 0.f, 1.f, 0.f);
+      if (grp) {
+        K.EM = maxwell_exp2(rho_n, pn[1], V, lam);
+        K.A = make_float4(f32_of(cB), f32_of(dtau), f32_of(inv), f32_of(g.rds));
+        if (shak) {
+          K.EO = maxwell_exp2(o_rho_n, po[1], oV, lo);
+          K.Q = make_float4(f32_of(-fma(s0, po[1], s1 * oV)), f32_of(s0), f32_of(s1), f32_of(ocB));
+          const double l2 = 2.0 * lo, lU = l2 * po[1], lV = l2 * oV;
+          K.TL = make_float4(f32_of(fma(lU, po[1], fma(lV, oV, g.Kb))), f32_of(-2.0 * lU), f32_of(-2.0 * lV),
+                             f32_of(l2));
+        }
+      }
+      s.cc[c] = K;
+    } else {
+      CellParam P;
+      P.upd = grp ? 1 : 0;
+      P.coll = coll;
+      P.rho_n = rho_n;
+      P.U = pn[1];
+      P.V = V;
+      P.l2 = EXP64_LOG2E * lam;
+      P.cB = cB;
+      P.dtau = dtau;
+      P.inv = inv;
+      P.o_rho_n = o_rho_n;
+      P.oU = po[1];
+      P.oV = oV;
+      P.olam = lo;
+      P.ocB = ocB;
+      P.s0 = s0;
+      P.s1 = s1;
+      s.cp[c] = P;
     }
-    s.cc[c] = K;
   }
+  if (!res) return;  // uniform over the launch
   // deterministic block partials: interior (grp 1) and boundary (grp 2) sums
-  for (int half = 0; half < 2; ++half) {
-    bool take = grp == half + 1;
-    for (int k = 0; k < 8; ++k) red[threadIdx.x][k] = take ? rr[k] : 0.0;
-    __syncthreads();
-    for (int st = BS / 2; st >= 1; st >>= 1) {
-      if (threadIdx.x < st)
-        for (int k = 0; k < 8; ++k) red[threadIdx.x][k] += red[threadIdx.x + st][k];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0)
-      for (int k = 0; k < 8; ++k) s.blockres[(long)lb * 16 + half * 8 + k] = red[0][k];
-    __syncthreads();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double x[16];
+  for (int k = 0; k < 8; ++k) {
+    x[k] = grp == 1 ? rr[k] : 0.0;
+    x[8 + k] = grp == 2 ? rr[k] : 0.0;
+  }
+  const double sum = warp_sums<16>(x, lane);
+  if ((lane & 1) == 0) red[wid][lane >> 1] = sum;
+  __syncthreads();
+  if (threadIdx.x < 16) {
+    double a = red[0][threadIdx.x];
+    for (int k = 1; k < BS / 32; ++k) a += red[k][threadIdx.x];
+    s.blockres[(long)lb * 16 + threadIdx.x] = a;
   }
 }
 
 // residual = sqrt(sumRes N) / (sumAvg + 1e-7) + sqrt(boundary sumRes 2) / (...)
 // (src/Solver/solver_update.jl:86-88, :239-241; update_boundary.jl:41-44, :284-288).
 template <bool GRP = false>
-__global__ void k_residual(DevState sp) {
+__global__ void __launch_bounds__(256) k_residual(DevState sp) {
+  pdl_wait();
+  pdl_next();
   int lb;
   const int gr = group_member<GRP, GK_RES>(sp, lb);
   KB_GROUP_STATE(GRP, sp, gr);
-  __shared__ double red[256][16];
+  __shared__ double red[8][16];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   double acc[16];
   for (int k = 0; k < 16; ++k) acc[k] = 0.0;
-  for (int b = threadIdx.x; b < s.res_blocks; b += blockDim.x)
+  for (int b = threadIdx.x; b < s.res_blocks; b += 256)
     for (int k = 0; k < 16; ++k) acc[k] += s.blockres[(long)b * 16 + k];
-  for (int k = 0; k < 16; ++k) red[threadIdx.x][k] = acc[k];
+  const double sum = warp_sums<16>(acc, lane);
+  if ((lane & 1) == 0) red[wid][lane >> 1] = sum;
   __syncthreads();
-  for (int st = 128; st >= 1; st >>= 1) {
-    if (threadIdx.x < st)
-      for (int k = 0; k < 16; ++k) red[threadIdx.x][k] += red[threadIdx.x + st][k];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
+  if (wid != 0) return;
+  double t = red[0][lane & 15];
+  for (int k = 1; k < 8; ++k) t += red[k][lane & 15];
+  // lane k < 4: component k (sums k and 4 + k of the interior, 8 + k and 12 + k
+  // of the boundary cells)
+  const double a = __shfl_down_sync(0xffffffffu, t, 4), b = __shfl_down_sync(0xffffffffu, t, 8),
+               c = __shfl_down_sync(0xffffffffu, t, 12);
+  if (lane < 4) {
     const Geo& g = s.g;
     double n = g.D == 1 ? double(g.nx) : double(g.nx) * g.ny;
-    for (int k = 0; k < 4; ++k) {
-      double r = sqrt(red[0][k] * n) / (red[0][4 + k] + 1.e-7);
-      r += sqrt(red[0][8 + k] * 2) / (red[0][12 + k] + 1.e-7);
-      s.residual[k] = r;
-    }
+    double r = sqrt(t * n) / (a + 1.e-7);
+    r += sqrt(b * 2) / (c + 1.e-7);
+    s.residual[lane] = r;
   }
 }
 
@@ -620,8 +669,8 @@ __device__ __forceinline__ FaceCtx<R> make_ctx(const DevState& s, int f, int kin
     x.wU = R(r.d == 0 ? wp[1] : wp[2]);
     x.wV = R(D == 1 ? 0.0 : (r.d == 0 ? wp[2] : -wp[1]));
     x.wlam = R(lw);
-    x.wrn = R(D == 1 ? rho * sqrt(lw / PI) : rho * (lw / PI));
-    x.wcB = R(g.Kb / (2.0 * lw));
+    x.wrn = R(D == 1 ? rho * sqrt64(lw * (1.0 / PI)) : rho * (lw * (1.0 / PI)));
+    x.wcB = R(g.Kb * (0.5 * rcp64(lw)));
     x.wsc = R(D == 2 ? (r.d == 0 ? g.dy : g.dx) * dt : dt);
   }
   return x;
@@ -675,6 +724,8 @@ __device__ __forceinline__ void ctx_flux(const FaceCtx<R>& x, const R* __restric
 // in the new buffers.  pass 0: x sides, pass 1: y sides.  One block per ghost cell.
 template <typename R>
 __global__ void k_ghost(DevState s, int pass) {
+  pdl_wait();
+  pdl_next();
   const Geo& g = s.g;
   int t = blockIdx.x;
   int dst = -1, src = -1;
@@ -900,6 +951,16 @@ __global__ void k_init_eq(DevState s, R* __restrict__ H, R* __restrict__ Bq) {
 
 // ------------------------------------------------------------- launchers
 
+// Launch of a step kernel in its chain (launch_after).
+template <typename... P, typename... A>
+static void go(void (*fn)(P...), unsigned blocks, int threads, cudaStream_t st, A... a) {
+  std::tuple<P...> v(a...);
+  std::apply([&](P&... x) {
+    void* args[] = {(void*)&x...};
+    launch_after((const void*)fn, dim3(blocks), dim3((unsigned)threads), 0, st, args);
+  }, v);
+}
+
 static inline unsigned nblk(long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 // Every kernel of a step asks for the largest shared-memory carveout, the one
@@ -930,9 +991,8 @@ int launch_reconstruct(DevState& s, cudaStream_t st) {
   long n = (long)s.g.nx * s.g.ny * s.g.D;
   if (s.g.interp == 1) return 0;
   const int bs = item_bs(s, n);
-  void (*fn)(DevState) = s.prec != 0 ? k_wslope<true> : k_wslope<false>;
-  prefer_max_shared((const void*)fn);
-  fn<<<nblk(n, bs), bs, 0, st>>>(s);
+  prefer_max_shared((const void*)k_wslope<>);
+  go(k_wslope<>, nblk(n, bs), bs, st, s);
   return 1;
 }
 
@@ -951,7 +1011,7 @@ int launch_face_param(DevState& s, double dt, cudaStream_t st) {
   const int bs = item_bs(s, nf);
   void (*fn)(DevState, double) = s.g.D == 2 ? face_param_fn<2>(s.flux, fast) : face_param_fn<1>(s.flux, fast);
   prefer_max_shared((const void*)fn);
-  fn<<<nblk(nf, bs), bs, 0, st>>>(s, dt);
+  go(fn, nblk(nf, bs), bs, st, s, dt);
   return 1;
 }
 
@@ -961,7 +1021,7 @@ int launch_wall(DevState& s, double dt, cudaStream_t st) {
   if (s.g.D == 1) fn = s.prec == 0 ? k_wall<double, 1> : k_wall<float, 1>;
   else fn = s.prec == 0 ? k_wall<double, 2> : k_wall<float, 2>;
   prefer_max_shared((const void*)fn);
-  fn<<<(unsigned)s.nwall, WALL_T, 0, st>>>(s, dt);
+  go(fn, (unsigned)s.nwall, WALL_T, st, s, dt);
   return 1;
 }
 
@@ -973,18 +1033,18 @@ int launch_evolve(DevState& s, double dt, cudaStream_t st) {
 }
 
 template <int BS>
-static void cell_param_bs(DevState& s, double dt, cudaStream_t st) {
+static void cell_param_bs(DevState& s, double dt, bool res, cudaStream_t st) {
   const bool fast = s.prec != 0;
-  void (*fn)(DevState, double);
+  void (*fn)(DevState, double, int);
   if (s.g.D == 1) fn = fast ? k_cell_param<1, true, BS> : k_cell_param<1, false, BS>;
   else fn = fast ? k_cell_param<2, true, BS> : k_cell_param<2, false, BS>;
   prefer_max_shared((const void*)fn);
-  fn<<<s.res_blocks, BS, 0, st>>>(s, dt);
+  go(fn, (unsigned)s.res_blocks, BS, st, s, dt, res ? 1 : 0);
 }
 
-int launch_cell_param(DevState& s, double dt, cudaStream_t st) {
-  if (s.cell_bs == 32) cell_param_bs<32>(s, dt, st);
-  else cell_param_bs<256>(s, dt, st);
+int launch_cell_param(DevState& s, double dt, cudaStream_t st, bool res) {
+  if (s.cell_bs == 32) cell_param_bs<32>(s, dt, res, st);
+  else cell_param_bs<256>(s, dt, res, st);
   return 1;
 }
 
@@ -1001,12 +1061,12 @@ static int finish_t(DevState& s, cudaStream_t st, bool res) {
     t.cur ^= 1;
     int nrow = D == 2 ? s.g.nyt : 1;
     prefer_max_shared((const void*)k_ghost<R>);
-    if (s.g.ngx > 0) { k_ghost<R><<<2 * s.g.ngx * nrow, 128, 0, st>>>(t, 0); ++n; }
-    if (D == 2 && s.g.ngy > 0) { k_ghost<R><<<2 * s.g.ngy * s.g.nxt, 128, 0, st>>>(t, 1); ++n; }
+    if (s.g.ngx > 0) { go(k_ghost<R>, (unsigned)(2 * s.g.ngx * nrow), 128, st, t, 0); ++n; }
+    if (D == 2 && s.g.ngy > 0) { go(k_ghost<R>, (unsigned)(2 * s.g.ngy * s.g.nxt), 128, st, t, 1); ++n; }
   }
   if (res) {
     prefer_max_shared((const void*)k_residual<false>);
-    k_residual<false><<<1, 256, 0, st>>>(s);
+    go(k_residual<false>, 1u, 256, st, s);
     ++n;
   }
   return n;
@@ -1015,37 +1075,37 @@ static int finish_t(DevState& s, cudaStream_t st, bool res) {
 // ---- grouped launches (kb_group.cu): the per-face / per-cell kernels of one
 // step of the 2D FP32 form over all members of a group; ls.grp points at
 // the step's member table, the block counts are the members' summed.
-void group_small(int kind, const DevState& ls, int flux, int blocks, cudaStream_t st) {
+void group_small(int kind, const DevState& ls, int flux, int blocks, bool res, cudaStream_t st) {
   if (blocks <= 0) return;
   const void* fn = nullptr;
   switch (kind) {
     case GK_WSLOPE:
-      fn = (const void*)k_wslope<true, true>;
+      fn = (const void*)k_wslope<true>;
       prefer_max_shared(fn);
-      k_wslope<true, true><<<blocks, 32, 0, st>>>(ls);
+      go(k_wslope<true>, (unsigned)blocks, 32, st, ls);
       break;
     case GK_FACE: {
       void (*f)(DevState, double) = flux == FLUX_KFVS ? k_face_param<2, FLUX_KFVS, true, true>
                                     : flux == FLUX_KCU ? k_face_param<2, FLUX_KCU, true, true>
                                                        : k_face_param<2, FLUX_UGKS, true, true>;
       prefer_max_shared((const void*)f);
-      f<<<blocks, 32, 0, st>>>(ls, 0.0);
+      go(f, (unsigned)blocks, 32, st, ls, 0.0);
       break;
     }
     case GK_WALL:
       fn = (const void*)k_wall<float, 2, true>;
       prefer_max_shared(fn);
-      k_wall<float, 2, true><<<blocks, WALL_T, 0, st>>>(ls, 0.0);
+      go(k_wall<float, 2, true>, (unsigned)blocks, WALL_T, st, ls, 0.0);
       break;
     case GK_CELL:
       fn = (const void*)k_cell_param<2, true, 32, true>;
       prefer_max_shared(fn);
-      k_cell_param<2, true, 32, true><<<blocks, 32, 0, st>>>(ls, 0.0);
+      go(k_cell_param<2, true, 32, true>, (unsigned)blocks, 32, st, ls, 0.0, res ? 1 : 0);
       break;
     case GK_RES:
       fn = (const void*)k_residual<true>;
       prefer_max_shared(fn);
-      k_residual<true><<<blocks, 256, 0, st>>>(ls);
+      go(k_residual<true>, (unsigned)blocks, 256, st, ls);
       break;
     default:
       break;
@@ -1058,7 +1118,7 @@ int launch_finish(DevState& s, cudaStream_t st, bool res) {
 }
 
 int launch_update(DevState& s, double dt, cudaStream_t st, bool res) {
-  int n = launch_cell_param(s, dt, st);
+  int n = launch_cell_param(s, dt, st, res);
   n += launch_march(s, dt, st);
   n += launch_finish(s, st, res);
   return n;

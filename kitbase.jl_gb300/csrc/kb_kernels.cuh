@@ -42,7 +42,6 @@ struct DevState {
   double* prim;     // [ncell][4]
   double* sw;       // [ncell][2][4]
   FaceParam* fp;    // [nface]
-  FaceParamF* fpf;  // [nface]
   double* fw;       // [nface][4] global frame
   double* wall;     // [nface][4] wall prim, global frame (only wall faces read)
   double* rhow;     // [nface] Maxwell wall density
@@ -51,8 +50,8 @@ struct DevState {
   int nwall;
   double* q;        // [ncell][2]
   CellParam* cp;    // [ncell]
-  CellParamF* cpf;  // [ncell]
-  FaceCoef32* fc;   // [nface] FP32 coefficient blocks
+  FaceCoef32* fc;   // [nface] FP32 coefficient blocks (FP32 form)
+  FaceCoef64* fc64; // [nface] FP64 coefficient blocks (FP64 form)
   CellCoef32* cc;   // [ncell] FP32 cell coefficients
   double* blockres; // [nblocks][16] residual partials
   float2* mpart;    // [velocity boxes][2][nface][4] pass-A partials of the row-ring form
@@ -124,7 +123,8 @@ __device__ __forceinline__ int group_member(const DevState& sp, int& lb) {
 
 // Grouped launch of a per-face / per-cell step kernel (kind GK_WSLOPE,
 // GK_FACE, GK_WALL, GK_CELL or GK_RES) over `blocks` blocks (kb_kernels.cu).
-void group_small(int kind, const DevState& ls, int flux, int blocks, cudaStream_t st);
+// res: with the residual's partial sums (GK_CELL).
+void group_small(int kind, const DevState& ls, int flux, int blocks, bool res, cudaStream_t st);
 
 // Face classification for the current configuration (host computes, uploads).
 void face_kinds_host(const Geo& g, signed char* kind);
@@ -140,7 +140,7 @@ int launch_update(DevState& s, double dt, cudaStream_t st, bool res = true);
 // evolve = face_param + moments + wall; update = cell_param + march + finish.
 int launch_face_param(DevState& s, double dt, cudaStream_t st);
 int launch_wall(DevState& s, double dt, cudaStream_t st);
-int launch_cell_param(DevState& s, double dt, cudaStream_t st);
+int launch_cell_param(DevState& s, double dt, cudaStream_t st, bool res = true);
 int launch_finish(DevState& s, cudaStream_t st, bool res = true);
 
 // Pass A (face moments, heat flux) and pass B (pointwise update), kb_march.cu.

@@ -48,10 +48,9 @@ __device__ __forceinline__ float vl_diff(int rule, float qm, float q0, float qp,
   return 0.f;
 }
 __device__ __forceinline__ double vl_diff(int rule, double qm, double q0, double qp, double epsd) {
-  double a = q0 - qm, b = qp - q0;
-  if (rule == 1) return (a * fabs(b) + b * fabs(a)) / (fabs(a) + fabs(b) + epsd);
-  if (rule == 2) return b;
-  if (rule == 3) return a;
+  if (rule == 1) return vl64(qm, q0, qp, epsd);
+  if (rule == 2) return qp - q0;
+  if (rule == 3) return q0 - qm;
   return 0.0;
 }
 
@@ -98,11 +97,66 @@ struct BAcc<double> {
 
 // ------------------------------------------------------------------ pass A
 
+__device__ __forceinline__ double bacc_value(BAcc<double>& a) { return a.p; }
+__device__ __forceinline__ DF bacc_value(BAcc<float>& a) {
+  a.flush();
+  return a.d;
+}
+// fw of N faces of a warp's segment from its lanes' moments acc[f][k]: all sums
+// in one reduce-scatter, then a lane for each (face, moment), so the FP64
+// conversion and addition are one warp instruction each for all of them.  The
+// faces are p = p0 .. p0 + N - 1 of the line; `live` of them are stored (those
+// of kind 1).  Moments: mass, normal and tangential momentum, twice the energy.
+template <int N, int D, int DIR, typename A>
+__device__ __forceinline__ void store_fw(const DevState& s, A (*acc)[4], int line, int p0, int live, int lane) {
+  decltype(bacc_value(acc[0][0])) x[4 * N];
+#pragma unroll
+  for (int k = 0; k < 4 * N; ++k) x[k] = bacc_value(acc[k >> 2][k & 3]);
+  double S = f64_total(warp_sums<4 * N>(x, lane));
+  constexpr int W = 32 / (4 * N);  // lanes per value
+  const int v = lane / W, f = v >> 2, k = v & 3;
+  if (lane % W != 0 || f >= live) return;
+  const int p = p0 + f;
+  const int fi = DIR == 0 ? line * (s.g.nx + 1) + p : s.nface_x + p * s.g.nx + line;
+  if (s.kind[fi] != 1) return;
+  double* out = s.fw + (long)fi * 4;
+  const double* fwa = s.fp[fi].fwa;
+  if (k == 3) S *= 0.5;
+  if (D == 1) {  // energy in slot 2
+    if (k == 2) out[3] = 0.0;
+    else out[k == 3 ? 2 : k] = fwa[k == 3 ? 2 : k] + S;
+  } else {
+    const double x0 = fwa[k] + S;
+    if (DIR == 0) out[k] = x0;
+    else out[k == 1 ? 2 : (k == 2 ? 1 : k)] = k == 2 ? -x0 : x0;  // global_frame with n = (0, 1)
+  }
+}
+// the old heat flux of N cells p0 .. of the line, `live` of them
+template <int N, int DIR, typename A>
+__device__ __forceinline__ void store_q(const DevState& s, A (*qa)[2], int line, int p0, int live, int lane) {
+  decltype(bacc_value(qa[0][0])) x[2 * N];
+#pragma unroll
+  for (int k = 0; k < 2 * N; ++k) x[k] = bacc_value(qa[k >> 1][k & 1]);
+  const double S = 0.5 * f64_total(warp_sums<2 * N>(x, lane));
+  constexpr int W = 32 / (2 * N);
+  const int v = lane / W, c = v >> 1;
+  if (lane % W != 0 || c >= live) return;
+  const int cc = DIR == 0 ? cell_index(s.g, p0 + c, line) : cell_index(s.g, line, p0 + c);
+  s.q[(long)cc * 2 + (v & 1)] = S;
+}
+
 // DIR 0: x faces, segments along x in each row; DIR 1: y faces, segments
 // along y in each column.  Face f of a segment sits between cells p-1 and p
 // along the line with p = p0 + f; cells p0-2 .. p0+TS+1 form the window.
-template <typename R, int D, int FLUX, int TS, bool SHAK, int DIR>
+// FP64 form.  Bound by the FP64 pipe: one upwind slope per face and velocity
+// (Newton reciprocal) and the transport flux as one multiply-add on the slope:
+// about 33 FP64 instructions per face and velocity, 80 with both cells' slopes
+// and IEEE divisions (128 x 128 cells x 32 x 32 velocities: see store_fw).
+template <int D, int FLUX, int TS, bool SHAK, int DIR>
 __global__ void __launch_bounds__(128) k_mom(DevState s) {
+  using R = double;
+  pdl_wait();
+  pdl_next();
   const Geo& g = s.g;
   const int lane = threadIdx.x & 31;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -147,8 +201,8 @@ __global__ void __launch_bounds__(128) k_mom(DevState s) {
     t4[f] = R(0);
     if (act[f]) {
       const FaceParam& P = s.fp[fidx[f]];
-      t3[f] = R(P.tr[0]);
-      t4[f] = R(P.tr[1] / dd);
+      t3[f] = P.tr[0];
+      t4[f] = P.tr[1] * (DIR == 0 ? g.rdx : g.rdy);
     }
   }
   R oU[TS], oV[TS];
@@ -174,8 +228,7 @@ __global__ void __launch_bounds__(128) k_mom(DevState s) {
 
   auto run = [&](auto fast_tag) {
   constexpr bool FAST = decltype(fast_tag)::value;
-  int it = 0;
-  for (int v0 = 0; v0 < g.nvel; v0 += 32, ++it) {
+  for (int v0 = 0; v0 < g.nvel; v0 += 32) {
     const int v = v0 + lane;
     const bool ok = v < g.nvel;
     R u = ok ? U[v] : R(0);
@@ -189,52 +242,33 @@ __global__ void __launch_bounds__(128) k_mom(DevState s) {
       hx[w] = ldq(H, base[w] + v, (FAST || ex[w]) && ok);
       bx[w] = ldq(Bq, base[w] + v, (FAST || ex[w]) && ok);
     }
-    R dh[TS + 2], db[TS + 2];  // slopes of cells w = 1 .. TS+2
-#pragma unroll
-    for (int w = 1; w <= TS + 2; ++w) {
-      dh[w - 1] = slope<FAST>(rule[w], hx[w - 1], hx[w], hx[w + 1], epsd);
-      db[w - 1] = slope<FAST>(rule[w], bx[w - 1], bx[w], bx[w + 1], epsd);
-    }
+    // only the upwind cell's slope of each face, its stencil picked by sign
     const bool pos = un >= R(0);
-    const R c2 = un * un + ut * ut;
-    const R un2 = un * un;
+    const R un2 = un * un, c2 = D == 2 ? un2 + ut * ut : un2;
+    const R ou = om * un, ot = om * ut, oc = om * c2;
 #pragma unroll
     for (int f = 0; f < TS + 1; ++f) {
       if (FAST ? f == TS : !act[f]) continue;
-      R hu = pos ? hx[f + 1] : hx[f + 2];
-      R bu = pos ? bx[f + 1] : bx[f + 2];
-      R su = pos ? dh[f] : dh[f + 1];
-      R sb = pos ? db[f] : db[f + 1];
-      R hf = hu + (pos ? R(0.5) : R(-0.5)) * su;
-      R bf = bu + (pos ? R(0.5) : R(-0.5)) * sb;
-      R Th = t3[f] * un * hf - t4[f] * un2 * su;
-      R Tb = t3[f] * un * bf - t4[f] * un2 * sb;
-      R wT = om * Th;
-      acc[f][0].add(wT);
-      acc[f][1].add(wT * un);
-      if (D == 2) acc[f][2].add(wT * ut);
-      acc[f][3].add(wT * c2 + om * Tb);
+      const int ru = FAST ? 1 : (pos ? rule[f + 1] : rule[f + 2]);
+      const R h0 = pos ? hx[f + 1] : hx[f + 2], b0 = pos ? bx[f + 1] : bx[f + 2];
+      const R su = vl_diff(ru, pos ? hx[f] : hx[f + 1], h0, pos ? hx[f + 2] : hx[f + 3], epsd);
+      const R sb = vl_diff(ru, pos ? bx[f] : bx[f + 1], b0, pos ? bx[f + 2] : bx[f + 3], epsd);
+      // t3 un (q + side s) - t4 un^2 s
+      const R a = t3[f] * un, k = fma(pos ? R(0.5) : R(-0.5), a, -t4[f] * un2);
+      const R Th = fma(k, su, a * h0), Tb = fma(k, sb, a * b0);
+      acc[f][0].p = fma(om, Th, acc[f][0].p);
+      acc[f][1].p = fma(ou, Th, acc[f][1].p);
+      if (D == 2) acc[f][2].p = fma(ot, Th, acc[f][2].p);
+      acc[f][3].p = fma(oc, Th, fma(om, Tb, acc[f][3].p));
     }
     if (SHAK) {
 #pragma unroll
       for (int c = 0; c < TS; ++c) {
         R cu = u - oU[c];
         R cv = vv - oV[c];
-        R c2o = cu * cu + cv * cv;
-        R hc = hx[c + 2], bc = bx[c + 2];
-        qa[c][0].add(om * cu * c2o * hc + om * cu * bc);
-        if (D == 2) qa[c][1].add(om * cv * c2o * hc + om * cv * bc);
-      }
-    }
-    if ((it & 3) == 3) {
-#pragma unroll
-      for (int f = 0; f < TS + 1; ++f)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) acc[f][k].flush();
-#pragma unroll
-      for (int c = 0; c < (SHAK ? TS : 1); ++c) {
-        qa[c][0].flush();
-        qa[c][1].flush();
+        const R t = om * fma(D == 2 ? fma(cu, cu, cv * cv) : cu * cu, hx[c + 2], bx[c + 2]);
+        qa[c][0].p = fma(cu, t, qa[c][0].p);
+        if (D == 2) qa[c][1].p = fma(cv, t, qa[c][1].p);
       }
     }
   }
@@ -244,50 +278,9 @@ __global__ void __launch_bounds__(128) k_mom(DevState s) {
   for (int f = 0; f < TS; ++f) fast = fast && act[f];
   if (fast) run(std::true_type{});
   else run(std::false_type{});
-#pragma unroll
-  for (int f = 0; f < TS + 1; ++f) {
-    if (!act[f]) continue;
-    double S0 = acc[f][0].total(), S1 = acc[f][1].total();
-    double S2 = D == 2 ? acc[f][2].total() : 0.0;
-    double S3 = acc[f][3].total();
-    if (lane == 0) {
-      const FaceParam& P = s.fp[fidx[f]];
-      double fl[4];
-      fl[0] = P.fwa[0] + S0;
-      fl[1] = P.fwa[1] + S1;
-      if (D == 1) {
-        fl[2] = P.fwa[2] + 0.5 * S3;
-        fl[3] = 0.0;
-      } else {
-        fl[2] = P.fwa[2] + S2;
-        fl[3] = P.fwa[3] + 0.5 * S3;
-      }
-      double* out = s.fw + (long)fidx[f] * 4;
-      if (DIR == 1) {  // global_frame with n = (0, 1)
-        out[0] = fl[0];
-        out[1] = -fl[2];
-        out[2] = fl[1];
-        out[3] = fl[3];
-      } else {
-        out[0] = fl[0];
-        out[1] = fl[1];
-        out[2] = fl[2];
-        out[3] = fl[3];
-      }
-    }
-  }
-  if (SHAK) {
-#pragma unroll
-    for (int c = 0; c < TS; ++c) {
-      double q0 = qa[c][0].total();
-      double q1 = D == 2 ? qa[c][1].total() : 0.0;
-      if (lane == 0 && c < ncell) {
-        long cc = base[c + 2] / vs;
-        s.q[cc * 2 + 0] = 0.5 * q0;
-        s.q[cc * 2 + 1] = 0.5 * q1;
-      }
-    }
-  }
+  store_fw<TS, D, DIR>(s, acc, line, p0, nf, lane);
+  if (nf > TS) store_fw<1, D, DIR>(s, acc + TS, line, p0 + TS, 1, lane);
+  if (SHAK) store_q<TS, DIR>(s, qa, line, p0, ncell, lane);
 }
 
 // Pass A, FP32 form: the stencil window of a CTA segment (4 warps x TS faces
@@ -318,6 +311,8 @@ __global__ void __launch_bounds__(MOM_THREADS) k_mom_st(const __grid_constant__ 
                                                         const __grid_constant__ CUtensorMap tmb,
                                                         DevState sp) {
   using R = float;
+  pdl_wait();
+  pdl_next();
   int lb;
   const int gr = group_member<GRP, DIR == 0 ? GK_MOMX : GK_MOMY>(sp, lb);
   KB_GROUP_STATE(GRP, sp, gr);
@@ -398,9 +393,9 @@ __global__ void __launch_bounds__(MOM_THREADS) k_mom_st(const __grid_constant__ 
     t3[f] = R(0);
     t4[f] = R(0);
     if (act[f]) {
-      const FaceParam& P = s.fp[fidx[f]];
-      t3[f] = R(P.tr[0]);
-      t4[f] = R(P.tr[1] / dd);
+      const float4 T = s.fc[fidx[f]].T;  // transport coefficients, T.y over the cell size
+      t3[f] = T.x;
+      t4[f] = T.y;
     }
   }
   R oU[TS], oV[TS];
@@ -409,8 +404,8 @@ __global__ void __launch_bounds__(MOM_THREADS) k_mom_st(const __grid_constant__ 
     for (int c = 0; c < TS; ++c) {
       bool e;
       const int cc = win_cell(wid * TS + c + 2, e);
-      oU[c] = e ? R(s.prim[(long)cc * 4 + 1]) : R(0);
-      oV[c] = (e && D == 2) ? R(s.prim[(long)cc * 4 + 2]) : R(0);
+      oU[c] = e ? f32_of(s.prim[(long)cc * 4 + 1]) : R(0);
+      oV[c] = (e && D == 2) ? f32_of(s.prim[(long)cc * 4 + 2]) : R(0);
     }
   }
   BAcc<R> acc[TS + 1][4];
@@ -604,51 +599,10 @@ __global__ void __launch_bounds__(MOM_THREADS) k_mom_st(const __grid_constant__ 
         mbar_wait(&full[k % MOM_P], (k / MOM_P) & 1);
     return;
   }
-#pragma unroll
-  for (int f = 0; f < TS + 1; ++f) {
-    if (!act[f]) continue;
-    double S0 = acc[f][0].total(), S1 = acc[f][1].total();
-    double S2 = D == 2 ? acc[f][2].total() : 0.0;
-    double S3 = acc[f][3].total();
-    if (lane == 0) {
-      const FaceParam& P = s.fp[fidx[f]];
-      double fl[4];
-      fl[0] = P.fwa[0] + S0;
-      fl[1] = P.fwa[1] + S1;
-      if (D == 1) {
-        fl[2] = P.fwa[2] + 0.5 * S3;
-        fl[3] = 0.0;
-      } else {
-        fl[2] = P.fwa[2] + S2;
-        fl[3] = P.fwa[3] + 0.5 * S3;
-      }
-      double* out = s.fw + (long)fidx[f] * 4;
-      if (DIR == 1) {  // global_frame with n = (0, 1)
-        out[0] = fl[0];
-        out[1] = -fl[2];
-        out[2] = fl[1];
-        out[3] = fl[3];
-      } else {
-        out[0] = fl[0];
-        out[1] = fl[1];
-        out[2] = fl[2];
-        out[3] = fl[3];
-      }
-    }
-  }
-  if (SHAK) {
-#pragma unroll
-    for (int c = 0; c < TS; ++c) {
-      double q0 = qa[c][0].total();
-      double q1 = D == 2 ? qa[c][1].total() : 0.0;
-      if (lane == 0 && c < ncell) {
-        bool e;
-        const long cc = win_cell(wid * TS + c + 2, e);
-        s.q[cc * 2 + 0] = 0.5 * q0;
-        s.q[cc * 2 + 1] = 0.5 * q1;
-      }
-    }
-  }
+  if (nf == 0) return;  // the producer warp, and warps past the line's end
+  store_fw<TS, D, DIR>(s, acc, line, p0w, nf, lane);
+  if (nf > TS) store_fw<1, D, DIR>(s, acc + TS, line, p0w + TS, 1, lane);
+  if (SHAK) store_q<TS, DIR>(s, qa, line, p0w, ncell, lane);
 }
 
 // ------------------------------------------------------------------ pass B
@@ -688,35 +642,24 @@ struct FEv<float> {
   }
 };
 
-// FP64: direct formulas of the reference with the interface prim.
+// FP64: the same form, with FaceCoef64.
 template <>
 struct FEv<double> {
-  FP<double> P;
-  double dd;  // cell size along the face normal
-  double wU, wV, wlam, wrn, wcB, wsc, rot;
+  Quad64 E, T, G, C, Dd;
   int kind;
-  __device__ __forceinline__ void load(const DevState& s, int f, bool pos) {
-    (void)pos;
-    kind = s.kind[f];
+  __device__ __forceinline__ void load_interior(const FaceCoef64& c, bool pos) {
+    kind = 1;
+    E = c.E;
+    T = c.T;
+    G = c.G;
+    C = pos ? c.Cp : c.Cm;
+    Dd = pos ? c.Dp : c.Dm;
+  }
+  __device__ __forceinline__ void load(const FaceCoef64& c, int kd, bool pos) {
+    kind = kd;
     if (kind == 0) return;
-    const Geo& g = s.g;
-    FaceGeo r = face_geo(g, f);
-    dd = r.d == 0 ? g.dx : g.dy;
-    if (kind == 1) {
-      P = load_fp<double>(s, f);
-    } else {
-      const double* wp = s.wall + (long)f * 4;
-      double lw = g.D == 1 ? wp[2] : wp[3];
-      double rho = s.rhow[f];
-      wU = r.d == 0 ? wp[1] : wp[2];
-      wV = g.D == 1 ? 0.0 : (r.d == 0 ? wp[2] : -wp[1]);
-      wlam = lw;
-      wrn = g.D == 1 ? rho * sqrt(lw / PI) : rho * (lw / PI);
-      wcB = g.Kb / (2.0 * lw);
-      wsc = g.D == 2 ? (r.d == 0 ? g.dy : g.dx) : 1.0;
-      int p0 = r.d == 0 ? r.fi : r.fj;
-      rot = p0 == 0 ? 1.0 : -1.0;
-    }
+    load_interior(c, pos);
+    kind = kd;
   }
 };
 
@@ -740,8 +683,7 @@ struct Mono {
 template <int D, int FLUX, bool FAST = false>
 __device__ __forceinline__ void eval_face(const FEv<float>& e, const Mono<float>& M, float side,
                                           float hu, float bu, float su, float sb, float hc,
-                                          float bc, double dt, float& fh, float& fb) {
-  (void)dt;
+                                          float bc, const double*, float& fh, float& fb) {
   if (!FAST && e.kind == 0) {
     fh = 0.f;
     fb = 0.f;
@@ -789,41 +731,62 @@ __device__ __forceinline__ void eval_face(const FEv<float>& e, const Mono<float>
   fb += Hu * pb;
 }
 
+// FP64: tab is the table of exp2_tab.
 template <int D, int FLUX, bool FAST = false>
 __device__ __forceinline__ void eval_face(const FEv<double>& e, const Mono<double>& M,
                                           double side, double hu, double bu, double su,
-                                          double sb, double hc, double bc, double dt,
+                                          double sb, double hc, double bc, const double* tab,
                                           double& fh, double& fb) {
   if (!FAST && e.kind == 0) {
     fh = 0.0;
     fb = 0.0;
     return;
   }
-  const double un = M.un, ut = M.ut;
+  const double un = M.un;
+  auto maxwell = [&]() {
+    const double du = un - e.E.y;
+    double c2 = du * du;
+    if (D == 2) {
+      const double dv = M.ut - e.E.z;
+      c2 = fma(dv, dv, c2);
+    }
+    return e.E.x * exp2_tab(e.E.w, c2, tab);
+  };
   if (!FAST && e.kind == 2) {
-    bool in = un * e.rot >= 0.0;
     double hw, bw;
-    if (in) {
-      double du = un - e.wU, ee = du * du;
-      if (D == 2) {
-        double dv = ut - e.wV;
-        ee += dv * dv;
-      }
-      hw = e.wrn * exp(-e.wlam * ee);
-      bw = hw * e.wcB;
+    if (un * e.T.w >= 0.0) {
+      hw = maxwell();
+      bw = hw * e.T.z;
     } else {
       hw = hc;
       bw = bc;
     }
-    fh = un * hw * e.wsc * dt;
-    fb = un * bw * e.wsc * dt;
+    const double a = un * e.T.x;
+    fh = a * hw;
+    fb = a * bw;
     return;
   }
-  const double hf = hu + side * su;
-  const double bf = bu + side * sb;
-  double Th, Tb;
-  face_flux<double, FLUX, D>(e.P, dt, un, ut, side > 0.0, hf, bf, su / e.dd, sb / e.dd, fh, fb,
-                             Th, Tb);
+  const double a = e.T.x * un, k = fma(side, a, -e.T.y * M.n2);
+  fh = fma(k, su, a * hu);
+  fb = fma(k, sb, a * bu);
+  if (FLUX == FLUX_KFVS) return;
+  double ph = e.T.z, pb = e.T.w;
+  if (FLUX == FLUX_UGKS) {
+    double ih = fma(e.C.w, M.c2, fma(e.C.y, un, e.C.x)), ib = fma(e.Dd.w, M.c2, fma(e.Dd.y, un, e.Dd.x));
+    if (D == 2) {
+      ih = fma(e.C.z, M.ut, ih);
+      ib = fma(e.Dd.z, M.ut, ib);
+    }
+    ph = fma(e.G.y, M.c2, fma(un, ih, ph));
+    pb = fma(e.G.w, M.c2, fma(un, ib, pb));
+    if (D == 2) {
+      ph = fma(e.G.x, M.ut, ph);
+      pb = fma(e.G.z, M.ut, pb);
+    }
+  }
+  const double Hu = maxwell() * un;
+  fh = fma(Hu, ph, fh);
+  fb = fma(Hu, pb, fb);
 }
 
 // Pointwise relaxation of one cell value (step!, src/Solver/step_2f.jl:32-63, :210-248).
@@ -843,51 +806,44 @@ __device__ __forceinline__ void relax(const CellCoef32& k, bool shak, float u, f
   bn = (b0 + db * k.A.w + k.A.y * MB) * k.A.z;
 }
 
-__device__ __forceinline__ void relax(const CP<double>& C, double ds, double u, double vv,
+__device__ __forceinline__ void relax(const CellParam& C, double rds, double u, double vv,
                                       double Kf, int D, double h0, double b0, double dh,
-                                      double db, double& hn, double& bn) {
+                                      double db, const double* tab, double& hn, double& bn) {
   if (!C.upd) {
     hn = h0;
     bn = b0;
     return;
   }
-  double du = u - C.U, e = du * du;
+  const double du = u - C.U;
+  double e = du * du;
   if (D == 2) {
-    double dv = vv - C.V;
-    e += dv * dv;
+    const double dv = vv - C.V;
+    e = fma(dv, dv, e);
   }
-  double MH = C.rho_n * exp(-C.lam * e);
-  double MB = MH * Kf / (2.0 * C.lam);
+  double MH = C.rho_n * exp2_tab(C.l2, e, tab), MB = MH * C.cB;
   if (C.coll == COLL_SHAKHOV) {
-    double ou = u - C.oU, oe = ou * ou, cq = ou * C.s0;
+    const double ou = u - C.oU;
+    double oe = ou * ou, cq = ou * C.s0;
     if (D == 2) {
-      double ov = vv - C.oV;
-      oe += ov * ov;
-      cq += ov * C.s1;
+      const double ov = vv - C.oV;
+      oe = fma(ov, ov, oe);
+      cq = fma(ov, C.s1, cq);
     }
-    double OH = C.o_rho_n * exp(-C.olam * oe);
-    double OB = OH * Kf / (2.0 * C.olam);
-    double tl = 2.0 * C.olam * oe + Kf;
-    MH += cq * (tl - 5.0) * OH;
-    MB += cq * (tl - 3.0) * OB;
+    const double S = cq * (C.o_rho_n * exp2_tab(EXP64_LOG2E * C.olam, oe, tab));
+    const double tl = fma(2.0 * C.olam, oe, Kf - 3.0);
+    MH = fma(S, tl - 2.0, MH);
+    MB = fma(S * tl, C.ocB, MB);
   }
-  hn = (h0 + dh / ds + C.dtau * MH) / (1.0 + C.dtau);
-  bn = (b0 + db / ds + C.dtau * MB) / (1.0 + C.dtau);
+  hn = fma(C.dtau, MH, fma(dh, rds, h0)) * C.inv;
+  bn = fma(C.dtau, MB, fma(db, rds, b0)) * C.inv;
 }
 
-// Load face f's evaluation state: FP32 from its coefficient block c (global
-// memory or staged in shared memory), FP64 from the FaceParam table.
-template <bool FAST>
-__device__ __forceinline__ void face_load(FEv<float>& e, const DevState& s, int f,
-                                          const FaceCoef32& c, bool pos) {
+// Load face f's evaluation state from its coefficient block c (global memory or
+// staged in shared memory).
+template <bool FAST, typename R, typename FC>
+__device__ __forceinline__ void face_load(FEv<R>& e, const DevState& s, int f, const FC& c, bool pos) {
   if (FAST) e.load_interior(c, pos);
   else e.load(c, s.kind[f], pos);
-}
-template <bool FAST>
-__device__ __forceinline__ void face_load(FEv<double>& e, const DevState& s, int f,
-                                          const FaceCoef32& c, bool pos) {
-  (void)c;
-  e.load(s, f, pos);
 }
 
 // Shared-memory staging of the FP32 coefficient blocks of a pass-B strip:
@@ -919,7 +875,15 @@ static_assert(sizeof(FaceCoef32) % 16 == 0 && sizeof(CellCoef32) % 16 == 0,
 // the last velocity compute on a clamped velocity and store nothing, so every
 // thread reaches every barrier.
 template <typename R, int D, int FLUX, int TX, int BS>
-__global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / BS) k_march(DevState s, double dt, int RY) {
+__global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / BS) k_march(DevState s, int RY) {
+  using FC = typename FaceCoefOf<R>::T;
+  __shared__ double tab[sizeof(R) == 8 ? EXP64_N : 1];
+  if (sizeof(R) == 8) {
+    exp64_load(tab, threadIdx.x, BS);
+    __syncthreads();
+  }
+  pdl_wait();
+  pdl_next();
   constexpr bool STAGE = sizeof(R) == 4 && D == 2;
   using SL = MarchStage<TX>;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -993,8 +957,10 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
   const R sys = py ? R(0.5) : R(-0.5);
   const R epsx = R(1.e-7 * g.dx), epsy = R(1.e-7 * g.dy);
   const bool shak = s.coll == COLL_SHAKHOV;
-  const double ds = D == 1 ? g.dx : g.dx * g.dy;
   const double Kf = g.Kb;
+  const FC* fct;
+  if constexpr (sizeof(R) == 4) fct = s.fc;
+  else fct = s.fc64;
 
   bool exx[TX + 4];
   int rx[TX + 4];
@@ -1033,13 +999,13 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
     const int r = j - j0;
     return smem + SL::Y0 + ((r / MARCH_CH) & 1) * SL::BUF + (r % MARCH_CH) * SL::ROW;
   };
-  auto xcoef = [&](int j) -> const FaceCoef32* {
-    if (STAGE) return (const FaceCoef32*)(stage_row(j) + SL::XF);
-    return s.fc + (long)j * (g.nx + 1) + i0;
+  auto xcoef = [&](int j) -> const FC* {
+    if (STAGE) return (const FC*)(stage_row(j) + SL::XF);
+    return fct + (long)j * (g.nx + 1) + i0;
   };
-  auto ycoef = [&](int j) -> const FaceCoef32* {  // y faces above row j
-    if (STAGE) return (const FaceCoef32*)(stage_row(j) + SL::YF);
-    return s.fc + s.nface_x + (long)(j + 1) * g.nx + i0;
+  auto ycoef = [&](int j) -> const FC* {  // y faces above row j
+    if (STAGE) return (const FC*)(stage_row(j) + SL::YF);
+    return fct + s.nface_x + (long)(j + 1) * g.nx + i0;
   };
   auto ccoef = [&](int j) -> const CellCoef32* {
     if (STAGE) return (const CellCoef32*)(stage_row(j) + SL::CC);
@@ -1061,8 +1027,7 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
       await(0);
       if (failed >= 0) j1 = j0;  // no rows: straight to the bounded clean-up
     }
-    const FaceCoef32* y0c =
-        STAGE ? (const FaceCoef32*)smem : s.fc + s.nface_x + (long)j0 * g.nx + i0;
+    const FC* y0c = STAGE ? (const FC*)smem : fct + s.nface_x + (long)j0 * g.nx + i0;
     const int rlo = slope_rule(g, 1, j0 - 1), rhi = slope_rule(g, 1, j0);
 #pragma unroll
     for (int c = 0; c < TX; ++c) {
@@ -1081,7 +1046,7 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
         su = vl_diff(rhi, wh[0][c], wh[1][c], wh[2][c], epsy);
         sb = vl_diff(rhi, wb[0][c], wb[1][c], wb[2][c], epsy);
       }
-      eval_face<D, FLUX>(e, MY, sys, hu, bu, su, sb, wh[1][c], wb[1][c], dt, fyh[c], fyb[c]);
+      eval_face<D, FLUX>(e, MY, sys, hu, bu, su, sb, wh[1][c], wb[1][c], tab, fyh[c], fyb[c]);
     }
   } else {
     tile(0, wh[1], wb[1]);
@@ -1095,8 +1060,8 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
     const bool qx = SG == 0 ? px : (SG == 1 || SG == 2);
     const bool qy = SG == 0 ? py : (SG == 1 || SG == 3);
     const R qxs = qx ? R(0.5) : R(-0.5), qys = qy ? R(0.5) : R(-0.5);
-    const FaceCoef32* xc = xcoef(j);
-    const FaceCoef32* yc = ycoef(j);
+    const FC* xc = xcoef(j);
+    const FC* yc = ycoef(j);
     const CellCoef32* cc = ccoef(j);
     // prefetch the next window row and the next row's halo
     if (D == 2 && j + 1 < j1) {
@@ -1138,17 +1103,11 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
           su = slope<FAST>(rhi, wh[1][c], wh[2][c], wh[3][c], epsy);
           sb = slope<FAST>(rhi, wb[1][c], wb[2][c], wb[3][c], epsy);
         }
-        eval_face<D, FLUX, FAST>(e, MY, qys, hu, bu, su, sb, wh[1][c], wb[1][c], dt, fyh2[c],
+        eval_face<D, FLUX, FAST>(e, MY, qys, hu, bu, su, sb, wh[1][c], wb[1][c], tab, fyh2[c],
                                  fyb2[c]);
       }
     }
-    // x slopes of cells w = 1 .. TX+2 and the x faces of row j
-    R dh[TX + 2], db[TX + 2];
-#pragma unroll
-    for (int w = 1; w <= TX + 2; ++w) {
-      dh[w - 1] = slope<FAST>(rx[w], xh[w - 1], xh[w], xh[w + 1], epsx);
-      db[w - 1] = slope<FAST>(rx[w], xb[w - 1], xb[w], xb[w + 1], epsx);
-    }
+    // x faces of row j, each with the upwind cell's slope
     R fxh[TX + 1], fxb[TX + 1];
 #pragma unroll
     for (int f = 0; f <= TX; ++f) {
@@ -1156,13 +1115,14 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
       e.kind = 0;
       const int fi = i0 + f;
       if (FAST || f <= ncol) face_load<FAST>(e, s, j * (g.nx + 1) + fi, xc[f], qx);
+      const int ru = FAST ? 1 : (qx ? rx[f + 1] : rx[f + 2]);
       R hu = qx ? xh[f + 1] : xh[f + 2];
       R bu = qx ? xb[f + 1] : xb[f + 2];
-      R su = qx ? dh[f] : dh[f + 1];
-      R sb = qx ? db[f] : db[f + 1];
+      R su = vl_diff(ru, qx ? xh[f] : xh[f + 1], hu, qx ? xh[f + 2] : xh[f + 3], epsx);
+      R sb = vl_diff(ru, qx ? xb[f] : xb[f + 1], bu, qx ? xb[f + 2] : xb[f + 3], epsx);
       R hc = fi == 0 ? xh[f + 2] : xh[f + 1];
       R bc = fi == 0 ? xb[f + 2] : xb[f + 1];
-      eval_face<D, FLUX, FAST>(e, MX, qxs, hu, bu, su, sb, hc, bc, dt, fxh[f], fxb[f]);
+      eval_face<D, FLUX, FAST>(e, MX, qxs, hu, bu, su, sb, hc, bc, tab, fxh[f], fxb[f]);
     }
     // update the cells of row j
     const long ro = (long)(j + g.ngy) * rows;
@@ -1180,8 +1140,8 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
         const CellCoef32 k = cc[c];
         relax(k, shak, u, vv, MX.c2, xh[c + 2], xb[c + 2], dhh, dbb, hn, bn);
       } else {
-        const CP<double> C = load_cp<double>(s, cell_index(g, i0 + c, j));
-        relax(C, ds, u, vv, Kf, D, xh[c + 2], xb[c + 2], dhh, dbb, hn, bn);
+        relax(s.cp[cell_index(g, i0 + c, j)], g.rds, u, vv, Kf, D, xh[c + 2], xb[c + 2], dhh, dbb, tab, hn,
+              bn);
       }
       if (vok) {
         Ho[ro + coff[c + 2]] = hn;
@@ -1295,6 +1255,8 @@ __global__ void __launch_bounds__(M3_BS) k_march3(const __grid_constant__ CUtens
                                                   const __grid_constant__ CUtensorMap tmb,
                                                   DevState sp, int RY) {
   static_assert(NS >= 6, "the ring holds the 4-row window plus at least one row ahead");
+  pdl_wait();
+  pdl_next();
   int lb;
   const int gr = group_member<GRP, GK_MARCH>(sp, lb);
   KB_GROUP_STATE(GRP, sp, gr);
@@ -1426,7 +1388,7 @@ __global__ void __launch_bounds__(M3_BS) k_march3(const __grid_constant__ CUtens
       hc = Hv(Si, w);
       bc = Bv(Si, w);
     }
-    eval_face<D, FLUX, FAST>(e, MY, sy, h0, b0, su, sb, hc, bc, 0.0, fh, fb);
+    eval_face<D, FLUX, FAST>(e, MY, sy, h0, b0, su, sb, hc, bc, nullptr, fh, fb);
   };
 
   float fyh[TX], fyb[TX];  // flux through the y faces below the current row
@@ -1475,7 +1437,7 @@ __global__ void __launch_bounds__(M3_BS) k_march3(const __grid_constant__ CUtens
         hc = Hv(Sj, fi == 0 ? f + 2 : f + 1);
         bc = Bv(Sj, fi == 0 ? f + 2 : f + 1);
       }
-      eval_face<D, FLUX, FAST>(e, MX, sx, xs[f + 1], xt[f + 1], su, sb, hc, bc, 0.0, fxh[f],
+      eval_face<D, FLUX, FAST>(e, MX, sx, xs[f + 1], xt[f + 1], su, sb, hc, bc, nullptr, fxh[f],
                                fxb[f]);
     }
     // relax and store the cells of row j
@@ -1587,8 +1549,8 @@ __device__ __forceinline__ void eval_face2(const FEv<float>& e, const Mono2& M, 
                                            float2 hu, float2 bu, float2 su, float2 sb,
                                            float2 hc, float2 bc, float2& fh, float2& fb) {
   if (!FAST && e.kind != 1) {
-    eval_face<D, FLUX>(e, M.lane(0), side.x, hu.x, bu.x, su.x, sb.x, hc.x, bc.x, 0.0, fh.x, fb.x);
-    eval_face<D, FLUX>(e, M.lane(1), side.y, hu.y, bu.y, su.y, sb.y, hc.y, bc.y, 0.0, fh.y, fb.y);
+    eval_face<D, FLUX>(e, M.lane(0), side.x, hu.x, bu.x, su.x, sb.x, hc.x, bc.x, nullptr, fh.x, fb.x);
+    eval_face<D, FLUX>(e, M.lane(1), side.y, hu.y, bu.y, su.y, sb.y, hc.y, bc.y, nullptr, fh.y, fb.y);
     return;
   }
   const float2 hf = f2fma(side, su, hu), bf = f2fma(side, sb, bu);
@@ -1647,6 +1609,8 @@ __global__ void __launch_bounds__(M4_THREADS * G, G == 2 ? 4 : 1) k_march4(const
                                                        const __grid_constant__ CUtensorMap tmb,
                                                        DevState s, int RY) {
   static_assert(NS >= 6, "the ring holds the 4-row window plus at least one row ahead");
+  pdl_wait();
+  pdl_next();
   using L = M3Layout<TX, NS>;
   constexpr int D = 2;
   extern __shared__ __align__(1024) unsigned char smem4[];
@@ -1800,8 +1764,8 @@ __global__ void __launch_bounds__(M4_THREADS * G, G == 2 ? 4 : 1) k_march4(const
         ea.Dd = (pya ? yc[cg + c].Dp : yc[cg + c].Dm);
         eb.C = (pyb ? yc[cg + c].Cp : yc[cg + c].Cm);
         eb.Dd = (pyb ? yc[cg + c].Dp : yc[cg + c].Dm);
-        eval_face<D, FLUX>(ea, MY.lane(0), sy.x, h0.x, b0.x, su.x, sb.x, 0.f, 0.f, 0.0, fh.x, fb.x);
-        eval_face<D, FLUX>(eb, MY.lane(1), sy.y, h0.y, b0.y, su.y, sb.y, 0.f, 0.f, 0.0, fh.y, fb.y);
+        eval_face<D, FLUX>(ea, MY.lane(0), sy.x, h0.x, b0.x, su.x, sb.x, 0.f, 0.f, nullptr, fh.x, fb.x);
+        eval_face<D, FLUX>(eb, MY.lane(1), sy.y, h0.y, b0.y, su.y, sb.y, 0.f, 0.f, nullptr, fh.y, fb.y);
         return;
       }
       e.C = cpa[0];
@@ -1881,9 +1845,9 @@ __global__ void __launch_bounds__(M4_THREADS * G, G == 2 ? 4 : 1) k_march4(const
           eb.C = (pxb ? xc[cg + f].Cp : xc[cg + f].Cm);
           eb.Dd = (pxb ? xc[cg + f].Dp : xc[cg + f].Dm);
           eval_face<D, FLUX>(ea, MX.lane(0), sx.x, xs[f + 1].x, xt[f + 1].x, su.x, sb.x, 0.f,
-                             0.f, 0.0, fxh[f].x, fxb[f].x);
+                             0.f, nullptr, fxh[f].x, fxb[f].x);
           eval_face<D, FLUX>(eb, MX.lane(1), sx.y, xs[f + 1].y, xt[f + 1].y, su.y, sb.y, 0.f,
-                             0.f, 0.0, fxh[f].y, fxb[f].y);
+                             0.f, nullptr, fxh[f].y, fxb[f].y);
           continue;
         }
         const float4* cp = pxa ? &xc[cg + f].Cp : &xc[cg + f].Cm;
@@ -1981,7 +1945,8 @@ static void mom_st_go(DevState& s, cudaStream_t st) {
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                          cudaSharedmemCarveoutMaxShared);
   });
-  kern<<<(unsigned)nblk, MOM_THREADS, SL::BYTES, st>>>(tm[0], tm[1], s);
+  void* args[] = {(void*)&tm[0], (void*)&tm[1], (void*)&s};
+  launch_after((const void*)kern, dim3((unsigned)nblk), dim3(MOM_THREADS), SL::BYTES, st, args);
 }
 
 template <typename R, int D, int FLUX, int TS>
@@ -1993,22 +1958,18 @@ static int mom_go(DevState& s, cudaStream_t st) {
     if (D == 2) mom_st_go<D, FLUX, TS, false, 1>(s, st);
     return D == 2 ? 2 : 1;
   }
-  int n = 0;
-  long wx = (long)((g.nx + TS - 1) / TS) * g.ny;
-  prefer_max_shared((const void*)k_mom<R, D, FLUX, TS, true, 0>);
-  prefer_max_shared((const void*)k_mom<R, D, FLUX, TS, false, 0>);
-  prefer_max_shared((const void*)k_mom<R, D, FLUX, TS, false, 1>);
-  if (s.coll == COLL_SHAKHOV)
-    k_mom<R, D, FLUX, TS, true, 0><<<nblk2(wx * 32, 128), 128, 0, st>>>(s);
-  else
-    k_mom<R, D, FLUX, TS, false, 0><<<nblk2(wx * 32, 128), 128, 0, st>>>(s);
-  ++n;
-  if (D == 2) {
-    long wy = (long)((g.ny + TS - 1) / TS) * g.nx;
-    k_mom<R, D, FLUX, TS, false, 1><<<nblk2(wy * 32, 128), 128, 0, st>>>(s);
-    ++n;
+  if constexpr (sizeof(R) == 8) {
+    void* args[] = {(void*)&s};
+    auto run = [&](auto kern, long warps) {
+      prefer_max_shared((const void*)kern);
+      launch_after((const void*)kern, dim3(nblk2(warps * 32, 128)), dim3(128), 0, st, args);
+    };
+    const long wx = (long)((g.nx + TS - 1) / TS) * g.ny, wy = (long)((g.ny + TS - 1) / TS) * g.nx;
+    if (s.coll == COLL_SHAKHOV) run(k_mom<D, FLUX, TS, true, 0>, wx);
+    else run(k_mom<D, FLUX, TS, false, 0>, wx);
+    if (D == 2) run(k_mom<D, FLUX, TS, false, 1>, wy);
   }
-  return n;
+  return D;
 }
 
 template <typename R, int D, int FLUX>
@@ -2021,13 +1982,14 @@ static int mom_t(DevState& s, cudaStream_t st) {
 }
 
 template <typename R, int D, int FLUX, int TX, int BS>
-static void march_go(DevState& s, double dt, cudaStream_t st) {
+static void march_go(DevState& s, cudaStream_t st) {
   const Geo& g = s.g;
   const int ry = s.tune[KB_TUNE_MARCH_RY] > 0 ? s.tune[KB_TUNE_MARCH_RY] : RY_MARCH;
   dim3 grid((g.nx + TX - 1) / TX, D == 2 ? (g.ny + ry - 1) / ry : 1, (g.nvel + BS - 1) / BS);
   const int smem = sizeof(R) == 4 && D == 2 ? MarchStage<TX>::BYTES : 0;
   prefer_max_shared((const void*)k_march<R, D, FLUX, TX, BS>);
-  k_march<R, D, FLUX, TX, BS><<<grid, BS, smem, st>>>(s, dt, ry);
+  void* args[] = {(void*)&s, (void*)&ry};
+  launch_after((const void*)k_march<R, D, FLUX, TX, BS>, grid, dim3(BS), smem, st, args);
 }
 
 // FP32 2D pass B (k_march3): the tensor maps of the current h / b buffers for
@@ -2054,7 +2016,8 @@ static void march3_go(DevState& s, cudaStream_t st) {
                          cudaSharedmemCarveoutMaxShared);
   });
   dim3 grid((g.nvel + M3_BS - 1) / M3_BS, (g.nx + TX - 1) / TX, (g.ny + ry - 1) / ry);
-  kern<<<grid, PAIR ? M4_THREADS * G : M3_BS, L::BYTES, st>>>(tm[0], tm[1], s, ry);
+  void* args[] = {(void*)&tm[0], (void*)&tm[1], (void*)&s, (void*)&ry};
+  launch_after((const void*)kern, grid, dim3(PAIR ? M4_THREADS * G : M3_BS), L::BYTES, st, args);
 }
 
 // FP32: the autotuned shapes (TX 2 or 4 columns, 64 or 128 threads);
@@ -2062,7 +2025,7 @@ static void march3_go(DevState& s, cudaStream_t st) {
 template <typename R, int D, int FLUX>
 static int march_t(DevState& s, double dt, cudaStream_t st) {
   if constexpr (sizeof(R) == 8) {
-    march_go<R, D, FLUX, 2, 64>(s, dt, st);
+    march_go<R, D, FLUX, 2, 64>(s, st);
   } else {
     const int tx = s.tune[KB_TUNE_MARCH_TX] > 0 ? s.tune[KB_TUNE_MARCH_TX] : TX_MARCH;
     const int bs = s.tune[KB_TUNE_MARCH_BS] > 0 ? s.tune[KB_TUNE_MARCH_BS] : 128;
@@ -2079,11 +2042,11 @@ static int march_t(DevState& s, double dt, cudaStream_t st) {
       }
     } else {
       if (tx == 2) {
-        if (bs == 64) march_go<R, D, FLUX, 2, 64>(s, dt, st);
-        else march_go<R, D, FLUX, 2, 128>(s, dt, st);
+        if (bs == 64) march_go<R, D, FLUX, 2, 64>(s, st);
+        else march_go<R, D, FLUX, 2, 128>(s, st);
       } else {
-        if (bs == 64) march_go<R, D, FLUX, 4, 64>(s, dt, st);
-        else march_go<R, D, FLUX, 4, 128>(s, dt, st);
+        if (bs == 64) march_go<R, D, FLUX, 4, 64>(s, st);
+        else march_go<R, D, FLUX, 4, 128>(s, st);
       }
     }
   }

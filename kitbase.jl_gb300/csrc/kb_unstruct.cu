@@ -39,6 +39,7 @@
 #include "../../include/kitgpu.h"
 #include "kb_device.cuh"
 #include "kb_kernels.cuh"
+#include "kb_tma.cuh"
 
 namespace kb {
 
@@ -69,12 +70,14 @@ struct UsDev {
   double* tmax;   // [1]
   double* residual;  // [4]
   int* status;
+  double hg, rmu;    // 0.5 / (gamma - 1), 1 / (2 mu_ref)
+  float Kbf, mu2f, om1f, prf;  // Kb, 2 mu_ref, 1 - omega, 0.8 (1 - Pr) in FP32
+  Pow64 tau_pow;     // lambda^(omega - 1) of the collision time
   double K, Kb, gamma, mu_ref, omega, Pr, umax, vmax;  // Kb = K (2F) or 0 (1F: b absent)
 };
 
 constexpr int US_T = 128;
 constexpr int US_W = US_T / 32;
-constexpr int US_BLK = 8;  // velocities summed plainly before a compensated flush
 
 // explicitly rounded arithmetic (never contracted), so that both cells of a
 // face form its flux and moments bit-identically
@@ -100,30 +103,6 @@ __device__ __forceinline__ float rfma(float a, float b, float c) { return __fmaf
 // Each face flux is formed with explicitly rounded operations (never
 // contracted) from the same inputs in both of its cells, so both see the
 // same per-velocity values.
-template <typename R>
-struct UsFace {
-  R n1, n2, a, l;  // flux = ((a vn) s) l: FP64 a = dt, l = len; FP32 a = dt len, l = 1
-  R sg, sgn;       // sg and sg |n|^2
-  int nb;          // the other cell
-  bool left;       // the cell is the face's first cell
-};
-
-template <typename R>
-__device__ __forceinline__ void us_flux(const UsFace<R>& F, R u, R v, R hc, R bc, R hn, R bn,
-                                        R& fh, R& fb) {
-  const R vn = rfma(u, F.n1, rmul(v, F.n2));
-  const bool own = (vn >= R(0)) == F.left;
-  const R hs = own ? hc : hn, bs = own ? bc : bn;
-  const R av = rmul(F.a, vn);
-  if (sizeof(R) == 8) {
-    fh = rmul(rmul(av, hs), F.l);
-    fb = rmul(rmul(av, bs), F.l);
-  } else {
-    fh = rmul(av, hs);
-    fb = rmul(av, bs);
-  }
-}
-
 constexpr int US_CB = 32;   // most cells of one CTA (one lane each in the cell phase)
 constexpr int US_NM = 8;    // block sums per cell: 5 moments, 2 heat-flux sums, 1 spare
 constexpr int US_NP = 16;   // per-cell parameters of the relaxation
@@ -137,7 +116,7 @@ __device__ __forceinline__ DF us_merge(DF a, DF b) { return df_merge(a, b); }
 __device__ __forceinline__ double us_shfl(double a, int m) { return __shfl_xor_sync(0xffffffffu, a, m); }
 __device__ __forceinline__ DF us_shfl(DF a, int m) { return df_shfl_xor(a, m); }
 __device__ __forceinline__ double us_value(double a) { return a; }
-__device__ __forceinline__ double us_value(DF a) { return (double)a.hi + (double)a.lo; }
+__device__ __forceinline__ double us_value(DF a) { return f64_of(a.hi) + f64_of(a.lo); }
 template <typename V>
 __device__ __forceinline__ double us_reduce8(const V (&x)[8], int lane) {
   const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
@@ -239,7 +218,7 @@ template <> struct UsGeoRow<double> { using T = UsG64; };
 // spill); the FP64 form 3.
 template <typename R, bool SHAK>
 __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
-    k_us_step(UsDev d, double dt, int cb, const R* __restrict__ hin,
+    k_us_step(UsDev d, double dt, int cb, int res, const R* __restrict__ hin,
                                                   const R* __restrict__ bin, R* __restrict__ hout,
                                                   R* __restrict__ bout) {
   using R2 = typename Vec2<R>::T;
@@ -252,6 +231,8 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
   GR* GS = (GR*)(D + (long)cb * 2 * d.vstride);  // [cb][3] face geometry
   int4* RS = (int4*)(GS + 3 * cb);               // [cb] cell and neighbours
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  // the exponential's table from L1: shared memory goes to the flux sums
+  const double* tab = EXP64_TAB;
   const int c0 = blockIdx.x * cb;
   const int nloc = min(cb, d.nstep - c0);
   const R2* U2 = (const R2*)(FAST ? (const void*)d.uf : (const void*)d.u);
@@ -267,33 +248,36 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
   // staged in shared memory first.
   us_stage_rec(d, c0, nloc, RS, GS);
   __syncthreads();
+  // up to here only what no step writes
+  pdl_wait();
+  pdl_next();
   for (int i = wid; i < nloc; i += US_W) {
     const int4 rec = RS[i];
     const int c = rec.x;
-    UsFace<R> F[3];
+    // per face: the outward normal (FP64: times dt len), dt len, |n|^2
+    R no[3][2], aa[3], nn[3];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       UsGeo<R> geo;
       us_geo(GS[3 * i + j], geo);
-      F[j].n1 = geo.n1;
-      F[j].n2 = geo.n2;
-      F[j].a = FAST ? rmul(rdt, geo.len) : R(dt);
-      F[j].l = FAST ? R(1) : geo.len;
-      F[j].sgn = geo.sgn;
-      F[j].left = geo.sgn > R(0);
-      F[j].sg = F[j].left ? R(1) : R(-1);
+      const bool left = geo.sgn > R(0);
+      aa[j] = rmul(rdt, geo.len);
+      nn[j] = fabs(geo.sgn);
+      no[j][0] = left ? geo.n1 : -geo.n1;
+      no[j][1] = left ? geo.n2 : -geo.n2;
+      if (!FAST) {
+        no[j][0] = rmul(aa[j], no[j][0]);
+        no[j][1] = rmul(aa[j], no[j][1]);
+      }
     }
-    F[0].nb = rec.y;
-    F[1].nb = rec.z;
-    F[2].nb = rec.w;
     const R2* Hc = (const R2*)(hin + (long)c * vs);
     const R2* Bc = (const R2*)(bin + (long)c * vs);
-    const R2* H0 = (const R2*)(hin + (long)F[0].nb * vs);
-    const R2* B0 = (const R2*)(bin + (long)F[0].nb * vs);
-    const R2* H1 = (const R2*)(hin + (long)F[1].nb * vs);
-    const R2* B1 = (const R2*)(bin + (long)F[1].nb * vs);
-    const R2* H2 = (const R2*)(hin + (long)F[2].nb * vs);
-    const R2* B2 = (const R2*)(bin + (long)F[2].nb * vs);
+    const R2* H0 = (const R2*)(hin + (long)rec.y * vs);
+    const R2* B0 = (const R2*)(bin + (long)rec.y * vs);
+    const R2* H1 = (const R2*)(hin + (long)rec.z * vs);
+    const R2* B1 = (const R2*)(bin + (long)rec.z * vs);
+    const R2* H2 = (const R2*)(hin + (long)rec.w * vs);
+    const R2* B2 = (const R2*)(bin + (long)rec.w * vs);
     R Uo = R(0), Vo = R(0);
     if (shak) {
       Uo = R(d.prim[4L * c + 1]);
@@ -301,20 +285,8 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
     }
     R2* Dh = (R2*)(D + (long)i * 2 * vs);
     R2* Db = (R2*)(D + (long)i * 2 * vs + vs);
-    R pp[US_NM];
     Acc<R> acc[US_NM];
-#pragma unroll
-    for (int k = 0; k < US_NM; ++k) pp[k] = R(0);
-    int blk = 0;
     if constexpr (FAST) {
-      float no[3][2], aa[3], nn[3];
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        no[j][0] = F[j].left ? F[j].n1 : -F[j].n1;
-        no[j][1] = F[j].left ? F[j].n2 : -F[j].n2;
-        aa[j] = F[j].a;
-        nn[j] = fabsf(F[j].sgn);
-      }
       float2 Pk[US_NM];
 #pragma unroll
       for (int k = 0; k < US_NM; ++k) Pk[k] = make_float2(0.f, 0.f);
@@ -368,44 +340,40 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
       for (int e = 0; e < 2; ++e) {
         const R u = e ? u2.y : u2.x, vv = e ? v2.y : v2.x, om = e ? w2.y : w2.x;
         const R hc = e ? hc2.y : hc2.x, bc = e ? bc2.y : bc2.x;
-        R fh0, fb0, fh1, fb1, fh2, fb2;
-        us_flux(F[0], u, vv, hc, bc, e ? h0.y : h0.x, e ? b0.y : b0.x, fh0, fb0);
-        us_flux(F[1], u, vv, hc, bc, e ? h1.y : h1.x, e ? b1.y : b1.x, fh1, fb1);
-        us_flux(F[2], u, vv, hc, bc, e ? h2.y : h2.x, e ? b2.y : b2.x, fh2, fb2);
-        const R dh = F[0].sg * fh0 + F[1].sg * fh1 + F[2].sg * fh2;
-        const R db = F[0].sg * fb0 + F[1].sg * fb1 + F[2].sg * fb2;
-        const R dn = F[0].sgn * fh0 + F[1].sgn * fh1 + F[2].sgn * fh2;
+        R dh = R(0), db = R(0), dn = R(0);
+        // outward flux a vo times the upwind value: the neighbour forms exactly
+        // the negated one
+        auto face = [&](int j, R hn, R bn) {
+          const R ao = rfma(u, no[j][0], rmul(vv, no[j][1]));
+          const bool own = nonneg64(ao);
+          const R fh = rmul(ao, own ? hc : hn), fb = rmul(ao, own ? bc : bn);
+          dh += fh;
+          db += fb;
+          dn = fma(nn[j], fh, dn);
+        };
+        face(0, e ? h0.y : h0.x, e ? b0.y : b0.x);
+        face(1, e ? h1.y : h1.x, e ? b1.y : b1.x);
+        face(2, e ? h2.y : h2.x, e ? b2.y : b2.x);
         if (e) { dh2.y = dh; db2.y = db; } else { dh2.x = dh; db2.x = db; }
         const R wn = om * dn;
-        pp[0] += om * dh;
-        pp[1] += u * wn;
-        pp[2] += vv * wn;
-        pp[3] += (u * u + vv * vv) * wn;
-        pp[4] += om * db;
+        acc[0].s = fma(om, dh, acc[0].s);
+        acc[1].s = fma(u, wn, acc[1].s);
+        acc[2].s = fma(vv, wn, acc[2].s);
+        acc[3].s = fma(fma(u, u, vv * vv), wn, acc[3].s);
+        acc[4].s = fma(om, db, acc[4].s);
         if (shak) {  // heat_flux 2F2V of the old state (src/Theory/theory_moments.jl:567-578)
           const R cu = u - Uo, cv = vv - Vo;
-          const R t = om * ((cu * cu + cv * cv) * hc + bc);
-          pp[5] += cu * t;
-          pp[6] += cv * t;
+          const R t = om * fma(fma(cu, cu, cv * cv), hc, bc);
+          acc[5].s = fma(cu, t, acc[5].s);
+          acc[6].s = fma(cv, t, acc[6].s);
         }
       }
       Dh[q] = dh2;
       Db[q] = db2;
-      if (++blk == US_BLK) {
-#pragma unroll
-        for (int k = 0; k < US_NM; ++k) {
-          acc[k].add(pp[k]);
-          pp[k] = R(0);
-        }
-        blk = 0;
-      }
     }
     decltype(acc[0].s) x[US_NM];
 #pragma unroll
-    for (int k = 0; k < US_NM; ++k) {
-      acc[k].add(pp[k]);
-      x[k] = acc[k].s;
-    }
+    for (int k = 0; k < US_NM; ++k) x[k] = acc[k].s;
     const double t = us_reduce8(x, lane);
     if ((lane & 3) == 0) S[i * US_NM + (lane >> 2)] = t;
   }
@@ -428,56 +396,59 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
         wo[k] = w[k];
         w[k] -= A[k] * ia;
       }
-      conserve_prim<FAST>(w, 4, d.gamma, pn);
+      conserve_prim<4>(w, d.hg, pn);
       for (int k = 0; k < 4; ++k) {
         p[k] = pn[k];
-        rr[k] = (w[k] - wo[k]) * (w[k] - wo[k]);
-        rr[4 + k] = fabs(w[k]);
+        if (res) {
+          const double dw = w[k] - wo[k];
+          rr[k] = dw * dw;
+          rr[4 + k] = fabs(w[k]);
+        }
       }
-      if (!(pn[0] > 0.0) || !(pn[3] > 0.0) || !isfinite(pn[0]) || !isfinite(pn[3])) atomicOr(d.status, 1);
+      if (!pos64(pn[0]) || !pos64(pn[3])) atomicOr(d.status, 1);
       R* Pc = P + lane * US_NP;
       if constexpr (FAST) {
         // The relaxation's FP32 coefficients are formed in FP32: FP64
         // division runs on GB300's slow FP64 pipe while the CTA's other
         // warps wait at the barrier.
-        const float rho = (float)pn[0], lam = (float)pn[3], Kb = (float)d.Kb;
-        const float tau = (float)(2.0 * d.mu_ref) * powf(lam, (float)(1.0 - d.omega)) / rho;
-        const float k = (float)dt / tau;
+        const float rho = f32_of(pn[0]), lam = f32_of(pn[3]), Kb = d.Kbf;
+        const float tau = d.mu2f * powf(lam, d.om1f) / rho;
+        const float k = rdt / tau;
         Pc[0] = rho * (lam * (float)(1.0 / PI));  // Maxwellian amplitude
-        Pc[1] = R(pn[1]);
-        Pc[2] = R(pn[2]);
+        Pc[1] = f32_of(pn[1]);
+        Pc[2] = f32_of(pn[2]);
         Pc[3] = lam;
         Pc[4] = Kb / (2.f * lam);  // B / H
         Pc[5] = k;
         Pc[6] = 1.f / (1.f + k);
-        Pc[7] = R(ia);
+        Pc[7] = f32_of(ia);
         if (shak) {  // shakhov 2F2V of the old state (src/Theory/theory_equilibrium.jl:227-238)
-          const float ro = (float)rho_o, lo = (float)lam_o;
-          const float sfac = (float)(0.8 * (1.0 - d.Pr)) * (lo * lo) / ro;
-          Pc[8] = sfac * 0.5f * (float)Sc[5];
-          Pc[9] = sfac * 0.5f * (float)Sc[6];
+          const float ro = f32_of(rho_o), lo = f32_of(lam_o);
+          const float sfac = d.prf * (lo * lo) / ro;
+          Pc[8] = sfac * 0.5f * f32_of(Sc[5]);
+          Pc[9] = sfac * 0.5f * f32_of(Sc[6]);
           Pc[10] = ro * (lo * (float)(1.0 / PI));
           Pc[11] = Kb / (2.f * lo);
           Pc[12] = lo;
-          Pc[13] = R(U_o);
-          Pc[14] = R(V_o);
+          Pc[13] = f32_of(U_o);
+          Pc[14] = f32_of(V_o);
         }
       } else {
-        const double k = dt / vhs_time<FAST>(pn[0], pn[3], d.mu_ref, d.omega);
-        Pc[0] = R(pn[0] * (pn[3] / PI));  // Maxwellian amplitude
+        const double k = dt * d.rmu * pn[0] * pow_tab(pn[3], d.tau_pow, tab);
+        Pc[0] = R(pn[0] * (pn[3] * (1.0 / PI)));  // Maxwellian amplitude
         Pc[1] = R(pn[1]);
         Pc[2] = R(pn[2]);
-        Pc[3] = R(pn[3]);
-        Pc[4] = R(d.Kb / (2.0 * pn[3]));  // B / H
+        Pc[3] = R(EXP64_LOG2E * pn[3]);
+        Pc[4] = R(d.Kb * (0.5 * rcp64(pn[3])));  // B / H
         Pc[5] = R(k);
-        Pc[6] = R(1.0 / (1.0 + k));
+        Pc[6] = R(rcp64(1.0 + k));
         Pc[7] = R(ia);
         if (shak) {  // shakhov 2F2V of the old state (src/Theory/theory_equilibrium.jl:227-238)
-          const double sfac = 0.8 * (1.0 - d.Pr) * (lam_o * lam_o) / rho_o;
-          Pc[8] = R(sfac * 0.5 * Sc[5]);
-          Pc[9] = R(sfac * 0.5 * Sc[6]);
-          Pc[10] = R(rho_o * (lam_o / PI));
-          Pc[11] = R(d.Kb / (2.0 * lam_o));
+          // the heat-flux factors times the old Maxwellian's amplitude
+          const double sfac = 0.4 * (1.0 - d.Pr) * (lam_o * lam_o) * (lam_o * (1.0 / PI));
+          Pc[8] = R(sfac * Sc[5]);
+          Pc[9] = R(sfac * Sc[6]);
+          Pc[11] = R(d.Kb * (0.5 * rcp64(lam_o)));
           Pc[12] = R(lam_o);
           Pc[13] = R(U_o);
           Pc[14] = R(V_o);
@@ -486,8 +457,10 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
     }
     // residual partials of update! (src/Solver/solver_update.jl:465-467)
     // summed over the CTA's cells in a fixed order
-    const double t = us_reduce8(rr, lane);
-    if ((lane & 3) == 0) d.bres[8L * blockIdx.x + (lane >> 2)] = t;
+    if (res) {
+      const double t = us_reduce8(rr, lane);
+      if ((lane & 3) == 0) d.bres[8L * blockIdx.x + (lane >> 2)] = t;
+    }
   }
   __syncthreads();
 
@@ -541,18 +514,17 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
       for (int e = 0; e < 2; ++e) {
         const R u = e ? u2.y : u2.x, vv = e ? v2.y : v2.x;
         const R du = u - U, dv = vv - V;
-        R MH = rn * mexp(-lam * (du * du + dv * dv));
+        R MH = rn * exp2_tab(lam, fma(du, du, dv * dv), tab);  // lam: EXP64_LOG2E lambda
         R MB = MH * cB;
         if (shak) {
-          const R cu = u - Uo, cv = vv - Vo, c2 = cu * cu + cv * cv;
-          const R MHo = orn * mexp(-olam * c2), MBo = MHo * ocB;
-          const R fq = fq0 * cu + fq1 * cv;
-          const R tl = R(2) * olam * c2;
-          MH += fq * (tl + Km5) * MHo;
-          MB += fq * (tl + Km3) * MBo;
+          const R cu = u - Uo, cv = vv - Vo, c2 = fma(cu, cu, cv * cv);
+          const R fq = fma(fq0, cu, fq1 * cv) * exp2_tab(EXP64_LOG2E * olam, c2, tab);
+          const R tl = fma(R(2) * olam, c2, Km3);
+          MH = fma(fq, tl - R(2), MH);
+          MB = fma(fq * tl, ocB, MB);
         }
-        const R hn = ((e ? hc2.y : hc2.x) - (e ? dh2.y : dh2.x) * ia + kk * MH) * i1k;
-        const R bn = ((e ? bc2.y : bc2.x) - (e ? db2.y : db2.x) * ia + kk * MB) * i1k;
+        const R hn = fma(kk, MH, fma(e ? dh2.y : dh2.x, -ia, e ? hc2.y : hc2.x)) * i1k;
+        const R bn = fma(kk, MB, fma(e ? db2.y : db2.x, -ia, e ? bc2.y : bc2.x)) * i1k;
         if (e) { ho.y = hn; bo.y = bn; } else { ho.x = hn; bo.x = bn; }
       }
       Ho[q] = ho;
@@ -572,6 +544,8 @@ template <typename R>
 __global__ void __launch_bounds__(US_T) k_us_avg(UsDev d, int first, const R* __restrict__ hin,
                                                  const R* __restrict__ bin, R* hout, R* bout) {
   const int c = d.avg_list[first + blockIdx.x];
+  pdl_wait();
+  pdl_next();
   int id[2] = {c, c}, m = 0;
   for (int j = 0; j < 3; ++j)
     if (d.cell_nb[3 * c + j] != -1 && m < 2) id[m++] = d.cell_nb[3 * c + j];
@@ -579,7 +553,7 @@ __global__ void __launch_bounds__(US_T) k_us_avg(UsDev d, int first, const R* __
     double* w = d.w + 4L * c;
     for (int k = 0; k < 4; ++k) w[k] = 0.5 * (d.w[4L * id[0] + k] + d.w[4L * id[1] + k]);
     double pn[4];
-    conserve_prim<false>(w, 4, d.gamma, pn);
+    conserve_prim<4>(w, d.hg, pn);
     for (int k = 0; k < 4; ++k) d.prim[4L * c + k] = pn[k];
   }
   const long vs = d.vstride;
@@ -602,6 +576,8 @@ __global__ void __launch_bounds__(US_T) k_us_avg(UsDev d, int first, const R* __
 __global__ void __launch_bounds__(256) k_us_residual(UsDev d, int nblk) {
   __shared__ double red[8][256];
   double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  pdl_wait();
+  pdl_next();
   for (int b = threadIdx.x; b < nblk; b += 256)
     for (int k = 0; k < 8; ++k) a[k] += d.bres[8L * b + k];
   for (int k = 0; k < 8; ++k) red[k][threadIdx.x] = a[k];
@@ -833,9 +809,16 @@ extern "C" int kb_us_create(const kb_config_t* cfg, int32_t ncell, int32_t nface
   d.K = cfg->K;
   d.Kb = cfg->nf == 1 ? 0.0 : cfg->K;
   d.gamma = cfg->gamma;
+  d.hg = 0.5 / (cfg->gamma - 1.0);
+  d.rmu = 1.0 / (2.0 * cfg->mu_ref);
+  d.tau_pow = kb::pow64_of(cfg->omega - 1.0);
   d.mu_ref = cfg->mu_ref;
   d.omega = cfg->omega;
   d.Pr = cfg->Pr;
+  d.Kbf = float(d.Kb);
+  d.mu2f = float(2.0 * cfg->mu_ref);
+  d.om1f = float(1.0 - cfg->omega);
+  d.prf = float(0.8 * (1.0 - cfg->Pr));
   d.umax = cfg->umax;
   d.vmax = cfg->vmax;
   auto bail = [&](int rc) {
@@ -1027,7 +1010,7 @@ extern "C" int kb_us_timestep(kb_us_t* U, double cfl, double sim_time, double ma
 }
 
 template <typename R>
-static void us_enqueue_step(kb_us* U, double dt) {
+static void us_enqueue_step(kb_us* U, double dt, bool last) {
   const kb::UsDev& d = U->d;
   const R* hin = (const R*)U->h[U->cur];
   const R* bin = (const R*)U->b[U->cur];
@@ -1036,16 +1019,17 @@ static void us_enqueue_step(kb_us* U, double dt) {
   if (d.nstep) {
     const int grid = (d.nstep + U->cb - 1) / U->cb;
     U->nblk = grid;
-    if (d.coll == KB_COLL_SHAKHOV)
-      kb::k_us_step<R, true><<<grid, kb::US_T, U->smem, U->stream>>>(d, dt, U->cb, hin, bin, hout, bout);
-    else
-      kb::k_us_step<R, false><<<grid, kb::US_T, U->smem, U->stream>>>(d, dt, U->cb, hin, bin, hout, bout);
+    int res = last ? 1 : 0;
+    void* args[] = {(void*)&d, &dt, &U->cb, &res, &hin, &bin, &hout, &bout};
+    const void* fn = d.coll == KB_COLL_SHAKHOV ? (const void*)kb::k_us_step<R, true> : (const void*)kb::k_us_step<R, false>;
+    kb::launch_after(fn, dim3((unsigned)grid), dim3(kb::US_T), U->smem, U->stream, args);
     U->launches++;
   }
   for (size_t l = 0; l + 1 < U->level_first.size(); ++l) {
     const int n = U->level_first[l + 1] - U->level_first[l];
     if (n == 0) continue;
-    kb::k_us_avg<R><<<n, kb::US_T, 0, U->stream>>>(d, U->level_first[l], hin, bin, hout, bout);
+    void* args[] = {(void*)&d, &U->level_first[l], &hin, &bin, &hout, &bout};
+    kb::launch_after((const void*)kb::k_us_avg<R>, dim3((unsigned)n), dim3(kb::US_T), 0, U->stream, args);
     U->launches++;
   }
   U->cur ^= 1;
@@ -1056,11 +1040,12 @@ extern "C" int kb_us_step(kb_us_t* U, double dt, int32_t nsteps, double* residua
   const kb::UsDev& d = U->d;
   for (int s = 0; s < nsteps; ++s) {
     if (U->prec == KB_PREC_FP64)
-      us_enqueue_step<double>(U, dt);
+      us_enqueue_step<double>(U, dt, s == nsteps - 1);
     else
-      us_enqueue_step<float>(U, dt);
+      us_enqueue_step<float>(U, dt, s == nsteps - 1);
   }
-  kb::k_us_residual<<<1, 256, 0, U->stream>>>(d, U->nblk);
+  void* rargs[] = {(void*)&d, &U->nblk};
+  kb::launch_after((const void*)kb::k_us_residual, dim3(1), dim3(256), 0, U->stream, rargs);
   U->launches++;
   if (cudaStreamSynchronize(U->stream) != cudaSuccess)
     return usfail(KB_ERR_CUDA, std::string("kb_us_step: ") + cudaGetErrorString(cudaGetLastError()));
