@@ -323,6 +323,9 @@ int kb_create(const kb_config_t* cfg, const double* u, const double* v, const do
     fv[k] = (float)hv[k];
     fw[k] = (float)hw[k];
   }
+  g.tensor = c.dim == 2;
+  for (int k = 0; k < g.nvel && g.tensor; ++k)
+    g.tensor = hu[k] == hu[k % g.nu] && hv[k] == hv[k - k % g.nu];
   if (cudaMemcpy((void*)h->s.u, hu.data(), sizeof(double) * g.vstride, cudaMemcpyHostToDevice) ||
       cudaMemcpy((void*)h->s.v, hv.data(), sizeof(double) * g.vstride, cudaMemcpyHostToDevice) ||
       cudaMemcpy((void*)h->s.wt, hw.data(), sizeof(double) * g.vstride, cudaMemcpyHostToDevice) ||
@@ -473,11 +476,7 @@ int kb_upload_state(kb_handle_t* h, const double* w, const double* prim, const d
     KB_CUDA(cudaMemsetAsync(h->s.b[0], 0, (size_t)h->ncell * h->vstride * (h->s.prec == KB_PREC_FP64 ? 8 : 4),
                             h->stream));
   }
-  // both ping-pong buffers start equal: ghost cells of fix / Maxwell solves are
-  // never rewritten, so the second buffer must hold them too
-  size_t dist = (size_t)h->ncell * h->vstride * (h->s.prec == KB_PREC_FP64 ? 8 : 4);
-  KB_CUDA(cudaMemcpyAsync(h->s.h[1], h->s.h[0], dist, cudaMemcpyDeviceToDevice, h->stream));
-  KB_CUDA(cudaMemcpyAsync(h->s.b[1], h->s.b[0], dist, cudaMemcpyDeviceToDevice, h->stream));
+  KB_TRY(check_launch(h, kb::launch_ghost_dup(h->s, h->stream)));
   KB_TRY(sync(h));
   h->evolved = false;
   return KB_OK;
@@ -501,9 +500,6 @@ int kb_init_equilibrium(kb_handle_t* h, const double* w, const double* prim) {
   KB_CUDA(cudaMemsetAsync(h->s.status, 0, sizeof(int), h->stream));
   h->s.cur = 0;
   KB_TRY(check_launch(h, kb::launch_init_equilibrium(h->s, h->stream)));
-  size_t dist = (size_t)h->ncell * h->vstride * (h->s.prec == KB_PREC_FP64 ? 8 : 4);
-  KB_CUDA(cudaMemcpyAsync(h->s.h[1], h->s.h[0], dist, cudaMemcpyDeviceToDevice, h->stream));
-  KB_CUDA(cudaMemcpyAsync(h->s.b[1], h->s.b[0], dist, cudaMemcpyDeviceToDevice, h->stream));
   KB_TRY(sync(h));
   h->evolved = false;
   return KB_OK;

@@ -69,8 +69,8 @@ __global__ void k_batch_timestep(BatchDev B, const double* umax, double cfl, dou
   double m = 0.0;
   for (int i = threadIdx.x; i < nx; i += blockDim.x) {
     const double* p = B.prim + (B.cell_off[b] + i + ng) * 4;
-    double sos = pow(0.5 * B.gamma / p[2], 0.5);
-    m = fmax(m, (fmax(umax[b], fabs(p[1])) + sos) / B.dx[b]);
+    const double sos = sqrt64((0.5 * B.gamma) * rcp64(p[2]));
+    m = fmax(m, (fmax(umax[b], fabs(p[1])) + sos) * B.rdx[b]);
   }
   red[threadIdx.x] = m;
   __syncthreads();

@@ -40,6 +40,7 @@ struct Geo {
   // 2F models, 0 for the 1F models, which carry no b (src/Solver/step_1f.jl)
   double Kb;
   int nf;  // distributions per cell: 2 (h, b) or 1 (f, held in h; b stays 0)
+  int tensor;  // 2D velocity grid u[k] = u[k mod nu], v[k] = v[k - k mod nu]
   // formed once on the host (geo_consts): FP64 divisions are dear on the device
   double rdx, rdy;   // 1 / dx, 1 / dy
   double rds;        // 1 / cell size (dx, or dx dy)

@@ -908,10 +908,9 @@ __global__ void k_timestep(DevState s, double umax, double vmax, double* out) {
   for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
     int i = (int)(t % g.nx), j = (int)(t / g.nx);
     const double* p = s.prim + (long)cell_index(g, i, j) * 4;
-    double sos = pow(0.5 * g.gamma / p[g.NW - 1], 0.5);
-    double v;
-    if (g.D == 1) v = (fmax(umax, fabs(p[1])) + sos) / g.dx;
-    else v = (fmax(umax, fabs(p[1])) + sos) / g.dx + (fmax(vmax, fabs(p[2])) + sos) / g.dy;
+    const double sos = sqrt64((0.5 * g.gamma) * rcp64(p[g.NW - 1]));
+    double v = (fmax(umax, fabs(p[1])) + sos) * g.rdx;
+    if (g.D == 2) v = fma(fmax(vmax, fabs(p[2])) + sos, g.rdy, v);
     m = fmax(m, v);
   }
   red[threadIdx.x] = m;
@@ -926,26 +925,129 @@ __global__ void k_timestep(DevState s, double umax, double vmax, double* out) {
 
 // Equilibrium initial distributions of init_fvm (src/Solver/solver_init.jl:
 // 119-141, :285-325): h = maxwellian(u, prim) (src/Theory/theory_equilibrium.jl:
-// 8-25), b = h K / (2 lambda), for every cell incl. ghosts.  One block per cell.
+// 8-25), b = h K / (2 lambda), for every cell incl. ghosts into buffer 0, and
+// for ghost cells, which some boundaries never rewrite, into both buffers.
+// One block per cell.
+__device__ __forceinline__ bool ghost_cell(const Geo& g, long c) {
+  const int i = (int)(c % g.nxt) - g.ngx, j = (int)(c / g.nxt) - g.ngy;
+  return i < 0 || i >= g.nx || j < 0 || j >= g.ny;
+}
+constexpr int INIT_T = 128;
 template <typename R>
-__global__ void k_init_eq(DevState s, R* __restrict__ H, R* __restrict__ Bq) {
+__global__ void __launch_bounds__(INIT_T) k_init_eq(DevState s) {
   const Geo& g = s.g;
   const long c = blockIdx.x;
   const double* p = s.prim + c * 4;
   const double rho = p[0], U = p[1], V = g.D == 2 ? p[2] : 0.0, lam = p[g.NW - 1];
-  const double rn = g.D == 1 ? rho * sqrt(lam / PI) : rho * (lam / PI);
-  const double cB = g.Kb / (2.0 * lam);
-  const long vs = g.vstride;
-  for (int v = threadIdx.x; v < g.nvel; v += blockDim.x) {
+  const double rn = g.D == 1 ? rho * sqrt64(lam * (1.0 / PI)) : rho * (lam * (1.0 / PI));
+  const double cB = g.Kb * (0.5 * rcp64(lam)), l2 = EXP64_LOG2E * lam;
+  const int nb = ghost_cell(g, c) ? 2 : 1;
+  for (int v = threadIdx.x; v < g.nvel; v += INIT_T) {
     const double du = s.u[v] - U;
     double e = du * du;
     if (g.D == 2) {
       const double dv = s.v[v] - V;
-      e += dv * dv;
+      e = fma(dv, dv, e);
     }
-    const double M = rn * exp(-lam * e);
-    H[c * vs + v] = (R)M;
-    Bq[c * vs + v] = (R)(M * cB);
+    const double M = rn * exp2_tab(l2, e, EXP64_TAB), MB = M * cB;
+    for (int k = 0; k < nb; ++k) {
+      ((R*)s.h[k])[c * g.vstride + v] = (R)M;
+      ((R*)s.b[k])[c * g.vstride + v] = (R)MB;
+    }
+  }
+}
+// The same when the velocity grid is a product of nu and nv abscissae
+// (Geo::tensor): the Maxwellian is then a product too, so a cell takes nu + nv
+// exponentials instead of nu nv.  FP64: two products per point.  FP32: the
+// factors and K / (2 lambda) as pairs of floats, whose products carry about 47
+// bits before the one rounding to FP32, because the FP64 pipe would bound the
+// kernel (512^2 cells x 64^2 velocities: 49.6 ms with an FP64 exponential per
+// point, bound by writing h and b since).
+struct F2 {
+  float hi, lo;
+};
+__device__ __forceinline__ F2 f2_of(double x) {
+  F2 r;
+  r.hi = f32_of(x);
+  r.lo = f32_of(x - f64_of(r.hi));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  r.hi = __fmul_rn(a.hi, b.hi);
+  r.lo = fmaf(a.hi, b.hi, -r.hi) + fmaf(a.hi, b.lo, a.lo * b.hi);
+  return r;
+}
+template <typename R> struct InitPart;
+template <> struct InitPart<double> {
+  using T = double;
+  static __device__ double of(double x) { return x; }
+  static __device__ double mul(double a, double b) { return a * b; }
+  static __device__ double value(double a) { return a; }
+};
+template <> struct InitPart<float> {
+  using T = F2;
+  static __device__ F2 of(double x) { return f2_of(x); }
+  static __device__ F2 mul(F2 a, F2 b) { return f2_mul(a, b); }
+  static __device__ float value(F2 a) { return a.hi + a.lo; }
+};
+template <typename R>
+__global__ void __launch_bounds__(INIT_T) k_init_eq_product(DevState s) {
+  using IP = InitPart<R>;
+  using T = typename IP::T;
+  extern __shared__ __align__(16) unsigned char smi[];
+  const Geo& g = s.g;
+  const int nu = g.nu, nv = g.nvel / g.nu;
+  T* su = (T*)smi;    // rho lambda / pi exp(-lambda (u - U)^2)
+  T* sv = su + nu;    // exp(-lambda (v - V)^2)
+  const long c = blockIdx.x;
+  const double* p = s.prim + c * 4;
+  const double U = p[1], V = p[2], lam = p[3], l2 = EXP64_LOG2E * lam, rn = p[0] * (lam * (1.0 / PI));
+  const T cB = IP::of(g.Kb * (0.5 * rcp64(lam)));
+  for (int k = threadIdx.x; k < nu + nv; k += INIT_T) {
+    const bool first = k < nu;
+    const double d = first ? s.u[k] - U : s.v[(k - nu) * nu] - V;
+    const double e = exp2_tab(l2, d * d, EXP64_TAB);
+    su[k] = IP::of(first ? rn * e : e);  // sv follows su
+  }
+  __syncthreads();
+  const int nb = ghost_cell(g, c) ? 2 : 1;
+  const int di = INIT_T % nu, dj = INIT_T / nu;
+  int i = threadIdx.x % nu, j = threadIdx.x / nu;
+  for (int v = threadIdx.x; v < g.nvel; v += INIT_T) {
+    const T M = IP::mul(su[i], sv[j]);
+    const R h = IP::value(M), b = IP::value(IP::mul(M, cB));
+    for (int k = 0; k < nb; ++k) {
+      ((R*)s.h[k])[c * g.vstride + v] = h;
+      ((R*)s.b[k])[c * g.vstride + v] = b;
+    }
+    i += di;
+    j += dj;
+    if (i >= nu) {
+      i -= nu;
+      ++j;
+    }
+  }
+}
+// Ghost cells of buffer 0 into buffer 1 (after an upload); one block per ghost cell.
+template <typename R>
+__global__ void k_ghost_dup(DevState s) {
+  const Geo& g = s.g;
+  const int t = blockIdx.x, rows = 2 * g.ngy * g.nxt;
+  int i, j;
+  if (t < rows) {  // whole ghost rows
+    const int r = t / g.nxt;
+    i = t % g.nxt - g.ngx;
+    j = r < g.ngy ? r - g.ngy : g.ny + r - g.ngy;
+  } else {
+    const int q = t - rows, k = q % (2 * g.ngx);
+    j = q / (2 * g.ngx);
+    i = k < g.ngx ? k - g.ngx : g.nx + k - g.ngx;
+  }
+  const long o = (long)cell_index(g, i, j) * g.vstride;
+  for (int v = threadIdx.x; v < g.nvel; v += blockDim.x) {
+    ((R*)s.h[1])[o + v] = ((R*)s.h[0])[o + v];
+    ((R*)s.b[1])[o + v] = ((R*)s.b[0])[o + v];
   }
 }
 
@@ -1194,8 +1296,24 @@ int launch_timestep(const DevState& s, double umax, double vmax, double* out, cu
 }
 
 int launch_init_equilibrium(DevState& s, cudaStream_t st) {
-  if (s.prec == 0) k_init_eq<double><<<s.ncell, 128, 0, st>>>(s, (double*)s.h[0], (double*)s.b[0]);
-  else k_init_eq<float><<<s.ncell, 128, 0, st>>>(s, (float*)s.h[0], (float*)s.b[0]);
+  const Geo& g = s.g;
+  const size_t smem = 8 * (size_t)(g.nu + g.nvel / g.nu);
+  if (g.tensor && smem <= 48 * 1024) {
+    if (s.prec == 0) k_init_eq_product<double><<<s.ncell, INIT_T, smem, st>>>(s);
+    else k_init_eq_product<float><<<s.ncell, INIT_T, smem, st>>>(s);
+  } else if (s.prec == 0) {
+    k_init_eq<double><<<s.ncell, INIT_T, 0, st>>>(s);
+  } else {
+    k_init_eq<float><<<s.ncell, INIT_T, 0, st>>>(s);
+  }
+  return 1;
+}
+
+int launch_ghost_dup(DevState& s, cudaStream_t st) {
+  const int n = s.ncell - s.g.nx * s.g.ny;
+  if (n == 0) return 0;
+  if (s.prec == 0) k_ghost_dup<double><<<n, 128, 0, st>>>(s);
+  else k_ghost_dup<float><<<n, 128, 0, st>>>(s);
   return 1;
 }
 

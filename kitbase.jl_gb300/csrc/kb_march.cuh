@@ -122,6 +122,7 @@ __device__ __forceinline__ void store_fw(const DevState& s, A (*acc)[4], int lin
   double* out = s.fw + (long)fi * 4;
   const double* fwa = s.fp[fi].fwa;
   if (k == 3) S *= 0.5;
+  if constexpr (std::is_same<A, BAcc<float>>::value) S *= f64_of(s.fc[fi].T.x);  // sums over t3
   if (D == 1) {  // energy in slot 2
     if (k == 2) out[3] = 0.0;
     else out[k == 3 ? 2 : k] = fwa[k == 3 ? 2 : k] + S;
@@ -382,20 +383,17 @@ __global__ void __launch_bounds__(MOM_THREADS) k_mom_st(const __grid_constant__ 
   int rule[TS + 4];
 #pragma unroll
   for (int w = 0; w < TS + 4; ++w) rule[w] = slope_rule(g, DIR, p0w - 2 + w);
-  int fidx[TS + 1];
   bool act[TS + 1];
-  R t3[TS + 1], t4[TS + 1];
+  R ct[TS + 1];  // ratio of the transport coefficients (T.y is over the cell size)
 #pragma unroll
   for (int f = 0; f < TS + 1; ++f) {
     int p = p0w + f;
-    fidx[f] = DIR == 0 ? line * (g.nx + 1) + p : s.nface_x + p * g.nx + line;
-    act[f] = f < nf && s.kind[fidx[f]] == 1;
-    t3[f] = R(0);
-    t4[f] = R(0);
+    const int fi = DIR == 0 ? line * (g.nx + 1) + p : s.nface_x + p * g.nx + line;
+    act[f] = f < nf && s.kind[fi] == 1;
+    ct[f] = R(0);
     if (act[f]) {
-      const float4 T = s.fc[fidx[f]].T;  // transport coefficients, T.y over the cell size
-      t3[f] = T.x;
-      t4[f] = T.y;
+      const float4 T = s.fc[fi].T;
+      ct[f] = T.x > 0.f ? T.y / T.x : 0.f;
     }
   }
   R oU[TS], oV[TS];
@@ -442,8 +440,8 @@ __global__ void __launch_bounds__(MOM_THREADS) k_mom_st(const __grid_constant__ 
       bx[w] = Sw[SL::BOX + w * MOM_VC + vl];
     }
     const bool pos = SG == 0 ? un >= R(0) : SG == 1;
-    const R c2 = un * un + ut * ut;
-    const R un2 = un * un;
+    // moment weights of the flux un X (the face's factor t3 enters at the end)
+    const R ou = om * un, ou1 = ou * un, ot = ou * ut, oc = D == 2 ? fmaf(ot, ut, ou1 * un) : ou1 * un;
 #pragma unroll
     for (int f = 0; f < TS + 1; ++f) {
       if (FAST ? f == TS : !act[f]) continue;
@@ -484,25 +482,21 @@ __global__ void __launch_bounds__(MOM_THREADS) k_mom_st(const __grid_constant__ 
         su = pos ? sl : sr;
         sb = pos ? tl : tr;
       }
-      R hf = hu + (pos ? R(0.5) : R(-0.5)) * su;
-      R bf = bu + (pos ? R(0.5) : R(-0.5)) * sb;
-      R Th = t3[f] * un * hf - t4[f] * un2 * su;
-      R Tb = t3[f] * un * bf - t4[f] * un2 * sb;
-      R wT = om * Th;
-      acc[f][0].add(wT);
-      acc[f][1].add(wT * un);
-      if (D == 2) acc[f][2].add(wT * ut);
-      acc[f][3].add(wT * c2 + om * Tb);
+      // t3 un (q + side s) - t4 un^2 s = t3 un (q + (side - ct un) s)
+      const R k = fmaf(-ct[f], un, pos ? R(0.5) : R(-0.5));
+      const R X = fmaf(k, su, hu), Y = fmaf(k, sb, bu);
+      acc[f][0].p = fmaf(ou, X, acc[f][0].p);
+      acc[f][1].p = fmaf(ou1, X, acc[f][1].p);
+      if (D == 2) acc[f][2].p = fmaf(ot, X, acc[f][2].p);
+      acc[f][3].p = fmaf(oc, X, fmaf(ou, Y, acc[f][3].p));
     }
     if (SHAK) {
 #pragma unroll
       for (int c = 0; c < TS; ++c) {
-        R cu = u - oU[c];
-        R cv = vv - oV[c];
-        R c2o = cu * cu + cv * cv;
-        R hc = hx[c + 2], bc = bx[c + 2];
-        qa[c][0].add(om * cu * c2o * hc + om * cu * bc);
-        if (D == 2) qa[c][1].add(om * cv * c2o * hc + om * cv * bc);
+        const R cu = u - oU[c], cv = vv - oV[c];
+        const R t = om * fmaf(D == 2 ? fmaf(cu, cu, cv * cv) : cu * cu, hx[c + 2], bx[c + 2]);
+        qa[c][0].p = fmaf(cu, t, qa[c][0].p);
+        if (D == 2) qa[c][1].p = fmaf(cv, t, qa[c][1].p);
       }
     }
   };
@@ -1918,11 +1912,47 @@ __global__ void __launch_bounds__(M4_THREADS * G, G == 2 ? 4 : 1) k_march4(const
 
 // ----------------------------------------------------------- launch helpers
 
-constexpr int TS_MOM = 4;    // faces per warp in pass A
-constexpr int TX_MARCH = 4;  // columns per strip in pass B (FP32)
-constexpr int RY_MARCH = 32;
+constexpr int TX_MARCH = 4;  // columns per strip in pass B (FP32, 1D)
 
 static inline unsigned nblk2(long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
+
+// Launch shape of a pass: the caller's (kb_set_tuning) or, where that is 0, by
+// the size of the grid.
+struct Shape {
+  int tx, bs, ry, ts;
+};
+// Pass A: two faces per warp.  Four have half the warps and 30 more registers
+// a thread: 512^2 cells x 64^2 velocities 6.09 against 4.37 ms for both
+// directions, 64^2 x 28^2 113 against 46 us.
+// Pass B, FP32: two velocities per thread (4 columns, bs 64) unless nu is odd,
+// when pairs straddle two rows of the velocity grid and half of them take the
+// lane-by-lane path (131 x 97 cells x 37 x 29 velocities: 127 us with one
+// velocity per thread, 145 with two).  Rows per CTA: the most that leave some
+// 22 CTAs per multiprocessor (a CTA reads 4 halo rows for its ry rows, and the
+// last of too few long CTAs run alone): 64^2 x 28^2 ry 4 / 16 / 32: 41 / 51 /
+// 89 us, 128^2 x 48^2 ry 4 / 16 / 64: 265 / 240 / 285, 512^2 x 64^2 ry 8 / 64:
+// 6.72 / 6.14 ms.  When even 4 rows give fewer than two CTAs per
+// multiprocessor: 2 columns and one velocity per thread (16^2 x 48^2: 15.5
+// against 18.1 us).
+static inline Shape shape_of(const DevState& s) {
+  const Geo& g = s.g;
+  const auto cdiv = [](long a, long b) { return (a + b - 1) / b; };
+  Shape p = {s.tune[KB_TUNE_MARCH_TX], s.tune[KB_TUNE_MARCH_BS], s.tune[KB_TUNE_MARCH_RY], s.tune[KB_TUNE_MOM_TS]};
+  if (p.ts == 0) p.ts = 2;
+  if (s.prec == 0 || g.D == 1) {
+    if (p.tx == 0) p.tx = TX_MARCH;
+    if (p.bs == 0) p.bs = 128;
+    if (p.ry == 0) p.ry = 32;
+    return p;
+  }
+  const long boxes = cdiv(g.nvel, KB_TMA_VBOX);
+  const bool tiny = boxes * cdiv(g.nx, 4) * cdiv(g.ny, 4) < 2L * s.sm_count;
+  if (p.tx == 0) p.tx = tiny ? 2 : 4;
+  if (p.bs == 0) p.bs = tiny || g.nu % 2 != 0 ? 128 : 64;
+  for (int ry = 64; p.ry == 0; ry /= 2)
+    if (ry == 4 || boxes * cdiv(g.nx, p.tx) * cdiv(g.ny, ry) >= 22L * s.sm_count) p.ry = ry;
+  return p;
+}
 
 // FP32 pass A: one CTA (4 warps) per segment of 4 TS faces along a line;
 // its dynamic shared memory exceeds the default 48 KB for TS = 4, so the
@@ -1975,16 +2005,16 @@ static int mom_go(DevState& s, cudaStream_t st) {
 template <typename R, int D, int FLUX>
 static int mom_t(DevState& s, cudaStream_t st) {
   // 8: both face directions in one launch over row rings (2D FP32, BGK)
-  if (sizeof(R) == 4 && D == 2 && s.tune[KB_TUNE_MOM_TS] == 8 && s.coll == COLL_BGK && s.mpart)
-    return moments_ring(s, st);
-  if (s.tune[KB_TUNE_MOM_TS] == 2) return mom_go<R, D, FLUX, 2>(s, st);
-  return mom_go<R, D, FLUX, TS_MOM>(s, st);
+  const int ts = shape_of(s).ts;
+  if (sizeof(R) == 4 && D == 2 && ts == 8 && s.coll == COLL_BGK && s.mpart) return moments_ring(s, st);
+  if (ts == 2) return mom_go<R, D, FLUX, 2>(s, st);
+  return mom_go<R, D, FLUX, 4>(s, st);
 }
 
 template <typename R, int D, int FLUX, int TX, int BS>
 static void march_go(DevState& s, cudaStream_t st) {
   const Geo& g = s.g;
-  const int ry = s.tune[KB_TUNE_MARCH_RY] > 0 ? s.tune[KB_TUNE_MARCH_RY] : RY_MARCH;
+  int ry = shape_of(s).ry;
   dim3 grid((g.nx + TX - 1) / TX, D == 2 ? (g.ny + ry - 1) / ry : 1, (g.nvel + BS - 1) / BS);
   const int smem = sizeof(R) == 4 && D == 2 ? MarchStage<TX>::BYTES : 0;
   prefer_max_shared((const void*)k_march<R, D, FLUX, TX, BS>);
@@ -2000,7 +2030,7 @@ static void march3_go(DevState& s, cudaStream_t st) {
   constexpr bool PAIR = G > 0;  // G groups of 64 threads, two velocities each
   const Geo& g = s.g;
   using L = M3Layout<TX, NS>;
-  const int ry = s.tune[KB_TUNE_MARCH_RY] > 0 ? s.tune[KB_TUNE_MARCH_RY] : RY_MARCH;
+  int ry = shape_of(s).ry;
   const CUtensorMap* tm = (const CUtensorMap*)s.tmaps + ((TX == 4 ? 1 : 0) * 2 + s.cur) * 2;
   void (*kern)(CUtensorMap, CUtensorMap, DevState, int);
   if constexpr (PAIR) kern = k_march4<FLUX, TX, NS, G>;
@@ -2027,8 +2057,8 @@ static int march_t(DevState& s, double dt, cudaStream_t st) {
   if constexpr (sizeof(R) == 8) {
     march_go<R, D, FLUX, 2, 64>(s, st);
   } else {
-    const int tx = s.tune[KB_TUNE_MARCH_TX] > 0 ? s.tune[KB_TUNE_MARCH_TX] : TX_MARCH;
-    const int bs = s.tune[KB_TUNE_MARCH_BS] > 0 ? s.tune[KB_TUNE_MARCH_BS] : 128;
+    const Shape p = shape_of(s);
+    const int tx = p.tx, bs = p.bs;
     if constexpr (D == 2) {
       // bs 64: two velocities per thread, one 64-thread group per strip
       // (k_march4); tx 4 + bs 64 splits the strip between two groups; bs 128:

@@ -56,21 +56,29 @@ __device__ __forceinline__ float ma_reduce16(const float (&x)[16], int lane) {
   return r + __shfl_xor_sync(0xffffffffu, r, 1);
 }
 
-// Free-transport moments of one face for a velocity pair (k_mom_st's
-// per-velocity terms): Th = t3 un hf - t4 un^2 s, hf = hu +- s / 2, and
-// (sum w Th, sum w Th un, sum w Th ut, sum w (Th c^2 + Tb)).
-__device__ __forceinline__ float4 ma_moments(float t3, float t4, const Mono2& M, float2 side, float2 om,
+// Moment weights of a velocity pair in one face direction (k_mom_st's): om un
+// times 1, un, ut and c^2.
+struct MaWeight {
+  float2 o, o1, ot, oc;
+  __device__ __forceinline__ void set(float2 om, const Mono2& M) {
+    o = f2mul(om, M.un);
+    o1 = f2mul(o, M.un);
+    ot = f2mul(o, M.ut);
+    oc = f2fma(ot, M.ut, f2mul(o1, M.un));
+  }
+};
+// Free-transport moments of one face for a velocity pair, k_mom_st's
+// per-velocity terms: un X, X = q + (side - ct un) s; the face's factor t3
+// enters in k_mom_fin.
+__device__ __forceinline__ float4 ma_moments(float ct, const Mono2& M, const MaWeight& W, float2 side,
                                              float2 h0, float2 b0, float2 su, float2 sb) {
-  const float2 hf = f2fma(side, su, h0), bf = f2fma(side, sb, b0);
-  const float2 a = f2mul(f2s(t3), M.un);
-  const float2 c = f2mul(f2s(-t4), M.n2);
-  const float2 Th = f2fma(c, su, f2mul(a, hf));
-  const float2 Tb = f2fma(c, sb, f2mul(a, bf));
-  const float2 wT = f2mul(om, Th);
-  const float2 m1 = f2mul(wT, M.un), m2 = f2mul(wT, M.ut);
-  const float2 m3 = f2fma(wT, M.c2, f2mul(om, Tb));
-  return make_float4(wT.x + wT.y, m1.x + m1.y, m2.x + m2.y, m3.x + m3.y);
+  const float2 k = f2fma(f2s(-ct), M.un, side);
+  const float2 X = f2fma(k, su, h0), Y = f2fma(k, sb, b0);
+  const float2 m0 = f2mul(W.o, X), m1 = f2mul(W.o1, X), m2 = f2mul(W.ot, X);
+  const float2 m3 = f2fma(W.oc, X, f2mul(W.o, Y));
+  return make_float4(m0.x + m0.y, m1.x + m1.y, m2.x + m2.y, m3.x + m3.y);
 }
+__device__ __forceinline__ float ma_ratio(const float4& T) { return T.x > 0.f ? T.y / T.x : 0.f; }
 
 // G groups of 64 threads (two velocities each) split the strip's TX columns,
 // TX / G = 2 columns per group.
@@ -150,6 +158,9 @@ __global__ void __launch_bounds__(M4_THREADS * G, G == 2 ? 4 : 8)
   Mono2 MX, MY;
   MX.set(u, vv);
   MY.set(vv, make_float2(-u.x, -u.y));
+  MaWeight WX, WY;
+  WX.set(om, MX);
+  WY.set(om, MY);
   const bool pxa = u.x >= 0.f, pxb = u.y >= 0.f, pya = vv.x >= 0.f, pyb = vv.y >= 0.f;
   const float2 sx = make_float2(pxa ? 0.5f : -0.5f, pxb ? 0.5f : -0.5f);
   const float2 sy = make_float2(pya ? 0.5f : -0.5f, pyb ? 0.5f : -0.5f);
@@ -206,7 +217,7 @@ __global__ void __launch_bounds__(M4_THREADS * G, G == 2 ? 4 : 8)
       sb = slope2(ra, rb, bm, b0, bp, epsy);
     }
     const float4 T = ((const FaceCoef32*)(cslot(ql) + L::YF))[cg + c].T;
-    return ma_moments(T.x, T.y, MY, sy, om, h0, b0, su, sb);
+    return ma_moments(ma_ratio(T), MY, WY, sy, h0, b0, su, sb);
   };
   // moments of x face f (0 .. TXG) of the group in row j, window xs / xt
   auto xface = [&](int f, const float2* xs, const float2* xt, const FaceCoef32* xc,
@@ -221,7 +232,7 @@ __global__ void __launch_bounds__(M4_THREADS * G, G == 2 ? 4 : 8)
       sb = slope2(rxa[f + 1], rxb[f + 1], xt[f], xt[f + 1], xt[f + 2], epsx);
     }
     const float4 T = xc[cg + f].T;
-    return ma_moments(T.x, T.y, MX, sx, om, xs[f + 1], xt[f + 1], su, sb);
+    return ma_moments(ma_ratio(T), MX, WX, sx, xs[f + 1], xt[f + 1], su, sb);
   };
 
   // reduce a warp's 16 row values over its 64 velocities and write the
@@ -378,8 +389,9 @@ __global__ void k_mom_fin(DevState s, int nchunk) {
     d.hi = y.z; d.lo = y.w; a[3] = df_merge(a[3], d);
   }
   const FaceParam& P = s.fp[f];
-  const double S0 = (double)a[0].hi + a[0].lo, S1 = (double)a[1].hi + a[1].lo;
-  const double S2 = (double)a[2].hi + a[2].lo, S3 = (double)a[3].hi + a[3].lo;
+  const double t3 = f64_of(s.fc[f].T.x);
+  const double S0 = f64_total(a[0]) * t3, S1 = f64_total(a[1]) * t3, S2 = f64_total(a[2]) * t3,
+               S3 = f64_total(a[3]) * t3;
   const double fl0 = P.fwa[0] + S0, fl1 = P.fwa[1] + S1, fl2 = P.fwa[2] + S2;
   const double fl3 = P.fwa[3] + 0.5 * S3;
   double* out = s.fw + f * 4;

@@ -597,9 +597,9 @@ __global__ void k_us_tmax(UsDev d) {
   __shared__ double red[256];
   double m = 0.0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d.ncell; c += gridDim.x * blockDim.x) {
-    const double sos = pow(0.5 * d.gamma / d.prim[4L * c + 3], 0.5);
+    const double sos = sqrt64((0.5 * d.gamma) * rcp64(d.prim[4L * c + 3]));
     const double um = d.umax + sos, vm = d.vmax + sos;
-    m = fmax(m, sqrt(um * um + vm * vm) / d.cell_mindx[c]);
+    m = fmax(m, sqrt64(fma(um, um, vm * vm)) * rcp64(d.cell_mindx[c]));
   }
   red[threadIdx.x] = m;
   __syncthreads();

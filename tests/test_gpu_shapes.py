@@ -1,0 +1,56 @@
+"""The launch shapes a solve takes by its size (no kb_set_tuning), on both
+sides of each rule, against the oracle; and the device-built equilibrium on
+velocity grids that are and are not products."""
+import numpy as np
+import pytest
+
+import kitgpu
+from kitgpu.solver import Handle, initial_cells, kb_config
+from cases import cavity, oracle_for, quadrant, rho_u_t_error
+
+pytestmark = pytest.mark.gpu
+
+# grids of fewer than two CTAs per multiprocessor, of just more, with odd nu
+# (one velocity per thread), and long enough for more than 4 rows per CTA
+SHAPES = [("tiny", cavity(nx=9, ny=13, nu=12, nv=10)), ("tiny-odd", cavity(nx=20, ny=11, nu=13, nv=9)),
+          ("pairs", cavity(nx=32, ny=33, nu=28, nv=28)), ("odd", cavity(nx=33, ny=30, nu=29, nv=28)),
+          ("rows", quadrant(nx=66, ny=150, nu=28, nv=28, flux="kfvs")),
+          ("rows-ugks", quadrant(nx=65, ny=130, nu=32, nv=32))]
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-12), ("fp32", 1e-5)])
+@pytest.mark.parametrize("name,cfg", SHAPES, ids=[c[0] for c in SHAPES])
+def test_default_shapes_against_oracle(gpu_lib, name, cfg, prec, tol):
+    KS, ctr, *faces, t = kitgpu.initialize(cfg, precision=prec)
+    orc = oracle_for(KS)
+    dt = kitgpu.timestep(KS, ctr, 0.0)
+    kitgpu.step(KS, ctr, dt, 3)
+    orc.step(dt, 3)
+    got, ref = ctr.handle.download(), orc.get_state()
+    assert max(rho_u_t_error(got["prim"], ref[1])) < tol
+    for k, x in (("h", ref[2]), ("b", ref[3])):
+        assert np.max(np.abs(got[k] - x)) < tol * np.max(np.abs(x)), k
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-14), ("fp32", 1.2e-7)])
+def test_equilibrium_on_any_velocity_grid(gpu_lib, prec, tol):
+    """A velocity grid in another order is no product of abscissae: the same
+    equilibrium, velocity by velocity (each value rounded once from 47 bits or
+    more), and the same in the ghost cells of both buffers."""
+    KS = kitgpu.solver_set(quadrant(nx=7, ny=6, nu=13, nv=10))
+    vs = KS.vs
+    u, v, w = (vs.flat(x) for x in (vs.u, vs.v, vs.weights))
+    perm = np.random.default_rng(1).permutation(len(u))
+    W, P = initial_cells(KS)
+    out = []
+    for order in (np.arange(len(u)), perm):
+        h = Handle(kb_config(KS, prec), u[order], v[order], w[order])
+        h.init_equilibrium(W, P)
+        s = h.download()
+        back = np.argsort(order)
+        out.append((s["h"][:, back], s["b"][:, back]))
+    l = P[:, 3:4]
+    H = P[:, :1] * (l / np.pi) * np.exp(-l * ((u[None] - P[:, 1:2]) ** 2 + (v[None] - P[:, 2:3]) ** 2))
+    for a in out:
+        for got, ref in zip(a, (H, H * KS.gas.K / (2.0 * l))):
+            assert np.max(np.abs(got - ref) / ref) < tol + 30 * 2 ** -52
