@@ -1934,17 +1934,37 @@ struct Shape {
 // 6.72 / 6.14 ms.  When even 4 rows give fewer than two CTAs per
 // multiprocessor: 2 columns and one velocity per thread (16^2 x 48^2: 15.5
 // against 18.1 us).
+// FP64: one warp nearly fills its quarter's FP64 pipe, so what counts is the
+// work of the busiest quarter (pass A: warps of ts faces) or multiprocessor
+// (pass B: CTAs of 4 x ry cells, 3 units a row and 1 for the first y faces).
+// Pass A, us, ts 2 / 4: 16^2 cells x 16^2 velocities 62 / 108, 40 x 90 x 13 x 30
+// 263 / 293, 64^2 x 28^2 620 / 554, 64^2 x 16^2 181 / 175.  Pass B, us, ry
+// 4 / 8 / 16 / 32, same order: 59 / 105 / 197 / 197, 402 / 417 / 512 / 423,
+// 1053 / 1033 / 1081 / 1248, 409 / 393 / 386 / 432; the rule is within 5 % of
+// the best of each.
 static inline Shape shape_of(const DevState& s) {
   const Geo& g = s.g;
   const auto cdiv = [](long a, long b) { return (a + b - 1) / b; };
   Shape p = {s.tune[KB_TUNE_MARCH_TX], s.tune[KB_TUNE_MARCH_BS], s.tune[KB_TUNE_MARCH_RY], s.tune[KB_TUNE_MOM_TS]};
-  if (p.ts == 0) p.ts = 2;
   if (s.prec == 0 || g.D == 1) {
+    const long sms = s.sm_count;
     if (p.tx == 0) p.tx = TX_MARCH;
     if (p.bs == 0) p.bs = 128;
-    if (p.ry == 0) p.ry = 32;
+    if (p.ts == 0) {
+      const auto cost = [&](int ts) { return cdiv(g.ny * cdiv(g.nx, ts), 4 * sms) * ts; };
+      p.ts = s.prec == 0 && cost(4) <= cost(2) ? 4 : 2;
+    }
+    if (p.ry == 0) {
+      const auto cost = [&](int ry) {
+        return cdiv(cdiv(g.nx, p.tx) * cdiv(g.ny, ry) * cdiv(g.nvel, p.bs), sms) * (3 * ry + 1);
+      };
+      p.ry = 32;
+      for (int ry = 16; ry >= 4; ry /= 2)
+        if (cost(ry) <= cost(p.ry)) p.ry = ry;
+    }
     return p;
   }
+  if (p.ts == 0) p.ts = 2;
   const long boxes = cdiv(g.nvel, KB_TMA_VBOX);
   const bool tiny = boxes * cdiv(g.nx, 4) * cdiv(g.ny, 4) < 2L * s.sm_count;
   if (p.tx == 0) p.tx = tiny ? 2 : 4;

@@ -32,11 +32,13 @@ def test_default_shapes_against_oracle(gpu_lib, name, cfg, prec, tol):
         assert np.max(np.abs(got[k] - x)) < tol * np.max(np.abs(x)), k
 
 
-@pytest.mark.parametrize("prec,tol", [("fp64", 1e-14), ("fp32", 1.2e-7)])
+@pytest.mark.parametrize("prec,tol", [("fp64", 0.0), ("fp32", 1.05 * 2 ** -24)])
 def test_equilibrium_on_any_velocity_grid(gpu_lib, prec, tol):
     """A velocity grid in another order is no product of abscissae: the same
-    equilibrium, velocity by velocity (each value rounded once from 47 bits or
-    more), and the same in the ghost cells of both buffers."""
+    equilibrium, velocity by velocity, in all cells.  On either side the
+    exponent x carries 2.5 roundings, so a value 2.5 x 2^-53, and 8 more
+    roundings follow; FP32 rounds it once more (values near 1e-36 have the low
+    halves of their products among the denormals: 5 % of a rounding)."""
     KS = kitgpu.solver_set(quadrant(nx=7, ny=6, nu=13, nv=10))
     vs = KS.vs
     u, v, w = (vs.flat(x) for x in (vs.u, vs.v, vs.weights))
@@ -50,7 +52,9 @@ def test_equilibrium_on_any_velocity_grid(gpu_lib, prec, tol):
         back = np.argsort(order)
         out.append((s["h"][:, back], s["b"][:, back]))
     l = P[:, 3:4]
-    H = P[:, :1] * (l / np.pi) * np.exp(-l * ((u[None] - P[:, 1:2]) ** 2 + (v[None] - P[:, 2:3]) ** 2))
+    x = l * ((u[None] - P[:, 1:2]) ** 2 + (v[None] - P[:, 2:3]) ** 2)
+    H = P[:, :1] * (l / np.pi) * np.exp(-x)
+    tol += 2 * (2.5 * x.max() + 8) * 2 ** -53
     for a in out:
         for got, ref in zip(a, (H, H * KS.gas.K / (2.0 * l))):
-            assert np.max(np.abs(got - ref) / ref) < tol + 30 * 2 ** -52
+            assert np.max(np.abs(got - ref) / ref) < tol
