@@ -156,6 +156,8 @@ struct kb_batch {
   cudaStream_t stream = nullptr;
   std::vector<void*> allocs;
   std::vector<int> nx, ng, nu, nus;
+  std::vector<double> dx, mu;
+  std::vector<long> vel_off_h;
   std::vector<long> cell_off, elem_off, dense_off;  // dense_off: caller layout [cell][nu]
   long ndense = 0, nseg = 0;
   double* d_stage = nullptr;
@@ -163,7 +165,7 @@ struct kb_batch {
   cudaGraphExec_t graph = nullptr;
   int graph_cur = -1, graph_launches = 0;
   int64_t launches = 0;
-  // FP32 segment kernel: shape (cells per segment, threads, persistent grid)
+  // FP32 segment kernel: shape (faces per CTA, threads, persistent grid)
   // and its launch; segment tables are rebuilt when the shape changes
   int seg = 16, seg_t = 128, persist = 0;
   const void* seg_fn = nullptr;
@@ -172,13 +174,12 @@ struct kb_batch {
   int* d_segi0 = nullptr;
   int* d_segfirst = nullptr;
   int* d_nseg = nullptr;
-  long seg_cap = 0;  // capacity of the segment tables (segments of 8 cells)
+  long seg_cap = 0;  // capacity of the segment tables (segments of 7 cells)
   // pool form (kb_pool_*): instance slots that requests join and leave, and
   // first-fit allocators of the cell, element and velocity ranges
   bool pool = false;
   std::vector<char> used;
   std::map<long, long> free_cells, free_elems, free_vels;  // offset -> length
-  std::vector<long> vel_off_h;
 };
 
 static int bfail(int code, const std::string& m) {
@@ -221,12 +222,17 @@ const std::vector<kb::SegVariant>& kb::seg_variants() {
 // consecutive).  Waits for the stream; invalidates the step graph.
 static int batch_tables(kb_batch* B, int seg) {
   std::vector<int> seg_b, seg_i0, seg_first(B->n), nseg(B->n);
+  std::vector<kb::SegDesc> seg_d;
   for (int b = 0; b < B->n; ++b) {
     seg_first[b] = (int)seg_b.size();
     nseg[b] = B->pool && !B->used[b] ? 0 : (B->nx[b] + seg - 1) / seg;
     for (int k = 0; k < nseg[b]; ++k) {
       seg_b.push_back(b);
       seg_i0.push_back(k * seg);
+      if (B->prec == KB_PREC_FP32)
+        seg_d.push_back({b, k * seg, B->nx[b], B->ng[b], B->nu[b], B->nus[b], (int)B->vel_off_h[b], 0,
+                         B->cell_off[b], B->elem_off[b], 1.0 / B->dx[b], float(1.e-7 * B->dx[b]),
+                         2.f * float(B->mu[b])});
     }
   }
   if ((long)seg_b.size() > B->seg_cap) return bfail(KB_ERR_ARG, "batch shape: segment table overflow");
@@ -234,6 +240,8 @@ static int batch_tables(kb_batch* B, int seg) {
   bool ok = true;
   ok &= cudaMemcpy(B->d_segb, seg_b.data(), sizeof(int) * seg_b.size(), cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(B->d_segi0, seg_i0.data(), sizeof(int) * seg_i0.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+  ok &= cudaMemcpy((void*)B->d.seg_d, seg_d.data(), sizeof(kb::SegDesc) * seg_d.size(), cudaMemcpyHostToDevice) ==
+        cudaSuccess;
   ok &= cudaMemcpy(B->d_segfirst, seg_first.data(), sizeof(int) * B->n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(B->d_nseg, nseg.data(), sizeof(int) * B->n, cudaMemcpyHostToDevice) == cudaSuccess;
   if (!ok) {
@@ -260,7 +268,7 @@ static int batch_set_shape(kb_batch* B, int seg, int threads, int persist) {
     if (v.seg == seg && v.threads == threads) var = &v;
   if (!var) return bfail(KB_ERR_ARG, "batch shape: no segment kernel for " + std::to_string(seg) +
                                          " cells x " + std::to_string(threads) + " threads");
-  int rc = batch_tables(B, seg);
+  int rc = batch_tables(B, var->cells);
   if (rc != KB_OK) return rc;
   bool ok = true;
   const int smem = var->smem(B->d.sst_max, B->d.nu4_max);
@@ -278,6 +286,7 @@ static int batch_set_shape(kb_batch* B, int seg, int threads, int persist) {
     cudaGetLastError();
     return bfail(KB_ERR_CUDA, "batch shape: kernel attributes refused");
   }
+  B->seg = seg;
   B->seg_t = threads;
   B->persist = persist ? 1 : 0;
   B->seg_fn = var->fn;
@@ -335,7 +344,7 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
     dx[b] = (x1[b] - x0[b]) / nx[b];
     rdx[b] = 1.0 / dx[b];
     rmu[b] = 1.0 / (2.0 * mu[b]);
-    seg_cap += (nx[b] + 7) / 8;  // the shortest segment length the tuner offers
+    seg_cap += (nx[b] + 6) / 7 + 1;  // the shortest segment length the tuner offers (a pool's members: one more)
   }
   int dev = 0, sms = 1;
   cudaGetDevice(&dev);
@@ -345,6 +354,9 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
     seg_cap = 0;
     for (int b = 0; b < n; ++b) seg_cap += (nx[b] + seg64 - 1) / seg64;
   }
+  B->dx = dx;
+  B->mu = mu;
+  B->vel_off_h.assign(vel_off.begin(), vel_off.end());
   B->ndense = dense;
   B->seg_cap = seg_cap;
   B->ncell = cells;
@@ -373,6 +385,7 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   BALLOC(d_nus, int, n);
   BALLOC(d_segb, int, B->seg_cap);
   BALLOC(d_segi0, int, B->seg_cap);
+  BALLOC(B->d.seg_d, const kb::SegDesc, B->prec == KB_PREC_FP32 ? B->seg_cap : 0);
   BALLOC(d_segfirst, int, n);
   BALLOC(d_nseg, int, n);
   BALLOC(d_respart, double, B->seg_cap * 8);
@@ -649,8 +662,8 @@ static int batch_launch(kb_batch* B, int cur, bool res) {
     const float* bin = (const float*)B->bq[cur];
     float* hout = (float*)B->h[cur ^ 1];
     float* bout = (float*)B->bq[cur ^ 1];
-    int slot = -1;
-    void* args[] = {(void*)&B->d, (void*)&hin, (void*)&bin, (void*)&hout, (void*)&bout, (void*)&slot};
+    int slot = -1, want = res;
+    void* args[] = {(void*)&B->d, (void*)&hin, (void*)&bin, (void*)&hout, (void*)&bout, (void*)&slot, (void*)&want};
     if (B->seg_grid > 0) {  // an empty pool has no segments
       kb::launch_after(B->seg_fn, dim3((unsigned)B->seg_grid), dim3((unsigned)B->seg_t),
                        (size_t)B->seg_smem, B->stream, args);
@@ -865,6 +878,8 @@ extern "C" int kb_pool_add(kb_batch_t* B, int32_t nx, int32_t ngx, int32_t nu, d
   B->elem_off[b] = eo;
   B->vel_off_h[b] = vo;
   const double dx = (x1 - x0) / nx;
+  B->dx[b] = dx;
+  B->mu[b] = mu_ref;
   bool ok = put1(B->d.nx, b, (int)nx) && put1(B->d.ng, b, (int)ngx) && put1(B->d.nu, b, (int)nu) &&
             put1(B->d.nus, b, (int)nus) && put1(B->d.cell_off, b, co) && put1(B->d.elem_off, b, eo) &&
             put1(B->d.vel_off, b, (int)vo) && put1(B->d.dx, b, dx) && put1(B->d.mu, b, mu_ref) &&

@@ -16,6 +16,17 @@
 
 namespace kb {
 
+// What a segment CTA needs before it can ask for its window, in one load.
+struct alignas(16) SegDesc {
+  int b, i0;              // instance, first cell
+  int nx, ng, nu, ns;     // the instance's (BatchDev)
+  int vo, pad;            // velocity table offset
+  long c0, e0;            // first cell, first distribution element
+  double rdx;             // 1 / dx
+  float epsd, mu2;        // 1e-7 dx, 2 mu
+};
+static_assert(sizeof(SegDesc) == 64, "four 16-byte loads");
+
 struct BatchDev {
   int n;                 // instances
   const int* nx;         // physical cells
@@ -54,6 +65,7 @@ struct BatchDev {
   // seg_first[b] (nseg[b] of them)
   const int* seg_b;
   const int* seg_i0;
+  const SegDesc* seg_d;  // FP32 kernel: the same and the instance's constants
   const int* seg_first;
   const int* nseg;
   double* respart;       // [segments][8] residual partial sums
@@ -78,15 +90,17 @@ inline void seg_gas(BatchDev& d) {
   d.tau_pow = pow64_of(d.omega - 1.0);
 }
 
-// van Leer slope times dx: one reciprocal and one multiply (subnormals
-// flushed), the division the FP32 passes of the 2D solver use as well
-__device__ __forceinline__ float bvl(float qm, float q0, float qp, float epsd) {
-  const float a = q0 - qm, b = qp - q0;
-  float r;
-  asm("div.approx.ftz.f32 %0, %1, %2;"
-      : "=f"(r)
-      : "f"(a * fabsf(b) + b * fabsf(a)), "f"(fabsf(a) + fabsf(b) + epsd));
-  return r;
+// Half the van Leer slope times dx from the differences a = q0 - qm and
+// b = qp - q0, two at once: (a |b| + b |a|) / (|a| + |b| + eps) is
+// 2 a b / (a + b +- eps) where a b > 0 and zero elsewhere (one reciprocal and
+// one multiply, subnormals flushed).
+__device__ __forceinline__ float2 bvl2(float2 a, float2 b, float eps) {
+  const float2 p = p2mul(a, b), d = p2add(a, b);
+  const float2 e = p2add(d, make_float2(copysignf(eps, d.x), copysignf(eps, d.y)));
+  float rx, ry;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rx) : "f"(e.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ry) : "f"(e.y));
+  return p2mul(make_float2(fmaxf(p.x, 0.f), fmaxf(p.y, 0.f)), make_float2(rx, ry));
 }
 
 // 1D slope rule: van Leer everywhere inside when ghosts exist, boundary cells
@@ -96,15 +110,6 @@ __device__ __forceinline__ int brule(int i, int nx, int ng) {
   if (ng == 0 && (i == 0 || i == nx - 1)) return 0;
   return 1;
 }
-
-// Blocked FP32 sum, flushed into a double-float accumulator.
-struct BSum {
-  float p;
-  DF d;
-  __device__ __forceinline__ void init() { p = 0.f; d.hi = d.lo = 0.f; }
-  __device__ __forceinline__ void add(float x) { p += x; }
-  __device__ __forceinline__ void flush() { df_add(d, p); p = 0.f; }
-};
 
 // e^x on the MUFU unit (2^(x log2 e), results below 2^-126 flushed to zero)
 __device__ __forceinline__ float fexp(float x) {
@@ -124,6 +129,15 @@ __device__ __forceinline__ float seg_maxwell(float u, float ulo, float rn, float
                                              float lam) {
   const float du = (u - Uh) + (ulo - Ul);
   return rn * fexp(-lam * du * du);
+}
+
+// Two at once, of the difference du and -lambda (the same roundings)
+__device__ __forceinline__ float2 seg_maxwell2(float2 du, float2 rn, float2 nlam) {
+  const float2 x = p2mul(p2mul(p2mul(nlam, du), du), p2s(1.4426950408889634f));
+  float2 y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(x.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(x.y));
+  return p2mul(rn, y);
 }
 
 // FP32 coefficients of one cell's Maxwellian from its FP64 prim [rho, U,
@@ -218,61 +232,79 @@ __device__ __forceinline__ void seg_clock_rate(const BatchDev& B, int slot, doub
 // the pointwise update all need only the old state inside that window, so
 // the step is one pass over HBM (each value read once, plus a 2-cell halo on
 // each side, and written once).  The window arrives by bulk async copies, one
-// per row, into rows whose stride is = 4 (mod 32) floats so that the face
+// per row, into rows whose stride is = 16 (mod 32) floats so that the face
 // threads read without bank conflicts.  Per-instance residuals are summed
 // by k_batch_seg_res after the step, in segment order (deterministic).
+//
+// What bounds it: instruction issue.  512 shock structures (115,000 cells of 48
+// to 200 velocities, 210 MB a step, 31 us of HBM) take 164 us a step: the face
+// moments about 65 (two thirds of it the exact sums), the pointwise update 54,
+// the FP64 cell warp 18, the window's latency the rest.  189 us before packed
+// pairs, one descriptor load in front of the window (five dependent ones took
+// 6,200 of a CTA's 36,000 cycles), sums merged by shuffles instead of by the
+// cell warp, and two chunks of cells per thread instead of one velocity per
+// thread (half the threads idle at 64 velocities).  At most 96 registers, five
+// CTAs per multiprocessor: 178 us with 80 (spills), 195 with 120 (four CTAs).
 constexpr int SEG_MAXNU = 256;
-constexpr int SEG_CC = 4;  // float4 coefficient blocks per cell
-__host__ __device__ inline int seg_stride(int nus) { return (nus + 31) / 32 * 32 + 4; }
-// Thread mapping of a segment CTA of SEG cells and T threads: FT threads per
-// face in the face-moment phase (SEG + 1 faces), then one warp of the CTA with
-// a lane per cell in the cell phase and beside it NWH warps with QT threads
-// per cell in the heat-flux phase, one thread per velocity in the pointwise
-// phase.
+constexpr int SEG_CC = 7;  // float4 coefficient blocks per pair of cells
+__host__ __device__ inline int seg_stride(int nus) { return (nus + 15) / 32 * 32 + 16; }
+// Thread mapping of a segment CTA of SEG cells and T threads: a group of FT
+// threads, a power of two, for each of the SEG + 1 faces in the face-moment
+// phase (its sums are merged by shuffles); then one warp with a lane per cell;
+// then one velocity and two chunks of cells per thread.
 template <int SEG, int T>
 struct SegShape {
   static constexpr int ROWS = SEG + 4;  // window cells
   static constexpr int FT = T / (SEG + 1);
-  static constexpr int QRAW = (T - 32) / SEG;
-  static constexpr int QT = QRAW >= 8 ? 8 : (QRAW >= 4 ? 4 : (QRAW >= 2 ? 2 : 1));
-  static constexpr int NWH = (QT * SEG + 31) / 32;
-  static constexpr int NV = 3 * (SEG + 1);  // face moments merged by the cell warp
-  static constexpr int ML = 8 * NV <= 32 ? 8 : (4 * NV <= 32 ? 4 : (2 * NV <= 32 ? 2 : 1));  // lanes for each
-  static_assert(SEG <= 32 && T % 32 == 0 && FT >= 1 && QRAW >= 1 && 1 + NWH <= T / 32,
+  static_assert(SEG <= 31 && (SEG + 1) % 4 == 0 && T >= 64 && FT * (SEG + 1) == T && FT >= 4 && FT <= 32 &&
+                    (FT & (FT - 1)) == 0,
                 "segment shape");
 };
 // Dynamic shared memory of a segment CTA, sized by the batch's largest row
-// stride and velocity count: h and b windows, velocity tables (hi, weight,
-// lo), fw, the 16-byte aligned cell coefficients, the face-moment partials,
-// the old w of the stepped cells and their old Maxwellian coefficients.
+// stride and velocity count: h and b windows, velocity tables (hi, lo,
+// weight), fw, the old w of the stepped cells, the coefficients of the cell
+// pairs, the old Maxwellian coefficients and the heat fluxes.
 template <int SEG, int T>
 __host__ __device__ inline int seg_smem(int sst_max, int nu4_max) {
-  return 2 * (SEG + 4) * sst_max * 4 + 3 * nu4_max * 4 + (SEG + 1) * 3 * 8 + 16 +
-         SEG * SEG_CC * 16 + T * 6 * 4 + SEG * 3 * 8 + SEG * 32 + 8 * 8;
+  return 2 * (SEG + 4) * sst_max * 4 + 3 * nu4_max * 4 + (SEG + 1) / 2 * SEG_CC * 16 + SEG * 32 +
+         (SEG + 1) * 3 * 8 + SEG * 3 * 8 + (SEG + 1) * 4;
 }
 template <int SEG, int T>
 __host__ __device__ inline int seg_smem_max() {
   return seg_smem<SEG, T>(seg_stride((SEG_MAXNU + 3) / 4 * 4), SEG_MAXNU);
 }
 
+// Sums of 4 values over a group of FT lanes: two levels that halve the values
+// a lane carries, then plain ones.  Lane q of the group returns the total of
+// value q / (FT / 4), merged in a fixed order.
+template <int FT>
+__device__ __forceinline__ DF seg_sums(DF (&x)[4], int lane) {
+  DF y[2];
+  const bool u1 = lane & (FT / 2), u0 = lane & (FT / 4);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) y[k] = df_merge(u1 ? x[2 + k] : x[k], df_shfl_xor(u1 ? x[k] : x[2 + k], FT / 2));
+  DF z = df_merge(u0 ? y[1] : y[0], df_shfl_xor(u0 ? y[0] : y[1], FT / 4));
+#pragma unroll
+  for (int m = FT / 8; m >= 1; m >>= 1) z = df_merge(z, df_shfl_xor(z, m));
+  return z;
+}
+
 // Segment k covers cells [seg_i0[k], seg_i0[k] + SEG) of instance seg_b[k].
 // A CTA takes segments k = blockIdx.x, blockIdx.x + gridDim.x, ...: one
 // segment each when the grid has a CTA per segment, or a persistent loop
 // when the grid is the number of CTAs that fit on the GPU at once.
-// slot: see BatchDev::clock (-1: the instances' own dt).
+// slot: see BatchDev::clock (-1: the instances' own dt).  res: the residual's
+// partial sums are wanted.
 template <int SEG, int SEG_T>
-__global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __restrict__ Hin,
-                                                     const float* __restrict__ Bin,
-                                                     float* __restrict__ Hout,
-                                                     float* __restrict__ Bout, int slot) {
+__global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
+    k_batch_seg(BatchDev B, const float* __restrict__ Hin, const float* __restrict__ Bin,
+                float* __restrict__ Hout, float* __restrict__ Bout, int slot, int res) {
   using SH = SegShape<SEG, SEG_T>;
   constexpr int SEG_ROWS = SH::ROWS;
-  constexpr int SEG_FT = SH::FT;
-  constexpr int QT = SH::QT;
+  constexpr int FT = SH::FT;
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ unsigned long long bar;
-  __shared__ float sconst[5];  // T3, T4, 1/dx, 1e-7 dx, 2 mu
-  __shared__ double srdx;      // 1/dx
+  __shared__ float sconst[2];  // T3, T4
   // An FP64 instruction holds a quarter of the multiprocessor for 64 cycles
   // whatever its active lanes, so the FP64 cell phase is one warp's, written
   // for few instructions (about 30; the divisions, conversions and compares
@@ -287,48 +319,32 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
   __syncthreads();
   unsigned phase = 0;  // completed window copies of this CTA (mbarrier parity)
   for (int k = blockIdx.x; k < B.nseg_all; k += gridDim.x) {
-  const int b = B.seg_b[k], i0 = B.seg_i0[k];
-  const int nx = B.nx[b], ng = B.ng[b], nu = B.nu[b], ns = B.nus[b];
+  const SegDesc sd = B.seg_d[k];
+  const int b = sd.b, i0 = sd.i0, nx = sd.nx, ng = sd.ng, nu = sd.nu, ns = sd.ns;
   const int i1 = min(i0 + SEG, nx);
-  const long c0 = B.cell_off[b], e0 = B.elem_off[b];
-  const float* Hi = Hin + e0;
-  const float* Bi = Bin + e0;
-  float* Ho = Hout + e0;
-  float* Bo = Bout + e0;
+  const long c0 = sd.c0;
+  const float* Hi = Hin + sd.e0;
+  const float* Bi = Bin + sd.e0;
+  float* Ho = Hout + sd.e0;
+  float* Bo = Bout + sd.e0;
   const int sst = seg_stride(ns);
+  // window rows r0 .. r1-1 (cells incl. ghosts), smem row = cell - r0
+  const int r0 = max(i0 - 2, -ng), r1 = min(i1 + 2, nx + ng), nrow = r1 - r0;
   float* sH = (float*)sm;
   float* sB = sH + SEG_ROWS * B.sst_max;
   float* sU = sB + SEG_ROWS * B.sst_max;
   float* sW = sU + B.nu4_max;
-  float* sUl = sW + B.nu4_max;               // low parts of the velocities
-  for (int v = tid; v < nu; v += SEG_T) {
-    sU[v] = B.uf[B.vel_off[b] + v];
-    sUl[v] = B.ul[B.vel_off[b] + v];
-    sW[v] = B.wtf[B.vel_off[b] + v];
-  }
+  float* sUl = sW + B.nu4_max;  // low parts of the velocities
+  // [(SEG + 1) / 2][SEG_CC] coefficients of cell pairs
+  float4* scc = (float4*)(sUl + B.nu4_max);
+  float4* smc = scc + (SEG + 1) / 2 * SEG_CC;  // [SEG][2] see B.mc
+  double* sfw = (double*)(smc + SEG * 2);      // [SEG + 1][3]
+  double* swo = sfw + (SEG + 1) * 3;           // [SEG][3] w
+  float* sq = (float*)(swo + SEG * 3);         // [SEG + 1] heat flux of the cell right of the face
   // up to here only what no step writes
   pdl_wait();
   pdl_next();
-  bool skip = !B.active[b];
-  if (slot >= 0) {
-    const SegClock c = seg_clock(B, slot);
-    skip = skip || c.stop;
-    if (k == 0 && tid == 0) seg_clock_next(B, slot, c);
-  }
-  if (skip) {  // converged or past the end: carry this segment's cells over
-    for (long t = tid; t < (long)(i1 - i0) * ns; t += SEG_T) {
-      const long o = (long)(i0 + ng) * ns + t;
-      Ho[o] = Hi[o];
-      Bo[o] = Bi[o];
-    }
-    __syncthreads();  // the velocity tables are reused by the next segment
-    continue;  // CTA-uniform
-  }
-  double* sfw = (double*)(sUl + B.nu4_max);  // [SEG + 1][3]
-  // [SEG][SEG_CC] float4 cell coefficients, 16-byte aligned
-  float4* scc = (float4*)(((unsigned long long)(sfw + (SEG + 1) * 3) + 15) & ~15ull);
-  // window rows r0 .. r1-1 (cells incl. ghosts), smem row = cell - r0
-  const int r0 = max(i0 - 2, -ng), r1 = min(i1 + 2, nx + ng), nrow = r1 - r0;
+  // The window first: it is on its way while the rest is read (one load deep).
   if (tid < 32) {
     if (lane == 0) mbar_expect(&bar, 2u * nrow * ns * 4u);
     __syncwarp();
@@ -339,29 +355,31 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
       bulk_g2s(dst, src, (unsigned)ns * 4u, &bar);
     }
   }
-  if (tid == 0) {
-    const double rdx0 = B.rdx[b], dt0 = slot >= 0 ? seg_clock(B, slot).dt : B.dt[b];
-    sconst[0] = f32_of(dt0);
-    sconst[1] = f32_of(0.5 * dt0 * dt0 * rdx0);
-    sconst[2] = f32_of(rdx0);
-    sconst[3] = f32_of(1.e-7 * B.dx[b]);
-    sconst[4] = f32_of(B.mu[b]) * 2.f;
-    srdx = rdx0;
+  bool skip = !B.active[b];
+  const int ca = max(i0, 1), cb = min(i1, nx - 1);  // stepped cells [ca, cb); may be none
+  const int ncell = cb - ca;
+  for (int v = tid; v < ns; v += SEG_T) {  // zero weight up to the row's end
+    sU[v] = v < nu ? B.uf[sd.vo + v] : 0.f;
+    sUl[v] = v < nu ? B.ul[sd.vo + v] : 0.f;
+    sW[v] = v < nu ? B.wtf[sd.vo + v] : 0.f;
   }
-  // the old w and Maxwellian coefficients of the stepped cells, while the
-  // window is on its way
-  const int fa = max(i0, 1), fb = min(i1, nx - 1);
-  const int ca = max(i0, 1), cb = min(i1, nx - 1);  // stepped cells [ca, cb)
-  float* sred = (float*)(scc + SEG * SEG_CC);  // [SEG_T][6]: face-moment DF partials
-  double* swo = (double*)(sred + SEG_T * 6);   // [SEG][3] w
-  float4* smc = (float4*)(((unsigned long long)(swo + SEG * 3) + 15) & ~15ull);  // [SEG][2] see B.mc
-  if (tid < cb - ca) {
+  if (tid < ncell) {  // old w and Maxwellian coefficients of the stepped cells
     const long c = c0 + ca + tid + ng;
     swo[tid * 3 + 0] = B.w[c * 4 + 0];
     swo[tid * 3 + 1] = B.w[c * 4 + 1];
     swo[tid * 3 + 2] = B.w[c * 4 + 2];
     smc[tid * 2] = ((const float4*)(B.mc + c * 8))[0];
     smc[tid * 2 + 1] = ((const float4*)(B.mc + c * 8))[1];
+  }
+  if (slot >= 0) {
+    const SegClock c = seg_clock(B, slot);
+    skip = skip || c.stop;
+    if (k == 0 && tid == 0) seg_clock_next(B, slot, c);
+  }
+  if (tid == SEG_T - 1) {
+    const double dt0 = slot >= 0 ? seg_clock(B, slot).dt : B.dt[b];
+    sconst[0] = f32_of(dt0);
+    sconst[1] = f32_of(0.5 * dt0 * dt0 * sd.rdx);
   }
   // one thread waits for the window; the others wait at the CTA barrier
   const bool ok = tid == 0 ? mbar_wait(&bar, phase & 1) : true;
@@ -373,123 +391,177 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
     return;
   }
   ++phase;
-  const float epsd = sconst[3];
+  const int dB = SEG_ROWS * B.sst_max;  // from a value of h to the same of b
+  if (skip) {  // converged or past the end: carry this segment's cells over
+    for (int i = i0; i < i1; ++i)
+      for (int v = tid; v < ns; v += SEG_T) {
+        Ho[(long)(i + ng) * ns + v] = sH[(i - r0) * sst + v];
+        Bo[(long)(i + ng) * ns + v] = sH[(i - r0) * sst + v + dB];
+      }
+    __syncthreads();  // the window is reused by the next segment
+    continue;  // CTA-uniform
+  }
+  const int fa = ca, fb = cb;  // faces fa .. fb: the left faces of the stepped cells and the last one's right face
+  const float epsd = sd.epsd;
   const float T3 = sconst[0], T4 = sconst[1];
-  auto rowH = [&](int c) { return sH + (c - r0) * sst; };
-  auto rowB = [&](int c) { return sB + (c - r0) * sst; };
-
-  // ---- face moments of faces fa .. fb: SEG_FT threads per face (velocities
-  // v = q mod SEG_FT), so the SEG + 1 faces keep all four warps busy
+  const bool shak = B.coll == COLL_SHAKHOV;
+  // The pointwise phase's split: a thread takes one velocity and two chunks of
+  // L cells in packed arithmetic.  Chunks of ceil(ncell / 2, 4, 8) cells: the
+  // one with the least rounds of the CTA times (cells + half a cell for the
+  // chunk's first face), so that 48 velocities fill 128 threads as well as 128
+  // or 160 do.
+  int L = (ncell + 1) >> 1, ngrp = 1;
   {
-    const int j = tid / SEG_FT, q = tid - j * SEG_FT;
+    int best = ((nu + SEG_T - 1) / SEG_T) * (2 * L + 1);
+#pragma unroll
+    for (int lg = 2; (1 << lg) <= (SEG < 7 ? SEG + 1 : 8); ++lg) {
+      const int l = (ncell + (1 << lg) - 1) >> lg, g = 1 << (lg - 1);
+      const int c = ((nu * g + SEG_T - 1) / SEG_T) * (2 * l + 1);
+      if (c < best) {
+        best = c;
+        L = l;
+        ngrp = g;
+      }
+    }
+  }
+
+  // ---- face moments of faces fa .. fb and heat flux of the cells right of
+  // them: FT threads per face (velocity pairs q mod FT).  A half-warp reads 16
+  // pairs: rows of 16 (mod 32) floats put two faces' pairs on all the banks.
+  {
+    const int j = tid / FT, q = tid % FT;
     const int f = fa + j;
     // Each moment term enters as an exact pair: the FP32 products w fh,
     // w fh u, w fh u^2, w fb with their rounding errors (FMA), added with
-    // error-free sums (TwoSum).  In a supersonic flow the energy flux is
-    // large and the flux difference between a cell's two faces small, so
-    // FP32 rounding of the terms or of running partial sums would enter w as
-    // a bias of relative size ~1e-7 of the flux every step -- amplified in
-    // T = 1 / (2 lambda) by the kinetic-to-thermal energy ratio (~35 at
-    // Mach 8), it grew to 1e-5 of T within a few hundred steps.
-    DF m0, m1, m2;
-    m0.hi = m0.lo = m1.hi = m1.lo = m2.hi = m2.lo = 0.f;
-    float l0 = 0.f, l1 = 0.f, l2 = 0.f;  // sums of the products' rounding errors
-    if (j <= SEG && f <= fb) {
+    // error-free sums (TwoSum), the two velocities in packed arithmetic.  In a
+    // supersonic flow the energy flux is large and the flux difference between
+    // a cell's two faces small, so FP32 rounding of the terms or of running
+    // partial sums would enter w as a bias of relative size ~1e-7 of the flux
+    // every step -- amplified in T = 1 / (2 lambda) by the kinetic-to-thermal
+    // energy ratio (~35 at Mach 8), it grew to 1e-5 of T within a few hundred
+    // steps.
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 s0 = zero, s1 = zero, s2 = zero, sb = zero, sq2 = zero;  // sums
+    float2 l0 = zero, l1 = zero, l2 = zero, lb = zero, lq = zero;  // their rounding errors
+    float2 e0 = zero, e1 = zero, e2 = zero;                        // and the products'
+    if (f <= fb) {
       const int iL = f - 1, iR = f;
-      const int rL = brule(iL, nx, ng), rR = brule(iR, nx, ng);
-      for (int v = q; v < nu; v += SEG_FT) {
-        const float u = sU[v];
-        const bool pos = u >= 0.f;
-        const int c = pos ? iL : iR;
-        const int r = pos ? rL : rR;
-        const float* hc = rowH(c);
-        const float* bc = rowB(c);
-        const float h0 = hc[v], b0 = bc[v];
-        float sh = 0.f, sb = 0.f;
-        if (r == 1) {
-          sh = bvl(hc[v - sst], h0, hc[v + sst], epsd);
-          sb = bvl(bc[v - sst], b0, bc[v + sst], epsd);
+      const bool vlL = brule(iL, nx, ng) == 1, vlR = brule(iR, nx, ng) == 1;
+      // window offsets of the three cells around the upwind one (clamped where
+      // the slope rule reads no neighbour): iL's for u >= 0, iR's otherwise
+      const int oL = (iL - r0) * sst, oR = (iR - r0) * sst;
+      const int oLL = (max(iL - 1, r0) - r0) * sst, oRR = (min(iR + 1, r1 - 1) - r0) * sst;
+      const bool hf = shak && j < ncell;
+      const float Uh = hf ? smc[j * 2].y : 0.f, Ul = hf ? smc[j * 2 + 1].x : 0.f;
+      float2 pq = zero;  // heat-flux terms, eight at a time
+      int it = 0;
+      for (int v = 2 * q; v < nu; v += 2 * FT, ++it) {
+        const float2 u = *(const float2*)(sU + v), w = *(const float2*)(sW + v);
+        const bool px = u.x >= 0.f, py = u.y >= 0.f;
+        const float* m = sH + (px ? oLL : oL) + v;
+        const float* c = sH + (px ? oL : oR) + v;
+        const float* r = sH + (px ? oR : oRR) + v;
+        float2 hm = *(const float2*)m, h0 = *(const float2*)c, hp = *(const float2*)r;
+        float2 bm = *(const float2*)(m + dB), b0 = *(const float2*)(c + dB), bp = *(const float2*)(r + dB);
+        if (px != py) {  // the one pair that straddles u = 0
+          m = sH + (py ? oLL : oL) + v + 1;
+          c = sH + (py ? oL : oR) + v + 1;
+          r = sH + (py ? oR : oRR) + v + 1;
+          hm.y = *m;
+          h0.y = *c;
+          hp.y = *r;
+          bm.y = m[dB];
+          b0.y = c[dB];
+          bp.y = r[dB];
         }
-        const float side = pos ? 0.5f : -0.5f;
-        const float hf = h0 + side * sh, bf = b0 + side * sb;
-        const float fh = T3 * u * hf - T4 * (u * u) * sh;
-        const float fbb = T3 * u * bf - T4 * (u * u) * sb;
-        // rounded products that the compiler may not fuse into a later add
-        // (a fused product would no longer match its error term)
-        const float wv = sW[v];
-        const float t0 = __fmul_rn(wv, fh), e0 = fmaf(wv, fh, -t0);  // w fh = t0 + e0 exactly
-        const float t1 = __fmul_rn(t0, u), e1 = fmaf(t0, u, -t1);
-        const float c1 = fmaf(e0, u, e1);                            // w fh u = t1 + c1
-        const float t2 = __fmul_rn(t1, u), e2 = fmaf(t1, u, -t2);
-        const float tb = __fmul_rn(wv, fbb), eb = fmaf(wv, fbb, -tb);
-        df_add(m0, t0);
-        df_add(m1, t1);
-        df_add(m2, t2);
-        df_add(m2, tb);
-        l0 += e0;
-        l1 += c1;
-        l2 += fmaf(c1, u, e2) + eb;                       // w (fh u^2 + fb) = t2 + tb + ...
+        const float2 sh = bvl2(p2sub(h0, hm), p2sub(hp, h0), epsd), sv = bvl2(p2sub(b0, bm), p2sub(bp, b0), epsd);
+        // T3 u (h0 +- s / 2) - T4 u^2 s = T3 u h0 + |u| (T3 / 2 - T4 |u|) s
+        const float2 au = make_float2(fabsf(u.x), fabsf(u.y));
+        const float2 Tu = p2mul(p2s(T3), u);
+        float2 cs = p2mul(au, p2fma(p2s(-2.f * T4), au, p2s(T3)));
+        cs.x = (px ? vlL : vlR) ? cs.x : 0.f;
+        cs.y = (py ? vlL : vlR) ? cs.y : 0.f;
+        const float2 fh = p2fma(Tu, h0, p2mul(cs, sh)), fbv = p2fma(Tu, b0, p2mul(cs, sv));
+        // rounded products and, negated, their errors: w fh = t0 - n0 exactly
+        const float2 nw = make_float2(-w.x, -w.y), nu2 = make_float2(-u.x, -u.y);
+        const float2 t0 = p2mul(w, fh), n0 = p2fma(nw, fh, t0);
+        const float2 tb = p2mul(w, fbv), nb = p2fma(nw, fbv, tb);
+        const float2 t1 = p2mul(t0, u), n1 = p2fma(n0, u, p2fma(nu2, t0, t1));  // w fh u = t1 - n1
+        const float2 t2 = p2mul(t1, u), n2 = p2add(p2fma(n1, u, p2fma(nu2, t1, t2)), nb);
+        p2df_add(s0, l0, t0);
+        p2df_add(s1, l1, t1);
+        p2df_add(s2, l2, t2);
+        p2df_add(sb, lb, tb);
+        e0 = p2add(e0, n0);
+        e1 = p2add(e1, n1);
+        e2 = p2add(e2, n2);  // w (fh u^2 + fb) = t2 + tb - n2
+        if (hf) {  // heat_flux 2F1V of cell iR: the row right of or at the upwind one
+          const float2 ul = *(const float2*)(sUl + v);
+          const float2 hc = make_float2(px ? hp.x : h0.x, py ? hp.y : h0.y);
+          const float2 bc = make_float2(px ? bp.x : b0.x, py ? bp.y : b0.y);
+          const float2 cu = p2add(p2sub(u, p2s(Uh)), p2sub(ul, p2s(Ul)));
+          pq = p2fma(p2mul(w, cu), p2fma(p2mul(cu, cu), hc, bc), pq);
+          if ((it & 7) == 7) {
+            p2df_add(sq2, lq, pq);
+            pq = zero;
+          }
+        }
       }
+      p2df_add(sq2, lq, pq);
     }
-    // each thread's pairs, merged per face below in thread order: both
-    // segments that share a face map it to the same threads q, so they
-    // compute bit-identical fw (conservation holds exactly)
-    float* o = sred + tid * 6;
-    o[0] = m0.hi;
-    o[1] = m0.lo + l0;
-    o[2] = m1.hi;
-    o[3] = m1.lo + l1;
-    o[4] = m2.hi;
-    o[5] = m2.lo + l2;
+    // merged over the face's threads in a fixed order: both segments that
+    // share a face map its velocities to the same threads q, so they compute
+    // bit-identical fw (conservation holds exactly)
+    const auto fold = [](float2 s, float2 lo) {
+      DF d;
+      d.hi = s.x;
+      d.lo = lo.x + lo.y;
+      df_add(d, s.y);
+      return d;
+    };
+    DF x[4] = {fold(s0, p2sub(l0, e0)), fold(s1, p2sub(l1, e1)), fold(s2, p2sub(p2add(l2, lb), e2)), fold(sq2, lq)};
+    df_add(x[2], sb.x);
+    df_add(x[2], sb.y);
+    const DF t = seg_sums<FT>(x, lane);
+    const int m = q / (FT / 4);
+    if (q % (FT / 4) == 0) {
+      const float half = m < 2 ? 1.f : 0.5f;
+      if (m < 3) sfw[j * 3 + m] = f64_of(half * t.hi) + f64_of(half * t.lo);
+      else sq[j] = half * (t.hi + t.lo);
+    }
   }
-  __syncthreads();  // face partials in shared memory
-  // The cell warp: merge the face moments, then the FP64 cell update; NWH other
-  // warps meanwhile: the old heat flux (Shakhov) of the stepped cells.
-  constexpr int NW = SEG_T / 32;
-  const int role = (wid + (int)(((unsigned)k * 2654435761u) >> 29)) % NW;
+  __syncthreads();  // face moments and heat fluxes in shared memory
+  // Coefficient block n of cell ca + j: the cells of a pair sit side by side
+  auto coef = [&](int j, int n) {
+    const int g = j / (2 * L), r = j - 2 * L * g;
+    const int hi = r >= L ? 1 : 0;
+    return (float*)(scc + (g * L + r - hi * L) * SEG_CC) + 2 * n + hi;
+  };
+  // The cell warp: the FP64 cell update.
+  const int role = (wid + (int)(((unsigned)k * 2654435761u) >> 29)) % (SEG_T / 32);
   if (role == 0) {
     // residual terms of the cell: a convergence monitor, summed in FP32 below
     float rr[6] = {0, 0, 0, 0, 0, 0};
     double rate = 0.0;  // CFL rate of the cell's new state (slot >= 0)
-    // face f = fa + jf, moment m: the SEG_FT partials of its threads, in order
-    // (ML lanes take every ML-th and join)
-    for (int r = 0; r < SH::NV; r += 32 / SH::ML) {
-      const int t0 = r + lane / SH::ML, ql = lane % SH::ML;
-      const int jf = t0 / 3, m = t0 - 3 * jf;
-      const float* o = sred + jf * SEG_FT * 6 + 2 * m;
-      const bool live = t0 < SH::NV && fa + jf <= fb;
-      DF d;
-      d.hi = live ? o[6 * ql] : 0.f;
-      d.lo = live ? o[6 * ql + 1] : 0.f;
-      for (int t = ql + SH::ML; live && t < SEG_FT; t += SH::ML) {
-        DF e;
-        e.hi = o[6 * t];
-        e.lo = o[6 * t + 1];
-        d = df_merge(d, e);
-      }
-#pragma unroll
-      for (int x = 1; x < SH::ML; x <<= 1) d = df_merge(d, df_shfl_xor(d, x));
-      const float half = m == 2 ? 0.5f : 1.f;
-      if (live && ql == 0) sfw[jf * 3 + m] = f64_of(half * d.hi) + f64_of(half * d.lo);
-    }
-    __syncwarp();
     // ---- cell parameters of the stepped cells (one lane per cell, FP64)
-    if (lane < cb - ca) {
-      const double rdx = srdx;
+    if (lane < ncell) {
+      const double rdx = sd.rdx;
       const int i = ca + lane;
       const long c = c0 + i + ng;
       double* w = B.w + c * 4;
       double* p = B.prim + c * 4;
-      const double* fL = sfw + (i - fa) * 3;
-      const double* fR = sfw + (i + 1 - fa) * 3;
+      const double* fL = sfw + lane * 3;
+      const double* fR = fL + 3;
       double wn[3];
 #pragma unroll
       for (int m = 0; m < 3; ++m) {
         const double d = fL[m] - fR[m];
         wn[m] = fma(d, rdx, swo[lane * 3 + m]);
-        const float df = f32_of(d) * sconst[2];  // the change of w
-        rr[m] = df * df;
-        rr[3 + m] = fabsf(f32_of(wn[m]));
+        if (res) {
+          const float df = f32_of(d) * f32_of(rdx);  // the change of w
+          rr[m] = df * df;
+          rr[3 + m] = fabsf(f32_of(wn[m]));
+        }
         w[m] = wn[m];
       }
       // conserve_prim (src/Theory/theory_macro.jl:185-206), hg = 0.5 / (gamma - 1)
@@ -513,132 +585,139 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
       // relaxation rate and is formed in FP32.
       SegMax mn;  // the new Maxwellian
       mn.set(pn, B.K);
-      const float tau = sconst[4] * powf(mn.lam, B.om1f) / f32_of(pn[0]);
+      const float tau = sd.mu2 * powf(mn.lam, B.om1f) / f32_of(pn[0]);
       const float dtt = sconst[0] / tau;
       // the old Maxwellian's coefficients are the ones this cell's update
       // formed from the same prim one step earlier (or the set-up formed from
       // the initial prim): read instead of recomputed
       const float4 mo = smc[lane * 2];
-      float4* kc = scc + lane * SEG_CC;
-      // new Maxwellian: density factor, U (hi), lambda, K / (2 lambda)
-      kc[0] = make_float4(mn.rn, mn.Uh, mn.lam, mn.cB);
-      // dt / tau, 1 / (1 + dt / tau), old Maxwellian (Shakhov) density factor and U (hi)
-      kc[1] = make_float4(dtt, 1.f / (1.f + dtt), mo.x, mo.y);
-      // old lambda, K / (2 lambda); .z (the Shakhov heat-flux factor) comes
-      // from the heat-flux warps; .w the low part of U
-      float* k2 = (float*)(kc + 2);
-      k2[0] = mo.z;
-      k2[1] = mo.w;
-      k2[3] = mn.Ul;
-      kc[3] = make_float4(smc[lane * 2 + 1].x, 0.f, 0.f, 0.f);
+      // new Maxwellian: density factor, U (hi, lo), -lambda, K / (2 lambda);
+      // dt / tau, 1 / (1 + dt / tau); old Maxwellian (Shakhov): density factor,
+      // U (hi, lo), -lambda, K / (2 lambda), and the heat-flux factor
+      // 0.8 (1 - Pr) lambda^2 / rho q of the old state
+      const float kc[13] = {mn.rn, mn.Uh, mn.Ul, -mn.lam, mn.cB, dtt, 1.f / (1.f + dtt),
+                            mo.x,  mo.y,  smc[lane * 2 + 1].x, -mo.z, mo.w,
+                            shak ? B.prf * (mo.z * mo.z) / f32_of(swo[lane * 3]) * sq[lane] : 0.f};
+      float* kp = coef(lane, 0);
+#pragma unroll
+      for (int n = 0; n < 13; ++n) kp[2 * n] = kc[n];
       seg_store_coef(B, c, mn);
     }
-    // residual partial sums of the segment, in a fixed shuffle order
+    if (res) {  // this segment's residual partial sums (k_batch_seg_res adds them up)
 #pragma unroll
-    for (int m = 0; m < 6; ++m) {
+      for (int m = 0; m < 6; ++m) {
 #pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) rr[m] += __shfl_xor_sync(0xffffffffu, rr[m], o);
-    }
-    // this segment's residual partial sums (k_batch_seg_res adds them up)
-    if (lane == 0) {
-      double* pr = B.respart + (long)k * 8;
-#pragma unroll
-      for (int m = 0; m < 6; ++m) pr[m] = f64_of(rr[m]);
-    }
-    if (slot >= 0) seg_clock_rate(B, slot, rate, c0, ng, i0, i1, nx, srdx, lane);
-  } else if (role <= SH::NWH) {
-    // ---- old heat flux of the stepped cells, QT threads per cell, and the
-    // Shakhov factor 0.8 (1 - Pr) lambda^2 / rho q of the cell coefficients
-    const int lt = (role - 1) * 32 + lane, jc = lt / QT, q = lt % QT;
-    const int i = ca + jc;
-    float qf = 0.f;
-    if (B.coll == COLL_SHAKHOV) {
-      BSum sm4;
-      sm4.init();
-      if (i < cb) {
-        const float Uc = smc[jc * 2].y, Ul = smc[jc * 2 + 1].x;  // U as an FP32 pair
-        const float* hc = rowH(i);
-        const float* bc = rowB(i);
-        int it = 0;
-        for (int v = q; v < nu; v += QT, ++it) {
-          const float cu = (sU[v] - Uc) + (sUl[v] - Ul);
-          sm4.add(sW[v] * cu * (cu * cu * hc[v] + bc[v]));
-          if ((it & 7) == 7) sm4.flush();
-        }
+        for (int o = 16; o >= 1; o >>= 1) rr[m] += __shfl_xor_sync(0xffffffffu, rr[m], o);
       }
-      sm4.flush();
-      DF d = sm4.d;
+      if (lane == 0) {
+        double* pr = B.respart + (long)k * 8;
 #pragma unroll
-      for (int m = 1; m < QT; m <<= 1) d = df_merge(d, df_shfl_xor(d, m));
-      if (i < cb) {
-        const float lof = smc[jc * 2].z;
-        qf = B.prf * (lof * lof) / f32_of(swo[jc * 3]) * (0.5f * (d.hi + d.lo));
+        for (int m = 0; m < 6; ++m) pr[m] = f64_of(rr[m]);
       }
     }
-    if (q == 0 && jc < SEG && i < cb) ((float*)(scc + jc * SEG_CC + 2))[2] = qf;
+    if (slot >= 0) seg_clock_rate(B, slot, rate, c0, ng, i0, i1, nx, sd.rdx, lane);
   }
   __syncthreads();  // cell coefficients ready for the pointwise update
-  // ---- pointwise KFVS flux + relaxation, one thread per velocity.  Every
-  // upwind cell of a segment away from ghost-less ends takes the van Leer
+  // ---- pointwise KFVS flux + relaxation: a thread marches two chunks of L
+  // cells at its velocity, in packed arithmetic, each window row read once.
+  // Every upwind cell of a segment away from ghost-less ends takes the van Leer
   // slope, so that form skips the per-face slope rule.
-  const float idx = sconst[2];
+  for (int v = tid; v < nu; v += SEG_T) {  // fixed end cells keep their state
+    if (i0 == 0) {
+      Ho[(long)ng * ns + v] = sH[(0 - r0) * sst + v];
+      Bo[(long)ng * ns + v] = sH[(0 - r0) * sst + v + dB];
+    }
+    if (i1 == nx) {
+      Ho[(long)(nx - 1 + ng) * ns + v] = sH[(nx - 1 - r0) * sst + v];
+      Bo[(long)(nx - 1 + ng) * ns + v] = sH[(nx - 1 - r0) * sst + v + dB];
+    }
+  }
+  const float2 idx = p2s(f32_of(sd.rdx));
   const bool all_vl = ng > 0 || (ca >= 2 && cb <= nx - 2);
   auto pointwise = [&](auto vl_tag) {
     constexpr bool VL = decltype(vl_tag)::value;
-    for (int v = tid; v < nu; v += SEG_T) {
-      const float u = sU[v], ulo = sUl[v];
+    for (int it = tid; it < nu * ngrp; it += SEG_T) {
+      int v = it, g = 0;
+      for (; v >= nu; ++g) v -= nu;
+      const int a0 = ca + 2 * L * g;                      // the chunks' first cells
+      const int nA = min(L, cb - a0), nB = cb - (a0 + L);  // and numbers (nB may be below 1 or above L)
+      if (nA <= 0) continue;
+      const float u = sU[v], au = fabsf(u);
       const bool pos = u >= 0.f;
-      const float side = pos ? 0.5f : -0.5f;
-      const float Tu = T3 * u, Tuu = T4 * (u * u);
-      if (i0 == 0) {  // fixed end cells keep their state
-        Ho[(long)ng * ns + v] = rowH(0)[v];
-        Bo[(long)ng * ns + v] = rowB(0)[v];
-      }
-      if (i1 == nx) {
-        Ho[(long)(nx - 1 + ng) * ns + v] = rowH(nx - 1)[v];
-        Bo[(long)(nx - 1 + ng) * ns + v] = rowB(nx - 1)[v];
-      }
-      // flux through face f, whose upwind cell row starts at hc / bc
-      auto face = [&](int f, const float* hc, const float* bc, float& fh, float& fbv) {
-        const float h0 = hc[0], b0 = bc[0];
-        float sh = 0.f, sb = 0.f;
-        if (VL || brule(pos ? f - 1 : f, nx, ng) == 1) {
-          sh = bvl(hc[-sst], h0, hc[sst], epsd);
-          sb = bvl(bc[-sst], b0, bc[sst], epsd);
+      const float2 Tu = p2s(T3 * u), cs = p2s(au * fmaf(-2.f * T4, au, T3));
+      const float2 u2 = p2s(u), ul2 = p2s(sUl[v]);
+      // the upwind cell of a chunk's first face and the rows around it; past
+      // the window's ends (no slope there, or beyond the second chunk's last
+      // cell) the row stays the end one
+      const int cA = a0 - (pos ? 1 : 0), cB = cA + L;
+      const int last = (r1 - 1 - r0) * sst;
+      const float* hv = sH + v;
+      int oA = (cA - r0) * sst, oB = min((cB - r0) * sst, last);
+      const int mA = VL ? oA - sst : max(oA - sst, 0), mB = min((cB - 1 - r0) * sst, last);
+      float2 hm = make_float2(hv[mA], hv[mB]), bm = make_float2(hv[mA + dB], hv[mB + dB]);
+      float2 h0 = make_float2(hv[oA], hv[oB]), b0 = make_float2(hv[oA + dB], hv[oB + dB]);
+      float2 dh = p2sub(h0, hm), db = p2sub(b0, bm);
+      float2 hp, bp, dhp, dbp;
+      // the flux out of the upwind cells (cA + k, cB + k); moves hp, bp one on
+      auto face = [&](int k, float2& fh, float2& fb) {
+        oA = VL ? oA + sst : min(oA + sst, last);
+        oB = min(oB + sst, last);
+        hp = make_float2(hv[oA], hv[oB]);
+        bp = make_float2(hv[oA + dB], hv[oB + dB]);
+        dhp = p2sub(hp, h0);
+        dbp = p2sub(bp, b0);
+        float2 c = cs;
+        if (!VL) {
+          c.x = brule(cA + k, nx, ng) == 1 ? c.x : 0.f;
+          c.y = brule(cB + k, nx, ng) == 1 ? c.y : 0.f;
         }
-        fh = Tu * (h0 + side * sh) - Tuu * sh;
-        fbv = Tu * (b0 + side * sb) - Tuu * sb;
+        fh = p2fma(Tu, h0, p2mul(c, bvl2(dh, dhp, epsd)));
+        fb = p2fma(Tu, b0, p2mul(c, bvl2(db, dbp, epsd)));
       };
-      if (ca >= cb) continue;
-      // hr / br: row of cell i at this velocity; the upwind cell of face i + 1
-      // is i (pos) or i + 1
-      const int up = pos ? 0 : sst;
-      const float* hr = rowH(ca) + v;
-      const float* br = rowB(ca) + v;
-      float fhL, fbL;
-      face(ca, hr - sst + up, br - sst + up, fhL, fbL);
-      float* ph = Ho + (long)(ca + ng) * ns + v;
-      float* pb = Bo + (long)(ca + ng) * ns + v;
-      const float4* kc = scc;
-      for (int i = ca; i < cb; ++i, hr += sst, br += sst, ph += ns, pb += ns, kc += SEG_CC) {
-        float fhR, fbR;
-        face(i + 1, hr + up, br + up, fhR, fbR);
-        const float4 k0 = kc[0], k1 = kc[1], k2 = kc[2];
-        const float h0 = hr[0], b0 = br[0];
-        const float M = seg_maxwell(u, ulo, k0.x, k0.y, k2.w, k0.z);
-        float MH = M, MB = M * k0.w;
-        if (B.coll == COLL_SHAKHOV) {
-          const float ou = (u - k1.w) + (ulo - kc[3].x);
-          const float OH = k1.z * fexp(-k2.x * ou * ou);
-          const float cq = k2.z * ou;
-          const float tl = 2.f * k2.x * ou * ou + B.Kf;
-          MH += cq * (tl - 5.f) * OH;
-          MB += cq * (tl - 3.f) * OH * k2.y;
+      float2 fhL, fbL;
+      face(0, fhL, fbL);
+      long o = (long)(a0 + ng) * ns + v;
+      const long oL = (long)L * ns;
+      const float4* kc = scc + g * L * SEG_CC;
+      for (int k = 0; k < nA; ++k, o += ns, kc += SEG_CC) {
+        hm = h0;
+        bm = b0;
+        h0 = hp;
+        b0 = bp;
+        dh = dhp;
+        db = dbp;
+        float2 fhR, fbR;
+        face(k + 1, fhR, fbR);
+        // the cells themselves: upwind of the right face where u >= 0, of the
+        // left one otherwise
+        const float2 hc = make_float2(pos ? h0.x : hm.x, pos ? h0.y : hm.y);
+        const float2 bc = make_float2(pos ? b0.x : bm.x, pos ? b0.y : bm.y);
+        const float4 k0 = kc[0], k1 = kc[1], k2 = kc[2], k3 = kc[3];
+        const float2 du = p2add(p2sub(u2, make_float2(k0.z, k0.w)), p2sub(ul2, make_float2(k1.x, k1.y)));
+        const float2 M = seg_maxwell2(du, make_float2(k0.x, k0.y), make_float2(k1.z, k1.w));
+        float2 MH = M, MB = p2mul(M, make_float2(k2.x, k2.y));
+        if (shak) {
+          const float4 k4 = kc[4], k5 = kc[5];
+          const float2 qf = *(const float2*)(kc + 6);
+          const float2 ou = p2add(p2sub(u2, make_float2(k4.x, k4.y)), p2sub(ul2, make_float2(k4.z, k4.w)));
+          const float2 nl = make_float2(k5.x, k5.y);
+          const float2 OH = seg_maxwell2(ou, make_float2(k3.z, k3.w), nl);
+          const float2 y = p2mul(p2mul(nl, ou), ou);  // -lambda ou^2
+          const float2 cq = p2mul(p2mul(qf, ou), OH);
+          MH = p2fma(cq, p2fma(y, p2s(-2.f), p2s(B.Kf - 5.f)), MH);
+          MB = p2fma(p2mul(cq, make_float2(k5.z, k5.w)), p2fma(y, p2s(-2.f), p2s(B.Kf - 3.f)), MB);
         }
         // (h + div + dt/tau MH) / (1 + dt/tau) written as a correction of h,
         // so that an equilibrium cell (MH == h, div == 0) stays bit-exact
-        *ph = h0 + ((fhL - fhR) * idx + k1.x * (MH - h0)) * k1.y;
-        *pb = b0 + ((fbL - fbR) * idx + k1.x * (MB - b0)) * k1.y;
+        const float2 dt2 = make_float2(k2.z, k2.w), i1k = make_float2(k3.x, k3.y);
+        const float2 nh = p2fma(p2fma(p2sub(fhL, fhR), idx, p2mul(dt2, p2sub(MH, hc))), i1k, hc);
+        const float2 nb = p2fma(p2fma(p2sub(fbL, fbR), idx, p2mul(dt2, p2sub(MB, bc))), i1k, bc);
+        Ho[o] = nh.x;
+        Bo[o] = nb.x;
+        if (k < nB) {
+          Ho[o + oL] = nh.y;
+          Bo[o + oL] = nb.y;
+        }
         fhL = fhR;
         fbL = fbR;
       }
@@ -653,7 +732,8 @@ __global__ void __launch_bounds__(SEG_T) k_batch_seg(BatchDev B, const float* __
 
 // One compiled shape of the segment kernel.
 struct SegVariant {
-  int seg, threads;
+  int seg, threads;               // the shape's name: faces per CTA, threads
+  int cells;                      // cells per segment
   const void* fn;                 // k_batch_seg<seg, threads>
   int (*smem)(int sst_max, int nu4_max);
   int smem_max;

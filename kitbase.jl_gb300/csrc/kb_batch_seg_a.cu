@@ -5,10 +5,10 @@
 namespace kb {
 
 void seg_variants_a(std::vector<SegVariant>& out) {
-  out.push_back({8, 64, (const void*)k_batch_seg<8, 64>, seg_smem<8, 64>, seg_smem_max<8, 64>()});
-  out.push_back({16, 64, (const void*)k_batch_seg<16, 64>, seg_smem<16, 64>, seg_smem_max<16, 64>()});
-  out.push_back({16, 128, (const void*)k_batch_seg<16, 128>, seg_smem<16, 128>, seg_smem_max<16, 128>()});
-  out.push_back({16, 256, (const void*)k_batch_seg<16, 256>, seg_smem<16, 256>, seg_smem_max<16, 256>()});
+  out.push_back({8, 64, 7, (const void*)k_batch_seg<7, 64>, seg_smem<7, 64>, seg_smem_max<7, 64>()});
+  out.push_back({16, 64, 15, (const void*)k_batch_seg<15, 64>, seg_smem<15, 64>, seg_smem_max<15, 64>()});
+  out.push_back({16, 128, 15, (const void*)k_batch_seg<15, 128>, seg_smem<15, 128>, seg_smem_max<15, 128>()});
+  out.push_back({16, 256, 15, (const void*)k_batch_seg<15, 256>, seg_smem<15, 256>, seg_smem_max<15, 256>()});
 }
 
 }  // namespace kb

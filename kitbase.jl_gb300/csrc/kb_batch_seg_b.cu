@@ -5,8 +5,8 @@
 namespace kb {
 
 void seg_variants_b(std::vector<SegVariant>& out) {
-  out.push_back({32, 128, (const void*)k_batch_seg<32, 128>, seg_smem<32, 128>, seg_smem_max<32, 128>()});
-  out.push_back({32, 256, (const void*)k_batch_seg<32, 256>, seg_smem<32, 256>, seg_smem_max<32, 256>()});
+  out.push_back({32, 128, 31, (const void*)k_batch_seg<31, 128>, seg_smem<31, 128>, seg_smem_max<31, 128>()});
+  out.push_back({32, 256, 31, (const void*)k_batch_seg<31, 256>, seg_smem<31, 256>, seg_smem_max<31, 256>()});
 }
 
 }  // namespace kb

@@ -321,6 +321,18 @@ __device__ __forceinline__ void pdf_slope(const double* p, const double* s, doub
 
 // ------------------------------------------- compensated FP32 accumulation
 
+// Packed FP32 pair arithmetic: one instruction for two values.
+__device__ __forceinline__ float2 p2add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 p2mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 p2fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 p2sub(float2 a, float2 b) {
+  unsigned long long A = *reinterpret_cast<unsigned long long*>(&a);
+  unsigned long long B = *reinterpret_cast<unsigned long long*>(&b), C;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(C) : "l"(A), "l"(B));
+  return *reinterpret_cast<float2*>(&C);
+}
+__device__ __forceinline__ float2 p2s(float x) { return make_float2(x, x); }
+
 // Double-float accumulator: (hi, lo) with |lo| <= ulp(hi)/2 after each add.
 // Knuth's TwoSum makes every addition error-free, so the pair carries about
 // 44 significant bits; it is converted exactly to FP64 (hi + lo) before the
@@ -334,6 +346,13 @@ __device__ __forceinline__ void df_add(DF& a, float x) {
   float e = (a.hi - (s - bp)) + (x - bp);
   a.hi = s;
   a.lo += e;
+}
+// df_add of two independent sums at once
+__device__ __forceinline__ void p2df_add(float2& hi, float2& lo, float2 x) {
+  const float2 s = p2add(hi, x);
+  const float2 bp = p2sub(s, hi);
+  lo = p2add(lo, p2add(p2sub(hi, p2sub(s, bp)), p2sub(x, bp)));
+  hi = s;
 }
 __device__ __forceinline__ DF df_merge(DF a, DF b) {
   float s = a.hi + b.hi;

@@ -17,14 +17,14 @@ bool line_covers(const kb_config_t& c) {
          c.bc[0] == KB_BC_FIX && c.bc[1] == KB_BC_FIX && c.nu <= SEG_MAXNU;
 }
 
-static const SegVariant kLine32 = {4, 128, (const void*)k_batch_seg<4, 128>, seg_smem<4, 128>,
-                                   seg_smem_max<4, 128>()};
+static const SegVariant kLine32 = {4, 128, 3, (const void*)k_batch_seg<3, 128>, seg_smem<3, 128>,
+                                   seg_smem_max<3, 128>()};
 
 int line_seg(int prec, int nx, int sms) {
-  return prec == KB_PREC_FP64 ? seg64_cells(nx, sms) : kLine32.seg;
+  return prec == KB_PREC_FP64 ? seg64_cells(nx, sms) : kLine32.cells;
 }
 
-// ints: nx, ng, nu, nus, vel_off, active, seg_first, nseg, then seg_b and
+// the segments' descriptors; ints: nx, ng, nu, nus, vel_off, active, seg_first, nseg, then seg_b and
 // seg_i0; longs: cell_off, elem_off; doubles: dx, dt, mu, 1/dx, 1/(2 mu),
 // clock[10], respart, FP64 mc64; floats: ul, FP32 mc
 static int line_nseg(const kb_config_t& c, int seg) { return (c.nx + seg - 1) / seg; }
@@ -33,12 +33,13 @@ static size_t line_doubles(const kb_config_t& c, int seg) { return 18 + 8 * (siz
 static size_t line_floats(const kb_config_t& c, int ncell) { return (size_t)(c.nu + 3) / 4 * 4 + 8 * (size_t)ncell; }
 static size_t line_ints(const kb_config_t& c, int seg) { return 8 + 2 * (size_t)line_nseg(c, seg); }
 size_t line_bytes(const kb_config_t& c, int ncell, int seg) {
-  return 8 * line_doubles(c, seg) + 4 * line_floats(c, ncell) + 4 * line_ints(c, seg);
+  return sizeof(SegDesc) * (size_t)line_nseg(c, seg) + 8 * line_doubles(c, seg) + 4 * line_floats(c, ncell) + 4 * line_ints(c, seg);
 }
 
 bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int seg, void* mem) {
   const int ns = line_nseg(c, seg);
-  double* D = (double*)mem;
+  SegDesc* G = (SegDesc*)mem;
+  double* D = (double*)(G + ns);
   float* F = (float*)(D + line_doubles(c, seg));
   int* I = (int*)(F + line_floats(c, ncell));
   std::vector<double> hd(line_doubles(c, seg), 0.0);
@@ -54,7 +55,11 @@ bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int 
   const int head[8] = {c.nx, c.ngx, c.nu, s.g.vstride, 0, 1, 0, ns};
   for (int k = 0; k < 8; ++k) hi[k] = head[k];
   for (int k = 0; k < ns; ++k) hi[8 + ns + k] = k * seg;  // seg_b stays 0
-  if (cudaMemcpy(D, hd.data(), 8 * hd.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+  std::vector<SegDesc> hg(ns);
+  for (int k = 0; k < ns; ++k)
+    hg[k] = {0, k * seg, c.nx, c.ngx, c.nu, s.g.vstride, 0, 0, 0, 0, hd[5], float(1.e-7 * s.g.dx), 2.f * float(s.g.mu_ref)};
+  if (cudaMemcpy(G, hg.data(), sizeof(SegDesc) * hg.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(D, hd.data(), 8 * hd.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(F, hf.data(), 4 * hf.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(I, hi.data(), 4 * hi.size(), cudaMemcpyHostToDevice) != cudaSuccess)
     return false;
@@ -70,6 +75,7 @@ bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int 
   d.nseg = I + 7;
   d.seg_b = I + 8;
   d.seg_i0 = I + 8 + ns;
+  d.seg_d = G;
   d.cell_off = (const long*)D;
   d.elem_off = (const long*)(D + 1);
   d.dx = D + 2;
@@ -135,7 +141,8 @@ int line_step(Line& L, DevState& s, bool res, int slot, cudaStream_t st) {
     const float* bin = (const float*)s.b[cur];
     float* hout = (float*)s.h[cur ^ 1];
     float* bout = (float*)s.b[cur ^ 1];
-    void* args[] = {(void*)&L.d, (void*)&hin, (void*)&bin, (void*)&hout, (void*)&bout, (void*)&slot};
+    int want = res || slot >= 0;
+    void* args[] = {(void*)&L.d, (void*)&hin, (void*)&bin, (void*)&hout, (void*)&bout, (void*)&slot, (void*)&want};
     launch_after(L.f32->fn, dim3((unsigned)L.d.nseg_all), dim3((unsigned)L.f32->threads), (size_t)L.smem, st, args);
   }
   s.cur = cur ^ 1;

@@ -135,18 +135,7 @@ template <typename R> struct Vec2;
 template <> struct Vec2<float> { using T = float2; };
 template <> struct Vec2<double> { using T = double2; };
 
-// Packed FP32 pair arithmetic (one instruction for both velocities of a
-// lane's pair) and the base-2 exponential of a pre-scaled argument.
-__device__ __forceinline__ float2 p2add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 p2mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 p2fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 p2sub(float2 a, float2 b) {
-  unsigned long long A = *reinterpret_cast<unsigned long long*>(&a);
-  unsigned long long B = *reinterpret_cast<unsigned long long*>(&b), C;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(C) : "l"(A), "l"(B));
-  return *reinterpret_cast<float2*>(&C);
-}
-__device__ __forceinline__ float2 p2s(float x) { return make_float2(x, x); }
+// The base-2 exponential of a pre-scaled argument.
 __device__ __forceinline__ float us_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
