@@ -587,7 +587,7 @@ static int timed_step(kb_handle* h, double dt, cudaEvent_t* ev) {
   cudaEventRecord(ev[1], st);
   n += kb::launch_face_param(h->s, dt, st);
   cudaEventRecord(ev[2], st);
-  n += kb::launch_moments(h->s, st);
+  n += kb::launch_moments(h->s, dt, false, st);
   cudaEventRecord(ev[3], st);
   n += kb::launch_wall(h->s, dt, st);
   cudaEventRecord(ev[4], st);

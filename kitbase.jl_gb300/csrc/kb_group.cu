@@ -52,10 +52,10 @@ __global__ void k_group_gather(const DevState* states, int n, double* out) {
   out[r * 5 + 4] = (double)*s.status;
 }
 
-template <bool SHAK, int DIR>
-void launch_mom(const DevState& ls, int blocks, cudaStream_t st) {
+template <bool SHAK>
+void launch_mom(const DevState& ls, const int* blocks, cudaStream_t st) {
   using SL = kb::MomStage<G_TS>;
-  auto kern = kb::k_mom_st<2, kb::FLUX_KCU, G_TS, SHAK, DIR, true>;
+  auto kern = kb::k_mom_st<2, kb::FLUX_KCU, G_TS, SHAK, true>;
   static std::once_flag once[64];
   int dev = 0;
   cudaGetDevice(&dev);
@@ -66,8 +66,12 @@ void launch_mom(const DevState& ls, int blocks, cudaStream_t st) {
   });
   CUtensorMap unused;  // the grouped kernel reads the members' maps from the table
   std::memset(&unused, 0, sizeof(unused));
-  void* args[] = {(void*)&unused, (void*)&unused, (void*)&ls};
-  kb::launch_after((const void*)kern, dim3((unsigned)blocks), dim3(kb::MOM_THREADS), SL::BYTES, st, args);
+  int nbx = blocks[kb::GK_MOMX], nby = blocks[kb::GK_MOMY];
+  const unsigned n = (unsigned)(nbx + nby + blocks[kb::GK_WALL]);
+  double dt = 0.0;  // the members' own
+  void* args[] = {(void*)&unused, (void*)&unused, (void*)&unused, (void*)&unused,
+                  (void*)&ls,     (void*)&dt,     (void*)&nbx,    (void*)&nby};
+  kb::launch_after((const void*)kern, dim3(n), dim3(kb::MOM_THREADS), SL::BYTES, st, args);
 }
 
 void launch_march(const DevState& ls, int blocks, cudaStream_t st) {
@@ -287,15 +291,13 @@ int kb_group_step_async(kb_group_t* G, int32_t nsteps) {
     const DevState& ls = G->ls[(G->parity + k) & 1];
     kb::group_small(kb::GK_WSLOPE, ls, G->flux, G->blocks[kb::GK_WSLOPE], false, G->stream);
     kb::group_small(kb::GK_FACE, ls, G->flux, G->blocks[kb::GK_FACE], false, G->stream);
-    if (shak) launch_mom<true, 0>(ls, G->blocks[kb::GK_MOMX], G->stream);
-    else launch_mom<false, 0>(ls, G->blocks[kb::GK_MOMX], G->stream);
-    launch_mom<false, 1>(ls, G->blocks[kb::GK_MOMY], G->stream);
-    kb::group_small(kb::GK_WALL, ls, G->flux, G->blocks[kb::GK_WALL], false, G->stream);
+    if (shak) launch_mom<true>(ls, G->blocks, G->stream);
+    else launch_mom<false>(ls, G->blocks, G->stream);
     const bool last = k == nsteps - 1;  // the chunk reports the last step's residual
     kb::group_small(kb::GK_CELL, ls, G->flux, G->blocks[kb::GK_CELL], last, G->stream);
     launch_march(ls, G->blocks[kb::GK_MARCH], G->stream);
     if (last) kb::group_small(kb::GK_RES, ls, G->flux, G->blocks[kb::GK_RES], true, G->stream);
-    nl += 5 + last + (G->blocks[kb::GK_WSLOPE] > 0) + (G->blocks[kb::GK_WALL] > 0);
+    nl += 4 + last + (G->blocks[kb::GK_WSLOPE] > 0);
   }
   // the members' current buffers moved with the steps
   G->parity = (G->parity + nsteps) & 1;

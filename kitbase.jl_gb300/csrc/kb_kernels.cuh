@@ -87,17 +87,16 @@ struct GroupTab {
   const int* start;         // [GK_N][n + 1] first block of each member per kernel kind
 };
 
-// The member a block of a grouped launch belongs to, and the block's index in
+// The member block b of a grouped launch belongs to, and the block's index in
 // that member's own launch (a plain launch: member 0, the block itself).
 template <bool GRP, int KIND>
-__device__ __forceinline__ int group_member(const DevState& sp, int& lb) {
+__device__ __forceinline__ int group_member(const DevState& sp, int& lb, int b = blockIdx.x) {
   if constexpr (!GRP) {
-    lb = blockIdx.x;
+    lb = b;
     return 0;
   } else {
     const GroupTab& t = *sp.grp;
     const int* st = t.start + KIND * (t.n + 1);
-    const int b = blockIdx.x;
     int lo = 0, hi = t.n - 1;  // the last member whose first block is <= b
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -122,7 +121,7 @@ __device__ __forceinline__ int group_member(const DevState& sp, int& lb) {
   const DevState& s = (GRP) ? s_member_ : (sp)
 
 // Grouped launch of a per-face / per-cell step kernel (kind GK_WSLOPE,
-// GK_FACE, GK_WALL, GK_CELL or GK_RES) over `blocks` blocks (kb_kernels.cu).
+// GK_FACE, GK_CELL or GK_RES) over `blocks` blocks (kb_kernels.cu).
 // res: with the residual's partial sums (GK_CELL).
 void group_small(int kind, const DevState& ls, int flux, int blocks, bool res, cudaStream_t st);
 
@@ -144,7 +143,7 @@ int launch_cell_param(DevState& s, double dt, cudaStream_t st, bool res = true);
 int launch_finish(DevState& s, cudaStream_t st, bool res = true);
 
 // Pass A (face moments, heat flux) and pass B (pointwise update), kb_march.cu.
-int launch_moments(DevState& s, cudaStream_t st);
+int launch_moments(DevState& s, double dt, bool wall, cudaStream_t st);  // wall: the wall faces too
 // Pass A of the 2D FP32 BGK step in one launch over row rings plus the
 // partial sum (kb_mom4.cu); returns the number of launches.
 int moments_ring(DevState& s, cudaStream_t st);

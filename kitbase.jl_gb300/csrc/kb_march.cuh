@@ -27,6 +27,7 @@
 #include "kb_kernels.cuh"
 #include "kb_flux.cuh"
 #include "kb_tma.cuh"
+#include "kb_wall.cuh"
 
 namespace kb {
 
@@ -152,15 +153,13 @@ __device__ __forceinline__ void store_q(const DevState& s, A (*qa)[2], int line,
 // FP64 form.  Bound by the FP64 pipe: one upwind slope per face and velocity
 // (Newton reciprocal) and the transport flux as one multiply-add on the slope:
 // about 33 FP64 instructions per face and velocity, 80 with both cells' slopes
-// and IEEE divisions (128 x 128 cells x 32 x 32 velocities: see store_fw).
+// and IEEE divisions.
 template <int D, int FLUX, int TS, bool SHAK, int DIR>
-__global__ void __launch_bounds__(128) k_mom(DevState s) {
+__device__ __forceinline__ void mom_line(const DevState& s, int blk) {
   using R = double;
-  pdl_wait();
-  pdl_next();
   const Geo& g = s.g;
   const int lane = threadIdx.x & 31;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int gw = (blk * (int)blockDim.x + (int)threadIdx.x) >> 5;
   const int n = DIR == 0 ? g.nx : g.ny;          // cells along the line
   const int ng = DIR == 0 ? g.ngx : g.ngy;
   const int nlines = DIR == 0 ? g.ny : g.nx;
@@ -284,6 +283,24 @@ __global__ void __launch_bounds__(128) k_mom(DevState s) {
   if (SHAK) store_q<TS, DIR>(s, qa, line, p0, ncell, lane);
 }
 
+// Pass A in one launch: the first nbx blocks take the x faces (and the old heat
+// flux), the next nby the y faces, the rest the wall faces.
+// None needs another's results, and one after the other each left
+// multiprocessors idle.  FP32 cavities, a step, three launches / one: 16^2 cells x
+// 16^2 velocities 49 / 37 us, 24^2 x 40^2 105 / 80, 40^2 x 25^2 79 / 70, 73^2 x
+// 18^2 103 / 97, 128^2 x 48^2 562 / 545 (80^2 x 40^2 229 / 233).  The walls come
+// last: their CTAs are few and long, and in front they kept the moments' slots
+// (64^2 x 28^2: 118 us, last 110).
+template <int D, int FLUX, int TS, bool SHAK>
+__global__ void __launch_bounds__(128) k_mom(DevState s, double dt, int nbx, int nby) {
+  pdl_wait();
+  pdl_next();
+  const int b = blockIdx.x;
+  if (b < nbx) mom_line<D, FLUX, TS, SHAK, 0>(s, b);
+  else if (D == 2 && b < nbx + nby) mom_line<D, FLUX, TS, false, 1>(s, b - nbx);
+  else wall_face<double, D>(s, dt, b - nbx - nby);
+}
+
 // Pass A, FP32 form: the stencil window of a CTA segment (4 warps x TS faces
 // along one line) is streamed through shared memory in chunks of MOM_VC
 // velocities, MOM_P chunks in flight: one TMA tensor box per distribution
@@ -307,15 +324,12 @@ struct MomStage {
 };
 constexpr int MOM_THREADS = 160;  // 4 consumer warps + 1 producer warp
 
-template <int D, int FLUX, int TS, bool SHAK, int DIR, bool GRP = false>
-__global__ void __launch_bounds__(MOM_THREADS) k_mom_st(const __grid_constant__ CUtensorMap tmh,
-                                                        const __grid_constant__ CUtensorMap tmb,
-                                                        DevState sp) {
+template <int D, int FLUX, int TS, bool SHAK, int DIR, bool GRP>
+__device__ __forceinline__ void mom_st_line(const CUtensorMap& tmh, const CUtensorMap& tmb, const DevState& sp,
+                                            int blk) {
   using R = float;
-  pdl_wait();
-  pdl_next();
   int lb;
-  const int gr = group_member<GRP, DIR == 0 ? GK_MOMX : GK_MOMY>(sp, lb);
+  const int gr = group_member<GRP, DIR == 0 ? GK_MOMX : GK_MOMY>(sp, lb, blk);
   KB_GROUP_STATE(GRP, sp, gr);
   // a grouped launch reads each member's tensor maps from global memory
   const CUtensorMap* mh = GRP ? sp.grp->maps + gr * 6 + DIR * 2 : &tmh;
@@ -597,6 +611,20 @@ __global__ void __launch_bounds__(MOM_THREADS) k_mom_st(const __grid_constant__ 
   store_fw<TS, D, DIR>(s, acc, line, p0w, nf, lane);
   if (nf > TS) store_fw<1, D, DIR>(s, acc + TS, line, p0w + TS, 1, lane);
   if (SHAK) store_q<TS, DIR>(s, qa, line, p0w, ncell, lane);
+}
+
+// The FP32 form of k_mom's launch; tx*, ty*: the tensor maps of the x and y passes.
+template <int D, int FLUX, int TS, bool SHAK, bool GRP = false>
+__global__ void __launch_bounds__(MOM_THREADS)
+    k_mom_st(const __grid_constant__ CUtensorMap txh, const __grid_constant__ CUtensorMap txb,
+             const __grid_constant__ CUtensorMap tyh, const __grid_constant__ CUtensorMap tyb, DevState s, double dt,
+             int nbx, int nby) {
+  pdl_wait();
+  pdl_next();
+  const int b = blockIdx.x;
+  if (b < nbx) mom_st_line<D, FLUX, TS, SHAK, 0, GRP>(txh, txb, s, b);
+  else if (D == 2 && b < nbx + nby) mom_st_line<D, FLUX, TS, false, 1, GRP>(tyh, tyb, s, b - nbx);
+  else wall_face<float, D, GRP>(s, dt, b - nbx - nby);
 }
 
 // ------------------------------------------------------------------ pass B
@@ -1977,15 +2005,18 @@ static inline Shape shape_of(const DevState& s) {
 // FP32 pass A: one CTA (4 warps) per segment of 4 TS faces along a line;
 // its dynamic shared memory exceeds the default 48 KB for TS = 4, so the
 // limit is raised once per device.
-template <int D, int FLUX, int TS, bool SHAK, int DIR>
-static void mom_st_go(DevState& s, cudaStream_t st) {
+template <int D, int FLUX, int TS, bool SHAK>
+static void mom_st_go(DevState& s, double dt, int nwall, cudaStream_t st) {
   const Geo& g = s.g;
   using SL = MomStage<TS>;
-  const int n = DIR == 0 ? g.nx : g.ny, nlines = DIR == 0 ? g.ny : g.nx;
-  const long nblk = (long)nlines * ((n + SL::NF - 1) / SL::NF);
-  auto kern = k_mom_st<D, FLUX, TS, SHAK, DIR>;
-  const CUtensorMap* tm =
-      (const CUtensorMap*)s.tmaps + 8 + ((DIR * 2 + (TS == 4 ? 1 : 0)) * 2 + s.cur) * 2;
+  const auto blocks = [](int n, int nlines) { return nlines * ((n + SL::NF - 1) / SL::NF); };
+  int nbx = blocks(g.nx, g.ny);
+  int nby = D == 2 ? blocks(g.ny, g.nx) : 0;
+  auto kern = k_mom_st<D, FLUX, TS, SHAK>;
+  const auto maps = [&](int dir) {
+    return (const CUtensorMap*)s.tmaps + 8 + ((dir * 2 + (TS == 4 ? 1 : 0)) * 2 + s.cur) * 2;
+  };
+  const CUtensorMap *tx = maps(0), *ty = D == 2 ? maps(1) : tx;
   static std::once_flag once[64];  // per device; thread-safe for concurrent host threads
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1995,40 +2026,38 @@ static void mom_st_go(DevState& s, cudaStream_t st) {
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                          cudaSharedmemCarveoutMaxShared);
   });
-  void* args[] = {(void*)&tm[0], (void*)&tm[1], (void*)&s};
-  launch_after((const void*)kern, dim3((unsigned)nblk), dim3(MOM_THREADS), SL::BYTES, st, args);
+  void* args[] = {(void*)&tx[0], (void*)&tx[1], (void*)&ty[0], (void*)&ty[1], (void*)&s, (void*)&dt, (void*)&nbx, (void*)&nby};
+  launch_after((const void*)kern, dim3((unsigned)(nwall + nbx + nby)), dim3(MOM_THREADS), SL::BYTES, st, args);
 }
 
 template <typename R, int D, int FLUX, int TS>
-static int mom_go(DevState& s, cudaStream_t st) {
+static int mom_go(DevState& s, double dt, int nwall, cudaStream_t st) {
   const Geo& g = s.g;
   if constexpr (sizeof(R) == 4) {
-    if (s.coll == COLL_SHAKHOV) mom_st_go<D, FLUX, TS, true, 0>(s, st);
-    else mom_st_go<D, FLUX, TS, false, 0>(s, st);
-    if (D == 2) mom_st_go<D, FLUX, TS, false, 1>(s, st);
-    return D == 2 ? 2 : 1;
-  }
-  if constexpr (sizeof(R) == 8) {
-    void* args[] = {(void*)&s};
-    auto run = [&](auto kern, long warps) {
-      prefer_max_shared((const void*)kern);
-      launch_after((const void*)kern, dim3(nblk2(warps * 32, 128)), dim3(128), 0, st, args);
-    };
+    if (s.coll == COLL_SHAKHOV) mom_st_go<D, FLUX, TS, true>(s, dt, nwall, st);
+    else mom_st_go<D, FLUX, TS, false>(s, dt, nwall, st);
+  } else {
     const long wx = (long)((g.nx + TS - 1) / TS) * g.ny, wy = (long)((g.ny + TS - 1) / TS) * g.nx;
-    if (s.coll == COLL_SHAKHOV) run(k_mom<D, FLUX, TS, true, 0>, wx);
-    else run(k_mom<D, FLUX, TS, false, 0>, wx);
-    if (D == 2) run(k_mom<D, FLUX, TS, false, 1>, wy);
+    int nbx = (int)nblk2(wx * 32, 128);
+    int nby = D == 2 ? (int)nblk2(wy * 32, 128) : 0;
+    const void* kern = s.coll == COLL_SHAKHOV ? (const void*)k_mom<D, FLUX, TS, true>
+                                              : (const void*)k_mom<D, FLUX, TS, false>;
+    prefer_max_shared(kern);
+    void* args[] = {(void*)&s, (void*)&dt, (void*)&nbx, (void*)&nby};
+    launch_after(kern, dim3((unsigned)(nwall + nbx + nby)), dim3(128), 0, st, args);
   }
-  return D;
+  return 1;
 }
 
 template <typename R, int D, int FLUX>
-static int mom_t(DevState& s, cudaStream_t st) {
+static int mom_t(DevState& s, double dt, bool wall, cudaStream_t st) {
   // 8: both face directions in one launch over row rings (2D FP32, BGK)
   const int ts = shape_of(s).ts;
-  if (sizeof(R) == 4 && D == 2 && ts == 8 && s.coll == COLL_BGK && s.mpart) return moments_ring(s, st);
-  if (ts == 2) return mom_go<R, D, FLUX, 2>(s, st);
-  return mom_go<R, D, FLUX, 4>(s, st);
+  if (sizeof(R) == 4 && D == 2 && ts == 8 && s.coll == COLL_BGK && s.mpart)
+    return moments_ring(s, st) + (wall ? launch_wall(s, dt, st) : 0);
+  const int nwall = wall ? s.nwall : 0;
+  if (ts == 2) return mom_go<R, D, FLUX, 2>(s, dt, nwall, st);
+  return mom_go<R, D, FLUX, 4>(s, dt, nwall, st);
 }
 
 template <typename R, int D, int FLUX, int TX, int BS>
@@ -2108,8 +2137,8 @@ static int march_t(DevState& s, double dt, cudaStream_t st) {
 // One precision x flux: the pass A and pass B launchers of both dimensions.
 #define KB_MARCH_INSTANCE(R, FLUX, NAME)                                          \
   namespace kb {                                                                \
-  int moments_##NAME(DevState& s, cudaStream_t st) {                            \
-    return s.g.D == 1 ? mom_t<R, 1, FLUX>(s, st) : mom_t<R, 2, FLUX>(s, st);     \
+  int moments_##NAME(DevState& s, double dt, bool wall, cudaStream_t st) {      \
+    return s.g.D == 1 ? mom_t<R, 1, FLUX>(s, dt, wall, st) : mom_t<R, 2, FLUX>(s, dt, wall, st); \
   }                                                                             \
   int march_##NAME(DevState& s, double dt, cudaStream_t st) {                   \
     return s.g.D == 1 ? march_t<R, 1, FLUX>(s, dt, st) : march_t<R, 2, FLUX>(s, dt, st); \

@@ -6,7 +6,7 @@ import pytest
 
 import kitgpu
 from kitgpu.solver import Handle, initial_cells, kb_config
-from cases import cavity, oracle_for, quadrant, rho_u_t_error
+from cases import cavity, oracle_for, quadrant, rho_u_t_error, sod
 
 pytestmark = pytest.mark.gpu
 
@@ -58,3 +58,22 @@ def test_equilibrium_on_any_velocity_grid(gpu_lib, prec, tol):
     for a in out:
         for got, ref in zip(a, (H, H * KS.gas.K / (2.0 * l))):
             assert np.max(np.abs(got - ref) / ref) < tol
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("name,cfg", [("cavity", cavity(nx=21, ny=18, nu=12, nv=10)),
+                                      ("cavity-bgk-odd", cavity(nx=9, ny=16, nu=13, nv=9, flux="ugks", coll="bgk")),
+                                      ("line", sod(nx=37, nu=33, flux="kcu", bc="maxwell"))],
+                         ids=["cavity", "cavity-bgk-odd", "line"])
+def test_stages_one_by_one_equal_whole_steps(gpu_lib, name, cfg, prec):
+    """A whole step takes the walls in the moment passes' launch, the timed
+    stages launch them apart: the same sums, bit for bit."""
+    out = []
+    for timed in (False, True):
+        KS, ctr, *faces, t = kitgpu.initialize(cfg, precision=prec)
+        dt = kitgpu.timestep(KS, ctr, 0.0)
+        ctr.handle.set_timing(timed)
+        kitgpu.step(KS, ctr, dt, 4)
+        out.append(ctr.handle.download())
+    for k in ("w", "prim", "h", "b"):
+        assert np.array_equal(out[0][k], out[1][k]), k
