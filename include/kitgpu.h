@@ -401,7 +401,7 @@ int kb_us_timestep(kb_us_t* us, double cfl, double sim_time, double max_time, do
 int kb_us_step(kb_us_t* us, double dt, int32_t nsteps, double* residual);
 int kb_us_info(kb_us_t* us, int64_t* launches);
 /* Kernel shape of the step: stepped cells per CTA (1..32; 0 = the default,
- * as many as fit 32 KB of per-velocity flux sums).  No reference
+ * up to 12, by the velocity grid and in FP64 by the mesh).  No reference
  * counterpart (launch tuning). */
 int kb_us_set_tuning(kb_us_t* us, int32_t cells_per_cta);
 int kb_us_get_tuning(kb_us_t* us, int32_t* cells_per_cta);

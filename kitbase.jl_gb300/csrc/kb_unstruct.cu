@@ -169,12 +169,20 @@ struct UsGeo {
 // Stage the records of a CTA's nloc cells (cell, neighbours, per-face
 // geometry) into shared memory: one coalesced read per CTA, so the warps'
 // cell loops hold no prefetched record in registers.
-__device__ __forceinline__ void us_stage_rec(const UsDev& d, int c0, int nloc, int4* RS, float4* GS) {
-  for (int t = threadIdx.x; t < nloc; t += US_T) RS[t] = __ldg(d.step_rec + c0 + t);
+__device__ __forceinline__ void us_stage_rec(const UsDev& d, int c0, int nloc, int4* RS, float4* GS, float* P) {
+  for (int t = threadIdx.x; t < nloc; t += US_T) {
+    const int4 r = __ldg(d.step_rec + c0 + t);
+    RS[t] = r;
+    P[t * US_NP + 7] = f32_of(__ldg(d.cell_iarea + r.x));
+  }
   for (int t = threadIdx.x; t < 3 * nloc; t += US_T) GS[t] = __ldg(d.step_geo32 + 3L * c0 + t);
 }
-__device__ __forceinline__ void us_stage_rec(const UsDev& d, int c0, int nloc, int4* RS, UsG64* GS) {
-  for (int t = threadIdx.x; t < nloc; t += US_T) RS[t] = __ldg(d.step_rec + c0 + t);
+__device__ __forceinline__ void us_stage_rec(const UsDev& d, int c0, int nloc, int4* RS, UsG64* GS, double* P) {
+  for (int t = threadIdx.x; t < nloc; t += US_T) {
+    const int4 r = __ldg(d.step_rec + c0 + t);
+    RS[t] = r;
+    P[t * US_NP + 7] = __ldg(d.cell_iarea + r.x);
+  }
   for (int t = threadIdx.x; t < 3 * nloc; t += US_T) GS[t] = d.step_geo64[3L * c0 + t];
 }
 __device__ __forceinline__ void us_geo(const float4& q, UsGeo<float>& g) {
@@ -194,9 +202,10 @@ template <> struct UsGeoRow<float> { using T = float4; };
 template <> struct UsGeoRow<double> { using T = UsG64; };
 
 // One CTA of US_T threads steps cb consecutive cells of the step list:
-// (1) each warp takes cells wid, wid + 4, ..., forms Dh, Db (kept in shared
-// memory, two velocities per lane and iteration) and the cell's velocity
-// sums (blocked, compensated in the FP32 form); (2) warp 0 does each cell's
+// (1) each warp takes cells wid, wid + 4, ..., forms h, b less the fluxes out of
+// the cell (kept in shared memory, two velocities per lane and iteration, so
+// that (3) reads no row again: 612 -> 534 us a step of 294,912 triangles of 256
+// velocities) and the cell's velocity sums (blocked, compensated in the FP32 form); (2) warp 0 does each cell's
 // FP64 algebra on its own lane (w update, conserve_prim, residual partials,
 // tau, equilibrium and Shakhov parameters); (3) the warps relax h, b of
 // their cells.  The FP32 form takes its face geometry from an FP32 table and
@@ -207,15 +216,16 @@ template <> struct UsGeoRow<double> { using T = UsG64; };
 // spill); the FP64 form 3.
 template <typename R, bool SHAK>
 __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
-    k_us_step(UsDev d, double dt, int cb, int res, const R* __restrict__ hin,
+    k_us_step(UsDev d, double dt, int cb, int lp, int res, const R* __restrict__ hin,
                                                   const R* __restrict__ bin, R* __restrict__ hout,
                                                   R* __restrict__ bout) {
   using R2 = typename Vec2<R>::T;
   constexpr bool FAST = sizeof(R) == 4;
   extern __shared__ __align__(16) unsigned char us_smem[];
-  double* S = (double*)us_smem;                  // [cb][US_NM]
-  R* P = (R*)(S + cb * US_NM);                   // [cb][US_NP] (room for doubles)
-  R* D = (R*)(S + cb * (US_NM + US_NP));         // [cb][2][vstride]: Dh, Db
+  double* S = (double*)us_smem;                  // [cb << lp][US_NM]
+  R* P = (R*)(S + (cb << lp) * US_NM);           // [cb][US_NP] (room for doubles)
+  // [cb][2][vstride]: h, b less the fluxes out of the cell
+  R* D = (R*)(S + (cb << lp) * US_NM + cb * US_NP);
   using GR = typename UsGeoRow<R>::T;
   GR* GS = (GR*)(D + (long)cb * 2 * d.vstride);  // [cb][3] face geometry
   int4* RS = (int4*)(GS + 3 * cb);               // [cb] cell and neighbours
@@ -235,13 +245,17 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
   // (1) face fluxes and velocity sums.  The records of the CTA's cells (the
   // cell, its three neighbours, and per face n1, n2, len and sg |n|^2) are
   // staged in shared memory first.
-  us_stage_rec(d, c0, nloc, RS, GS);
+  us_stage_rec(d, c0, nloc, RS, GS, P);
   __syncthreads();
   // up to here only what no step writes
   pdl_wait();
   pdl_next();
-  for (int i = wid; i < nloc; i += US_W) {
+  for (int item = wid; item < (nloc << lp); item += US_W) {
+    // a cell, or (FP64, small meshes) every 2^lp-th round of its velocities
+    const int i = FAST ? item : item >> lp;
+    const int q0 = FAST ? lane : lane + 32 * (item & ((1 << lp) - 1)), dq = FAST ? 32 : 32 << lp;
     const int4 rec = RS[i];
+    const R ia = P[i * US_NP + 7];
     const int c = rec.x;
     // per face: the outward normal (FP64: times dt len), dt len, |n|^2
     R no[3][2], aa[3], nn[3];
@@ -280,7 +294,7 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
 #pragma unroll
       for (int k = 0; k < US_NM; ++k) Pk[k] = make_float2(0.f, 0.f);
       const float2 Uo2 = p2s(Uo), Vo2 = p2s(Vo);
-      for (int q = lane; q < np; q += 32) {
+      for (int q = q0; q < np; q += dq) {
         const float2 u2 = U2[q], v2 = V2[q], w2 = W2[q];
         const float2 hc2 = Hc[q], bc2 = Bc[q];
         const float2 h0 = H0[q], b0 = B0[q], h1 = H1[q], b1 = B1[q], h2 = H2[q], b2 = B2[q];
@@ -297,8 +311,8 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
         dh2 = p2add(dh2, fh);
         db2 = p2add(db2, fb);
         dn2 = p2fma(p2s(nn[2]), fh, dn2);
-        Dh[q] = dh2;
-        Db[q] = db2;
+        Dh[q] = p2fma(dh2, p2s(-ia), hc2);
+        Db[q] = p2fma(db2, p2s(-ia), bc2);
         const float2 wn = p2mul(w2, dn2);
         Pk[0] = p2fma(w2, dh2, Pk[0]);
         Pk[1] = p2fma(u2, wn, Pk[1]);
@@ -320,7 +334,7 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
         acc[k].add(Pk[k].y);
       }
     } else
-    for (int q = lane; q < np; q += 32) {
+    for (int q = q0; q < np; q += dq) {
       const R2 u2 = U2[q], v2 = V2[q], w2 = W2[q];
       const R2 hc2 = Hc[q], bc2 = Bc[q];
       const R2 h0 = H0[q], b0 = B0[q], h1 = H1[q], b1 = B1[q], h2 = H2[q], b2 = B2[q];
@@ -343,7 +357,8 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
         face(0, e ? h0.y : h0.x, e ? b0.y : b0.x);
         face(1, e ? h1.y : h1.x, e ? b1.y : b1.x);
         face(2, e ? h2.y : h2.x, e ? b2.y : b2.x);
-        if (e) { dh2.y = dh; db2.y = db; } else { dh2.x = dh; db2.x = db; }
+        const R xh = fma(dh, -ia, hc), xb = fma(db, -ia, bc);
+        if (e) { dh2.y = xh; db2.y = xb; } else { dh2.x = xh; db2.x = xb; }
         const R wn = om * dn;
         acc[0].s = fma(om, dh, acc[0].s);
         acc[1].s = fma(u, wn, acc[1].s);
@@ -364,7 +379,7 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
 #pragma unroll
     for (int k = 0; k < US_NM; ++k) x[k] = acc[k].s;
     const double t = us_reduce8(x, lane);
-    if ((lane & 3) == 0) S[i * US_NM + (lane >> 2)] = t;
+    if ((lane & 3) == 0) S[item * US_NM + (lane >> 2)] = t;
   }
   __syncthreads();
 
@@ -374,7 +389,13 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
     double rr[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     if (lane < nloc) {
       const int c = RS[lane].x;
-      const double* Sc = S + lane * US_NM;
+      double Sc[US_NM];
+#pragma unroll
+      for (int k = 0; k < US_NM; ++k) Sc[k] = S[(lane << lp) * US_NM + k];
+      if (!FAST)
+        for (int t = 1; t < 1 << lp; ++t)
+#pragma unroll
+          for (int k = 0; k < (SHAK ? 7 : 5); ++k) Sc[k] += S[((lane << lp) + t) * US_NM + k];
       double* w = d.w + 4L * c;
       double* p = d.prim + 4L * c;
       const double rho_o = p[0], U_o = p[1], V_o = p[2], lam_o = p[3];
@@ -410,7 +431,6 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
         Pc[4] = Kb / (2.f * lam);  // B / H
         Pc[5] = k;
         Pc[6] = 1.f / (1.f + k);
-        Pc[7] = f32_of(ia);
         if (shak) {  // shakhov 2F2V of the old state (src/Theory/theory_equilibrium.jl:227-238)
           const float ro = f32_of(rho_o), lo = f32_of(lam_o);
           const float sfac = d.prf * (lo * lo) / ro;
@@ -431,7 +451,6 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
         Pc[4] = R(d.Kb * (0.5 * rcp64(pn[3])));  // B / H
         Pc[5] = R(k);
         Pc[6] = R(rcp64(1.0 + k));
-        Pc[7] = R(ia);
         if (shak) {  // shakhov 2F2V of the old state (src/Theory/theory_equilibrium.jl:227-238)
           // the heat-flux factors times the old Maxwellian's amplitude
           const double sfac = 0.4 * (1.0 - d.Pr) * (lam_o * lam_o) * (lam_o * (1.0 / PI));
@@ -455,11 +474,13 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
 
   // (3) relaxation of h, b
   const R Km5 = R(d.Kb - 5.0), Km3 = R(d.Kb - 3.0);
-  for (int i = wid; i < nloc; i += US_W) {
+  for (int item = wid; item < (nloc << lp); item += US_W) {
+    const int i = FAST ? item : item >> lp;
+    const int q0 = FAST ? lane : lane + 32 * (item & ((1 << lp) - 1)), dq = FAST ? 32 : 32 << lp;
     const int c = RS[i].x;
     const R* Pc = P + i * US_NP;
     const R rn = Pc[0], U = Pc[1], V = Pc[2], lam = Pc[3], cB = Pc[4];
-    const R kk = Pc[5], i1k = Pc[6], ia = Pc[7];
+    const R kk = Pc[5], i1k = Pc[6];
     R fq0 = R(0), fq1 = R(0), orn = R(0), ocB = R(0), olam = R(0), Uo = R(0), Vo = R(0);
     if (shak) {
       fq0 = Pc[8];
@@ -470,16 +491,14 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
       Uo = Pc[13];
       Vo = Pc[14];
     }
-    const R2* Hc = (const R2*)(hin + (long)c * vs);
-    const R2* Bc = (const R2*)(bin + (long)c * vs);
     const R2* Dh = (const R2*)(D + (long)i * 2 * vs);
     const R2* Db = (const R2*)(D + (long)i * 2 * vs + vs);
     R2* Ho = (R2*)(hout + (long)c * vs);
     R2* Bo = (R2*)(bout + (long)c * vs);
     if constexpr (FAST) {
       const float nl = -float(LOG2E) * lam, onl = -float(LOG2E) * olam;
-      for (int q = lane; q < np; q += 32) {
-        const float2 u2 = U2[q], v2 = V2[q], hc2 = Hc[q], bc2 = Bc[q], dh2 = Dh[q], db2 = Db[q];
+      for (int q = q0; q < np; q += dq) {
+        const float2 u2 = U2[q], v2 = V2[q];
         const float2 du = p2sub(u2, p2s(U)), dv = p2sub(v2, p2s(V));
         float2 MH = p2mul(p2s(rn), p2ex2(p2mul(p2s(nl), p2fma(du, du, p2mul(dv, dv)))));
         float2 MB = p2mul(p2s(cB), MH);
@@ -492,12 +511,12 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
           MH = p2fma(p2mul(fq, p2add(tl, p2s(Km5))), MHo, MH);
           MB = p2fma(p2mul(fq, p2add(tl, p2s(Km3))), p2mul(p2s(ocB), MHo), MB);
         }
-        Ho[q] = p2mul(p2fma(p2s(kk), MH, p2fma(dh2, p2s(-ia), hc2)), p2s(i1k));
-        Bo[q] = p2mul(p2fma(p2s(kk), MB, p2fma(db2, p2s(-ia), bc2)), p2s(i1k));
+        Ho[q] = p2mul(p2fma(p2s(kk), MH, Dh[q]), p2s(i1k));
+        Bo[q] = p2mul(p2fma(p2s(kk), MB, Db[q]), p2s(i1k));
       }
     } else
-    for (int q = lane; q < np; q += 32) {
-      const R2 u2 = U2[q], v2 = V2[q], hc2 = Hc[q], bc2 = Bc[q], dh2 = Dh[q], db2 = Db[q];
+    for (int q = q0; q < np; q += dq) {
+      const R2 u2 = U2[q], v2 = V2[q], dh2 = Dh[q], db2 = Db[q];
       R2 ho, bo;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
@@ -512,8 +531,8 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
           MH = fma(fq, tl - R(2), MH);
           MB = fma(fq * tl, ocB, MB);
         }
-        const R hn = fma(kk, MH, fma(e ? dh2.y : dh2.x, -ia, e ? hc2.y : hc2.x)) * i1k;
-        const R bn = fma(kk, MB, fma(e ? db2.y : db2.x, -ia, e ? bc2.y : bc2.x)) * i1k;
+        const R hn = fma(kk, MH, e ? dh2.y : dh2.x) * i1k;
+        const R bn = fma(kk, MB, e ? db2.y : db2.x) * i1k;
         if (e) { ho.y = hn; bo.y = bn; } else { ho.x = hn; bo.x = bn; }
       }
       Ho[q] = ho;
@@ -631,6 +650,7 @@ struct kb_us {
   int cur = 0;
   std::vector<int> level_first;  // avg_list offsets of the dependency levels (+ end)
   int cb = 1;                    // stepped cells per CTA
+  int lp = 0;                    // log2 of the parts of a cell that warps take (FP64)
   int nblk = 0;                  // CTAs of the last step launch (residual partial rows)
   size_t smem = 0;               // dynamic shared memory of the step kernel
 };
@@ -688,18 +708,44 @@ static std::vector<int> us_levels(int ncell, const int32_t* cell_nb, const int32
 
 // Cells per CTA of the step kernel and its shared memory: the per-velocity
 // flux sums of cb cells (2 nvel values each) plus the per-cell sums,
-// parameters and staged records (cell, neighbours, face geometry).  cb = 0 picks the largest count up to 32 within 32 KB of flux
-// sums (at least one cell).
+// parameters and staged records (cell, neighbours, face geometry).  cb = 0 picks
+// the largest count up to 12 within 32 KB of flux sums (at least one cell), a
+// multiple of the four warps where it can be: 294,912 triangles of 256
+// velocities, FP32, BGK: 8 / 10 / 12 / 15 / 20 cells 488 / 492 / 460 / 534 / 623
+// us a step; 80,000 of 400: 8 / 10 / 12 215 / 270 / 274; 8,192 of 169, Shakhov:
+// 8 / 12 / 20 / 22 35 / 32 / 37 / 39.  In FP64, where a warp fills its quarter's
+// FP64 pipe, fewer cells and their velocities in two parts when that gives the
+// busiest quarter less work (a tenth of a cell's time is the cell phase, a
+// twentieth of a part's its sums): 800 triangles of 256 velocities 7 cells 69
+// us, 6 in two parts 59; 288 of 144 13 cells 96 us, 2 in two parts 33.
 static int us_set_cells_per_cta(kb_us* U, int cb) {
   const kb::UsDev& d = U->d;
   const size_t esz = U->prec == KB_PREC_FP64 ? 8 : 4;
   const size_t per = 2 * (size_t)d.vstride * esz + sizeof(int4) + 12 * esz;
-  if (cb == 0) cb = (int)std::max<size_t>(1, std::min<size_t>(kb::US_CB, (32u << 10) / per));
-  if (cb < 1 || cb > kb::US_CB) return usfail(KB_ERR_ARG, "cells per CTA must be 1 .. 32");
-  const size_t smem = (sizeof(double) * (kb::US_NM + kb::US_NP) + per) * cb;
-  int dev = 0, maxs = 0;
+  int lp = 0, dev = 0, maxs = 0, sms = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&maxs, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (cb == 0) {
+    cb = (int)std::max<size_t>(1, std::min<size_t>(12, (32u << 10) / per));
+    if (cb > kb::US_W) cb -= cb % kb::US_W;
+    if (U->prec == KB_PREC_FP64 && sms > 0) {
+      const auto cost = [&](int c, int l) {
+        const long ctas = (d.nstep + c - 1) / c, per_sm = (ctas + sms - 1) / sms;
+        const long items = (c << l) + kb::US_W - 1;
+        return per_sm * ((items / kb::US_W) * (1.0 / (1 << l) + 0.05) + 0.1);
+      };
+      const int c0 = cb;
+      for (int c = c0; c >= 1; --c)
+        for (int l = 0; l <= (d.vstride > 64 ? 1 : 0); ++l)
+          if (cost(c, l) < 0.97 * cost(cb, lp)) {
+            cb = c;
+            lp = l;
+          }
+    }
+  }
+  if (cb < 1 || cb > kb::US_CB) return usfail(KB_ERR_ARG, "cells per CTA must be 1 .. 32");
+  const size_t smem = (sizeof(double) * ((kb::US_NM << lp) + kb::US_NP) + per) * cb;
   if (smem > (size_t)maxs)
     return usfail(KB_ERR_CONFIG, "velocity grid too large for the unstructured step's shared memory");
   const bool sk = d.coll == KB_COLL_SHAKHOV;
@@ -713,6 +759,7 @@ static int us_set_cells_per_cta(kb_us* U, int cb) {
     return usfail(KB_ERR_CUDA, "kb_us: cudaFuncSetAttribute failed");
   }
   U->cb = cb;
+  U->lp = lp;
   U->smem = smem;
   return KB_OK;
 }
@@ -1009,7 +1056,7 @@ static void us_enqueue_step(kb_us* U, double dt, bool last) {
     const int grid = (d.nstep + U->cb - 1) / U->cb;
     U->nblk = grid;
     int res = last ? 1 : 0;
-    void* args[] = {(void*)&d, &dt, &U->cb, &res, &hin, &bin, &hout, &bout};
+    void* args[] = {(void*)&d, &dt, &U->cb, &U->lp, &res, &hin, &bin, &hout, &bout};
     const void* fn = d.coll == KB_COLL_SHAKHOV ? (const void*)kb::k_us_step<R, true> : (const void*)kb::k_us_step<R, false>;
     kb::launch_after(fn, dim3((unsigned)grid), dim3(kb::US_T), U->smem, U->stream, args);
     U->launches++;

@@ -1,0 +1,29 @@
+"""The default shape of the triangle-mesh step (cells per CTA, and in FP64 the
+parts of a cell that warps take) on meshes and velocity grids of several sizes,
+against a shape given by hand."""
+import numpy as np
+import pytest
+
+from kitgpu import unstruct as US
+from test_gpu_unstruct import _setup
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-13), ("fp32", 0.0)])
+@pytest.mark.parametrize("nx,ny,nv,coll", [(3, 3, 5, "bgk"), (5, 4, 9, "shakhov"), (13, 17, 11, "shakhov"), (41, 37, 12, "bgk")])
+def test_default_shape_equals_a_given_one(gpu_lib, nx, ny, nv, coll, prec, tol):
+    """FP32: the same sums, bit for bit.  FP64: a cell's sums may be formed in
+    two parts, a rounding apart (2^-53 of the sums a step, 6 steps, a condition
+    below 100: 1e-13)."""
+    KS, orc = _setup(dict(boundary="extra", collision=coll, nx=nx, ny=ny, nu=nv, nv=nv, jitter=0.2))
+    out = []
+    for cb in (0, 5):
+        hd = US.init_fvm(KS, prec)
+        if cb:
+            hd.set_tuning(cb)
+        hd.step(hd.timestep(), 6)
+        out.append(hd.download())
+        hd.close()
+    for k in ("w", "prim", "h", "b"):
+        assert np.max(np.abs(out[0][k] - out[1][k])) <= tol * np.max(np.abs(out[1][k])), k
