@@ -1959,9 +1959,10 @@ struct Shape {
 // 22 CTAs per multiprocessor (a CTA reads 4 halo rows for its ry rows, and the
 // last of too few long CTAs run alone): 64^2 x 28^2 ry 4 / 16 / 32: 41 / 51 /
 // 89 us, 128^2 x 48^2 ry 4 / 16 / 64: 265 / 240 / 285, 512^2 x 64^2 ry 8 / 64:
-// 6.72 / 6.14 ms.  When even 4 rows give fewer than two CTAs per
+// 6.72 / 6.14 ms.  When even 4 rows give fewer than eight CTAs per
 // multiprocessor: 2 columns and one velocity per thread (16^2 x 48^2: 15.5
-// against 18.1 us).
+// against 18.1 us; a whole step at 73^2 x 18^2, 7 CTAs: 83 against 96 us, 40^2 x
+// 25^2 66 / 69, but 54^2 x 32^2, 10 CTAs: 113 / 110).
 // FP64: one warp nearly fills its quarter's FP64 pipe, so what counts is the
 // work of the busiest quarter (pass A: warps of ts faces) or multiprocessor
 // (pass B: CTAs of 4 x ry cells, 3 units a row and 1 for the first y faces).
@@ -1994,7 +1995,7 @@ static inline Shape shape_of(const DevState& s) {
   }
   if (p.ts == 0) p.ts = 2;
   const long boxes = cdiv(g.nvel, KB_TMA_VBOX);
-  const bool tiny = boxes * cdiv(g.nx, 4) * cdiv(g.ny, 4) < 2L * s.sm_count;
+  const bool tiny = boxes * cdiv(g.nx, 4) * cdiv(g.ny, 4) < 8L * s.sm_count;
   if (p.tx == 0) p.tx = tiny ? 2 : 4;
   if (p.bs == 0) p.bs = tiny || g.nu % 2 != 0 ? 128 : 64;
   for (int ry = 64; p.ry == 0; ry /= 2)
