@@ -387,19 +387,17 @@ int kb_set_wall(kb_handle_t* h, int side, const double* host_prim) {
   const Geo& g = h->s.g;
   if (side < 0 || side >= 2 * g.D) return fail(KB_ERR_ARG, "kb_set_wall: side out of range");
   int n = side < 2 ? g.ny : g.nx;
-  std::vector<double> buf((size_t)h->nface * 4);
-  KB_CUDA(cudaMemcpy(buf.data(), h->s.wall, sizeof(double) * buf.size(), cudaMemcpyDeviceToHost));
+  std::vector<double> buf((size_t)n * 4, 0.0);
   for (int q = 0; q < n; ++q) {
-    int f;
-    if (side == 0) f = q * (g.nx + 1);
-    else if (side == 1) f = q * (g.nx + 1) + g.nx;
-    else if (side == 2) f = h->s.nface_x + q;
-    else f = h->s.nface_x + g.ny * g.nx + q;
-    for (int k = 0; k < 4; ++k) buf[(size_t)f * 4 + k] = k < g.NW ? host_prim[q * g.NW + k] : 0.0;
+    for (int k = 0; k < g.NW; ++k) buf[(size_t)q * 4 + k] = host_prim[q * g.NW + k];
     if (!(host_prim[q * g.NW + g.NW - 1] > 0.0))
       return fail(KB_ERR_ARG, "kb_set_wall: wall lambda must be positive");
   }
-  KB_CUDA(cudaMemcpy(h->s.wall, buf.data(), sizeof(double) * buf.size(), cudaMemcpyHostToDevice));
+  // the side's faces: one in each row of x faces, or a row of y faces
+  const long f0 = side == 0 ? 0 : (side == 1 ? g.nx : (side == 2 ? h->s.nface_x : h->s.nface_x + (long)g.ny * g.nx));
+  const size_t row = 4 * sizeof(double);
+  KB_CUDA(cudaMemcpy2D(h->s.wall + f0 * 4, side < 2 ? (g.nx + 1) * row : row, buf.data(), row, row, n,
+                       cudaMemcpyHostToDevice));
   return KB_OK;
 }
 

@@ -99,14 +99,14 @@ def mixed_stream(rate, duration, seed=20261203, max_steps=200, tol=1e-6, frac_1d
     return out
 
 
-# Launch shapes of the served 2D solves.  Served grids are small (16^2 to
-# 128^2 cells): the shapes that suit one large solve give them few CTAs, each
-# a long serial march.  Two-column strips of 8 rows with one velocity per
-# thread in the update pass and two faces per warp in the moment pass were
-# the fastest on every served size measured (16^2 x 21^2 to 128^2 x 48^2 cells
-# x velocities: 1.3-2x the default shapes).  Fixed rather than autotuned per
-# request: a tuning search would advance the request's own solution.
-SERVE_SHAPE_2D = dict(march_tx=2, march_ry=8, march_bs=128, mom_ts=2)
+# Launch shapes of the served 2D solves that keep a stream of their own: 0 is the
+# library's choice by the size of the grid, which is the fastest or within 2 % of
+# it on every size of the mix (a step, against two-column strips of 8 rows, one
+# velocity per thread and two faces per warp: 16^2 cells x 16^2 velocities 37 and
+# 43 us, 54^2 x 32^2 110 and 116, 80^2 x 40^2 233 and 252, 128^2 x 48^2 545 and 648).
+# Not autotuned per request: a tuning search would advance the request's own
+# solution.
+SERVE_SHAPE_2D = dict(march_tx=0, march_ry=0, march_bs=0, mom_ts=0)
 
 
 def estimate_bytes(cfg, precision):

@@ -265,21 +265,18 @@ class Faces:
 def initial_cells(KS):
     """Per-cell (w, prim) of init_fvm, all cells incl. ghosts, x fastest."""
     ps, ib, gas = KS.ps, KS.ib, KS.gas
-    if KS.dim == 1:
-        pts = [(x,) for x in ps.x]
-    else:
-        nxt, nyt = ps.x.shape
-        pts = [(ps.x[i, j], ps.y[i, j]) for j in range(nyt) for i in range(nxt)]
-    ws, ps_ = [], []
-    cache = {}
+    pts = zip(ps.x) if KS.dim == 1 else zip(ps.x.ravel(order="F"), ps.y.ravel(order="F"))
+    seen, ws, prims, which = {}, [], [], []  # the distinct states, and each cell's
     for pt in pts:
         w = np.asarray(ib.fw(*pt), dtype=np.float64)
         key = w.tobytes()
-        if key not in cache:
-            cache[key] = conserve_prim(w, gas.gamma)
-        ws.append(w)
-        ps_.append(cache[key])
-    return np.array(ws), np.array(ps_)
+        k = seen.get(key)
+        if k is None:
+            k = seen[key] = len(ws)
+            ws.append(w.copy())
+            prims.append(conserve_prim(w, gas.gamma))
+        which.append(k)
+    return np.array(ws)[which], np.array(prims)[which]
 
 
 def initial_state(KS):
