@@ -283,6 +283,7 @@ int kb_create(const kb_config_t* cfg, const double* u, const double* v, const do
   ALLOC(h->s.cc, kb::CellCoef32, f32 ? h->ncell : 0);
   ALLOC(h->s.blockres, double, (size_t)h->s.res_blocks * 16);
   h->s.mpart = nullptr;
+  h->s.mt = nullptr;
   h->s.grp = nullptr;
   if (c.precision == KB_PREC_FP32 && g.D == 2) {
     const size_t nbox = (size_t)(g.nvel + kb::KB_TMA_VBOX - 1) / kb::KB_TMA_VBOX;
@@ -326,6 +327,19 @@ int kb_create(const kb_config_t* cfg, const double* u, const double* v, const do
   g.tensor = c.dim == 2;
   for (int k = 0; k < g.nvel && g.tensor; ++k)
     g.tensor = hu[k] == hu[k % g.nu] && hv[k] == hv[k - k % g.nu];
+  // (a grid that leaves no room for the factors takes the exponentials)
+  if (g.tensor && !f32) {
+    void* mt = nullptr;
+    const size_t n = ((c.flux == KB_FLUX_KFVS ? 0 : (size_t)h->nface) +
+                      (c.collision == KB_COLL_SHAKHOV ? 2 : 1) * (size_t)h->ncell) * (size_t)(c.nu + c.nv);
+    if (cudaMalloc(&mt, n * sizeof(double)) == cudaSuccess) {
+      h->allocs.push_back(mt);
+      h->s.mt = (double*)mt;
+      h->bytes += (int64_t)(n * sizeof(double));
+    } else {
+      cudaGetLastError();
+    }
+  }
   if (cudaMemcpy((void*)h->s.u, hu.data(), sizeof(double) * g.vstride, cudaMemcpyHostToDevice) ||
       cudaMemcpy((void*)h->s.v, hv.data(), sizeof(double) * g.vstride, cudaMemcpyHostToDevice) ||
       cudaMemcpy((void*)h->s.wt, hw.data(), sizeof(double) * g.vstride, cudaMemcpyHostToDevice) ||

@@ -52,6 +52,10 @@ struct DevState {
   CellParam* cp;    // [ncell]
   FaceCoef32* fc;   // [nface] FP32 coefficient blocks (FP32 form)
   FaceCoef64* fc64; // [nface] FP64 coefficient blocks (FP64 form)
+  // FP64 2D on a product velocity grid, else null (k_maxwell_tab): the factors,
+  // nu + nv each, of the faces' Maxwellians (not KFVS), then of each cell's new
+  // and, Shakhov, old one
+  double* mt;
   CellCoef32* cc;   // [ncell] FP32 cell coefficients
   double* blockres; // [nblocks][16] residual partials
   float2* mpart;    // [velocity boxes][2][nface][4] pass-A partials of the row-ring form
@@ -138,6 +142,7 @@ int launch_update(DevState& s, double dt, cudaStream_t st, bool res = true);
 // The same step split into its kernel groups (per-stage timing):
 // evolve = face_param + moments + wall; update = cell_param + march + finish.
 int launch_face_param(DevState& s, double dt, cudaStream_t st);
+int launch_maxwell_tab(DevState& s, bool faces, cudaStream_t st);
 int launch_wall(DevState& s, double dt, cudaStream_t st);
 int launch_cell_param(DevState& s, double dt, cudaStream_t st, bool res = true);
 int launch_finish(DevState& s, cudaStream_t st, bool res = true);

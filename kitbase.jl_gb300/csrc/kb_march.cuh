@@ -699,6 +699,15 @@ struct Mono {
   }
 };
 
+// A Maxwellian at one velocity of a product grid: its factors on the two axes
+// (k_maxwell_tab), or none (t null): the exponential.
+struct Factors {
+  const double* t;
+  int iu, iv;  // this thread's entries
+  __device__ __forceinline__ bool has() const { return t != nullptr; }
+  __device__ __forceinline__ double at(long k) const { return t[k + iu] * t[k + iv]; }
+};
+
 // Interface flux of one face at this thread's velocity.  hu, bu: upwind cell
 // values; su, sb: upwind slopes times dx; side = +0.5 when the upwind cell is
 // on the left, -0.5 on the right; hc, bc: the interior cell of a wall face.
@@ -753,11 +762,19 @@ __device__ __forceinline__ void eval_face(const FEv<float>& e, const Mono<float>
   fb += Hu * pb;
 }
 
-// FP64: tab is the table of exp2_tab.
+// (the form shared with FP64, which has the factors of its Maxwellians)
+template <int D, int FLUX, bool FAST = false>
+__device__ __forceinline__ void eval_face(const FEv<float>& e, const Mono<float>& M, float side, float hu, float bu,
+                                          float su, float sb, float hc, float bc, const double* tab, const Factors&,
+                                          long, float& fh, float& fb) {
+  eval_face<D, FLUX, FAST>(e, M, side, hu, bu, su, sb, hc, bc, tab, fh, fb);
+}
+
+// FP64: tab is the table of exp2_tab, m the face's factors at offset mk.
 template <int D, int FLUX, bool FAST = false>
 __device__ __forceinline__ void eval_face(const FEv<double>& e, const Mono<double>& M,
                                           double side, double hu, double bu, double su,
-                                          double sb, double hc, double bc, const double* tab,
+                                          double sb, double hc, double bc, const double* tab, const Factors& m, long mk,
                                           double& fh, double& fb) {
   if (!FAST && e.kind == 0) {
     fh = 0.0;
@@ -766,6 +783,7 @@ __device__ __forceinline__ void eval_face(const FEv<double>& e, const Mono<doubl
   }
   const double un = M.un;
   auto maxwell = [&]() {
+    if (D == 2 && FLUX != FLUX_KFVS && m.has()) return m.at(mk);
     const double du = un - e.E.y;
     double c2 = du * du;
     if (D == 2) {
@@ -830,19 +848,26 @@ __device__ __forceinline__ void relax(const CellCoef32& k, bool shak, float u, f
 
 __device__ __forceinline__ void relax(const CellParam& C, double rds, double u, double vv,
                                       double Kf, int D, double h0, double b0, double dh,
-                                      double db, const double* tab, double& hn, double& bn) {
+                                      double db, const double* tab, const Factors& m, long mk, int nt, double& hn,
+                                      double& bn) {
   if (!C.upd) {
     hn = h0;
     bn = b0;
     return;
   }
-  const double du = u - C.U;
-  double e = du * du;
-  if (D == 2) {
-    const double dv = vv - C.V;
-    e = fma(dv, dv, e);
+  double MH;
+  if (m.has()) {
+    MH = m.at(mk);
+  } else {
+    const double du = u - C.U;
+    double e = du * du;
+    if (D == 2) {
+      const double dv = vv - C.V;
+      e = fma(dv, dv, e);
+    }
+    MH = C.rho_n * exp2_tab(C.l2, e, tab);
   }
-  double MH = C.rho_n * exp2_tab(C.l2, e, tab), MB = MH * C.cB;
+  double MB = MH * C.cB;
   if (C.coll == COLL_SHAKHOV) {
     const double ou = u - C.oU;
     double oe = ou * ou, cq = ou * C.s0;
@@ -851,7 +876,7 @@ __device__ __forceinline__ void relax(const CellParam& C, double rds, double u, 
       oe = fma(ov, ov, oe);
       cq = fma(ov, C.s1, cq);
     }
-    const double S = cq * (C.o_rho_n * exp2_tab(EXP64_LOG2E * C.olam, oe, tab));
+    const double S = cq * (m.has() ? m.at(mk + nt) : C.o_rho_n * exp2_tab(EXP64_LOG2E * C.olam, oe, tab));
     const double tl = fma(2.0 * C.olam, oe, Kf - 3.0);
     MH = fma(S, tl - 2.0, MH);
     MB = fma(S * tl, C.ocB, MB);
@@ -979,6 +1004,10 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
   const R sys = py ? R(0.5) : R(-0.5);
   const R epsx = R(1.e-7 * g.dx), epsy = R(1.e-7 * g.dy);
   const bool shak = s.coll == COLL_SHAKHOV;
+  const int nt = D == 2 ? g.nu + g.nvel / g.nu : 0;
+  const Factors fac = {D == 2 && sizeof(R) == 8 ? s.mt : nullptr, D == 2 ? v % g.nu : 0, D == 2 ? g.nu + v / g.nu : 0};
+  const long cfac = FLUX == FLUX_KFVS ? 0 : (long)(s.nface_x + s.nface_y) * nt;  // the cells' factors
+  const long cstep = shak ? 2 * nt : nt;
   const double Kf = g.Kb;
   const FC* fct;
   if constexpr (sizeof(R) == 4) fct = s.fc;
@@ -1068,7 +1097,8 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
         su = vl_diff(rhi, wh[0][c], wh[1][c], wh[2][c], epsy);
         sb = vl_diff(rhi, wb[0][c], wb[1][c], wb[2][c], epsy);
       }
-      eval_face<D, FLUX>(e, MY, sys, hu, bu, su, sb, wh[1][c], wb[1][c], tab, fyh[c], fyb[c]);
+      eval_face<D, FLUX>(e, MY, sys, hu, bu, su, sb, wh[1][c], wb[1][c], tab, fac,
+                         (long)(s.nface_x + j0 * g.nx + i0 + c) * nt, fyh[c], fyb[c]);
     }
   } else {
     tile(0, wh[1], wb[1]);
@@ -1125,8 +1155,8 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
           su = slope<FAST>(rhi, wh[1][c], wh[2][c], wh[3][c], epsy);
           sb = slope<FAST>(rhi, wb[1][c], wb[2][c], wb[3][c], epsy);
         }
-        eval_face<D, FLUX, FAST>(e, MY, qys, hu, bu, su, sb, wh[1][c], wb[1][c], tab, fyh2[c],
-                                 fyb2[c]);
+        eval_face<D, FLUX, FAST>(e, MY, qys, hu, bu, su, sb, wh[1][c], wb[1][c], tab, fac,
+                                 (long)(s.nface_x + (j + 1) * g.nx + i0 + c) * nt, fyh2[c], fyb2[c]);
       }
     }
     // x faces of row j, each with the upwind cell's slope
@@ -1144,7 +1174,8 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
       R sb = vl_diff(ru, qx ? xb[f] : xb[f + 1], bu, qx ? xb[f + 2] : xb[f + 3], epsx);
       R hc = fi == 0 ? xh[f + 2] : xh[f + 1];
       R bc = fi == 0 ? xb[f + 2] : xb[f + 1];
-      eval_face<D, FLUX, FAST>(e, MX, qxs, hu, bu, su, sb, hc, bc, tab, fxh[f], fxb[f]);
+      eval_face<D, FLUX, FAST>(e, MX, qxs, hu, bu, su, sb, hc, bc, tab, fac, (long)(j * (g.nx + 1) + fi) * nt, fxh[f],
+                               fxb[f]);
     }
     // update the cells of row j
     const long ro = (long)(j + g.ngy) * rows;
@@ -1162,8 +1193,8 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
         const CellCoef32 k = cc[c];
         relax(k, shak, u, vv, MX.c2, xh[c + 2], xb[c + 2], dhh, dbb, hn, bn);
       } else {
-        relax(s.cp[cell_index(g, i0 + c, j)], g.rds, u, vv, Kf, D, xh[c + 2], xb[c + 2], dhh, dbb, tab, hn,
-              bn);
+        const int ci = cell_index(g, i0 + c, j);
+        relax(s.cp[ci], g.rds, u, vv, Kf, D, xh[c + 2], xb[c + 2], dhh, dbb, tab, fac, cfac + ci * cstep, nt, hn, bn);
       }
       if (vok) {
         Ho[ro + coff[c + 2]] = hn;
@@ -1965,7 +1996,8 @@ struct Shape {
 // 25^2 66 / 69, but 54^2 x 32^2, 10 CTAs: 113 / 110).
 // FP64: one warp nearly fills its quarter's FP64 pipe, so what counts is the
 // work of the busiest quarter (pass A: warps of ts faces) or multiprocessor
-// (pass B: CTAs of 4 x ry cells, 3 units a row and 1 for the first y faces).
+// (pass B: rounds of the four CTAs of 2 columns, ry rows and 64 velocities that
+// it holds, 3 units a row and 1 for the first y faces).
 // Pass A, us, ts 2 / 4: 16^2 cells x 16^2 velocities 62 / 108, 40 x 90 x 13 x 30
 // 263 / 293, 64^2 x 28^2 620 / 554, 64^2 x 16^2 181 / 175.  Pass B, us, ry
 // 4 / 8 / 16 / 32, same order: 59 / 105 / 197 / 197, 402 / 417 / 512 / 423,
@@ -1985,7 +2017,7 @@ static inline Shape shape_of(const DevState& s) {
     }
     if (p.ry == 0) {
       const auto cost = [&](int ry) {
-        return cdiv(cdiv(g.nx, p.tx) * cdiv(g.ny, ry) * cdiv(g.nvel, p.bs), sms) * (3 * ry + 1);
+        return cdiv(cdiv(g.nx, 2) * cdiv(g.ny, ry) * cdiv(g.nvel, 64), 4 * sms) * (3 * ry + 1);
       };
       p.ry = 32;
       for (int ry = 16; ry >= 4; ry /= 2)
@@ -2067,6 +2099,7 @@ static void march_go(DevState& s, cudaStream_t st) {
   int ry = shape_of(s).ry;
   dim3 grid((g.nx + TX - 1) / TX, D == 2 ? (g.ny + ry - 1) / ry : 1, (g.nvel + BS - 1) / BS);
   const int smem = sizeof(R) == 4 && D == 2 ? MarchStage<TX>::BYTES : 0;
+  if (sizeof(R) == 8 && D == 2 && s.mt) launch_maxwell_tab(s, FLUX != FLUX_KFVS, st);
   prefer_max_shared((const void*)k_march<R, D, FLUX, TX, BS>);
   void* args[] = {(void*)&s, (void*)&ry};
   launch_after((const void*)k_march<R, D, FLUX, TX, BS>, grid, dim3(BS), smem, st, args);
@@ -2130,7 +2163,7 @@ static int march_t(DevState& s, double dt, cudaStream_t st) {
       }
     }
   }
-  return 1;
+  return sizeof(R) == 8 && D == 2 && s.mt ? 2 : 1;
 }
 
 }  // namespace kb

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import kitgpu
-from kitgpu.solver import Handle, initial_cells, kb_config
+from kitgpu.solver import Handle, initial_cells, kb_config, wall_states
 from cases import cavity, oracle_for, quadrant, rho_u_t_error, sod
 
 pytestmark = pytest.mark.gpu
@@ -77,3 +77,36 @@ def test_stages_one_by_one_equal_whole_steps(gpu_lib, name, cfg, prec):
         out.append(ctr.handle.download())
     for k in ("w", "prim", "h", "b"):
         assert np.array_equal(out[0][k], out[1][k]), k
+
+
+FACTORED = [("kcu-shakhov-walls", cavity(nx=9, ny=12, nu=11, nv=8)),
+            ("ugks-bgk-extra", quadrant(nx=10, ny=7, nu=9, nv=12)),
+            ("ugks-shakhov-extra", quadrant(nx=13, ny=9, nu=8, nv=13, coll="shakhov")),
+            ("kfvs-bgk-walls", cavity(nx=8, ny=9, nu=10, nv=7, flux="kfvs", coll="bgk")),
+            ("kfvs-shakhov-fix", quadrant(nx=17, ny=18, nu=8, nv=9, flux="kfvs", coll="shakhov", bc="fix", ng=0))]
+
+
+@pytest.mark.parametrize("name,cfg", FACTORED, ids=[c[0] for c in FACTORED])
+def test_factored_maxwellians_equal_exponentials(gpu_lib, name, cfg):
+    """FP64: a velocity grid in another order is no product, so its update takes
+    the exponentials where the ordered one takes products of factors: the same
+    states to the FP64 form's 1e-12 after 6 steps."""
+    KS = kitgpu.solver_set(cfg)
+    vs = KS.vs
+    u, v, w = (vs.flat(x) for x in (vs.u, vs.v, vs.weights))
+    perm = np.random.default_rng(2).permutation(len(u))
+    W, P = initial_cells(KS)
+    out = []
+    for order in (np.arange(len(u)), perm):
+        h = Handle(kb_config(KS, "fp64"), u[order], v[order], w[order])
+        h.init_equilibrium(W, P)
+        for side, prim in enumerate(wall_states(KS)):
+            if KS.set.boundary[side] == "maxwell":
+                h.set_wall(side, prim)
+        h.step(h.timestep(KS.set.cfl, 0.0, 1e9), 6)
+        s = h.download()
+        back = np.argsort(order)
+        out.append((s["prim"], s["h"][:, back], s["b"][:, back]))
+    assert max(rho_u_t_error(out[0][0], out[1][0])) < 1e-12
+    for x, y in zip(out[0][1:], out[1][1:]):
+        assert np.max(np.abs(x - y)) < 1e-12 * np.max(y)
