@@ -330,8 +330,8 @@ int kb_batch_set_dt(kb_batch_t* b, const double* dt);
 int kb_batch_step(kb_batch_t* b, int32_t nsteps, double tol, double* residual, int32_t* active);
 int kb_batch_info(kb_batch_t* b, int64_t* elems, int64_t* launches);
 /* Shape of the FP32 batch step kernel, chosen by the autotuner (kitgpu.tune):
- * params[0] cells per segment (8, 16, 32), params[1] threads per CTA (64, 128,
- * 256; compiled pairs: 8x64, 16x64, 16x128, 16x256, 32x128, 32x256), params[2]
+ * params[0] faces per CTA (8, 16, 32: segments of one cell less), params[1]
+ * threads per CTA (64, 128, 256; compiled pairs: 8x64, 16x64, 16x128, 16x256, 32x128, 32x256), params[2]
  * 1 for a persistent grid (as many CTAs as fit on the GPU, each looping over
  * segments) or 0 for one CTA per segment.  Call outside stream capture; the
  * FP64 batch ignores it.  No reference counterpart. */

@@ -352,7 +352,7 @@ int kb_create(const kb_config_t* cfg, const double* u, const double* v, const do
   if (cudaMemcpy(h->s.kind, kinds.data(), h->nface, cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(fail(KB_ERR_CUDA, "face kind upload failed"));
   {
-    // the wall faces, one CTA each in k_wall
+    // the wall faces, one CTA each (kb_wall.cuh)
     std::vector<int> walls;
     for (int f = 0; f < h->nface; ++f)
       if (kinds[f] == 2) walls.push_back(f);
@@ -673,7 +673,7 @@ int kb_step(kb_handle_t* h, double dt, int32_t nsteps, double* residual) {
     }
   } else {
     // A long run replays steps recorded as a CUDA graph: one graph launch for
-    // several steps instead of ~8 kernel launches per step, so small solves
+    // several steps instead of ~6 kernel launches per step, so small solves
     // are bound by their kernels rather than by launch latency.  The first
     // two steps run eagerly (modules load and function attributes are set
     // outside any capture); results are those of the eager steps, bit for bit.
@@ -790,7 +790,7 @@ int kb_step_async(kb_handle_t* h, double dt, int32_t nsteps) {
     KB_CUDA(cudaEventCreateWithFlags(&h->ev_done, cudaEventDisableTiming));
   }
   // A served request advances in equal chunks with one dt, so the chunk's
-  // ~8 kernels per step are recorded once per starting buffer as a CUDA graph
+  // ~6 kernels per step are recorded once per starting buffer as a CUDA graph
   // and replayed: one launch per chunk instead of hundreds keeps the host
   // from becoming the bottleneck when many small solves share the GPU.  The
   // first chunk of a shape runs eagerly (module loading and function

@@ -1,14 +1,16 @@
 // kb_march.cuh -- the two HBM passes of one DVM time step (kernel templates;
 // instantiated per precision and flux in kb_march_*.cu so they compile in parallel).
 //
-// Pass A (k_mom): fw of every interior face and the old heat flux q of every
-// cell.  A warp owns a line segment of TS faces (along x or y) and loops over
-// ALL velocities, lanes striding by 32; the cells of the segment stencil are
-// held in a register window, so each cell value is loaded once per segment
-// and each van Leer slope is formed once.  Per-lane partial sums are
-// compensated (FP32 blocks flushed into double-float accumulators on the FP32
-// path) and combined once per face by a fixed shuffle tree, so fw is
-// deterministic and each face has exactly one writer.
+// Pass A (k_mom, FP32: k_mom_st): fw of every interior face and the old heat
+// flux q of every cell; the wall faces (kb_wall.cuh) go in the same launch.  A
+// warp owns a line segment of TS faces (along x or y) and loops over ALL
+// velocities, lanes striding by 32; the cells of the segment stencil are held
+// in a register window, so each cell value is loaded once per segment, and each
+// face takes its upwind cell's van Leer slope.  Per-lane partial sums are
+// compensated in the FP32 form (FP32 blocks flushed into double-float
+// accumulators) and plain FP64 sums in the other, combined once per face by a
+// fixed shuffle tree, so fw is deterministic and each face has exactly one
+// writer.
 //
 // Pass B (k_march): the pointwise update of h and b.  A thread owns one
 // velocity; a CTA owns a strip of TX columns, a chunk of rows and a chunk of

@@ -1,7 +1,7 @@
 // kb_mom4.cu -- pass A of the 2D FP32 step (face moments fw) in one launch
 // over row rings, both face directions from one read of h and b.
 //
-// The two-launch form (k_mom_st, kb_march.cuh) streams every distribution
+// The line form (k_mom_st, kb_march.cuh) streams every distribution
 // twice per step, once along x lines and once along y lines.  This form
 // uses the row ring of the pointwise update (k_march4): a CTA owns 128
 // velocities of a strip of TX columns and RY rows and marches up the rows;
@@ -16,8 +16,8 @@
 // pairwise warp reduce-scatter and written as one partial per (velocity box,
 // warp of the group, face), so no warp waits on another; k_mom_fin then adds
 // all partials of a face in double-float in a fixed order (deterministic),
-// adds the analytic part of fw and rotates y faces to the global frame.  BGK only: the Shakhov heat flux of the old state stays
-// with the two-launch form.
+// adds the analytic part of fw and rotates y faces to the global frame.  BGK
+// only: the Shakhov heat flux of the old state stays with the line form.
 #include <mutex>
 
 #include "kb_march.cuh"

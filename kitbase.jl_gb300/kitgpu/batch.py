@@ -203,7 +203,8 @@ class Batch:
         return out
 
     def set_tuning(self, seg=16, threads=128, persist=0):
-        """Shape of the FP32 step kernel: cells per segment, threads per CTA,
+        """Shape of the FP32 step kernel: faces per CTA (segments of one
+        cell less), threads per CTA,
         persistent grid (kb_batch_set_tuning)."""
         arr = (ctypes.c_int32 * 3)(int(seg), int(threads), int(persist))
         N.check(self.lib.kb_batch_set_tuning(self.h, arr, 3))
