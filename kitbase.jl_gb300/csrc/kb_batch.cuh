@@ -161,27 +161,33 @@ __device__ __forceinline__ void seg_store_coef(const BatchDev& B, long cell, con
   mcc[1] = make_float4(m.Ul, 0.f, 0.f, 0.f);
 }
 
-// Equilibrium h, b of cell c (0-based incl. ghosts) of instance b into both
-// FP32 buffers (init_fvm, src/Solver/solver_init.jl:119-141); row padding zero.
+// Equilibrium h, b of cell c (0-based incl. ghosts) of instance b from the cell's
+// coefficients (B.mc) into the FP32 buffers (init_fvm,
+// src/Solver/solver_init.jl:119-141); row padding zero.  H0, B0: the buffer the
+// next step reads; the other one takes what no step writes, ghost cells and
+// padding.
 __device__ __forceinline__ void seg_init_cell(const BatchDev& B, int b, int c, float* H0, float* B0,
                                               float* H1, float* B1) {
-  SegMax m;
-  m.set(B.prim + (B.cell_off[b] + c) * 4, B.K);
-  if (threadIdx.x == 0) seg_store_coef(B, B.cell_off[b] + c, m);
-  const int nu = B.nu[b], ns = B.nus[b];
+  const float4* mc = (const float4*)(B.mc + (B.cell_off[b] + c) * 8);
+  const float4 m = mc[0];
+  const float Ul = mc[1].x;
+  const int nu = B.nu[b], ns = B.nus[b], ng = B.ng[b];
+  const bool ghost = c < ng || c >= ng + B.nx[b];
   const long e = B.elem_off[b] + (long)c * ns;
   const float* uf = B.uf + B.vel_off[b];
   const float* ul = B.ul + B.vel_off[b];
   for (int v = threadIdx.x; v < ns; v += blockDim.x) {
     float hv = 0.f, bv = 0.f;
     if (v < nu) {
-      hv = seg_maxwell(uf[v], ul[v], m.rn, m.Uh, m.Ul, m.lam);
-      bv = hv * m.cB;
+      hv = seg_maxwell(uf[v], ul[v], m.x, m.y, Ul, m.z);
+      bv = hv * m.w;
     }
     H0[e + v] = hv;
     B0[e + v] = bv;
-    H1[e + v] = hv;
-    B1[e + v] = bv;
+    if (ghost || v >= nu) {
+      H1[e + v] = hv;
+      B1[e + v] = bv;
+    }
   }
 }
 

@@ -24,6 +24,6 @@ void seg64_launch(const BatchDev& B, int seg, const double* hin, const double* b
 void seg_res_launch(const BatchDev& B, cudaStream_t st);
 // Maxwellian coefficients of every cell from its prim (BatchDev::mc64, mc).
 void seg64_mcache_launch(const BatchDev& B, int n, int max_cells, cudaStream_t st);
-void seg_mcache_launch(const BatchDev& B, int n, int max_cells, cudaStream_t st);
+void seg_mcache_launch(const BatchDev& B, int n, int max_cells, cudaStream_t st, int b0 = 0);
 
 }  // namespace kb

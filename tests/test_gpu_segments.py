@@ -79,3 +79,24 @@ def test_adaptive_lines_equal_single_steps(gpu_lib, prec, nsteps):
     tol = 1e-12 if prec == "fp64" else 1e-5
     assert max(rho_u_t_error(x["prim"], y["prim"])) < tol
     assert np.max(np.abs(x["h"] - y["h"])) < tol * np.max(y["h"])
+
+
+@pytest.mark.parametrize("before", [1, 2, 5])
+def test_pool_member_joins_after_any_number_of_steps(gpu_lib, before):
+    """A solve that joins a pool after an odd or even number of steps starts in
+    the buffer the next step reads: the state it has in a pool of its own, bit
+    for bit (cells and velocities that an earlier member held are taken again)."""
+    sets = KB.solver_sets([KB.shock_config(3.0, 61, 49), KB.shock_config(2.0, 40, 30), dict(KB.shock_config(4.0, 45, 33), nxg=1)])
+    outs = []
+    for alone in (False, True):
+        pool = KB.Pool(sets[0], max_instances=4, max_cells=400)
+        if not alone:
+            first = [pool.add(KS)[0] for KS in sets[:2]]
+            pool.step(before)
+            pool.remove(first[1])
+        slot = pool.add(sets[2])[0]
+        pool.step(7)
+        outs.append(pool.download(slot))
+        pool.close()
+    for k in ("w", "prim", "h", "b"):
+        assert np.array_equal(outs[0][k], outs[1][k]), k
