@@ -67,6 +67,7 @@ struct UsDev {
   double* w;      // [ncell][4]
   double* prim;   // [ncell][4]
   double* bres;   // [step CTAs][8]: sums of (w - w_old)^2, |w| over each CTA's cells, last step
+  double* bsum;   // [US_RES_CTAS][8]: sums of their rows (k_us_rows)
   double* tmax;   // [1]
   double* residual;  // [4]
   int* status;
@@ -609,16 +610,12 @@ __global__ void __launch_bounds__(US_T) k_us_avg(UsDev d, int first, const R* __
   }
 }
 
-// residual of update! US2F: sqrt(sum (w - w_old)^2 * ncell) / (sum |w| + 1e-7)
-// over the stepped cells (src/Solver/solver_update.jl:465-467) from the step
-// CTAs' partials: strided sums, then a fixed tree (deterministic)
-__global__ void __launch_bounds__(256) k_us_residual(UsDev d, int nblk) {
-  __shared__ double red[8][256];
+// Sums of the 8 columns of rows first, first + step, ... < n, then a fixed tree
+// over the CTA's 256 threads: red[k][0] (deterministic)
+__device__ __forceinline__ void us_sum_rows(const double* rows, int first, int n, int step, double (*red)[256]) {
   double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  pdl_wait();
-  pdl_next();
-  for (int b = threadIdx.x; b < nblk; b += 256)
-    for (int k = 0; k < 8; ++k) a[k] += d.bres[8L * b + k];
+  for (int b = first; b < n; b += step)
+    for (int k = 0; k < 8; ++k) a[k] += rows[8L * b + k];
   for (int k = 0; k < 8; ++k) red[k][threadIdx.x] = a[k];
   __syncthreads();
   for (int s = 128; s >= 1; s >>= 1) {
@@ -626,6 +623,28 @@ __global__ void __launch_bounds__(256) k_us_residual(UsDev d, int nblk) {
       for (int k = 0; k < 8; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + s];
     __syncthreads();
   }
+}
+
+// First level of the residual's sums on large meshes: FP64 additions at one
+// multiprocessor's rate bound a single CTA (24,448 rows: 81 us; a call of one step
+// of 294,912 triangles 590 -> 522 us).
+constexpr int US_RES_CTAS = 64, US_RES_ROWS = 2048;  // CTAs; rows that one CTA sums by itself
+__global__ void __launch_bounds__(256) k_us_rows(UsDev d, int nblk) {
+  __shared__ double red[8][256];
+  pdl_wait();
+  pdl_next();
+  us_sum_rows(d.bres, blockIdx.x * 256 + threadIdx.x, nblk, gridDim.x * 256, red);
+  if (threadIdx.x < 8) d.bsum[8 * blockIdx.x + threadIdx.x] = red[threadIdx.x][0];
+}
+
+// residual of update! US2F: sqrt(sum (w - w_old)^2 * ncell) / (sum |w| + 1e-7)
+// over the stepped cells (src/Solver/solver_update.jl:465-467) from the step
+// CTAs' partials or their sums (k_us_rows)
+__global__ void __launch_bounds__(256) k_us_residual(UsDev d, const double* rows, int n) {
+  __shared__ double red[8][256];
+  pdl_wait();
+  pdl_next();
+  us_sum_rows(rows, threadIdx.x, n, 256, red);
   if (threadIdx.x < 4)
     d.residual[threadIdx.x] = sqrt(red[threadIdx.x][0] * d.ncell) / (red[4 + threadIdx.x][0] + 1.e-7);
 }
@@ -937,6 +956,7 @@ extern "C" int kb_us_create(const kb_config_t* cfg, int32_t ncell, int32_t nface
   USALLOC(d.w, double, 4L * ncell);
   USALLOC(d.prim, double, 4L * ncell);
   USALLOC(d.bres, double, 8L * std::max(1, (int)steps.size()));
+  USALLOC(d.bsum, double, 8L * kb::US_RES_CTAS);
   USALLOC(U->stage, double, (long)ncell * d.nvel);
 #undef USALLOC
   for (void** q : {&U->h[0], &U->h[1], &U->b[0], &U->b[1]})
@@ -1127,7 +1147,16 @@ extern "C" int kb_us_step(kb_us_t* U, double dt, int32_t nsteps, double* residua
     else
       us_enqueue_step<float>(U, dt, s == nsteps - 1);
   }
-  void* rargs[] = {(void*)&d, &U->nblk};
+  const double* rows = d.bres;
+  int nrows = U->nblk;
+  if (nrows > kb::US_RES_ROWS) {
+    void* sargs[] = {(void*)&d, &U->nblk};
+    kb::launch_after((const void*)kb::k_us_rows, dim3(kb::US_RES_CTAS), dim3(256), 0, U->stream, sargs);
+    U->launches++;
+    rows = d.bsum;
+    nrows = kb::US_RES_CTAS;
+  }
+  void* rargs[] = {(void*)&d, &rows, &nrows};
   kb::launch_after((const void*)kb::k_us_residual, dim3(1), dim3(256), 0, U->stream, rargs);
   U->launches++;
   if (cudaStreamSynchronize(U->stream) != cudaSuccess)

@@ -53,3 +53,18 @@ def test_factored_maxwellians_equal_exponentials(gpu_lib, coll, nv, cb):
         out.append((s["w"], s["prim"], s["h"][:, back], s["b"][:, back]))
     for x, y in zip(*out):
         assert np.max(np.abs(x - y)) < 1e-12 * np.max(np.abs(y))
+
+
+@pytest.mark.parametrize("n", [44, 65])
+def test_residual_of_many_ctas(gpu_lib, n):
+    """One cell per CTA on meshes on either side of the 2,048 CTAs whose sums one
+    CTA adds by itself: the residual of 8 cells per CTA, to the rounding of a
+    sum of at most 10^4 terms of one sign (1e-11)."""
+    KS, orc = _setup(dict(boundary="extra", collision="bgk", nx=n // 2, ny=n, nu=5, nv=5, jitter=0.2))
+    res = []
+    for cb in (1, 8):
+        hd = US.init_fvm(KS, "fp64")
+        hd.set_tuning(cb)
+        res.append(np.array(hd.step(hd.timestep(), 3)))
+        hd.close()
+    assert np.all(np.abs(res[0] - res[1]) <= 1e-11 * np.abs(res[1])), res
