@@ -167,13 +167,22 @@ __device__ __forceinline__ int split64(double a, double b, double& f) {
 __device__ __forceinline__ double exp64_poly(double f) {
   return f * fma(fma(fma(EXP64_K4, f, EXP64_K3), f, EXP64_K2), f, EXP64_K1);
 }
-// 2^(a b / 256) for a b <= 0: 8 FP64 instructions.  Results below 2^-1021 are 0.
+// 2^(a b / 256): 8 FP64 instructions.  Results below 2^-1021 are 0, those from
+// 2^1023 up infinite, and not a number stays so.  The range is judged on the
+// whole pattern of t = a b + 1.5 2^52, which grows with t from one infinity to
+// the other (on each side of zero): from a b = -2^31 down, the integer no longer
+// fits the low word, and its wrapped value gave e^-x of x = 6e6 as -3e218.
 __device__ __forceinline__ double exp2_tab(double a, double b, const double* tab) {
-  double f;
-  const int n = split64(a, b, f);
-  const double t = tab[n & (EXP64_N - 1)];
-  const double e = fma(t, exp64_poly(f), t);
-  return n < -1021 * EXP64_N ? 0.0 : scale64(e, n >> 8);
+  constexpr double big = 6755399441055744.0;
+  const double t = fma(a, b, big);
+  const double f = fma(a, b, -(t - big));
+  const long long d = __double_as_longlong(t) - 0x4338000000000000ll;  // the integer, where it is in range
+  const int n = (int)d;
+  const double p = tab[n & (EXP64_N - 1)];
+  const double e = scale64(fma(p, exp64_poly(f), p), n >> 8);
+  if ((unsigned long long)(d + 1021 * EXP64_N) < 2044ull * EXP64_N) return e;
+  if ((__double2hiint(t) & 0x7fffffff) >= 0x7ff80000) return t;
+  return __hiloint2double(d < 0 ? 0 : 0x7ff00000, 0);
 }
 // -lambda (u - U)^2 as a 256th of a power of two: a = EXP64_LOG2E lambda
 constexpr double EXP64_LOG2E = -256.0 * 1.442695040888963407359924681001892137;
