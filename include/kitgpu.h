@@ -195,8 +195,10 @@ int kb_step_cfl(kb_handle_t* h, double cfl, double sim_time, double max_time, in
 int kb_step_async(kb_handle_t* h, double dt, int32_t nsteps);
 int kb_query(kb_handle_t* h, double* residual, int32_t* ready);
 
-/* Face fluxes of the last kb_evolve, materialised for inspection: fw in the
- * global frame [nface][dim+2], fh, fb [nface][nu*nv].  x faces first
+/* Face fluxes, materialised for inspection: fw in the global frame
+ * [nface][dim+2], of the last kb_evolve or of the last step of kb_step,
+ * kb_step_cfl or kb_step_async; fh, fb [nface][nu*nv], of the state now held
+ * (before kb_update: those of that kb_evolve).  x faces first
  * ((nx+1)*ny, i fastest), then y faces (nx*(ny+1)).  Faces that the
  * reference never computes for this configuration are returned as zero.
  * Any pointer may be NULL.  (face.fw / face.fh / face.fb of Interface2F,

@@ -499,6 +499,7 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   d.tol = 0.0;
   d.coll = base->collision;
   d.clock = nullptr;
+  d.fw = nullptr;
   if (B->prec == KB_PREC_FP64) {
     if (!kb::seg64_prepare()) return fail_out(bfail(KB_ERR_CUDA, "FP64 segment kernel attributes refused"));
     if ((rc = batch_tables(B, seg64)) != KB_OK) return fail_out(rc);

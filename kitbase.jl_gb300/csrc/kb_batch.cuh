@@ -51,6 +51,8 @@ struct BatchDev {
   float* mc;             // [cell][8] FP32 Maxwellian coefficients of the cell's current prim
                          // (SegMax: rn, U hi, lambda, K / (2 lambda), U lo), kept with prim
   double* residual;      // [n][4]
+  double* fw;            // [face][4] a single solve's face moments, null for ensembles: a step
+                         // asked for its residual leaves its own, on the end faces too (with ghosts)
   // Per-step time step of a single solve (kb_step_cfl), null otherwise.  Step
   // number m has slot m mod 3: [slot] the CFL rate of the state before it,
   // [3 + slot] the time before it; then cfl, the end time, umax and the number
@@ -195,6 +197,7 @@ __device__ __forceinline__ void seg_init_cell(const BatchDev& B, int b, int c, f
 struct SegClock {
   double dt, t;
   bool stop;  // the end time is reached: the state is carried over
+  bool last;  // this step reaches it: its residual and face moments are kept
 };
 // timestep (src/Solver/solver_main.jl:240-288) from the collected rate
 __device__ __forceinline__ SegClock seg_clock(const BatchDev& B, int slot) {
@@ -203,7 +206,9 @@ __device__ __forceinline__ SegClock seg_clock(const BatchDev& B, int slot) {
   c.t = B.clock[3 + slot];
   c.dt = B.clock[6] / B.clock[slot];
   c.dt = c.dt < tend - c.t ? c.dt : tend - c.t;
-  c.stop = !(c.t < tend - 1e-14 * fabs(tend)) || !(c.dt > 0.0);
+  const double end = tend - 1e-14 * fabs(tend);
+  c.stop = !(c.t < end) || !(c.dt > 0.0);
+  c.last = !(c.t + c.dt < end);
   return c;
 }
 // by one thread of the launch
@@ -299,9 +304,10 @@ __device__ __forceinline__ DF seg_sums(DF (&x)[4], int lane) {
 // A CTA takes segments k = blockIdx.x, blockIdx.x + gridDim.x, ...: one
 // segment each when the grid has a CTA per segment, or a persistent loop
 // when the grid is the number of CTAs that fit on the GPU at once.
-// slot: see BatchDev::clock (-1: the instances' own dt).  res: the residual's
-// partial sums are wanted.
-template <int SEG, int SEG_T>
+// res: the residual's partial sums are wanted.  ONE: the form of a single
+// solve, with its own time step (slot: BatchDev::clock, -1: B.dt) and face moments
+// (BatchDev::fw); a form of its own, because they cost the ensembles' 1.6 %.
+template <int SEG, int SEG_T, bool ONE = false>
 __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
     k_batch_seg(BatchDev B, const float* __restrict__ Hin, const float* __restrict__ Bin,
                 float* __restrict__ Hout, float* __restrict__ Bout, int slot, int res) {
@@ -311,6 +317,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ unsigned long long bar;
   __shared__ float sconst[2];  // T3, T4
+  __shared__ int sflag[2];     // (ONE) the step is past the end; its residual and face moments are kept
   // An FP64 instruction holds a quarter of the multiprocessor for 64 cycles
   // whatever its active lanes, so the FP64 cell phase is one warp's, written
   // for few instructions (about 30; the divisions, conversions and compares
@@ -361,7 +368,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
       bulk_g2s(dst, src, (unsigned)ns * 4u, &bar);
     }
   }
-  bool skip = !B.active[b];
+  const bool skip = !B.active[b];
   const int ca = max(i0, 1), cb = min(i1, nx - 1);  // stepped cells [ca, cb); may be none
   const int ncell = cb - ca;
   for (int v = tid; v < ns; v += SEG_T) {  // zero weight up to the row's end
@@ -377,13 +384,18 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
     smc[tid * 2] = ((const float4*)(B.mc + c * 8))[0];
     smc[tid * 2 + 1] = ((const float4*)(B.mc + c * 8))[1];
   }
-  if (slot >= 0) {
-    const SegClock c = seg_clock(B, slot);
-    skip = skip || c.stop;
-    if (k == 0 && tid == 0) seg_clock_next(B, slot, c);
-  }
   if (tid == SEG_T - 1) {
-    const double dt0 = slot >= 0 ? seg_clock(B, slot).dt : B.dt[b];
+    double dt0 = B.dt[b];
+    if (ONE) {
+      SegClock c = {dt0, 0.0, false, false};
+      if (slot >= 0) {
+        c = seg_clock(B, slot);
+        if (k == 0) seg_clock_next(B, slot, c);
+      }
+      dt0 = c.dt;
+      sflag[0] = c.stop;
+      sflag[1] = res || c.last;
+    }
     sconst[0] = f32_of(dt0);
     sconst[1] = f32_of(0.5 * dt0 * dt0 * sd.rdx);
   }
@@ -398,7 +410,8 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
   }
   ++phase;
   const int dB = SEG_ROWS * B.sst_max;  // from a value of h to the same of b
-  if (skip) {  // converged or past the end: carry this segment's cells over
+  const bool want = ONE ? sflag[1] != 0 : res != 0;
+  if (skip || (ONE && sflag[0])) {  // converged or past the end: carry this segment's cells over
     for (int i = i0; i < i1; ++i)
       for (int v = tid; v < ns; v += SEG_T) {
         Ho[(long)(i + ng) * ns + v] = sH[(i - r0) * sst + v];
@@ -407,7 +420,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
     __syncthreads();  // the window is reused by the next segment
     continue;  // CTA-uniform
   }
-  const int fa = ca, fb = cb;  // faces fa .. fb: the left faces of the stepped cells and the last one's right face
+  const int fa = ca;  // faces fa .. fa + ncell: the left faces of the stepped cells and the last one's right face
   const float epsd = sd.epsd;
   const float T3 = sconst[0], T4 = sconst[1];
   const bool shak = B.coll == COLL_SHAKHOV;
@@ -431,12 +444,17 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
     }
   }
 
-  // ---- face moments of faces fa .. fb and heat flux of the cells right of
+  // ---- face moments of those faces and heat flux of the cells right of
   // them: FT threads per face (velocity pairs q mod FT).  A half-warp reads 16
   // pairs: rows of 16 (mod 32) floats put two faces' pairs on all the banks.
   {
     const int j = tid / FT, q = tid % FT;
-    const int f = fa + j;
+    // the faces, then the ends' for BatchDev::fw (a segment with an end steps a
+    // cell less, so a group of threads is free for it)
+    const bool keep = ONE && want;
+    const int end0 = keep && ng > 0 && i0 == 0, end1 = keep && ng > 0 && i1 == nx;
+    const int f = j <= ncell ? fa + j : (j == ncell + 1 && end0 ? 0 : nx);
+    const bool live = j <= ncell + end0 + end1;
     // Each moment term enters as an exact pair: the FP32 products w fh,
     // w fh u, w fh u^2, w fb with their rounding errors (FMA), added with
     // error-free sums (TwoSum), the two velocities in packed arithmetic.  In a
@@ -450,7 +468,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
     float2 s0 = zero, s1 = zero, s2 = zero, sb = zero, sq2 = zero;  // sums
     float2 l0 = zero, l1 = zero, l2 = zero, lb = zero, lq = zero;  // their rounding errors
     float2 e0 = zero, e1 = zero, e2 = zero;                        // and the products'
-    if (f <= fb) {
+    if (live) {
       const int iL = f - 1, iR = f;
       const bool vlL = brule(iL, nx, ng) == 1, vlR = brule(iR, nx, ng) == 1;
       // window offsets of the three cells around the upwind one (clamped where
@@ -532,8 +550,13 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
     const int m = q / (FT / 4);
     if (q % (FT / 4) == 0) {
       const float half = m < 2 ? 1.f : 0.5f;
-      if (m < 3) sfw[j * 3 + m] = f64_of(half * t.hi) + f64_of(half * t.lo);
-      else sq[j] = half * (t.hi + t.lo);
+      if (m < 3) {
+        const double S = f64_of(half * t.hi) + f64_of(half * t.lo);
+        sfw[j * 3 + m] = S;
+        if (keep && live && (f > i0 || f <= 1)) B.fw[(long)f * 4 + m] = S;  // (face i0: the segment's before)
+      } else {
+        sq[j] = half * (t.hi + t.lo);
+      }
     }
   }
   __syncthreads();  // face moments and heat fluxes in shared memory
@@ -563,7 +586,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
       for (int m = 0; m < 3; ++m) {
         const double d = fL[m] - fR[m];
         wn[m] = fma(d, rdx, swo[lane * 3 + m]);
-        if (res) {
+        if (want) {
           const float df = f32_of(d) * f32_of(rdx);  // the change of w
           rr[m] = df * df;
           rr[3 + m] = fabsf(f32_of(wn[m]));
@@ -579,7 +602,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
       p[0] = pn[0];
       p[1] = pn[1];
       p[2] = pn[2];
-      if (slot >= 0) rate = seg_rate(B, pn, rdx);
+      if (ONE && slot >= 0) rate = seg_rate(B, pn, rdx);
       if (!pos64(pn[0]) || !pos64(pn[2])) atomicOr(B.status, 1);
       // w, prim and q stay FP64; the coefficients below feed only the FP32
       // pointwise update.  The Maxwellian's density factor, U and lambda are
@@ -609,7 +632,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
       for (int n = 0; n < 13; ++n) kp[2 * n] = kc[n];
       seg_store_coef(B, c, mn);
     }
-    if (res) {  // this segment's residual partial sums (k_batch_seg_res adds them up)
+    if (want) {  // this segment's residual partial sums (k_batch_seg_res adds them up)
 #pragma unroll
       for (int m = 0; m < 6; ++m) {
 #pragma unroll
@@ -621,7 +644,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
         for (int m = 0; m < 6; ++m) pr[m] = f64_of(rr[m]);
       }
     }
-    if (slot >= 0) seg_clock_rate(B, slot, rate, c0, ng, i0, i1, nx, sd.rdx, lane);
+    if (ONE && slot >= 0) seg_clock_rate(B, slot, rate, c0, ng, i0, i1, nx, sd.rdx, lane);
   }
   __syncthreads();  // cell coefficients ready for the pointwise update
   // ---- pointwise KFVS flux + relaxation: a thread marches two chunks of L

@@ -92,7 +92,8 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
                                                          int slot) {
   extern __shared__ __align__(16) unsigned char sm64[];
   __shared__ unsigned long long bar;
-  __shared__ double sdt[3];  // dt, time before the step, 1: the step is skipped
+  __shared__ double sdt;     // dt
+  __shared__ int sflag[2];   // the step is skipped; its residual and face moments are kept
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int k = blockIdx.x;
   const int b = B.seg_b[k], i0 = B.seg_i0[k];
@@ -127,20 +128,19 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
   pdl_wait();
   pdl_next();
   if (tid == 0) {
-    sdt[0] = B.dt[b];
-    sdt[2] = B.active[b] ? 0.0 : 1.0;
+    SegClock c = {B.dt[b], 0.0, B.active[b] == 0, false};
     if (slot >= 0) {
-      const SegClock c = seg_clock(B, slot);
-      sdt[0] = c.dt;
-      sdt[1] = c.t;
-      if (c.stop) sdt[2] = 1.0;
+      c = seg_clock(B, slot);
       if (k == 0) seg_clock_next(B, slot, c);
     }
+    sdt = c.dt;
+    sflag[0] = c.stop;
+    sflag[1] = want_res || c.last;
     mbar_init(&bar, 1);
     fence_async_smem();
   }
   __syncthreads();
-  if (sdt[2] != 0.0) {  // converged or past the end: carry this segment's cells over
+  if (sflag[0]) {  // converged or past the end: carry this segment's cells over
     for (long t = tid; t < (long)(i1 - i0) * ns; t += SEG64_T) {
       const long o = (long)(i0 + ng) * ns + t;
       Ho[o] = Hi[o];
@@ -156,11 +156,15 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
     bulk_g2s(sH, Hi + (long)(r0 + ng) * ns, bytes, &bar);
     bulk_g2s(sB, Bi + (long)(r0 + ng) * ns, bytes, &bar);
   }
-  const double dx = B.dx[b], dt = sdt[0];
+  const double dx = B.dx[b], dt = sdt;
   const double rdx = B.rdx[b];
   const double T4 = 0.5 * dt * dt * rdx;
   const int ca = max(i0, 1), cb = min(i1, nx - 1);  // stepped cells [ca, cb)
   const int nc = max(0, cb - ca), nf = nc > 0 ? nc + 1 : 0;  // faces ca .. cb
+  // then the ends' for BatchDev::fw (a segment with an end steps a cell less)
+  const bool want = sflag[1] != 0, keep = want && B.fw;
+  const int end0 = keep && ng > 0 && i0 == 0, end1 = keep && ng > 0 && i1 == nx, nfe = nf + end0 + end1;
+  const auto face = [&](int j) { return j < nf ? ca + j : (j == nf && end0 ? 0 : nx); };
   // the lane that updates a cell (of a warp that changes from segment to
   // segment: its number decides which quarter of the multiprocessor works)
   // reads its w and prim while the window is on its way
@@ -201,9 +205,9 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
   }
   const double epsd = 1.e-7 * dx;
   // ---- 1: fluxes.  fh = dt u (h + side s) - dt^2 u^2 / (2 dx) s = T h + K s
-  for (int t = tid; t < nf * nu; t += SEG64_T) {
+  for (int t = tid; t < nfe * nu; t += SEG64_T) {
     const int j = t / nu, v = t - j * nu;
-    const int up = ca + j - (nonneg64(sU[v]) ? 1 : 0);  // upwind cell
+    const int up = face(j) - (nonneg64(sU[v]) ? 1 : 0);  // upwind cell
     const int o = (up - r0) * ns + v;
     const double h0 = sH[o], b0 = sB[o];
     double sh = 0.0, sb = 0.0;
@@ -216,7 +220,7 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
   }
   __syncthreads();
   // ---- 2: moments of face ca + j and heat flux of cell ca + j
-  for (int j = wid; j < nf; j += SEG64_T / 32) {
+  for (int j = wid; j < nfe; j += SEG64_T / 32) {
     double m0 = 0.0, m1 = 0.0, m2 = 0.0, q = 0.0;
     const double* F = sF + j * ns;
     const double* G = sG + j * ns;
@@ -237,8 +241,13 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
     const double s = warp_sum4(m0, m1, m2, q, lane);
     if ((lane & 7) == 0) {
       const int m = lane >> 3;
-      if (m < 3) sfw[j * 4 + m] = m == 2 ? 0.5 * s : s;
-      else if (j < nc) sq[j * 4] = 0.5 * s;
+      const double S = m < 2 ? s : 0.5 * s;
+      if (m < 3) {
+        sfw[j * 4 + m] = S;
+        if (keep && (face(j) > i0 || face(j) <= 1)) B.fw[(long)face(j) * 4 + m] = S;  // (face i0: the segment's before)
+      } else if (j < nc) {
+        sq[j * 4] = S;
+      }
     }
   }
   __syncthreads();
@@ -278,7 +287,7 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
         p[m] = pn[m];
         B.mc64[cell * 4 + m] = mn[m];
       }
-      if (want_res) {
+      if (want) {
         for (int m = 0; m < 3; ++m) {
           const double d = wn[m] - wo[m];
           rr[m] = d * d;
@@ -288,7 +297,7 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
       if (!pos64(pn[0]) || !pos64(lam)) atomicOr(B.status, 1);
       if (slot >= 0) rate = seg_rate(B, pn, rdx);
     }
-    if (want_res) {
+    if (want) {
 #pragma unroll
       for (int m = 0; m < 6; ++m) rr[m] = warp_sum(rr[m]);
       if (lane == 0) {

@@ -17,7 +17,7 @@ bool line_covers(const kb_config_t& c) {
          c.bc[0] == KB_BC_FIX && c.bc[1] == KB_BC_FIX && c.nu <= SEG_MAXNU;
 }
 
-static const SegVariant kLine32 = {4, 128, 3, (const void*)k_batch_seg<3, 128>, seg_smem<3, 128>,
+static const SegVariant kLine32 = {4, 128, 3, (const void*)k_batch_seg<3, 128, true>, seg_smem<3, 128>,
                                    seg_smem_max<3, 128>()};
 
 int line_seg(int prec, int nx, int sms) {
@@ -95,6 +95,7 @@ bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int 
   d.w = s.w;
   d.prim = s.prim;
   d.residual = s.residual;
+  d.fw = s.fw;
   d.status = s.status;
   d.nseg_all = ns;
   d.sst_max = seg_stride(s.g.vstride);
@@ -135,13 +136,13 @@ int line_step(Line& L, DevState& s, bool res, int slot, cudaStream_t st) {
   const int cur = s.cur;
   if (s.prec == 0) {
     seg64_launch(L.d, L.seg, (const double*)s.h[cur], (const double*)s.b[cur], (double*)s.h[cur ^ 1],
-                 (double*)s.b[cur ^ 1], res || slot >= 0, slot, st);
+                 (double*)s.b[cur ^ 1], res, slot, st);
   } else {
     const float* hin = (const float*)s.h[cur];
     const float* bin = (const float*)s.b[cur];
     float* hout = (float*)s.h[cur ^ 1];
     float* bout = (float*)s.b[cur ^ 1];
-    int want = res || slot >= 0;
+    int want = res;
     void* args[] = {(void*)&L.d, (void*)&hin, (void*)&bin, (void*)&hout, (void*)&bout, (void*)&slot, (void*)&want};
     launch_after(L.f32->fn, dim3((unsigned)L.d.nseg_all), dim3((unsigned)L.f32->threads), (size_t)L.smem, st, args);
   }
