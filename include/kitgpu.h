@@ -179,7 +179,9 @@ int kb_step(kb_handle_t* h, double dt, int32_t nsteps, double* residual);
 /* nsteps steps, each with its own dt: before every step the CFL rate of the
  * current state is reduced on the device (as kb_timestep: timestep,
  * src/Solver/solver_main.jl:240-342) and dt = cfl / rate, clipped to
- * max_time - t; stops early once t reaches max_time.  time_out receives the
+ * max_time - t; stops early once t reaches max_time, and with
+ * KB_ERR_NUMERIC at the step whose state is not physical (the handle keeps
+ * that state).  time_out receives the
  * simulated time reached, residual (may be NULL) the last step's residual.
  * The per-step dt option of the time loop; solve! itself keeps the dt of the
  * initial state (src/Solver/solver_main.jl:12-76). */

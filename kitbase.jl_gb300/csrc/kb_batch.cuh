@@ -222,6 +222,12 @@ __device__ __forceinline__ void seg_clock_next(const BatchDev& B, int slot, cons
 __device__ __forceinline__ double seg_rate(const BatchDev& B, const double* p, double rdx) {
   return (fmax(B.clock[8], fabs(p[1])) + sqrt64((0.5 * B.gamma) * rcp64(p[2]))) * rdx;
 }
+// The rate of a state that no step may follow (not physical, or a wait that gave
+// up): the next step's dt is 0, and the state is carried over from there.
+__device__ __forceinline__ double seg_no_rate() { return __hiloint2double(0x7ff00000, 0); }
+__device__ __forceinline__ void seg_clock_max(const BatchDev& B, int slot, double rate) {
+  atomicMax((unsigned long long*)(B.clock + (slot + 1) % 3), (unsigned long long)__double_as_longlong(rate));
+}
 // The largest rate of a segment's cells (`rate`: the stepped cell of this
 // lane) and of the fixed ends among them into the next slot; one warp.  Rates
 // are positive, so their bits order like unsigned integers.
@@ -231,9 +237,7 @@ __device__ __forceinline__ void seg_clock_rate(const BatchDev& B, int slot, doub
   if (i1 == nx && lane == 1) rate = fmax(rate, seg_rate(B, B.prim + (c0 + nx - 1 + ng) * 4, rdx));
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) rate = fmax(rate, __shfl_xor_sync(0xffffffffu, rate, o));
-  if (lane == 0)
-    atomicMax((unsigned long long*)(B.clock + (slot + 1) % 3),
-              (unsigned long long)__double_as_longlong(rate));
+  if (lane == 0) seg_clock_max(B, slot, rate);
 }
 
 // ---- FP32 form: one CTA per segment of SEG cells, the whole step fused.
@@ -404,6 +408,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
   if (__syncthreads_or(!ok)) {  // CTA-uniform: bounded clean-up, then leave
     if (tid == 0) {
       atomicOr(B.status, 2);
+      if (ONE && slot >= 0) seg_clock_max(B, slot, seg_no_rate());
       mbar_wait(&bar, phase & 1);
     }
     return;
@@ -603,7 +608,10 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
       p[1] = pn[1];
       p[2] = pn[2];
       if (ONE && slot >= 0) rate = seg_rate(B, pn, rdx);
-      if (!pos64(pn[0]) || !pos64(pn[2])) atomicOr(B.status, 1);
+      if (!pos64(pn[0]) || !pos64(pn[2])) {
+        atomicOr(B.status, 1);
+        rate = seg_no_rate();
+      }
       // w, prim and q stay FP64; the coefficients below feed only the FP32
       // pointwise update.  The Maxwellian's density factor, U and lambda are
       // formed in FP64 and rounded once, and U is carried as an FP32 pair

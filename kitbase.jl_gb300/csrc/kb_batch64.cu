@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
   if (__syncthreads_or(!ok)) {  // CTA-uniform: bounded clean-up, then leave
     if (tid == 0) {
       atomicOr(B.status, 2);
+      if (slot >= 0) seg_clock_max(B, slot, seg_no_rate());
       mbar_wait(&bar, 0);
     }
     return;
@@ -294,8 +295,11 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
           rr[3 + m] = fabs(wn[m]);
         }
       }
-      if (!pos64(pn[0]) || !pos64(lam)) atomicOr(B.status, 1);
       if (slot >= 0) rate = seg_rate(B, pn, rdx);
+      if (!pos64(pn[0]) || !pos64(lam)) {
+        atomicOr(B.status, 1);
+        rate = seg_no_rate();
+      }
     }
     if (want) {
 #pragma unroll

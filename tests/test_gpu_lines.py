@@ -1,10 +1,11 @@
 """Single 1D solves that step in the fused segment kernels: what a call returns
-beside the state."""
+beside the state, and where it stops."""
 import numpy as np
 import pytest
 
 import kitgpu
-from cases import oracle_for, shock, sod
+from kitgpu._native import KitGPUError
+from cases import oracle_for, rho_u_t_error, shock, sod
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +51,41 @@ def test_face_moments_of_the_last_step(gpu_lib, how, name, cfg, prec, tol):
         # the sum of a face that has no flux of its own is rounding of its terms
         s = max(np.max(np.abs(ref[:, k])), 0.1 * np.max(np.abs(ref)))
         assert np.max(np.abs(fw[:, k] - ref[:, k])) < tol * s, k
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_adaptive_steps_stop_at_a_state_that_is_not_physical(gpu_lib, prec):
+    """A step far beyond the CFL limit leaves a negative density: the call fails,
+    and the handle holds the state that step left, as after single steps."""
+    out = []
+    for n in (1, 20):
+        KS, ctr, faces, orc, dt = _both(sod(nx=60, nu=33), prec)
+        with pytest.raises(KitGPUError) as e:
+            ctr.handle.step_cfl(40.0, 0.0, 1e9, n)
+        assert e.value.code == -4
+        out.append(ctr.handle.download())
+    assert np.any(out[0]["prim"] <= 0.0)
+    for k in ("w", "prim", "h", "b"):
+        assert np.array_equal(out[0][k], out[1][k], equal_nan=True), k
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("stop", [0.3, 7.5, 66.2])
+def test_end_time_inside_a_chunk(gpu_lib, stop, prec):
+    """An end time before the last step of a call: the shorter last step, then the
+    state is carried over; the time, state and residual of single steps."""
+    KS, a, fa, orc, dt = _both(sod(nx=70, nu=36), prec)
+    KS, b, fb, orc, dt = _both(sod(nx=70, nu=36), prec)
+    end = stop * dt
+    ta, ra = a.handle.step_cfl(KS.set.cfl, 0.0, end, 100)
+    t, rb = 0.0, None
+    while t < end * (1 - 1e-14):
+        d = b.handle.timestep(KS.set.cfl, t, end)
+        rb = b.handle.step(d, 1)
+        t += d
+    tol = 1e-12 if prec == "fp64" else 1e-5
+    assert abs(ta - end) <= 1e-13 * end and abs(t - end) <= 1e-13 * end
+    x, y = a.handle.download(), b.handle.download()
+    assert max(rho_u_t_error(x["prim"], y["prim"])) < tol
+    assert np.max(np.abs(x["h"] - y["h"])) < tol * np.max(y["h"])
+    assert np.allclose(ra, rb, rtol=1e-9 if prec == "fp64" else 1e-4)
