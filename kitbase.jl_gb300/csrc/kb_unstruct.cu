@@ -813,7 +813,9 @@ static int us_set_cells_per_cta(kb_us* U, int cb) {
                                                  : (const void*)kb::k_us_step<double, false>)
                                            : (sk ? (const void*)kb::k_us_step<float, true>
                                                  : (const void*)kb::k_us_step<float, false>);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // The limit belongs to the kernel, not to the handle, so it is the most that any
+  // handle may ask for: a handle's own size would lower it for the others.
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return usfail(KB_ERR_CUDA, "kb_us: cudaFuncSetAttribute failed");
