@@ -661,7 +661,8 @@ extern "C" int kb_batch_set_dt(kb_batch_t* B, const double* dt) {
 
 // One step from buffer `cur`.  The residual kernel sets residuals and
 // convergence flags; with tol = 0 no flag can change, so only the last step of
-// a call needs it (res).  Returns the kernels launched.
+// a call needs it (res).  Returns the kernels launched, or KB_ERR_CUDA when a
+// launch was refused (seen nowhere else).
 static int batch_launch(kb_batch* B, int cur, bool res) {
   int n = 0;
   if (B->prec == KB_PREC_FP32) {  // fused segments (one pass over HBM)
@@ -685,6 +686,8 @@ static int batch_launch(kb_batch* B, int cur, bool res) {
     kb::seg_res_launch(B->d, B->stream);
     ++n;
   }
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return bfail(KB_ERR_CUDA, std::string("batch step launch: ") + cudaGetErrorString(e));
   return n;
 }
 
@@ -699,10 +702,15 @@ static int batch_graph(kb_batch* B) {
   if (cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
     return bfail(KB_ERR_CUDA, "graph capture failed to start");
   const bool res = B->d.tol > 0.0;  // flags may change at every step
-  B->graph_launches = batch_launch(B, B->cur, res);
-  B->graph_launches += batch_launch(B, B->cur ^ 1, res);
-  if (cudaStreamEndCapture(B->stream, &g) != cudaSuccess)
-    return bfail(KB_ERR_CUDA, "graph capture failed");
+  const int n0 = batch_launch(B, B->cur, res), n1 = n0 < 0 ? n0 : batch_launch(B, B->cur ^ 1, res);
+  const cudaError_t ec = cudaStreamEndCapture(B->stream, &g);
+  cudaGetLastError();  // (a refused launch ends the capture too; the next call starts clean)
+  if (n1 < 0) {
+    if (ec == cudaSuccess) cudaGraphDestroy(g);
+    return n1;
+  }
+  if (ec != cudaSuccess) return bfail(KB_ERR_CUDA, "graph capture failed");
+  B->graph_launches = n0 + n1;
   cudaError_t e = cudaGraphInstantiate(&B->graph, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) return bfail(KB_ERR_CUDA, "graph instantiation failed");
@@ -733,7 +741,9 @@ extern "C" int kb_batch_step(kb_batch_t* B, int32_t nsteps, double tol, double* 
     }
   }
   for (; left > 0; --left) {
-    B->launches += batch_launch(B, B->cur, left == 1 || tol > 0.0);
+    const int k = batch_launch(B, B->cur, left == 1 || tol > 0.0);
+    if (k < 0) return k;
+    B->launches += k;
     B->cur ^= 1;
   }
   if (cudaStreamSynchronize(B->stream) != cudaSuccess)

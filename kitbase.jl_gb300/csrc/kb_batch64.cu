@@ -368,13 +368,13 @@ bool seg64_prepare() {
   return ok;
 }
 
-void seg64_launch(const BatchDev& B, int seg, const double* hin, const double* bin, double* hout,
-                  double* bout, bool want_res, int slot, cudaStream_t st) {
-  if (B.nseg_all <= 0) return;
+cudaError_t seg64_launch(const BatchDev& B, int seg, const double* hin, const double* bin, double* hout,
+                         double* bout, bool want_res, int slot, cudaStream_t st) {
+  if (B.nseg_all <= 0) return cudaSuccess;
   int nsm = B.nu4_max, res = want_res ? 1 : 0;
   void* args[] = {(void*)&B, &seg, &nsm, &hin, &bin, &hout, &bout, &res, &slot};
-  launch_after((const void*)k_batch_seg64, dim3((unsigned)B.nseg_all), dim3(SEG64_T),
-               (size_t)seg64_smem(seg, B.nu4_max), st, args);
+  return launch_after((const void*)k_batch_seg64, dim3((unsigned)B.nseg_all), dim3(SEG64_T),
+                      (size_t)seg64_smem(seg, B.nu4_max), st, args);
 }
 
 }  // namespace kb

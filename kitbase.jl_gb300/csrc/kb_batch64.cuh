@@ -18,8 +18,8 @@ int seg64_smem(int seg, int ns);
 bool seg64_prepare();
 // One step of every segment (B.nseg_all CTAs).  want_res: leave the segments'
 // residual sums in B.respart.  slot: see BatchDev::adapt (-1: dt from B.dt).
-void seg64_launch(const BatchDev& B, int seg, const double* hin, const double* bin, double* hout,
-                  double* bout, bool want_res, int slot, cudaStream_t st);
+cudaError_t seg64_launch(const BatchDev& B, int seg, const double* hin, const double* bin, double* hout,
+                         double* bout, bool want_res, int slot, cudaStream_t st);
 // Per-instance residual of the last step that left its sums (k_batch_seg_res).
 void seg_res_launch(const BatchDev& B, cudaStream_t st);
 // Maxwellian coefficients of every cell from its prim (BatchDev::mc64, mc).

@@ -134,8 +134,9 @@ int line_begin(Line& L, const DevState& s, double dt, cudaStream_t st) {
 
 int line_step(Line& L, DevState& s, bool res, int slot, cudaStream_t st) {
   const int cur = s.cur;
+  cudaError_t e;
   if (s.prec == 0) {
-    seg64_launch(L.d, L.seg, (const double*)s.h[cur], (const double*)s.b[cur], (double*)s.h[cur ^ 1],
+    e = seg64_launch(L.d, L.seg, (const double*)s.h[cur], (const double*)s.b[cur], (double*)s.h[cur ^ 1],
                  (double*)s.b[cur ^ 1], res, slot, st);
   } else {
     const float* hin = (const float*)s.h[cur];
@@ -144,8 +145,9 @@ int line_step(Line& L, DevState& s, bool res, int slot, cudaStream_t st) {
     float* bout = (float*)s.b[cur ^ 1];
     int want = res;
     void* args[] = {(void*)&L.d, (void*)&hin, (void*)&bin, (void*)&hout, (void*)&bout, (void*)&slot, (void*)&want};
-    launch_after(L.f32->fn, dim3((unsigned)L.d.nseg_all), dim3((unsigned)L.f32->threads), (size_t)L.smem, st, args);
+    e = launch_after(L.f32->fn, dim3((unsigned)L.d.nseg_all), dim3((unsigned)L.f32->threads), (size_t)L.smem, st, args);
   }
+  if (e != cudaSuccess) return 0;  // the caller's check reports it; the state stays the current one
   s.cur = cur ^ 1;
   if (!res) return 1;
   seg_res_launch(L.d, st);

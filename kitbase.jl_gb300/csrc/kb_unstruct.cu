@@ -1114,8 +1114,16 @@ extern "C" int kb_us_timestep(kb_us_t* U, double cfl, double sim_time, double ma
   return KB_OK;
 }
 
+// An error of the launches so far (a refused launch is seen nowhere else).
+static int us_launched(const char* what) {
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? KB_OK : usfail(KB_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+}
+
+// The next state becomes the current one only when its launches were taken; the
+// first that is refused ends the step (the averages write w and prim in place).
 template <typename R>
-static void us_enqueue_step(kb_us* U, double dt, bool last) {
+static int us_enqueue_step(kb_us* U, double dt, bool last) {
   const kb::UsDev& d = U->d;
   const R* hin = (const R*)U->h[U->cur];
   const R* bin = (const R*)U->b[U->cur];
@@ -1128,6 +1136,8 @@ static void us_enqueue_step(kb_us* U, double dt, bool last) {
     void* args[] = {(void*)&d, &dt, &U->cb, &U->lp, &U->fnu, &res, &hin, &bin, &hout, &bout};
     const void* fn = d.coll == KB_COLL_SHAKHOV ? (const void*)kb::k_us_step<R, true> : (const void*)kb::k_us_step<R, false>;
     kb::launch_after(fn, dim3((unsigned)grid), dim3(kb::US_T), U->smem, U->stream, args);
+    const int rc = us_launched("kb_us_step");
+    if (rc != KB_OK) return rc;
     U->launches++;
   }
   for (size_t l = 0; l + 1 < U->level_first.size(); ++l) {
@@ -1137,17 +1147,18 @@ static void us_enqueue_step(kb_us* U, double dt, bool last) {
     kb::launch_after((const void*)kb::k_us_avg<R>, dim3((unsigned)n), dim3(kb::US_T), 0, U->stream, args);
     U->launches++;
   }
-  U->cur ^= 1;
+  const int rc = us_launched("kb_us_step");
+  if (rc == KB_OK) U->cur ^= 1;
+  return rc;
 }
 
 extern "C" int kb_us_step(kb_us_t* U, double dt, int32_t nsteps, double* residual) {
   if (!U || nsteps < 0) return usfail(KB_ERR_ARG, "kb_us_step: bad argument");
   const kb::UsDev& d = U->d;
   for (int s = 0; s < nsteps; ++s) {
-    if (U->prec == KB_PREC_FP64)
-      us_enqueue_step<double>(U, dt, s == nsteps - 1);
-    else
-      us_enqueue_step<float>(U, dt, s == nsteps - 1);
+    const bool last = s == nsteps - 1;
+    const int rc = U->prec == KB_PREC_FP64 ? us_enqueue_step<double>(U, dt, last) : us_enqueue_step<float>(U, dt, last);
+    if (rc != KB_OK) return rc;
   }
   const double* rows = d.bres;
   int nrows = U->nblk;
@@ -1161,6 +1172,8 @@ extern "C" int kb_us_step(kb_us_t* U, double dt, int32_t nsteps, double* residua
   void* rargs[] = {(void*)&d, &rows, &nrows};
   kb::launch_after((const void*)kb::k_us_residual, dim3(1), dim3(256), 0, U->stream, rargs);
   U->launches++;
+  const int rc = us_launched("kb_us_step");
+  if (rc != KB_OK) return rc;
   if (cudaStreamSynchronize(U->stream) != cudaSuccess)
     return usfail(KB_ERR_CUDA, std::string("kb_us_step: ") + cudaGetErrorString(cudaGetLastError()));
   int st = 0;
