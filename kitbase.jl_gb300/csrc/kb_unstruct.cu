@@ -223,10 +223,12 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
   using R2 = typename Vec2<R>::T;
   constexpr bool FAST = sizeof(R) == 4;
   extern __shared__ __align__(16) unsigned char us_smem[];
-  double* S = (double*)us_smem;                  // [cb << lp][US_NM]
-  R* P = (R*)(S + (cb << lp) * US_NM);           // [cb][US_NP] (room for doubles)
+  double* S = (double*)us_smem;                  // [cb][US_NM]
+  // [cb][US_NP] (room for doubles); until the cell phase a second part's sums (lp 1)
+  // stand in the upper half
+  R* P = (R*)(S + cb * US_NM);
   // [cb][2][vstride]: h, b less the fluxes out of the cell
-  R* D = (R*)(S + (cb << lp) * US_NM + cb * US_NP);
+  R* D = (R*)(S + cb * US_NM + cb * US_NP);
   using GR = typename UsGeoRow<R>::T;
   unsigned char* rec = (unsigned char*)(D + (long)cb * 2 * d.vstride);
   // (in the FP32 form the other order costs 17 %: 9.5 against 11.2 ms for 20 steps
@@ -259,7 +261,7 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
   pdl_wait();
   pdl_next();
   for (int item = wid; item < (nloc << lp); item += US_W) {
-    // a cell, or (FP64, small meshes) every 2^lp-th round of its velocities
+    // a cell, or (FP64, small meshes, lp 1) every second round of its velocities
     const int i = FAST ? item : item >> lp;
     const int q0 = FAST ? lane : lane + 32 * (item & ((1 << lp) - 1)), dq = FAST ? 32 : 32 << lp;
     const int4 rec = RS[i];
@@ -387,7 +389,10 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
 #pragma unroll
     for (int k = 0; k < US_NM; ++k) x[k] = acc[k].s;
     const double t = us_reduce8(x, lane);
-    if ((lane & 3) == 0) S[item * US_NM + (lane >> 2)] = t;
+    if ((lane & 3) == 0) {
+      if (!FAST && (item & ((1 << lp) - 1))) P[i * US_NP + US_NM + (lane >> 2)] = R(t);
+      else S[i * US_NM + (lane >> 2)] = t;
+    }
   }
   __syncthreads();
 
@@ -399,11 +404,10 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
       const int c = RS[lane].x;
       double Sc[US_NM];
 #pragma unroll
-      for (int k = 0; k < US_NM; ++k) Sc[k] = S[(lane << lp) * US_NM + k];
-      if (!FAST)
-        for (int t = 1; t < 1 << lp; ++t)
+      for (int k = 0; k < US_NM; ++k) Sc[k] = S[lane * US_NM + k];
+      if (!FAST && lp)
 #pragma unroll
-          for (int k = 0; k < (SHAK ? 7 : 5); ++k) Sc[k] += S[((lane << lp) + t) * US_NM + k];
+        for (int k = 0; k < (SHAK ? 7 : 5); ++k) Sc[k] += double(P[lane * US_NP + US_NM + k]);
       double* w = d.w + 4L * c;
       double* p = d.prim + 4L * c;
       const double rho_o = p[0], U_o = p[1], V_o = p[2], lam_o = p[3];
@@ -769,34 +773,35 @@ static std::vector<int> us_levels(int ncell, const int32_t* cell_nb, const int32
 // busiest quarter less work (a tenth of a cell's time is the cell phase, a
 // twentieth of a part's its sums): 800 triangles of 256 velocities 7 cells 69
 // us, 6 in two parts 59; 288 of 144 13 cells 96 us, 2 in two parts 33.
+// The parts are the mesh's and velocity grid's, whatever cb is: they order a
+// cell's sums, and cb changes no result.
 static int us_set_cells_per_cta(kb_us* U, int cb) {
   const kb::UsDev& d = U->d;
   const size_t esz = U->prec == KB_PREC_FP64 ? 8 : 4;
   const size_t per = 2 * (size_t)d.vstride * esz + sizeof(int4) + 12 * esz;
-  int lp = 0, dev = 0, maxs = 0, sms = 1;
+  int dev = 0, maxs = 0, sms = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&maxs, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cb == 0) {
-    cb = (int)std::max<size_t>(1, std::min<size_t>(12, (32u << 10) / per));
-    if (cb > kb::US_W) cb -= cb % kb::US_W;
-    if (U->prec == KB_PREC_FP64 && sms > 0) {
-      const auto cost = [&](int c, int l) {
-        const long ctas = (d.nstep + c - 1) / c, per_sm = (ctas + sms - 1) / sms;
-        const long items = (c << l) + kb::US_W - 1;
-        return per_sm * ((items / kb::US_W) * (1.0 / (1 << l) + 0.05) + 0.1);
-      };
-      const int c0 = cb;
-      for (int c = c0; c >= 1; --c)
-        for (int l = 0; l <= (d.vstride > 64 ? 1 : 0); ++l)
-          if (cost(c, l) < 0.97 * cost(cb, lp)) {
-            cb = c;
-            lp = l;
-          }
-    }
+  int c0 = (int)std::max<size_t>(1, std::min<size_t>(12, (32u << 10) / per));
+  if (c0 > kb::US_W) c0 -= c0 % kb::US_W;
+  int best = c0, lp = 0;
+  if (U->prec == KB_PREC_FP64 && sms > 0) {
+    const auto cost = [&](int c, int l) {
+      const long ctas = (d.nstep + c - 1) / c, per_sm = (ctas + sms - 1) / sms;
+      const long items = (c << l) + kb::US_W - 1;
+      return per_sm * ((items / kb::US_W) * (1.0 / (1 << l) + 0.05) + 0.1);
+    };
+    for (int c = c0; c >= 1; --c)
+      for (int l = 0; l <= (d.vstride > 64 ? 1 : 0); ++l)
+        if (cost(c, l) < 0.97 * cost(best, lp)) {
+          best = c;
+          lp = l;
+        }
   }
+  if (cb == 0) cb = best;
   if (cb < 1 || cb > kb::US_CB) return usfail(KB_ERR_ARG, "cells per CTA must be 1 .. 32");
-  size_t smem = (sizeof(double) * ((kb::US_NM << lp) + kb::US_NP) + per) * cb;
+  size_t smem = (sizeof(double) * (kb::US_NM + kb::US_NP) + per) * cb;
   // The factors take the place of the face geometry.  Whether they are used
   // depends on the velocity grid alone (do they fit beside the most cells that
   // do?), so that the number of cells changes no result.

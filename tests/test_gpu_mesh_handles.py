@@ -1,5 +1,5 @@
-"""Triangle-mesh solves side by side: handles of different velocity grids
-and shapes stepped in turn."""
+"""Triangle-mesh solves side by side: handles of different velocity grids and
+shapes stepped in turn, and shapes that change no result."""
 import numpy as np
 import pytest
 
@@ -39,3 +39,21 @@ def test_handles_of_large_and_small_grids_in_turn(gpu_lib, coll, prec):
         got = hd.download()
         assert all(np.array_equal(got[k], ref[k]) for k in ("w", "prim", "h", "b"))
         hd.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,ny,nv,coll", [(3, 3, 5, "bgk"), (5, 4, 9, "shakhov"), (13, 17, 11, "shakhov"),
+                                           (20, 20, 16, "shakhov"), (12, 12, 12, "bgk"), (41, 37, 12, "bgk")])
+def test_cells_per_cta_change_no_result(gpu_lib, nx, ny, nv, coll, prec):
+    """The default and shapes given by hand: the same sums, bit for bit."""
+    KS = _mesh(nv, coll, nx, ny)
+    out = []
+    for cb in (0, 1, 2, 3, 5, 8, 12, 32):
+        hd = US.init_fvm(KS, prec)
+        if cb:
+            hd.set_tuning(cb)
+        hd.step(hd.timestep(), 6)
+        out.append(hd.download())
+        hd.close()
+    for o in out[1:]:
+        assert all(np.array_equal(o[k], out[0][k]) for k in ("w", "prim", "h", "b"))
