@@ -43,8 +43,9 @@
 
 namespace kb {
 
-// FP64 face record of a stepped cell (32-byte aligned, one vector load pair)
-struct alignas(32) UsG64 {
+// FP64 face record of a stepped cell; 16-byte aligned, as its place in shared
+// memory is for any number of cells
+struct alignas(16) UsG64 {
   double n1, n2, len, sgn;
 };
 
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
   // of 294,912 triangles x 256 velocities)
   GR* GS = (GR*)(FAST ? rec : rec + cb * sizeof(int4));               // [cb][3] face geometry
   int4* RS = (int4*)(FAST ? rec + 3 * cb * sizeof(GR) : rec);         // [cb] cell and neighbours
+  static_assert(alignof(GR) <= 16 && sizeof(GR) % 16 == 0, "records follow each other at 16-byte places");
   // FP64 on a product velocity grid (fnu: its nu, else 0): [cb][1 + SHAK][nu + nv]
   // factors of the new and the old Maxwellian, where the geometry was
   double* F = (double*)GS;
