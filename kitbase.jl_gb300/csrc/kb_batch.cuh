@@ -313,7 +313,7 @@ __device__ __forceinline__ DF seg_sums(DF (&x)[4], int lane) {
 // (BatchDev::fw); a form of its own, because they cost the ensembles' 1.6 %.
 template <int SEG, int SEG_T, bool ONE = false>
 __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
-    k_batch_seg(BatchDev B, const float* __restrict__ Hin, const float* __restrict__ Bin,
+    k_batch_seg(BatchDev B, const float* Hin, const float* Bin,
                 float* __restrict__ Hout, float* __restrict__ Bout, int slot, int res) {
   using SH = SegShape<SEG, SEG_T>;
   constexpr int SEG_ROWS = SH::ROWS;

@@ -85,8 +85,8 @@ __device__ __forceinline__ void seg_coef64(const BatchDev& B, const double* p, d
 // segment length or on what else is in the launch: a face's moments are
 // summed in the same lane order wherever the segment starts.
 __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, int nsm,
-                                                         const double* __restrict__ Hin,
-                                                         const double* __restrict__ Bin,
+                                                         const double* Hin,
+                                                         const double* Bin,
                                                          double* __restrict__ Hout,
                                                          double* __restrict__ Bout, int want_res,
                                                          int slot) {

@@ -79,7 +79,7 @@ __device__ __forceinline__ const float* vtab<float>(const DevState& s, int which
 // value of the upwind cell (h + s dx/2 from the left, h - s dx/2 from the
 // right) and that cell's slope (flux_kfvs.jl:35-63 / :98-140 wrappers).
 template <typename R>
-__device__ __forceinline__ R upwind_state(const R* __restrict__ q, long vs, int up, int step,
+__device__ __forceinline__ R upwind_state(const R* q, long vs, int up, int step,
                                           int rule, bool left, int v, R dsc, R dxh, R& slope) {
   R q0 = q[(long)up * vs + v];
   R qm = (rule == 1 || rule == 3) ? q[(long)(up - step) * vs + v] : R(0);

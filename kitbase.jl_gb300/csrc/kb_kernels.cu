@@ -570,8 +570,8 @@ __device__ __forceinline__ FaceCtx<R> make_ctx(const DevState& s, int f, int kin
 // Pointwise flux of one face at velocity v (face-local velocities un, ut);
 // c is the interior cell next to a wall face.
 template <typename R, int D, int FLUX>
-__device__ __forceinline__ void ctx_flux(const FaceCtx<R>& x, const R* __restrict__ H,
-                                         const R* __restrict__ Bq, long vs, int c, int v,
+__device__ __forceinline__ void ctx_flux(const FaceCtx<R>& x, const R* H,
+                                         const R* Bq, long vs, int c, int v,
                                          R un, R ut, R dt, R& fh, R& fb) {
   if (x.kind == 0) {
     fh = R(0);

@@ -72,8 +72,8 @@ __device__ __forceinline__ R slope(int rule, R qm, R q0, R qp, R epsd) {
 }
 
 template <typename R>
-__device__ __forceinline__ R ldq(const R* __restrict__ q, long idx, bool ok) {
-  return ok ? __ldg(q + idx) : R(0);
+__device__ __forceinline__ R ldq(const R* q, long idx, bool ok) {
+  return ok ? q[idx] : R(0);
 }
 
 // Blocked compensated accumulator: plain partial sums, flushed into a
@@ -172,8 +172,8 @@ __device__ __forceinline__ void mom_line(const DevState& s, int blk) {
   const int ncell = min(TS, n - p0);
   const int nf = ncell + (sg == nseg - 1 ? 1 : 0);  // faces p0 .. p0+nf-1
   const long vs = g.vstride;
-  const R* __restrict__ H = (const R*)s.h[s.cur];
-  const R* __restrict__ Bq = (const R*)s.b[s.cur];
+  const R* H = (const R*)s.h[s.cur];
+  const R* Bq = (const R*)s.b[s.cur];
   const R* __restrict__ U = vtab<R>(s, 0);
   const R* __restrict__ V = vtab<R>(s, 1);
   const R* __restrict__ W = vtab<R>(s, 2);
@@ -945,8 +945,8 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
   const int j0 = D == 2 ? blockIdx.y * RY : 0;
   int j1 = D == 2 ? min(g.ny, j0 + RY) : 1;
   const int vs = g.vstride;
-  const R* __restrict__ H = (const R*)s.h[s.cur];
-  const R* __restrict__ Bq = (const R*)s.b[s.cur];
+  const R* H = (const R*)s.h[s.cur];
+  const R* Bq = (const R*)s.b[s.cur];
   R* __restrict__ Ho = (R*)s.h[s.cur ^ 1];
   R* __restrict__ Bo = (R*)s.b[s.cur ^ 1];
 

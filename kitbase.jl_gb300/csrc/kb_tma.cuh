@@ -14,7 +14,10 @@ namespace kb {
 // chain writes, while that one still runs.  pdl_wait returns once the kernels
 // before are complete and their writes are visible: every kernel of a chain
 // calls it, in every thread that reads or writes what they do, before anything
-// else of theirs.
+// else of theirs.  What a kernel of the chain writes is not read-only for the
+// whole of the next, which is resident meanwhile: no pointer to it is const
+// __restrict__, and none of it is read by __ldg (both allow loads that this wait
+// does not order).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 inline cudaError_t launch_after(const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t st, void** args) {

@@ -218,8 +218,8 @@ template <> struct UsGeoRow<double> { using T = UsG64; };
 // spill); the FP64 form 3.
 template <typename R, bool SHAK>
 __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
-    k_us_step(UsDev d, double dt, int cb, int lp, int fnu, int res, const R* __restrict__ hin,
-                                                  const R* __restrict__ bin, R* __restrict__ hout,
+    k_us_step(UsDev d, double dt, int cb, int lp, int fnu, int res, const R* hin,
+                                                  const R* bin, R* __restrict__ hout,
                                                   R* __restrict__ bout) {
   using R2 = typename Vec2<R>::T;
   constexpr bool FAST = sizeof(R) == 4;
@@ -587,8 +587,8 @@ __global__ void __launch_bounds__(US_T, sizeof(R) == 4 ? (SHAK ? 6 : 7) : 3)
 // and the later ones not yet, and a later one's old h, b are read from the
 // input buffer (its output slot is written in a later level).
 template <typename R>
-__global__ void __launch_bounds__(US_T) k_us_avg(UsDev d, int first, const R* __restrict__ hin,
-                                                 const R* __restrict__ bin, R* hout, R* bout) {
+__global__ void __launch_bounds__(US_T) k_us_avg(UsDev d, int first, const R* hin,
+                                                 const R* bin, R* hout, R* bout) {
   const int c = d.avg_list[first + blockIdx.x];
   pdl_wait();
   pdl_next();
