@@ -304,6 +304,13 @@ __device__ __forceinline__ DF seg_sums(DF (&x)[4], int lane) {
   return z;
 }
 
+// A term of the residual in its sum's precision, and the sum in FP64
+template <typename R> __device__ __forceinline__ R seg_res_term(double x);
+template <> __device__ __forceinline__ double seg_res_term<double>(double x) { return x; }
+template <> __device__ __forceinline__ float seg_res_term<float>(double x) { return f32_of(x); }
+__device__ __forceinline__ double seg_res_sum(double x) { return x; }
+__device__ __forceinline__ double seg_res_sum(float x) { return f64_of(x); }
+
 // Segment k covers cells [seg_i0[k], seg_i0[k] + SEG) of instance seg_b[k].
 // A CTA takes segments k = blockIdx.x, blockIdx.x + gridDim.x, ...: one
 // segment each when the grid has a CTA per segment, or a persistent loop
@@ -574,8 +581,6 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
   // The cell warp: the FP64 cell update.
   const int role = (wid + (int)(((unsigned)k * 2654435761u) >> 29)) % (SEG_T / 32);
   if (role == 0) {
-    // residual terms of the cell: a convergence monitor, summed in FP32 below
-    float rr[6] = {0, 0, 0, 0, 0, 0};
     double rate = 0.0;  // CFL rate of the cell's new state (slot >= 0)
     // ---- cell parameters of the stepped cells (one lane per cell, FP64)
     if (lane < ncell) {
@@ -589,13 +594,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
       double wn[3];
 #pragma unroll
       for (int m = 0; m < 3; ++m) {
-        const double d = fL[m] - fR[m];
-        wn[m] = fma(d, rdx, swo[lane * 3 + m]);
-        if (want) {
-          const float df = f32_of(d) * f32_of(rdx);  // the change of w
-          rr[m] = df * df;
-          rr[3 + m] = fabsf(f32_of(wn[m]));
-        }
+        wn[m] = fma(fL[m] - fR[m], rdx, swo[lane * 3 + m]);
         w[m] = wn[m];
       }
       // conserve_prim (src/Theory/theory_macro.jl:185-206), hg = 0.5 / (gamma - 1)
@@ -641,15 +640,28 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
       seg_store_coef(B, c, mn);
     }
     if (want) {  // this segment's residual partial sums (k_batch_seg_res adds them up)
+      // squares of FP64 differences: a convergence monitor that the ensembles sum
+      // in FP32, a single solve in FP64
+      using RR = typename std::conditional<ONE, double, float>::type;
+      RR rr[6] = {0, 0, 0, 0, 0, 0};
+      if (lane < ncell) {
+        const double* w = B.w + (c0 + ca + lane + ng) * 4;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          const double wn = w[m], dw = wn - swo[lane * 3 + m];
+          rr[m] = seg_res_term<RR>(dw * dw);
+          rr[3 + m] = seg_res_term<RR>(fabs(wn));
+        }
+      }
 #pragma unroll
       for (int m = 0; m < 6; ++m) {
 #pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) rr[m] += __shfl_xor_sync(0xffffffffu, rr[m], o);
+        for (int o = (SEG + 1) / 2; o >= 1; o >>= 1) rr[m] += __shfl_xor_sync(0xffffffffu, rr[m], o);
       }
       if (lane == 0) {
         double* pr = B.respart + (long)k * 8;
 #pragma unroll
-        for (int m = 0; m < 6; ++m) pr[m] = f64_of(rr[m]);
+        for (int m = 0; m < 6; ++m) pr[m] = seg_res_sum(rr[m]);
       }
     }
     if (ONE && slot >= 0) seg_clock_rate(B, slot, rate, c0, ng, i0, i1, nx, sd.rdx, lane);

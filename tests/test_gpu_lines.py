@@ -1,5 +1,5 @@
 """Single 1D solves that step in the fused segment kernels: what a call returns
-beside the state, and where it stops."""
+beside the state (face moments, residual, time), and where it stops."""
 import numpy as np
 import pytest
 
@@ -89,3 +89,21 @@ def test_end_time_inside_a_chunk(gpu_lib, stop, prec):
     assert max(rho_u_t_error(x["prim"], y["prim"])) < tol
     assert np.max(np.abs(x["h"] - y["h"])) < tol * np.max(y["h"])
     assert np.allclose(ra, rb, rtol=1e-9 if prec == "fp64" else 1e-4)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("name,cfg", LINES, ids=[c[0] for c in LINES])
+def test_residual_is_the_change_of_w(gpu_lib, name, cfg, prec):
+    """sqrt(sum dw^2 nx) / (sum |w| + 1e-7) of the FP64 w, dw and its sums in FP64
+    in either precision of the distributions: nx roundings of terms of one
+    sign, and a few of the root and quotient (1e-13)."""
+    KS, ctr, faces, orc, dt = _both(cfg, prec)
+    ctr.handle.step(dt, 4)
+    before = ctr.handle.download()["w"]
+    r = ctr.handle.step(dt, 1)
+    after = ctr.handle.download()["w"]
+    nx, ng = KS.ps.nx, ctr.handle.cfg.ngx
+    i = slice(ng + 1, ng + nx - 1)  # the stepped cells
+    dw = after[i] - before[i]
+    want = np.sqrt(np.sum(dw * dw, 0) * nx) / (np.sum(np.abs(after[i]), 0) + 1e-7)
+    assert np.all(np.abs(r - want) <= 1e-13 * want), (r, want)
