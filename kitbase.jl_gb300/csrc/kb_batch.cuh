@@ -304,6 +304,18 @@ __device__ __forceinline__ DF seg_sums(DF (&x)[4], int lane) {
   return z;
 }
 
+// Relaxation factors of a single solve's cell, each rounded once to FP32:
+// dtt = dt / tau, tau = 2 mu lambda^(1 - omega) / rho (the power in FP32), and
+// 1 / (1 + dtt) of the rounded dtt, so that their product is dtt / (1 + dtt) also
+// where dtt is large; from dtm = dt / (2 mu) and om1 = omega - 1
+__device__ __forceinline__ void seg_relax(double dtm, double rho, float lam, float om1, float& dtt, float& i1t) {
+  dtt = f32_of(dtm * rho * f64_of(powf(lam, om1)));
+  i1t = f32_of(rcp64(1.0 + f64_of(dtt)));
+}
+// Its Shakhov factor 0.8 (1 - Pr) lambda^2 q / rho (of the old state)
+__device__ __forceinline__ float seg_heat(double c, double lam, double rho, double q) {
+  return f32_of(c * (lam * lam) * rcp64(rho) * q);
+}
 // A term of the residual in its sum's precision, and the sum in FP64
 template <typename R> __device__ __forceinline__ R seg_res_term(double x);
 template <> __device__ __forceinline__ double seg_res_term<double>(double x) { return x; }
@@ -329,6 +341,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
   __shared__ unsigned long long bar;
   __shared__ float sconst[2];  // T3, T4
   __shared__ int sflag[2];     // (ONE) the step is past the end; its residual and face moments are kept
+  __shared__ double sdtm;      // (ONE) dt / (2 mu)
   // An FP64 instruction holds a quarter of the multiprocessor for 64 cycles
   // whatever its active lanes, so the FP64 cell phase is one warp's, written
   // for few instructions (about 30; the divisions, conversions and compares
@@ -394,6 +407,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
     swo[tid * 3 + 2] = B.w[c * 4 + 2];
     smc[tid * 2] = ((const float4*)(B.mc + c * 8))[0];
     smc[tid * 2 + 1] = ((const float4*)(B.mc + c * 8))[1];
+    if (ONE) *(double*)&smc[tid * 2 + 1].z = B.prim[c * 4 + 2];
   }
   if (tid == SEG_T - 1) {
     double dt0 = B.dt[b];
@@ -404,6 +418,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
         if (k == 0) seg_clock_next(B, slot, c);
       }
       dt0 = c.dt;
+      sdtm = c.dt * B.rmu[b];
       sflag[0] = c.stop;
       sflag[1] = res || c.last;
     }
@@ -568,6 +583,7 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
         if (keep && live && (f > i0 || f <= 1)) B.fw[(long)f * 4 + m] = S;  // (face i0: the segment's before)
       } else {
         sq[j] = half * (t.hi + t.lo);
+        if (ONE && j < ncell) smc[j * 2 + 1].y = half * t.lo - (sq[j] - half * t.hi);
       }
     }
   }
@@ -580,6 +596,12 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
   };
   // The cell warp: the FP64 cell update.
   const int role = (wid + (int)(((unsigned)k * 2654435761u) >> 29)) % (SEG_T / 32);
+  if (ONE && role == 1 && shak && lane < ncell) {
+    // the heat-flux factor (below) in FP64, beside the cell warp
+    const double lo = *(const double*)&smc[lane * 2 + 1].z;
+    const double q = f64_of(sq[lane]) + f64_of(smc[lane * 2 + 1].y);
+    coef(lane, 0)[24] = seg_heat(0.8 * (1.0 - B.Pr), lo, swo[lane * 3], q);
+  }
   if (role == 0) {
     double rate = 0.0;  // CFL rate of the cell's new state (slot >= 0)
     // ---- cell parameters of the stepped cells (one lane per cell, FP64)
@@ -618,11 +640,17 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
       // at high Mach the energy is mostly kinetic, and an FP32-rounded U or
       // density factor would bias the moments of the equilibrium by more
       // than the FP32 split form's 1e-5 budget in T.  tau only sets the
-      // relaxation rate and is formed in FP32.
+      // relaxation rate: FP32 in the ensembles, and in a single solve, as in the
+      // general form, FP64 but for the power.
       SegMax mn;  // the new Maxwellian
       mn.set(pn, B.K);
-      const float tau = sd.mu2 * powf(mn.lam, B.om1f) / f32_of(pn[0]);
-      const float dtt = sconst[0] / tau;
+      float dtt, i1t;
+      if (ONE) {
+        seg_relax(sdtm, pn[0], mn.lam, -B.om1f, dtt, i1t);
+      } else {
+        dtt = sconst[0] / (sd.mu2 * powf(mn.lam, B.om1f) / f32_of(pn[0]));
+        i1t = 1.f / (1.f + dtt);
+      }
       // the old Maxwellian's coefficients are the ones this cell's update
       // formed from the same prim one step earlier (or the set-up formed from
       // the initial prim): read instead of recomputed
@@ -631,12 +659,12 @@ __global__ void __launch_bounds__(SEG_T, SEG < 7 ? 1 : 20 * 32 / SEG_T)
       // dt / tau, 1 / (1 + dt / tau); old Maxwellian (Shakhov): density factor,
       // U (hi, lo), -lambda, K / (2 lambda), and the heat-flux factor
       // 0.8 (1 - Pr) lambda^2 / rho q of the old state
-      const float kc[13] = {mn.rn, mn.Uh, mn.Ul, -mn.lam, mn.cB, dtt, 1.f / (1.f + dtt),
+      const float kc[13] = {mn.rn, mn.Uh, mn.Ul, -mn.lam, mn.cB, dtt, i1t,
                             mo.x,  mo.y,  smc[lane * 2 + 1].x, -mo.z, mo.w,
-                            shak ? B.prf * (mo.z * mo.z) / f32_of(swo[lane * 3]) * sq[lane] : 0.f};
+                            shak && !ONE ? B.prf * (mo.z * mo.z) / f32_of(swo[lane * 3]) * sq[lane] : 0.f};
       float* kp = coef(lane, 0);
 #pragma unroll
-      for (int n = 0; n < 13; ++n) kp[2 * n] = kc[n];
+      for (int n = 0; n < (ONE ? 12 : 13); ++n) kp[2 * n] = kc[n];
       seg_store_coef(B, c, mn);
     }
     if (want) {  // this segment's residual partial sums (k_batch_seg_res adds them up)
