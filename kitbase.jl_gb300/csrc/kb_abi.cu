@@ -294,7 +294,31 @@ int kb_create(const kb_config_t* cfg, const double* u, const double* v, const do
   ALLOC(h->d_scalar, double, 8);
   h->stage_elems = std::min<long>(h->ncell * (long)g.nvel, 32L << 20);
   h->stage_elems = std::max<long>(h->stage_elems, h->ncell * 4);
+  g.tensor = c.dim == 2;
+  for (int k = 0; k < g.nvel && g.tensor; ++k) g.tensor = u[k] == u[k % g.nu] && v[k] == v[k - k % g.nu];
+  h->s.mt_rows = h->s.mt_j0 = 0;
+  h->s.mt_j1 = g.ny;
+  // The factors of the update's Maxwellians stand in the staging buffer, which no
+  // step uses otherwise, for as many rows at a time as it holds: all of them
+  // unless the grid is beyond the buffer's limit (512^2 x 64^2: bands of 128
+  // rows) or has few velocities.  A buffer below 8 MB is raised to 8 rows; where
+  // even those don't fit, the update takes exponentials.  So the sizes alone say
+  // which of the two, and the bits of the results, a solve gets.
+  const long nt = c.nu + c.nv, few = std::min(8, g.ny);
+  if (g.tensor && !f32) {
+    const long need = kb::maxwell_entries(h->s, few) * nt;
+    if (need <= 1L << 20) h->stage_elems = std::max(h->stage_elems, need);
+    long rows = 0;
+    if (need <= h->stage_elems) {
+      const long first = kb::maxwell_entries(h->s, 0), each = kb::maxwell_entries(h->s, 1) - first;
+      rows = std::min<long>(g.ny, (h->stage_elems / nt - first) / each);
+      const long bands = (g.ny + rows - 1) / rows;
+      rows = (g.ny + bands - 1) / bands;
+    }
+    h->s.mt_rows = (int)rows;
+  }
   ALLOC(h->d_stage, double, h->stage_elems);
+  if (h->s.mt_rows) h->s.mt = h->d_stage;
 #undef ALLOC
   h->s.tmaps = nullptr;
   if (c.precision == KB_PREC_FP32 && (rc = make_tmaps(h)) != KB_OK) return bail(rc);
@@ -323,22 +347,6 @@ int kb_create(const kb_config_t* cfg, const double* u, const double* v, const do
     fu[k] = (float)hu[k];
     fv[k] = (float)hv[k];
     fw[k] = (float)hw[k];
-  }
-  g.tensor = c.dim == 2;
-  for (int k = 0; k < g.nvel && g.tensor; ++k)
-    g.tensor = hu[k] == hu[k % g.nu] && hv[k] == hv[k - k % g.nu];
-  // (a grid that leaves no room for the factors takes the exponentials)
-  if (g.tensor && !f32) {
-    void* mt = nullptr;
-    const size_t n = ((c.flux == KB_FLUX_KFVS ? 0 : (size_t)h->nface) +
-                      (c.collision == KB_COLL_SHAKHOV ? 2 : 1) * (size_t)h->ncell) * (size_t)(c.nu + c.nv);
-    if (cudaMalloc(&mt, n * sizeof(double)) == cudaSuccess) {
-      h->allocs.push_back(mt);
-      h->s.mt = (double*)mt;
-      h->bytes += (int64_t)(n * sizeof(double));
-    } else {
-      cudaGetLastError();
-    }
   }
   if (cudaMemcpy((void*)h->s.u, hu.data(), sizeof(double) * g.vstride, cudaMemcpyHostToDevice) ||
       cudaMemcpy((void*)h->s.v, hv.data(), sizeof(double) * g.vstride, cudaMemcpyHostToDevice) ||

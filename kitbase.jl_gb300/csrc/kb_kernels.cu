@@ -455,14 +455,16 @@ __global__ void __launch_bounds__(BS) k_cell_param(DevState sp, double dt_arg, i
 // follows its new one.  128^2 cells x 32^2 velocities, UGKS
 // and BGK: this kernel 71 us, the update 5,205 -> 3,989; 64^2 x 28^2, KCU and
 // Shakhov, walls: 24 us, 1,082 -> 739.
-__global__ void __launch_bounds__(256) k_maxwell_tab(DevState s, int nf) {
+// The entries: the band's x faces, its y faces, its cells (DevState::mt).
+__global__ void __launch_bounds__(256) k_maxwell_tab(DevState s, int faces) {
   pdl_wait();
   pdl_next();
   const Geo& g = s.g;
-  const int nt = g.nu + g.nvel / g.nu;
+  const int nt = g.nu + g.nvel / g.nu, rows = s.mt_j1 - s.mt_j0;
+  const int nfx = faces ? rows * (g.nx + 1) : 0, nf = faces ? nfx + (rows + 1) * g.nx : 0;
   const long t = (long)blockIdx.x * 256 + threadIdx.x;
   const int e = (int)(t / nt), a = (int)(t - (long)e * nt);
-  if (e >= nf + g.nx * g.ny) return;
+  if (e >= nf + g.nx * rows) return;
   const bool isu = a < g.nu;
   const double x = isu ? s.u[a] : s.v[(long)(a - g.nu) * g.nu];
   const double* tab = EXP64_TAB;
@@ -471,18 +473,19 @@ __global__ void __launch_bounds__(256) k_maxwell_tab(DevState s, int nf) {
     return isu ? amp * y : y;  // the amplitude goes with the first axis
   };
   if (e < nf) {
-    if (s.kind[e] == 0) return;
-    const Quad64 E = s.fc64[e].E;
+    const int f = e < nfx ? s.mt_j0 * (g.nx + 1) + e : s.nface_x + s.mt_j0 * g.nx + (e - nfx);
+    if (s.kind[f] == 0) return;
+    const Quad64 E = s.fc64[f].E;
     // y faces: normal v, tangential -u
-    const double U = e < s.nface_x ? (isu ? E.y : E.z) : (isu ? -E.z : E.y);
+    const double U = e < nfx ? (isu ? E.y : E.z) : (isu ? -E.z : E.y);
     s.mt[(long)e * nt + a] = factor(E.x, U, E.w);
     return;
   }
-  const int q = e - nf, j = q / g.nx, c = cell_index(g, q - j * g.nx, j);
-  const CellParam& C = s.cp[c];
+  const int q = e - nf, j = q / g.nx;
+  const CellParam& C = s.cp[cell_index(g, q - j * g.nx, s.mt_j0 + j)];
   if (!C.upd) return;
   const bool shak = s.coll == COLL_SHAKHOV;
-  double* o = s.mt + ((long)nf + (shak ? 2L : 1L) * c) * nt + a;
+  double* o = s.mt + ((long)nf + (shak ? 2L : 1L) * q) * nt + a;
   o[0] = factor(C.rho_n, isu ? C.U : C.V, C.l2);
   if (shak) o[nt] = factor(C.o_rho_n, isu ? C.oU : C.oV, EXP64_LOG2E * C.olam);
 }
@@ -1056,13 +1059,13 @@ int launch_face_param(DevState& s, double dt, cudaStream_t st) {
   return 1;
 }
 
-// The factors of the step's Maxwellians (DevState::mt) of the faces, when the
-// flux evaluates them, and of the cells.
-int launch_maxwell_tab(DevState& s, bool faces, cudaStream_t st) {
-  const int nf = faces ? s.nface_x + s.nface_y : 0;
-  const long n = ((long)nf + (long)s.g.nx * s.g.ny) * (s.g.nu + s.g.nvel / s.g.nu);
+// The factors of the step's Maxwellians (DevState::mt) of the band's faces, when
+// the flux evaluates them, and of its cells.
+int launch_maxwell_tab(const DevState& s, bool faces, cudaStream_t st) {
+  const long rows = s.mt_j1 - s.mt_j0, nx = s.g.nx;
+  const long n = ((faces ? (nx + 1) * rows + nx * (rows + 1) : 0) + nx * rows) * (s.g.nu + s.g.nvel / s.g.nu);
   prefer_max_shared((const void*)k_maxwell_tab);
-  go(k_maxwell_tab, (unsigned)((n + 255) / 256), 256, st, s, nf);
+  go(k_maxwell_tab, (unsigned)((n + 255) / 256), 256, st, s, faces ? 1 : 0);
   return 1;
 }
 

@@ -54,8 +54,10 @@ struct DevState {
   FaceCoef64* fc64; // [nface] FP64 coefficient blocks (FP64 form)
   // FP64 2D on a product velocity grid, else null (k_maxwell_tab): the factors,
   // nu + nv each, of the faces' Maxwellians (not KFVS), then of each cell's new
-  // and, Shakhov, old one
+  // and, Shakhov, old one, for mt_rows rows at a time; the update in hand takes
+  // the rows mt_j0 .. mt_j1 - 1 (all of them without factors)
   double* mt;
+  int mt_rows, mt_j0, mt_j1;
   CellCoef32* cc;   // [ncell] FP32 cell coefficients
   double* blockres; // [nblocks][16] residual partials
   float2* mpart;    // [velocity boxes][2][nface][4] pass-A partials of the row-ring form
@@ -142,7 +144,12 @@ int launch_update(DevState& s, double dt, cudaStream_t st, bool res = true);
 // The same step split into its kernel groups (per-stage timing):
 // evolve = face_param + moments + wall; update = cell_param + march + finish.
 int launch_face_param(DevState& s, double dt, cudaStream_t st);
-int launch_maxwell_tab(DevState& s, bool faces, cudaStream_t st);
+int launch_maxwell_tab(const DevState& s, bool faces, cudaStream_t st);
+// Entries of nu + nv factors that `rows` rows take.
+inline long maxwell_entries(const DevState& s, long rows) {
+  const long nx = s.g.nx, f = s.flux == FLUX_KFVS ? 0 : (nx + 1) * rows + nx * (rows + 1);
+  return f + (s.coll == COLL_SHAKHOV ? 2 : 1) * nx * rows;
+}
 int launch_wall(DevState& s, double dt, cudaStream_t st);
 int launch_cell_param(DevState& s, double dt, cudaStream_t st, bool res = true);
 int launch_finish(DevState& s, cudaStream_t st, bool res = true);

@@ -942,8 +942,8 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
   const int v = vok ? vraw : g.nvel - 1;
   const int i0 = blockIdx.x * TX;
   const int ncol = min(TX, g.nx - i0);
-  const int j0 = D == 2 ? blockIdx.y * RY : 0;
-  int j1 = D == 2 ? min(g.ny, j0 + RY) : 1;
+  const int j0 = D == 2 ? s.mt_j0 + blockIdx.y * RY : 0;
+  int j1 = D == 2 ? min(s.mt_j1, j0 + RY) : 1;
   const int vs = g.vstride;
   const R* H = (const R*)s.h[s.cur];
   const R* Bq = (const R*)s.b[s.cur];
@@ -1008,7 +1008,9 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
   const bool shak = s.coll == COLL_SHAKHOV;
   const int nt = D == 2 ? g.nu + g.nvel / g.nu : 0;
   const Factors fac = {D == 2 && sizeof(R) == 8 ? s.mt : nullptr, D == 2 ? v % g.nu : 0, D == 2 ? g.nu + v / g.nu : 0};
-  const long cfac = FLUX == FLUX_KFVS ? 0 : (long)(s.nface_x + s.nface_y) * nt;  // the cells' factors
+  // the factors of the band's y faces and cells follow those of its x faces
+  const int jb = s.mt_j0, nfx = FLUX == FLUX_KFVS ? 0 : (s.mt_j1 - jb) * (g.nx + 1);
+  const long cfac = FLUX == FLUX_KFVS ? 0 : (long)(nfx + (s.mt_j1 - jb + 1) * g.nx) * nt;
   const long cstep = shak ? 2 * nt : nt;
   const double Kf = g.Kb;
   const FC* fct;
@@ -1100,7 +1102,7 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
         sb = vl_diff(rhi, wb[0][c], wb[1][c], wb[2][c], epsy);
       }
       eval_face<D, FLUX>(e, MY, sys, hu, bu, su, sb, wh[1][c], wb[1][c], tab, fac,
-                         (long)(s.nface_x + j0 * g.nx + i0 + c) * nt, fyh[c], fyb[c]);
+                         (long)(nfx + (j0 - jb) * g.nx + i0 + c) * nt, fyh[c], fyb[c]);
     }
   } else {
     tile(0, wh[1], wb[1]);
@@ -1158,7 +1160,7 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
           sb = slope<FAST>(rhi, wb[1][c], wb[2][c], wb[3][c], epsy);
         }
         eval_face<D, FLUX, FAST>(e, MY, qys, hu, bu, su, sb, wh[1][c], wb[1][c], tab, fac,
-                                 (long)(s.nface_x + (j + 1) * g.nx + i0 + c) * nt, fyh2[c], fyb2[c]);
+                                 (long)(nfx + (j + 1 - jb) * g.nx + i0 + c) * nt, fyh2[c], fyb2[c]);
       }
     }
     // x faces of row j, each with the upwind cell's slope
@@ -1176,8 +1178,8 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
       R sb = vl_diff(ru, qx ? xb[f] : xb[f + 1], bu, qx ? xb[f + 2] : xb[f + 3], epsx);
       R hc = fi == 0 ? xh[f + 2] : xh[f + 1];
       R bc = fi == 0 ? xb[f + 2] : xb[f + 1];
-      eval_face<D, FLUX, FAST>(e, MX, qxs, hu, bu, su, sb, hc, bc, tab, fac, (long)(j * (g.nx + 1) + fi) * nt, fxh[f],
-                               fxb[f]);
+      eval_face<D, FLUX, FAST>(e, MX, qxs, hu, bu, su, sb, hc, bc, tab, fac, (long)((j - jb) * (g.nx + 1) + fi) * nt,
+                               fxh[f], fxb[f]);
     }
     // update the cells of row j
     const long ro = (long)(j + g.ngy) * rows;
@@ -1196,7 +1198,8 @@ __global__ void __launch_bounds__(BS, (sizeof(R) == 4 && TX < 4 ? 384 : 256) / B
         relax(k, shak, u, vv, MX.c2, xh[c + 2], xb[c + 2], dhh, dbb, hn, bn);
       } else {
         const int ci = cell_index(g, i0 + c, j);
-        relax(s.cp[ci], g.rds, u, vv, Kf, D, xh[c + 2], xb[c + 2], dhh, dbb, tab, fac, cfac + ci * cstep, nt, hn, bn);
+        relax(s.cp[ci], g.rds, u, vv, Kf, D, xh[c + 2], xb[c + 2], dhh, dbb, tab, fac,
+              cfac + ((j - jb) * g.nx + i0 + c) * cstep, nt, hn, bn);
       }
       if (vok) {
         Ho[ro + coff[c + 2]] = hn;
@@ -2096,15 +2099,24 @@ static int mom_t(DevState& s, double dt, bool wall, cudaStream_t st) {
 }
 
 template <typename R, int D, int FLUX, int TX, int BS>
-static void march_go(DevState& s, cudaStream_t st) {
+static int march_go(DevState& s, cudaStream_t st) {
   const Geo& g = s.g;
   int ry = shape_of(s).ry;
-  dim3 grid((g.nx + TX - 1) / TX, D == 2 ? (g.ny + ry - 1) / ry : 1, (g.nvel + BS - 1) / BS);
   const int smem = sizeof(R) == 4 && D == 2 ? MarchStage<TX>::BYTES : 0;
-  if (sizeof(R) == 8 && D == 2 && s.mt) launch_maxwell_tab(s, FLUX != FLUX_KFVS, st);
   prefer_max_shared((const void*)k_march<R, D, FLUX, TX, BS>);
-  void* args[] = {(void*)&s, (void*)&ry};
-  launch_after((const void*)k_march<R, D, FLUX, TX, BS>, grid, dim3(BS), smem, st, args);
+  const bool factors = sizeof(R) == 8 && D == 2 && s.mt;
+  const int rows = factors ? s.mt_rows : g.ny;
+  int n = 0;
+  DevState t = s;
+  for (t.mt_j0 = 0; t.mt_j0 < g.ny; t.mt_j0 += rows) {
+    t.mt_j1 = std::min(t.mt_j0 + rows, g.ny);
+    if (factors) n += launch_maxwell_tab(t, FLUX != FLUX_KFVS, st);
+    dim3 grid((g.nx + TX - 1) / TX, D == 2 ? (t.mt_j1 - t.mt_j0 + ry - 1) / ry : 1, (g.nvel + BS - 1) / BS);
+    void* args[] = {(void*)&t, (void*)&ry};
+    launch_after((const void*)k_march<R, D, FLUX, TX, BS>, grid, dim3(BS), smem, st, args);
+    ++n;
+  }
+  return n;
 }
 
 // FP32 2D pass B (k_march3): the tensor maps of the current h / b buffers for
@@ -2140,7 +2152,7 @@ static void march3_go(DevState& s, cudaStream_t st) {
 template <typename R, int D, int FLUX>
 static int march_t(DevState& s, double dt, cudaStream_t st) {
   if constexpr (sizeof(R) == 8) {
-    march_go<R, D, FLUX, 2, 64>(s, st);
+    return march_go<R, D, FLUX, 2, 64>(s, st);
   } else {
     const Shape p = shape_of(s);
     const int tx = p.tx, bs = p.bs;
@@ -2165,7 +2177,7 @@ static int march_t(DevState& s, double dt, cudaStream_t st) {
       }
     }
   }
-  return sizeof(R) == 8 && D == 2 && s.mt ? 2 : 1;
+  return 1;
 }
 
 }  // namespace kb

@@ -116,9 +116,7 @@ def estimate_bytes(cfg, precision):
     nvel = cfg["nu"] * (cfg["nv"] if d == 2 else 1)
     esz = 4 if precision == "fp32" else 8
     nface = (cfg["nx"] + 1) * (cfg.get("ny", 1) if d == 2 else 1) * (2 if d == 2 else 1)
-    # FP64 2D: the Maxwellians' factors of the faces and cells
-    factors = (nface + 2 * ncell) * (cfg["nu"] + cfg["nv"]) * 8 if d == 2 and precision != "fp32" else 0
-    return 4 * ncell * ((nvel + 3) // 4 * 4) * esz + ncell * 1024 + nface * 512 + factors + (1 << 20)
+    return 4 * ncell * ((nvel + 3) // 4 * 4) * esz + ncell * 1024 + nface * 512 + (1 << 20)
 
 
 def pool_bytes(max_cells, max_nu=256):
