@@ -275,6 +275,8 @@ int kb_launch_count(kb_handle_t* h, int64_t* count);
  * handle's stream.  Stages: 0 w slopes (reconstruct!), 1 face parameters,
  * 2 face moments (fw, heat flux), 3 Maxwell walls, 4 cell parameters
  * (w, prim, tau), 5 pointwise update of h and b, 6 ghost fill + residual.
+ * 1D KFVS lines with fixed ends and at most 256 velocities step in one fused
+ * kernel: its time is stage 5's, the stages before are empty.
  * kb_set_timing(h, 1) enables and resets the counters; kb_get_timing returns
  * the accumulated milliseconds and step counts per stage.  No reference
  * counterpart (the reference only wraps solve! in @showprogress). */
@@ -289,7 +291,9 @@ int kb_get_timing(kb_handle_t* h, double* ms, int64_t* count);
  * threads per CTA elsewhere; 128: one velocity per thread, 128 threads),
  * params[3] faces per warp of the moment pass (2, 4) along x and y lines,
  * or 8: both face directions in one launch over the update pass's row rings
- * (2D FP32 BGK; other solves keep the line form).  0 keeps the default.
+ * (2D FP32 BGK; other solves keep the line form).  0 keeps the default.  The
+ * fused kernel of 1D KFVS lines (see kb_set_timing) has no such shapes: the
+ * values are kept, but act on kb_evolve and kb_update alone.
  * No reference counterpart. */
 #define KB_NTUNE 4
 int kb_set_tuning(kb_handle_t* h, const int32_t* params, int32_t n);

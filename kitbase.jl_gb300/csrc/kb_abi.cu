@@ -602,6 +602,12 @@ int kb_update(kb_handle_t* h, double dt, double* residual) {
 static int timed_step(kb_handle* h, double dt, cudaEvent_t* ev) {
   cudaStream_t st = h->stream;
   int n = 0;
+  if (h->line.on) {  // one kernel does the step: all of its time is the update's
+    for (int k = 0; k < 6; ++k) cudaEventRecord(ev[k], st);
+    n = kb::line_step(h->line, h->s, true, -1, st, ev[6]);
+    cudaEventRecord(ev[7], st);
+    return n;
+  }
   cudaEventRecord(ev[0], st);
   n += kb::launch_reconstruct(h->s, st);
   cudaEventRecord(ev[1], st);
@@ -667,6 +673,7 @@ int kb_step(kb_handle_t* h, double dt, int32_t nsteps, double* residual) {
       KB_CUDA(cudaEventCreate(&e));
       h->events.push_back(e);
     }
+    if (h->line.on && nsteps > 0) KB_TRY(check_launch(h, kb::line_begin(h->line, h->s, dt, h->stream)));
     for (int s = 0; s < nsteps; ++s)
       KB_TRY(check_launch(h, timed_step(h, dt, &h->events[(size_t)s * (KB_NSTAGE + 1)])));
     KB_TRY(sync(h));

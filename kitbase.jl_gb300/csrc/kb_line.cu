@@ -132,7 +132,7 @@ int line_begin(Line& L, const DevState& s, double dt, cudaStream_t st) {
   return 1;
 }
 
-int line_step(Line& L, DevState& s, bool res, int slot, cudaStream_t st) {
+int line_step(Line& L, DevState& s, bool res, int slot, cudaStream_t st, cudaEvent_t mid) {
   const int cur = s.cur;
   cudaError_t e;
   if (s.prec == 0) {
@@ -149,6 +149,7 @@ int line_step(Line& L, DevState& s, bool res, int slot, cudaStream_t st) {
   }
   if (e != cudaSuccess) return 0;  // the caller's check reports it; the state stays the current one
   s.cur = cur ^ 1;
+  if (mid) cudaEventRecord(mid, st);
   if (!res) return 1;
   seg_res_launch(L.d, st);
   return 2;

@@ -32,6 +32,7 @@ bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int 
 // number of launches.
 int line_begin(Line& L, const DevState& s, double dt, cudaStream_t st);
 // One step (advances s.cur); res: with its residual.  slot: BatchDev::clock.
-int line_step(Line& L, DevState& s, bool res, int slot, cudaStream_t st);
+// mid: recorded between the step's kernel and the residual's.
+int line_step(Line& L, DevState& s, bool res, int slot, cudaStream_t st, cudaEvent_t mid = nullptr);
 
 }  // namespace kb

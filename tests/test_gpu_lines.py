@@ -107,3 +107,22 @@ def test_residual_is_the_change_of_w(gpu_lib, name, cfg, prec):
     dw = after[i] - before[i]
     want = np.sqrt(np.sum(dw * dw, 0) * nx) / (np.sum(np.abs(after[i]), 0) + 1e-7)
     assert np.all(np.abs(r - want) <= 1e-13 * want), (r, want)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_timed_steps_are_the_steps_of_a_solve(gpu_lib, prec):
+    """Stage timing (kb_set_timing) of a line times the kernels that its solve
+    runs: the same state and residual, bit for bit."""
+    out = []
+    for timed in (False, True):
+        KS, ctr, faces, orc, dt = _both(sod(nx=37, nu=33), prec)
+        ctr.handle.set_timing(timed)
+        r = ctr.handle.step(dt, 5)
+        if timed:
+            st = ctr.handle.timing()
+            assert all(n == 5 for _, n in st.values())
+            assert sum(ms for ms, _ in st.values()) > 0.0
+        s = ctr.handle.download()
+        out.append((r, s["w"], s["prim"], s["h"], s["b"], ctr.handle.faces(dt)[0]))
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
