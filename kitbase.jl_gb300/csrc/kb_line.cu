@@ -17,11 +17,41 @@ bool line_covers(const kb_config_t& c) {
          c.bc[0] == KB_BC_FIX && c.bc[1] == KB_BC_FIX && c.nu <= SEG_MAXNU;
 }
 
-static const SegVariant kLine32 = {4, 128, 3, (const void*)k_batch_seg<3, 128, true>, seg_smem<3, 128>,
-                                   seg_smem_max<3, 128>()};
+static const SegVariant kShort = {4, 128, 3, (const void*)k_batch_seg<3, 128, true>, seg_smem<3, 128>,
+                                  seg_smem_max<3, 128>()};
+static const SegVariant kLong = {16, 128, 15, (const void*)k_batch_seg<15, 128, true>, seg_smem<15, 128>,
+                                 seg_smem_max<15, 128>()};
 
-int line_seg(int prec, int nx, int sms) {
-  return prec == KB_PREC_FP64 ? seg64_cells(nx, sms) : kLine32.cells;
+// FP32: segments of three cells while the GPU holds all of them at once, and so a
+// step is one segment's latency; longer lines, whose segments queue, by fifteen,
+// which read 19 rows of the window for 15 cells and not 7 for 3, and run the
+// cell phase a fifth as often.  us a step, 3 / 15 cells (the general form):
+// 1000 x 100 7.2 / 9.2 (62), 2048 x 48 12.0 / 7.6 (59), 2048 x 256 15.5 / 13.5
+// (73), 20,000 x 256 117 / 51 (159), 100,000 x 48 436 / 84 (412), 400,000 x 48
+// 1,865 / 350 (1,551).
+static const SegVariant* line_variant(const kb_config_t& c, int vstride, int sms) {
+  for (const SegVariant* v : {&kShort, &kLong}) {
+    if (cudaFuncSetAttribute(v->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v->smem_max) != cudaSuccess)
+      return nullptr;
+    prefer_max_shared(v->fn);
+  }
+  int per = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kShort.fn, kShort.threads,
+                                                    kShort.smem(seg_stride(vstride), vstride)) != cudaSuccess)
+    return nullptr;
+  return (c.nx + kShort.cells - 1) / kShort.cells <= (long)per * sms ? &kShort : &kLong;
+}
+
+bool line_shape(Line& L, const kb_config_t& c, const DevState& s) {
+  if (s.prec == 0) {
+    L.seg = seg64_cells(c.nx, s.sm_count);
+    return seg64_prepare();
+  }
+  L.f32 = line_variant(c, s.g.vstride, s.sm_count);
+  if (!L.f32) return false;
+  L.seg = L.f32->cells;
+  L.smem = L.f32->smem(seg_stride(s.g.vstride), s.g.vstride);
+  return true;
 }
 
 // the segments' descriptors; ints: nx, ng, nu, nus, vel_off, active, seg_first, nseg, then seg_b and
@@ -36,7 +66,8 @@ size_t line_bytes(const kb_config_t& c, int ncell, int seg) {
   return sizeof(SegDesc) * (size_t)line_nseg(c, seg) + 8 * line_doubles(c, seg) + 4 * line_floats(c, ncell) + 4 * line_ints(c, seg);
 }
 
-bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int seg, void* mem) {
+bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, void* mem) {
+  const int seg = L.seg;
   const int ns = line_nseg(c, seg);
   SegDesc* G = (SegDesc*)mem;
   double* D = (double*)(G + ns);
@@ -107,17 +138,6 @@ bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int 
   seg_gas(d);
   d.tol = 0.0;
   d.coll = s.coll;
-  L.seg = seg;
-  if (s.prec == 0) {
-    if (!seg64_prepare()) return false;
-  } else {
-    L.f32 = &kLine32;
-    L.smem = kLine32.smem(d.sst_max, d.nu4_max);
-    if (cudaFuncSetAttribute(kLine32.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kLine32.smem_max) !=
-        cudaSuccess)
-      return false;
-    prefer_max_shared(kLine32.fn);
-  }
   L.on = true;
   return true;
 }

@@ -21,12 +21,13 @@ struct Line {
 // The solves the segment kernels cover: 1D2F1V, KFVS, fixed ends, van Leer,
 // at most 256 velocities.
 bool line_covers(const kb_config_t& c);
-// Cells per segment for a line of nx cells.
-int line_seg(int prec, int nx, int sms);
+// Choose the segment kernel and its cells per segment (L.seg, L.f32, L.smem);
+// outside any capture.
+bool line_shape(Line& L, const kb_config_t& c, const DevState& s);
 // Bytes of one allocation for the tables of nx cells (ncell incl. ghosts)
 size_t line_bytes(const kb_config_t& c, int ncell, int seg);
-// Fill `mem` (line_bytes) and L for the solve in s; outside any capture.
-bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, int seg, void* mem);
+// Fill `mem` (line_bytes) and L for the solve in s, after line_shape.
+bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, void* mem);
 // Before steps with time step dt (outside any capture): the step in device
 // memory and the Maxwellian coefficients of the current prim.  Returns the
 // number of launches.

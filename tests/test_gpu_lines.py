@@ -126,3 +126,28 @@ def test_timed_steps_are_the_steps_of_a_solve(gpu_lib, prec):
         out.append((r, s["w"], s["prim"], s["h"], s["b"], ctr.handle.faces(dt)[0]))
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("nx,nu", [(2048, 100), (5000, 33), (20011, 20)])
+def test_long_lines_against_oracle(gpu_lib, nx, nu):
+    """FP32 lines of more segments than the GPU holds at once."""
+    KS, ctr, faces, orc, dt = _both(sod(nx=nx, nu=nu), "fp32")
+    kitgpu.step(KS, ctr, dt, 8)
+    orc.step(dt, 8)
+    got, ref = ctr.handle.download(), orc.get_state()
+    assert max(rho_u_t_error(got["prim"], ref[1])) < 1e-5
+    for key, x in (("h", ref[2]), ("b", ref[3])):
+        assert np.max(np.abs(got[key] - x)) < 1e-5 * np.max(np.abs(x)), key
+
+
+def test_fp32_line_at_mach_8(gpu_lib):
+    """500 steps of a single Mach 8 shock in the FP32 split form: rho, U and T
+    within 1e-5 of FP64, as the ensembles' members."""
+    st = []
+    for prec in ("fp64", "fp32"):
+        KS, ctr, *faces, t = kitgpu.initialize(shock(nx=100, nu=128, Ma=8.0, ng=0), precision=prec)
+        if prec == "fp64":
+            dt = kitgpu.timestep(KS, ctr, 0.0)
+        kitgpu.step(KS, ctr, dt, 500)
+        st.append(ctr.handle.download()["prim"])
+    assert max(rho_u_t_error(st[1], st[0])) < 1e-5
