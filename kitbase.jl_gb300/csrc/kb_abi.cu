@@ -377,7 +377,7 @@ int kb_create(const kb_config_t* cfg, const double* u, const double* v, const do
   if (kb::line_covers(c)) {
     if (!kb::line_shape(h->line, c, h->s)) return bail(fail(KB_ERR_CUDA, "segment kernel attributes refused"));
     if ((rc = dev_alloc(h, &p, kb::line_bytes(c, (int)h->ncell, h->line.seg))) != KB_OK) return bail(rc);
-    if (!kb::line_init(h->line, c, h->s, (int)h->ncell, p))
+    if (!kb::line_init(h->line, c, h->s, u, (int)h->ncell, p))
       return bail(fail(KB_ERR_CUDA, "segment kernel set-up failed"));
   }
   // the set-up copies above are synchronous; wait for this handle's stream

@@ -54,46 +54,58 @@ bool line_shape(Line& L, const kb_config_t& c, const DevState& s) {
   return true;
 }
 
-// the segments' descriptors; ints: nx, ng, nu, nus, vel_off, active, seg_first, nseg, then seg_b and
-// seg_i0; longs: cell_off, elem_off; doubles: dx, dt, mu, 1/dx, 1/(2 mu),
-// clock[10], respart, FP64 mc64; floats: ul, FP32 mc
-static int line_nseg(const kb_config_t& c, int seg) { return (c.nx + seg - 1) / seg; }
-static size_t line_doubles(const kb_config_t& c, int seg) { return 18 + 8 * (size_t)line_nseg(c, seg); }
-// (8 floats or 4 doubles of Maxwellian coefficients per cell: the same room)
-static size_t line_floats(const kb_config_t& c, int ncell) { return (size_t)(c.nu + 3) / 4 * 4 + 8 * (size_t)ncell; }
-static size_t line_ints(const kb_config_t& c, int seg) { return 8 + 2 * (size_t)line_nseg(c, seg); }
-size_t line_bytes(const kb_config_t& c, int ncell, int seg) {
-  return sizeof(SegDesc) * (size_t)line_nseg(c, seg) + 8 * line_doubles(c, seg) + 4 * line_floats(c, ncell) + 4 * line_ints(c, seg);
-}
+// One allocation: the tables that kb_create uploads in one copy (the FP32 kernel's
+// descriptors, head, ul, ints), then the residual's sums and the Maxwellian
+// coefficients.
+struct LineHead {
+  long cell_off, elem_off;
+  double dx, dt, mu, rdx, rmu, clock[10], pad;
+};
+static_assert(sizeof(LineHead) % 16 == 0, "what follows is read by 16 bytes");
+struct LinePlan {
+  int ns;  // segments
+  size_t head, ul, ints, copy, respart, mc, total;  // byte offsets; copy: bytes uploaded
+  LinePlan(const kb_config_t& c, int ncell, int seg) {
+    const auto up = [](size_t x) { return (x + 15) / 16 * 16; };
+    ns = (c.nx + seg - 1) / seg;
+    head = c.precision == KB_PREC_FP64 ? 0 : sizeof(SegDesc) * (size_t)ns;
+    ul = head + sizeof(LineHead);
+    ints = up(ul + 4 * (size_t)c.nu);
+    copy = ints + 4 * (8 + (c.precision == KB_PREC_FP64 ? 2 * (size_t)ns : 0));  // nx, ng, nu, nus, vel_off, active,
+    respart = up(copy);                                                          // seg_first, nseg; FP64: seg_b, seg_i0
+    mc = respart + 64 * (size_t)ns;
+    total = mc + 32 * (size_t)ncell;  // 8 floats or 4 doubles of coefficients per cell
+  }
+};
+size_t line_bytes(const kb_config_t& c, int ncell, int seg) { return LinePlan(c, ncell, seg).total; }
 
-bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, void* mem) {
-  const int seg = L.seg;
-  const int ns = line_nseg(c, seg);
-  SegDesc* G = (SegDesc*)mem;
-  double* D = (double*)(G + ns);
-  float* F = (float*)(D + line_doubles(c, seg));
-  int* I = (int*)(F + line_floats(c, ncell));
-  std::vector<double> hd(line_doubles(c, seg), 0.0);
-  std::vector<float> hf(line_floats(c, ncell), 0.f);
-  std::vector<int> hi(line_ints(c, seg), 0);
-  hd[2] = s.g.dx;
-  hd[4] = s.g.mu_ref;
-  hd[5] = 1.0 / s.g.dx;
-  hd[6] = 1.0 / (2.0 * s.g.mu_ref);
-  std::vector<double> u(c.nu);
-  if (cudaMemcpy(u.data(), s.u, sizeof(double) * c.nu, cudaMemcpyDeviceToHost) != cudaSuccess) return false;
+bool line_init(Line& L, const kb_config_t& c, const DevState& s, const double* u, int ncell, void* mem) {
+  const LinePlan P(c, ncell, L.seg);
+  const int ns = P.ns, seg = L.seg;
+  std::vector<char> host(P.copy, 0);
+  LineHead& H = *(LineHead*)(host.data() + P.head);
+  H.dx = s.g.dx;
+  H.mu = s.g.mu_ref;
+  H.rdx = 1.0 / s.g.dx;
+  H.rmu = 1.0 / (2.0 * s.g.mu_ref);
+  float* hf = (float*)(host.data() + P.ul);
   for (int k = 0; k < c.nu; ++k) hf[k] = float(u[k] - (double)(float)u[k]);
+  int* hi = (int*)(host.data() + P.ints);
   const int head[8] = {c.nx, c.ngx, c.nu, s.g.vstride, 0, 1, 0, ns};
   for (int k = 0; k < 8; ++k) hi[k] = head[k];
-  for (int k = 0; k < ns; ++k) hi[8 + ns + k] = k * seg;  // seg_b stays 0
-  std::vector<SegDesc> hg(ns);
-  for (int k = 0; k < ns; ++k)
-    hg[k] = {0, k * seg, c.nx, c.ngx, c.nu, s.g.vstride, 0, 0, 0, 0, hd[5], float(1.e-7 * s.g.dx), 2.f * float(s.g.mu_ref)};
-  if (cudaMemcpy(G, hg.data(), sizeof(SegDesc) * hg.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(D, hd.data(), 8 * hd.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(F, hf.data(), 4 * hf.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(I, hi.data(), 4 * hi.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+  if (s.prec == 0) {
+    for (int k = 0; k < ns; ++k) hi[8 + ns + k] = k * seg;  // seg_b stays 0
+  } else {
+    SegDesc* G = (SegDesc*)host.data();
+    for (int k = 0; k < ns; ++k)
+      G[k] = {0, k * seg, c.nx, c.ngx, c.nu, s.g.vstride, 0, 0, 0, 0, H.rdx, float(1.e-7 * s.g.dx), 2.f * float(s.g.mu_ref)};
+  }
+  char* M = (char*)mem;
+  if (cudaMemcpy(M, host.data(), P.copy, cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemset(M + P.respart, 0, 64 * (size_t)ns) != cudaSuccess)
     return false;
+  const LineHead* D = (const LineHead*)(M + P.head);
+  int* I = (int*)(M + P.ints);
   BatchDev& d = L.d;
   d.n = 1;
   d.nx = I;
@@ -106,23 +118,23 @@ bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, void
   d.nseg = I + 7;
   d.seg_b = I + 8;
   d.seg_i0 = I + 8 + ns;
-  d.seg_d = G;
-  d.cell_off = (const long*)D;
-  d.elem_off = (const long*)(D + 1);
-  d.dx = D + 2;
-  d.dt = D + 3;
-  d.mu = D + 4;
-  d.rdx = D + 5;
-  d.rmu = D + 6;
-  d.clock = D + 7;
-  d.respart = D + 18;
+  d.seg_d = (const SegDesc*)M;
+  d.cell_off = &D->cell_off;
+  d.elem_off = &D->elem_off;
+  d.dx = &D->dx;
+  d.dt = &D->dt;
+  d.mu = &D->mu;
+  d.rdx = &D->rdx;
+  d.rmu = &D->rmu;
+  d.clock = (double*)D->clock;
+  d.respart = (double*)(M + P.respart);
   d.u = s.u;
   d.wt = s.wt;
   d.uf = s.uf;
   d.wtf = s.wtf;
-  d.ul = F;
-  d.mc = F + (c.nu + 3) / 4 * 4;
-  d.mc64 = (double*)d.mc;
+  d.ul = (const float*)(M + P.ul);
+  d.mc = (float*)(M + P.mc);
+  d.mc64 = (double*)(M + P.mc);
   d.w = s.w;
   d.prim = s.prim;
   d.residual = s.residual;

@@ -26,8 +26,9 @@ bool line_covers(const kb_config_t& c);
 bool line_shape(Line& L, const kb_config_t& c, const DevState& s);
 // Bytes of one allocation for the tables of nx cells (ncell incl. ghosts)
 size_t line_bytes(const kb_config_t& c, int ncell, int seg);
-// Fill `mem` (line_bytes) and L for the solve in s, after line_shape.
-bool line_init(Line& L, const kb_config_t& c, const DevState& s, int ncell, void* mem);
+// Fill `mem` (line_bytes) and L for the solve in s, after line_shape; u: the
+// host's velocities.
+bool line_init(Line& L, const kb_config_t& c, const DevState& s, const double* u, int ncell, void* mem);
 // Before steps with time step dt (outside any capture): the step in device
 // memory and the Maxwellian coefficients of the current prim.  Returns the
 // number of launches.
