@@ -378,7 +378,7 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   int *d_nus, *d_segb, *d_segi0, *d_segfirst, *d_nseg;
   double* d_respart;
   long *d_co, *d_eo;
-  double *d_dx, *d_rdx, *d_dt, *d_mu, *d_rmu, *d_mc64, *d_u, *d_w, *d_wv, *d_prim, *d_res;
+  double *d_dx, *d_rdx, *d_dt, *d_rmu, *d_mc64, *d_u, *d_w, *d_wv, *d_prim, *d_res;
   float *d_uf, *d_wf, *d_ul, *d_mc;
   BALLOC(d_nx, int, n);
   BALLOC(d_ng, int, n);
@@ -397,7 +397,6 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   BALLOC(d_eo, long, n);
   BALLOC(d_dx, double, n);
   BALLOC(d_dt, double, n);
-  BALLOC(d_mu, double, n);
   BALLOC(d_rdx, double, n);
   BALLOC(d_rmu, double, n);
   BALLOC(d_u, double, vels);
@@ -438,7 +437,6 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   ok &= cudaMemcpy(d_eo, B->elem_off.data(), sizeof(long) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_dx, dx.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_dt, dt.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
-  ok &= cudaMemcpy(d_mu, mu.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_rdx, rdx.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_rmu, rmu.data(), sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess;
   ok &= cudaMemcpy(d_u, u_all, sizeof(double) * vels, cudaMemcpyHostToDevice) == cudaSuccess;
@@ -476,7 +474,6 @@ extern "C" int kb_batch_create(const kb_config_t* base, int32_t n, const int32_t
   d.vel_off = d_vo;
   d.dx = d_dx;
   d.dt = d_dt;
-  d.mu = d_mu;
   d.rdx = d_rdx;
   d.rmu = d_rmu;
   d.u = d_u;
@@ -899,7 +896,7 @@ extern "C" int kb_pool_add(kb_batch_t* B, int32_t nx, int32_t ngx, int32_t nu, d
   B->mu[b] = mu_ref;
   bool ok = put1(B->d.nx, b, (int)nx) && put1(B->d.ng, b, (int)ngx) && put1(B->d.nu, b, (int)nu) &&
             put1(B->d.nus, b, (int)nus) && put1(B->d.cell_off, b, co) && put1(B->d.elem_off, b, eo) &&
-            put1(B->d.vel_off, b, (int)vo) && put1(B->d.dx, b, dx) && put1(B->d.mu, b, mu_ref) &&
+            put1(B->d.vel_off, b, (int)vo) && put1(B->d.dx, b, dx) &&
             put1(B->d.rdx, b, 1.0 / dx) && put1(B->d.rmu, b, 1.0 / (2.0 * mu_ref)) &&
             put1((const double*)B->d_umax, b, umax);
   std::vector<float> uf(nu), ul(nu), wf(nu);

@@ -39,7 +39,6 @@ struct BatchDev {
   const double* dx;      // cell size
   const double* rdx;     // 1 / dx
   const double* dt;      // time step
-  const double* mu;      // reference viscosity
   const double* rmu;     // 1 / (2 mu)
   const double* u;       // velocity tables (FP64)
   const double* wt;

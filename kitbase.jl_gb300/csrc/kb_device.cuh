@@ -64,13 +64,12 @@ inline void geo_consts(Geo& g) {
 }
 
 // Interface quantities of one face in the face-local frame.  KFVS uses only
-// `mult`; KCU adds the equilibrium part (prim, Mt[0..1], fwa); UGKS all of it.
+// `tr` and `len`; KCU adds the equilibrium part (prim, Mt[0..1], fwa); UGKS all of it.
 struct FaceParam {
   double prim[4];   // rho, U_n, U_t, lambda at the interface (1D: U_t = 0)
   double Mt[5];     // time integration coefficients
   double aL[4], aR[4], aT[4];
   double fwa[4];    // analytic (equilibrium) part of fw, local frame, times len
-  double mult;      // factor applied to the discrete moments (len or 1)
   double len;       // face length (1 in 1D)
   double Mxi2;      // <xi^4> moment of the interface Maxwellian
   double tr[2];     // transport coefficients incl. len: Th = tr0 un h_face - tr1 un^2 sh
@@ -372,11 +371,6 @@ __device__ __forceinline__ DF df_shfl_xor(DF a, int m) {
   r.lo = __shfl_xor_sync(0xffffffffu, a.lo, m);
   return r;
 }
-__device__ __forceinline__ double df_warp_sum(DF a) {
-#pragma unroll
-  for (int m = 16; m >= 1; m >>= 1) a = df_merge(a, df_shfl_xor(a, m));
-  return f64_of(a.hi) + f64_of(a.lo);
-}
 
 // Sums of N values over the warp (N a power of two, at most 32): a
 // reduce-scatter whose first log2 N levels halve the number of values a lane
@@ -422,14 +416,12 @@ struct Acc<double> {
   double s;
   __device__ __forceinline__ Acc() : s(0.0) {}
   __device__ __forceinline__ void add(double x) { s += x; }
-  __device__ __forceinline__ double total() { return warp_sum(s); }
 };
 template <>
 struct Acc<float> {
   DF s;
   __device__ __forceinline__ Acc() { s.hi = 0.f; s.lo = 0.f; }
   __device__ __forceinline__ void add(float x) { df_add(s, x); }
-  __device__ __forceinline__ double total() { return df_warp_sum(s); }
 };
 
 // exp of a Maxwellian exponent

@@ -160,7 +160,6 @@ __global__ void k_face_param(DevState sp, double dt_arg) {
   P.tr[0] = P.tr[1] = 0;
   double hl = 0.0;
   if (FLUX == FLUX_KFVS) {
-    P.mult = 1.0;
     P.tr[0] = dt * len;
     P.tr[1] = 0.5 * (dt * dt) * len;
   } else {
@@ -220,7 +219,6 @@ __global__ void k_face_param(DevState sp, double dt_arg) {
     double Muv[4] = {Mu[1], Mu[2], 0.0, 0.0};
     if (NW == 4) Muv[2] = Mu[1] * V;
     Muv[E] = 0.5 * fma(Mu[1], v2 + x1, Mu[3]);
-    P.mult = len;
     if (FLUX == FLUX_KCU) {
       const double tau = rcp64(itau) + fabs(pj) * rcp64(ps) * (2.0 * dt);
       P.Mt[1] = tau * (1.0 - t_exp_neg<FAST>(dt * rcp64(tau), tab));
@@ -831,12 +829,6 @@ static void conv_rows(T* dev, double* host, long ncell, int nvel, int vs, cudaSt
   k_conv_rows<T, OUT><<<(unsigned)((n + per - 1) / per), CONV_T, 0, st>>>(dev, host, n, (unsigned)nvel, vs);
 }
 
-__global__ void k_pack_w(double* dst4, const double* src, long ncell, int nw) {
-  long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncell) return;
-  for (int k = 0; k < 4; ++k) dst4[c * 4 + k] = k < nw ? src[c * nw + k] : 0.0;
-}
-
 // timestep: max over physical cells (src/Solver/solver_main.jl:240-342); one block.
 // Maximum over the physical cells of the CFL rate; each block reduces its
 // cells, then one atomic max per block on the bit pattern (the rates are
@@ -1235,11 +1227,6 @@ int launch_convert_out(double* dst, int prec, const void* src, long ncell, int n
     k_conv<double, double><<<nb, 256, 0, st>>>(dst, (const double*)src, ncell, nvel, nvel, vstride, cpb);
   else
     k_conv<double, float><<<nb, 256, 0, st>>>(dst, (const float*)src, ncell, nvel, nvel, vstride, cpb);
-  return 1;
-}
-
-int launch_pack_w(double* dst4, const double* src, long ncell, int nw, cudaStream_t st) {
-  k_pack_w<<<nblk(ncell, 256), 256, 0, st>>>(dst4, src, ncell, nw);
   return 1;
 }
 

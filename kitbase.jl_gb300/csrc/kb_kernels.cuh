@@ -170,7 +170,6 @@ int launch_convert_in(void* dst, int prec, const double* src, long ncell, int nv
                       cudaStream_t st);
 int launch_convert_out(double* dst, int prec, const void* src, long ncell, int nvel,
                        int vstride, cudaStream_t st);
-int launch_pack_w(double* dst4, const double* src, long ncell, int nw, cudaStream_t st);
 
 // Equilibrium h, b of every cell from its prim into buffer 0, of ghost cells
 // into both buffers.

@@ -59,7 +59,7 @@ bool line_shape(Line& L, const kb_config_t& c, const DevState& s) {
 // coefficients.
 struct LineHead {
   long cell_off, elem_off;
-  double dx, dt, mu, rdx, rmu, clock[10], pad;
+  double dx, dt, rdx, rmu, clock[10];
 };
 static_assert(sizeof(LineHead) % 16 == 0, "what follows is read by 16 bytes");
 struct LinePlan {
@@ -85,7 +85,6 @@ bool line_init(Line& L, const kb_config_t& c, const DevState& s, const double* u
   std::vector<char> host(P.copy, 0);
   LineHead& H = *(LineHead*)(host.data() + P.head);
   H.dx = s.g.dx;
-  H.mu = s.g.mu_ref;
   H.rdx = 1.0 / s.g.dx;
   H.rmu = 1.0 / (2.0 * s.g.mu_ref);
   float* hf = (float*)(host.data() + P.ul);
@@ -123,7 +122,6 @@ bool line_init(Line& L, const kb_config_t& c, const DevState& s, const double* u
   d.elem_off = &D->elem_off;
   d.dx = &D->dx;
   d.dt = &D->dt;
-  d.mu = &D->mu;
   d.rdx = &D->rdx;
   d.rmu = &D->rmu;
   d.clock = (double*)D->clock;

@@ -85,17 +85,12 @@ struct BAcc<float> {
   float p;
   DF d;
   __device__ __forceinline__ void init() { p = 0.f; d.hi = 0.f; d.lo = 0.f; }
-  __device__ __forceinline__ void add(float x) { p += x; }
   __device__ __forceinline__ void flush() { df_add(d, p); p = 0.f; }
-  __device__ __forceinline__ double total() { flush(); return df_warp_sum(d); }
 };
 template <>
 struct BAcc<double> {
   double p;
   __device__ __forceinline__ void init() { p = 0.0; }
-  __device__ __forceinline__ void add(double x) { p += x; }
-  __device__ __forceinline__ void flush() {}
-  __device__ __forceinline__ double total() { return warp_sum(p); }
 };
 
 // ------------------------------------------------------------------ pass A
@@ -1554,25 +1549,15 @@ __global__ void __launch_bounds__(M3_BS) k_march3(const __grid_constant__ CUtens
 
 // ------------------------------------ pass B, FP32 2D, two velocities per thread
 
-// Packed FP32 pair arithmetic (one instruction for both lanes of a float2).
-__device__ __forceinline__ float2 f2add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 f2mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 f2sub(float2 a, float2 b) {
-  unsigned long long A = *reinterpret_cast<unsigned long long*>(&a);
-  unsigned long long B = *reinterpret_cast<unsigned long long*>(&b), C;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(C) : "l"(A), "l"(B));
-  return *reinterpret_cast<float2*>(&C);
-}
-__device__ __forceinline__ float2 f2s(float s) { return make_float2(s, s); }
+// 2^x of both values of a pair
 __device__ __forceinline__ float2 f2ex2(float2 a) { return make_float2(ex2(a.x), ex2(a.y)); }
 
 // van Leer slope (times dx) of a pair, interior cells (rule 1)
 __device__ __forceinline__ float2 vl2(float2 qm, float2 q0, float2 qp, float epsd) {
-  const float2 a = f2sub(q0, qm), b = f2sub(qp, q0);
+  const float2 a = p2sub(q0, qm), b = p2sub(qp, q0);
   const float2 A = make_float2(fabsf(a.x), fabsf(a.y)), B = make_float2(fabsf(b.x), fabsf(b.y));
-  const float2 num = f2fma(b, A, f2mul(a, B));
-  const float2 den = f2add(f2add(A, B), f2s(epsd));
+  const float2 num = p2fma(b, A, p2mul(a, B));
+  const float2 den = p2add(p2add(A, B), p2s(epsd));
   return make_float2(fdiv_ftz(num.x, den.x), fdiv_ftz(num.y, den.y));
 }
 // general slope of a pair: per-lane rules (boundary cells)
@@ -1587,8 +1572,8 @@ struct Mono2 {
   __device__ __forceinline__ void set(float2 a, float2 b) {
     un = a;
     ut = b;
-    c2 = f2fma(a, a, f2mul(b, b));
-    n2 = f2mul(a, a);
+    c2 = p2fma(a, a, p2mul(b, b));
+    n2 = p2mul(a, a);
   }
   __device__ __forceinline__ Mono<float> lane(int k) const {
     Mono<float> M;
@@ -1611,28 +1596,28 @@ __device__ __forceinline__ void eval_face2(const FEv<float>& e, const Mono2& M, 
     eval_face<D, FLUX>(e, M.lane(1), side.y, hu.y, bu.y, su.y, sb.y, hc.y, bc.y, nullptr, fh.y, fb.y);
     return;
   }
-  const float2 hf = f2fma(side, su, hu), bf = f2fma(side, sb, bu);
-  const float2 a = f2mul(f2s(e.T.x), M.un);
-  const float2 c = f2mul(f2s(-e.T.y), M.n2);
-  fh = f2fma(c, su, f2mul(a, hf));
-  fb = f2fma(c, sb, f2mul(a, bf));
+  const float2 hf = p2fma(side, su, hu), bf = p2fma(side, sb, bu);
+  const float2 a = p2mul(p2s(e.T.x), M.un);
+  const float2 c = p2mul(p2s(-e.T.y), M.n2);
+  fh = p2fma(c, su, p2mul(a, hf));
+  fb = p2fma(c, sb, p2mul(a, bf));
   if (FLUX == FLUX_KFVS) return;
   const float2 Hm = f2ex2(
-      f2fma(f2s(e.E.w), M.c2, f2fma(f2s(e.E.z), M.ut, f2fma(f2s(e.E.y), M.un, f2s(e.E.x)))));
-  float2 ph = f2s(e.T.z), pb = f2s(e.T.w);
+      p2fma(p2s(e.E.w), M.c2, p2fma(p2s(e.E.z), M.ut, p2fma(p2s(e.E.y), M.un, p2s(e.E.x)))));
+  float2 ph = p2s(e.T.z), pb = p2s(e.T.w);
   if (FLUX == FLUX_UGKS) {
-    float2 ih = f2fma(f2s(e.C.w), M.c2, f2fma(f2s(e.C.y), M.un, f2s(e.C.x)));
-    float2 ib = f2fma(f2s(e.Dd.w), M.c2, f2fma(f2s(e.Dd.y), M.un, f2s(e.Dd.x)));
+    float2 ih = p2fma(p2s(e.C.w), M.c2, p2fma(p2s(e.C.y), M.un, p2s(e.C.x)));
+    float2 ib = p2fma(p2s(e.Dd.w), M.c2, p2fma(p2s(e.Dd.y), M.un, p2s(e.Dd.x)));
     if (D == 2) {
-      ih = f2fma(f2s(e.C.z), M.ut, ih);
-      ib = f2fma(f2s(e.Dd.z), M.ut, ib);
+      ih = p2fma(p2s(e.C.z), M.ut, ih);
+      ib = p2fma(p2s(e.Dd.z), M.ut, ib);
     }
-    ph = f2fma(f2s(e.G.y), M.c2, f2fma(f2s(e.G.x), M.ut, f2fma(M.un, ih, ph)));
-    pb = f2fma(f2s(e.G.w), M.c2, f2fma(f2s(e.G.z), M.ut, f2fma(M.un, ib, pb)));
+    ph = p2fma(p2s(e.G.y), M.c2, p2fma(p2s(e.G.x), M.ut, p2fma(M.un, ih, ph)));
+    pb = p2fma(p2s(e.G.w), M.c2, p2fma(p2s(e.G.z), M.ut, p2fma(M.un, ib, pb)));
   }
-  const float2 Hu = f2mul(Hm, M.un);
-  fh = f2fma(Hu, ph, fh);
-  fb = f2fma(Hu, pb, fb);
+  const float2 Hu = p2mul(Hm, M.un);
+  fh = p2fma(Hu, ph, fh);
+  fb = p2fma(Hu, pb, fb);
 }
 
 // pointwise relaxation of a velocity pair (same formulas as relax)
@@ -1640,19 +1625,19 @@ __device__ __forceinline__ void relax2(const CellCoef32& k, bool shak, float2 u,
                                        float2 c2, float2 h0, float2 b0, float2 dh, float2 db,
                                        float2& hn, float2& bn) {
   const float2 M = f2ex2(
-      f2fma(f2s(k.EM.w), c2, f2fma(f2s(k.EM.z), vv, f2fma(f2s(k.EM.y), u, f2s(k.EM.x)))));
-  float2 MH = M, MB = f2mul(M, f2s(k.A.x));
+      p2fma(p2s(k.EM.w), c2, p2fma(p2s(k.EM.z), vv, p2fma(p2s(k.EM.y), u, p2s(k.EM.x)))));
+  float2 MH = M, MB = p2mul(M, p2s(k.A.x));
   if (shak) {
     const float2 OH = f2ex2(
-        f2fma(f2s(k.EO.w), c2, f2fma(f2s(k.EO.z), vv, f2fma(f2s(k.EO.y), u, f2s(k.EO.x)))));
-    const float2 cq = f2mul(f2fma(f2s(k.Q.z), vv, f2fma(f2s(k.Q.y), u, f2s(k.Q.x))), OH);
+        p2fma(p2s(k.EO.w), c2, p2fma(p2s(k.EO.z), vv, p2fma(p2s(k.EO.y), u, p2s(k.EO.x)))));
+    const float2 cq = p2mul(p2fma(p2s(k.Q.z), vv, p2fma(p2s(k.Q.y), u, p2s(k.Q.x))), OH);
     const float2 tl =
-        f2fma(f2s(k.TL.w), c2, f2fma(f2s(k.TL.z), vv, f2fma(f2s(k.TL.y), u, f2s(k.TL.x))));
-    MH = f2fma(cq, f2add(tl, f2s(-5.f)), MH);
-    MB = f2fma(f2mul(cq, f2add(tl, f2s(-3.f))), f2s(k.Q.w), MB);
+        p2fma(p2s(k.TL.w), c2, p2fma(p2s(k.TL.z), vv, p2fma(p2s(k.TL.y), u, p2s(k.TL.x))));
+    MH = p2fma(cq, p2add(tl, p2s(-5.f)), MH);
+    MB = p2fma(p2mul(cq, p2add(tl, p2s(-3.f))), p2s(k.Q.w), MB);
   }
-  hn = f2mul(f2fma(f2s(k.A.y), MH, f2fma(dh, f2s(k.A.w), h0)), f2s(k.A.z));
-  bn = f2mul(f2fma(f2s(k.A.y), MB, f2fma(db, f2s(k.A.w), b0)), f2s(k.A.z));
+  hn = p2mul(p2fma(p2s(k.A.y), MH, p2fma(dh, p2s(k.A.w), h0)), p2s(k.A.z));
+  bn = p2mul(p2fma(p2s(k.A.y), MB, p2fma(db, p2s(k.A.w), b0)), p2s(k.A.z));
 }
 
 // Pass B in the 2D FP32 form with two adjacent velocities per thread: the
@@ -1782,8 +1767,8 @@ __global__ void __launch_bounds__(M4_THREADS * G, G == 2 ? 4 : 1) k_march4(const
   auto yface = [&](int ql, int c, auto fast_tag, auto same_tag, float2& fh, float2& fb) {
     constexpr bool FAST = decltype(fast_tag)::value;
     constexpr bool SAME = decltype(same_tag)::value;  // both lanes share their upwind sides
-    fh = f2s(0.f);
-    fb = f2s(0.f);
+    fh = p2s(0.f);
+    fb = p2s(0.f);
     if (!FAST && cg + c >= ncol) return;
     const int w = cg + c + 2;
     const int qa = pya ? ql - 1 : ql, qb = pyb ? ql - 1 : ql;  // stencil rows start
@@ -1829,7 +1814,7 @@ __global__ void __launch_bounds__(M4_THREADS * G, G == 2 ? 4 : 1) k_march4(const
       e.C = cpa[0];
       e.Dd = cpa[1];
     }
-    float2 hc = f2s(0.f), bc = f2s(0.f);
+    float2 hc = p2s(0.f), bc = p2s(0.f);
     if (!FAST) {
       const unsigned char* Si = slot(ql + 1 == 0 ? ql + 1 : ql);
       hc = Hp(Si, w);
@@ -1880,8 +1865,8 @@ __global__ void __launch_bounds__(M4_THREADS * G, G == 2 ? 4 : 1) k_march4(const
     float2 fxh[TXG + 1], fxb[TXG + 1];
 #pragma unroll
     for (int f = 0; f <= TXG; ++f) {
-      fxh[f] = f2s(0.f);
-      fxb[f] = f2s(0.f);
+      fxh[f] = p2s(0.f);
+      fxb[f] = p2s(0.f);
       if (!FAST && cg + f > ncol) continue;
       float2 su, sb;
       if (FAST) {
@@ -1912,7 +1897,7 @@ __global__ void __launch_bounds__(M4_THREADS * G, G == 2 ? 4 : 1) k_march4(const
         e.C = cp[0];
         e.Dd = cp[1];
       }
-      float2 hc = f2s(0.f), bc = f2s(0.f);
+      float2 hc = p2s(0.f), bc = p2s(0.f);
       if (!FAST) {
         hc = Hp(Sj, cg + (fi == 0 ? f + 2 : f + 1));
         bc = Bp(Sj, cg + (fi == 0 ? f + 2 : f + 1));
@@ -1924,8 +1909,8 @@ __global__ void __launch_bounds__(M4_THREADS * G, G == 2 ? 4 : 1) k_march4(const
 #pragma unroll
     for (int c = 0; c < TXG; ++c) {
       if (!FAST && cg + c >= ncol) continue;
-      const float2 dhh = f2sub(f2add(f2sub(fxh[c], fxh[c + 1]), fyh[c]), fyh2[c]);
-      const float2 dbb = f2sub(f2add(f2sub(fxb[c], fxb[c + 1]), fyb[c]), fyb2[c]);
+      const float2 dhh = p2sub(p2add(p2sub(fxh[c], fxh[c + 1]), fyh[c]), fyh2[c]);
+      const float2 dbb = p2sub(p2add(p2sub(fxb[c], fxb[c + 1]), fyb[c]), fyb2[c]);
       float2 hn, bn;
       relax2(cc[cg + c], shak, u, vv, MX.c2, Hp(Sj, cg + c + 2), Bp(Sj, cg + c + 2), dhh, dbb,
              hn, bn);

@@ -61,10 +61,10 @@ __device__ __forceinline__ float ma_reduce16(const float (&x)[16], int lane) {
 struct MaWeight {
   float2 o, o1, ot, oc;
   __device__ __forceinline__ void set(float2 om, const Mono2& M) {
-    o = f2mul(om, M.un);
-    o1 = f2mul(o, M.un);
-    ot = f2mul(o, M.ut);
-    oc = f2fma(ot, M.ut, f2mul(o1, M.un));
+    o = p2mul(om, M.un);
+    o1 = p2mul(o, M.un);
+    ot = p2mul(o, M.ut);
+    oc = p2fma(ot, M.ut, p2mul(o1, M.un));
   }
 };
 // Free-transport moments of one face for a velocity pair, k_mom_st's
@@ -72,10 +72,10 @@ struct MaWeight {
 // enters in k_mom_fin.
 __device__ __forceinline__ float4 ma_moments(float ct, const Mono2& M, const MaWeight& W, float2 side,
                                              float2 h0, float2 b0, float2 su, float2 sb) {
-  const float2 k = f2fma(f2s(-ct), M.un, side);
-  const float2 X = f2fma(k, su, h0), Y = f2fma(k, sb, b0);
-  const float2 m0 = f2mul(W.o, X), m1 = f2mul(W.o1, X), m2 = f2mul(W.ot, X);
-  const float2 m3 = f2fma(W.oc, X, f2mul(W.o, Y));
+  const float2 k = p2fma(p2s(-ct), M.un, side);
+  const float2 X = p2fma(k, su, h0), Y = p2fma(k, sb, b0);
+  const float2 m0 = p2mul(W.o, X), m1 = p2mul(W.o1, X), m2 = p2mul(W.ot, X);
+  const float2 m3 = p2fma(W.oc, X, p2mul(W.o, Y));
   return make_float4(m0.x + m0.y, m1.x + m1.y, m2.x + m2.y, m3.x + m3.y);
 }
 __device__ __forceinline__ float ma_ratio(const float4& T) { return T.x > 0.f ? T.y / T.x : 0.f; }
