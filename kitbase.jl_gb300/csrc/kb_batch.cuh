@@ -309,7 +309,10 @@ __device__ __forceinline__ DF seg_sums(DF (&x)[4], int lane) {
 // where dtt is large; from dtm = dt / (2 mu) and om1 = omega - 1
 __device__ __forceinline__ void seg_relax(double dtm, double rho, float lam, float om1, float& dtt, float& i1t) {
   dtt = f32_of(dtm * rho * f64_of(powf(lam, om1)));
-  i1t = f32_of(rcp64(1.0 + f64_of(dtt)));
+  // 1 / (1 + dtt): the sum as s + e exactly, its reciprocal corrected by one
+  // Newton step (FP32: the FP64 form holds the cell warp 0.2 us longer)
+  const float s = 1.f + dtt, b = s - 1.f, e = (1.f - (s - b)) + (dtt - b), r = __frcp_rn(s);
+  i1t = fmaf(r, fmaf(-s, r, 1.f) - e * r, r);
 }
 // Its Shakhov factor 0.8 (1 - Pr) lambda^2 q / rho (of the old state)
 __device__ __forceinline__ float seg_heat(double c, double lam, double rho, double q) {
