@@ -184,6 +184,13 @@ __device__ __forceinline__ double exp2_tab(double a, double b, const double* tab
   if ((__double2hiint(t) & 0x7fffffff) >= 0x7ff80000) return t;
   return __hiloint2double(d < 0 ? 0 : 0x7ff00000, 0);
 }
+// log2 x of a positive normal x within FP32's range: the FP32 value l, and
+// log2(1 + t), t = x 2^-l - 1, |t| < 1e-6, by two terms (the third is below 1e-18)
+__device__ __forceinline__ double log2_tab(double x, const double* tab) {
+  const double l = f64_of(log2f(f32_of(x)));
+  const double t = fma(x, exp2_tab(-EXP64_N, l, tab), -1.0);
+  return fma(t * 1.442695040888963407359924681001892137, fma(-0.5, t, 1.0), l);
+}
 // -lambda (u - U)^2 as a 256th of a power of two: a = EXP64_LOG2E lambda
 constexpr double EXP64_LOG2E = -256.0 * 1.442695040888963407359924681001892137;
 

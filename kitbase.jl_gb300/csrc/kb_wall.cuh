@@ -9,12 +9,14 @@
 namespace kb {
 
 // log2-form exponent of rho (lam/pi)^(D/2) exp(-lam ((un-U)^2 + (ut-V)^2)) as
-// E.x + E.y un + E.z ut + E.w c2; the log2 of the density factor in FP32.
-__device__ __forceinline__ float4 maxwell_exp2(double rho_n, double U, double V, double lam) {
+// E.x + E.y un + E.z ut + E.w c2; the log2 of the density factor in FP32, or (tab)
+// in FP64: a wall's Maxwellian is rounded to FP32 once.
+__device__ __forceinline__ float4 maxwell_exp2(double rho_n, double U, double V, double lam,
+                                               const double* tab = nullptr) {
   float4 E;
   const float rf = f32_of(rho_n);
   const double ll = lam * LOG2E, lU = ll * U, lV = ll * V;
-  E.x = rf > 0.f ? f32_of(f64_of(log2f(rf)) - fma(lU, U, lV * V)) : -200.f;
+  E.x = rf > 0.f ? f32_of((tab ? log2_tab(rho_n, tab) : f64_of(log2f(rf))) - fma(lU, U, lV * V)) : -200.f;
   E.y = f32_of(lU + lU);
   E.z = f32_of(lV + lV);
   E.w = f32_of(-ll);
@@ -138,7 +140,7 @@ __device__ __forceinline__ void wall_face(const DevState& sp, double dt_arg, int
     FaceCoef32 wc;
     float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
     wc.G = wc.Cp = wc.Dp = wc.Cm = wc.Dm = z;
-    wc.E = maxwell_exp2(rn, bw[1], bw[2], lw);
+    wc.E = maxwell_exp2(rn, bw[1], bw[2], lw, tab);
     wc.T = make_float4(f32_of(sc), 0.f, f32_of(cBw), rot > 0 ? 1.f : -1.f);
     s.fc[f] = wc;
   } else {
