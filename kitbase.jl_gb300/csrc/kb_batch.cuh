@@ -251,9 +251,10 @@ __device__ __forceinline__ void seg_clock_rate(const BatchDev& B, int slot, doub
 // by k_batch_seg_res after the step, in segment order (deterministic).
 //
 // What bounds it: instruction issue.  512 shock structures (115,000 cells of 48
-// to 200 velocities, 210 MB a step, 31 us of HBM) take 164 us a step: the face
+// to 200 velocities, 210 MB a step, 31 us of HBM) take 157 us a step: the face
 // moments about 65 (two thirds of it the exact sums), the pointwise update 54,
-// the FP64 cell warp 18, the window's latency the rest.  189 us before packed
+// the FP64 cell warp 18, the window's latency the rest.  164 us with the clock of
+// single solves in the same kernel, 189 before packed
 // pairs, one descriptor load in front of the window (five dependent ones took
 // 6,200 of a CTA's 36,000 cycles), sums merged by shuffles instead of by the
 // cell warp, and two chunks of cells per thread instead of one velocity per

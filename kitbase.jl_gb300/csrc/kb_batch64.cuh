@@ -17,7 +17,8 @@ int seg64_smem(int seg, int ns);
 // stream capture).  False when the device refuses.
 bool seg64_prepare();
 // One step of every segment (B.nseg_all CTAs).  want_res: leave the segments'
-// residual sums in B.respart.  slot: see BatchDev::adapt (-1: dt from B.dt).
+// residual sums in B.respart, and their face moments where B.fw is given.  slot:
+// see BatchDev::clock (-1: dt from B.dt).
 cudaError_t seg64_launch(const BatchDev& B, int seg, const double* hin, const double* bin, double* hout,
                          double* bout, bool want_res, int slot, cudaStream_t st);
 // Per-instance residual of the last step that left its sums (k_batch_seg_res).

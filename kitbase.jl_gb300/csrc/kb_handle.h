@@ -23,7 +23,8 @@ struct kb_handle {
   int64_t bytes = 0;
   int64_t launches = 0;
   std::vector<void*> allocs;
-  double* d_stage = nullptr;  // host-layout staging buffer for up/downloads
+  double* d_stage = nullptr;  // host-layout staging buffer for up/downloads; between
+                              // them the factors of an FP64 2D step (DevState::mt)
   long stage_elems = 0;
   double* d_scalar = nullptr; // [8] scratch scalars
   bool evolved = false;
@@ -34,7 +35,8 @@ struct kb_handle {
   // chunks of kb_step_async replayed as CUDA graphs: one executable graph per
   // starting buffer index, valid for one (dt, nsteps) and the current tuning
   cudaGraphExec_t agraph[2] = {nullptr, nullptr};
-  // kb_step's long runs: two steps recorded per starting buffer for one dt
+  // kb_step's long runs: two steps recorded per starting buffer for one dt (a
+  // line: 16, for any dt)
   cudaGraphExec_t sgraph[2] = {nullptr, nullptr};
   double sgraph_dt = 0.0;
   int64_t sgraph_launches = 0;

@@ -6,16 +6,17 @@
 // src/Solver/update_boundary.jl:575-594; timestep for unstructured cells,
 // src/Solver/solver_main.jl:398-420).
 //
-// One fused kernel per step, one CTA per stepped cell: the CTA reads its own
-// h, b and its three neighbours' (gathered through the index tables), forms
-// the first-order KFVS flux of each of its three faces for every velocity and
-// the faces' moments fw (block sums), updates w and prim, and relaxes h, b
-// with the fluxes formed again in a second sweep (the neighbours' values are
-// then in L1).  The face fluxes are never stored: each interior face is
-// formed by both of its cells, with the same inputs, the same operation
-// order (explicitly rounded operations, no contraction) and the same
-// velocity partition of the block sums, so both sides see bit-identical fw
-// and the update stays conservative.  New h, b go to the other buffer of a
+// One fused kernel per step; a CTA steps some consecutive cells of the step
+// list.  A warp takes a cell: it reads the cell's h, b and its three neighbours'
+// (gathered through the index tables), forms the first-order KFVS flux of the
+// three faces for every velocity, keeps h, b less the fluxes in shared memory and
+// sums the cell's moments; then one lane per cell updates w and prim, and the
+// warps relax h, b from shared memory, so that no row is read again.  The face
+// fluxes are never stored: each interior face is formed by both of its cells,
+// with the same inputs and explicitly rounded operations (no contraction), and
+// the order of a cell's sums is the mesh's and velocity grid's whatever the
+// number of cells per CTA, so both sides see the same fluxes and the update stays
+// conservative.  New h, b go to the other buffer of a
 // ping-pong pair (neighbours must read the old state); fixed cells hold the
 // same values in both.  The extrapolated boundary cells are then set in
 // dependency levels (see kb_us_create) that reproduce the reference's
