@@ -161,10 +161,7 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
   const double T4 = 0.5 * dt * dt * rdx;
   const int ca = max(i0, 1), cb = min(i1, nx - 1);  // stepped cells [ca, cb)
   const int nc = max(0, cb - ca), nf = nc > 0 ? nc + 1 : 0;  // faces ca .. cb
-  // then the ends' for BatchDev::fw (a segment with an end steps a cell less)
-  const bool want = sflag[1] != 0, keep = want && B.fw;
-  const int end0 = keep && ng > 0 && i0 == 0, end1 = keep && ng > 0 && i1 == nx, nfe = nf + end0 + end1;
-  const auto face = [&](int j) { return j < nf ? ca + j : (j == nf && end0 ? 0 : nx); };
+  const bool want = sflag[1] != 0;
   // the lane that updates a cell (of a warp that changes from segment to
   // segment: its number decides which quarter of the multiprocessor works)
   // reads its w and prim while the window is on its way
@@ -206,9 +203,8 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
   }
   const double epsd = 1.e-7 * dx;
   // ---- 1: fluxes.  fh = dt u (h + side s) - dt^2 u^2 / (2 dx) s = T h + K s
-  for (int t = tid; t < nfe * nu; t += SEG64_T) {
-    const int j = t / nu, v = t - j * nu;
-    const int up = face(j) - (nonneg64(sU[v]) ? 1 : 0);  // upwind cell
+  const auto flux = [&](int f, int v, double& fh, double& fb) {
+    const int up = f - (nonneg64(sU[v]) ? 1 : 0);  // upwind cell
     const int o = (up - r0) * ns + v;
     const double h0 = sH[o], b0 = sB[o];
     double sh = 0.0, sb = 0.0;
@@ -216,12 +212,16 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
       sh = vl64(sH[o - ns], h0, sH[o + ns], epsd);
       sb = vl64(sB[o - ns], b0, sB[o + ns], epsd);
     }
-    sF[j * ns + v] = fma(sK[v], sh, sT[v] * h0);
-    sG[j * ns + v] = fma(sK[v], sb, sT[v] * b0);
+    fh = fma(sK[v], sh, sT[v] * h0);
+    fb = fma(sK[v], sb, sT[v] * b0);
+  };
+  for (int t = tid; t < nf * nu; t += SEG64_T) {
+    const int j = t / nu, v = t - j * nu;
+    flux(ca + j, v, sF[j * ns + v], sG[j * ns + v]);
   }
   __syncthreads();
   // ---- 2: moments of face ca + j and heat flux of cell ca + j
-  for (int j = wid; j < nfe; j += SEG64_T / 32) {
+  for (int j = wid; j < nf; j += SEG64_T / 32) {
     double m0 = 0.0, m1 = 0.0, m2 = 0.0, q = 0.0;
     const double* F = sF + j * ns;
     const double* G = sG + j * ns;
@@ -242,13 +242,8 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
     const double s = warp_sum4(m0, m1, m2, q, lane);
     if ((lane & 7) == 0) {
       const int m = lane >> 3;
-      const double S = m < 2 ? s : 0.5 * s;
-      if (m < 3) {
-        sfw[j * 4 + m] = S;
-        if (keep && (face(j) > i0 || face(j) <= 1)) B.fw[(long)face(j) * 4 + m] = S;  // (face i0: the segment's before)
-      } else if (j < nc) {
-        sq[j * 4] = S;
-      }
+      if (m < 3) sfw[j * 4 + m] = m == 2 ? 0.5 * s : s;
+      else if (j < nc) sq[j * 4] = 0.5 * s;
     }
   }
   __syncthreads();
@@ -295,11 +290,9 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
           rr[3 + m] = fabs(wn[m]);
         }
       }
-      if (slot >= 0) rate = seg_rate(B, pn, rdx);
-      if (!pos64(pn[0]) || !pos64(lam)) {
-        atomicOr(B.status, 1);
-        rate = seg_no_rate();
-      }
+      const bool good = pos64(pn[0]) && pos64(lam);
+      if (!good) atomicOr(B.status, 1);
+      if (slot >= 0) rate = good ? seg_rate(B, pn, rdx) : seg_no_rate();
     }
     if (want) {
 #pragma unroll
@@ -345,6 +338,29 @@ __global__ void __launch_bounds__(SEG64_T) k_batch_seg64(BatchDev B, int seg, in
     const double* G = sG + j * ns + v;
     Ho[g] = fma(cc[4], MH, fma(F[0] - F[ns], rdx, sH[o])) * cc[5];
     Bo[g] = fma(cc[4], MB, fma(G[0] - G[ns], rdx, sB[o])) * cc[5];
+  }
+  // BatchDev::fw: the segment's faces but its first (the segment's before, if that
+  // steps any), and with ghosts those of the ends, which no cell reads
+  if (want && B.fw) {
+    for (int t = tid; t < nf * 3; t += SEG64_T) {
+      const int j = t / 3, m = t - j * 3;
+      if (ca + j > i0 || ca + j == 1) B.fw[(long)(ca + j) * 4 + m] = sfw[j * 4 + m];
+    }
+    const bool end = wid == 1 ? i0 == 0 : (wid == 2 && i1 == nx);
+    if (end && ng > 0) {
+      const int f = wid == 1 ? 0 : nx;
+      double m0 = 0.0, m1 = 0.0, m2 = 0.0;
+      for (int v = lane; v < nu; v += 32) {
+        double fh, fb;
+        flux(f, v, fh, fb);
+        m0 = fma(sW[v], fh, m0);
+        m1 = fma(sWu[v], fh, m1);
+        m2 = fma(sWu[v] * sU[v], fh, fma(sW[v], fb, m2));
+      }
+      const double s = warp_sum4(m0, m1, m2, 0.0, lane);
+      const int m = lane >> 3;
+      if ((lane & 7) == 0 && m < 3) B.fw[(long)f * 4 + m] = m == 2 ? 0.5 * s : s;
+    }
   }
 }
 
